@@ -1184,11 +1184,10 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
         const bool fine = c->copy1 || gi_type(c->gi, 0.5) == 1;
         cudaMemcpyAsync(&wsum, c->osum.p + (fine ? 0 : 1) * ldp + nent, sizeof(double),
                         cudaMemcpyDeviceToHost, c->stream);
-        const int64_t nb1 = (g1f.n + 8191) / 8192, nb2 = (g2f.n + 8191) / 8192;
+        const int64_t nb1 = diag_blocks(g1f.n), nb2 = diag_blocks(g2f.n);
         if ((e = c->diag.ensure(4 * (size_t)(nb1 + nb2))))
             return c->cuda_fail(e, "diagnostics");
-        launch_diagnostics(kStar1, g1f.dev(), c->diag.p, c->stream);
-        launch_diagnostics(kStar2, g2f.dev(), c->diag.p + 4 * nb1, c->stream);
+        launch_diagnostics(g1f.dev(), g2f.dev(), c->diag.p, c->stream);
         c->h_diag.resize(4 * (size_t)(nb1 + nb2));
         cudaMemcpyAsync(c->h_diag.data(), c->diag.p, c->h_diag.size() * sizeof(double),
                         cudaMemcpyDeviceToHost, c->stream);
@@ -1213,7 +1212,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
         double wd = 1.0 * gi_scale1(c->gi, 0.5) * wsum;
         scalars[LCG_OUT_WDWARF] = wd / 1 * sc;
         // comp_gravity1/2 (comp_gravity.cpp:20-155), comp_radius1/2 (comp_radius.cpp)
-        const int64_t nb1 = (g1f.n + 8191) / 8192, nb2 = (g2f.n + 8191) / 8192;
+        const int64_t nb1 = diag_blocks(g1f.n), nb2 = diag_blocks(g2f.n);
         double gm = pow(1000. * m.velocity_scale, 3) * m.tperiod * kDay / kTwoPi;
         double a = pow(gm / sq(kTwoPi / kDay / m.tperiod), 1. / 3.);
         double gscale = 100 * gm / sq(a);

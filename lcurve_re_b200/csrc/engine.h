@@ -285,8 +285,12 @@ void launch_scatter(const ScatterParams &p, const ReduceParams &r, const PhaseDe
 void launch_finalize(int32_t flags, const DatumRec *data, int32_t n, double *calc,
                      double *sfac_io, double *out, cudaStream_t s);
 // flux-weighted gravity / volume-averaged radius sums (comp_gravity.cpp,
-// comp_radius.cpp): out[0..3] = sum f*g, sum f, sum solid angle, sum volume
-void launch_diagnostics(int star, GridDev g, double *out, cudaStream_t s);
+// comp_radius.cpp) of the two stars' grids: per block of kDiagBlock faces, star
+// 1's diag_blocks(g1.n) blocks first, four partial sums (f*g, f, solid angle,
+// volume) to out
+constexpr int64_t kDiagBlock = 2048;
+inline int64_t diag_blocks(int64_t n) { return (n + kDiagBlock - 1) / kDiagBlock; }
+void launch_diagnostics(const GridDev &g1, const GridDev &g2, double *out, cudaStream_t s);
 // light_curve_comp_fast interpolation of the model at sampled points mc
 // (sample indices idx, m of them) to all n points; chi**2, wnok -> out[0..1].
 // dst row r = src row rows[r] (count rows of n doubles)
