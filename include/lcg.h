@@ -144,12 +144,9 @@ typedef struct lcg_options {
     int32_t precision;     /* LCG_PREC_FP64 or LCG_PREC_MIXED              */
     int32_t verbose;       /* print per-stage timings at destroy when > 0  */
     int32_t eclipse_warp;  /* Roche eclipse candidates up to which one warp
-                              bisects each face (the rest: one thread per
-                              face); -1 never. 0 automatic: one thread per
-                              face whenever the FP32 screen of the
-                              bisections serves the faces (mixed contexts,
-                              stars with r >= 0.01), else a warp per face
-                              up to twice the GPU's resident warps       */
+                              bisects each face by the plain bisection; 0
+                              (the default) and -1 never: one thread per
+                              boundary, from its root                    */
     int32_t reserved[4];
 } lcg_options;
 

@@ -36,7 +36,7 @@ SOURCES = {
     "components.cu": ["--fmad=false"],
     "walk.cu": ["--fmad=false"],
 }
-HEADERS = ["roche.cuh", "eclipse.cuh", "disc.cuh", "ecl_screen.cuh", "engine.h", "tma.cuh",
+HEADERS = ["roche.cuh", "eclipse.cuh", "disc.cuh", "ecl_root.cuh", "engine.h", "tma.cuh",
            "context.h", "fixed_phase.cuh", "mlp_tc.cuh"]
 
 

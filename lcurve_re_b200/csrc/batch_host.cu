@@ -706,7 +706,8 @@ extern "C" lcg_status lcg_light_curve_batch_resident(lcg_ctx *c, const lcg_model
                     ep.cosi = cos(ri);
                     ep.sini = sin(ri);
                     ep.delta = M.delta_phase;
-                    set_ecl_screen(ep, 1, star == kStar1 ? su.r1 : su.r2);  // batches are mixed
+                    ep.edge = make_edge_star(ep.comp_star, ep.q, ep.comp_spin, ep.cosi, ep.sini,
+                                             ep.comp_rref, ep.comp_pref);
                     X.eclipse_on = su.eclipse;
                 }
             }

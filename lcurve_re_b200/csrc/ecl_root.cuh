@@ -1,0 +1,375 @@
+// ecl_root.cuh — the eclipse boundary of a line of sight from its root.
+//
+// ingress_egress (ingress_egress.cpp:61-86) bisects the phase at which the
+// line of sight to a surface element leaves the eclipsing star: about twenty
+// tests Roche::fblink (fblink.cpp:34-104) per boundary, each a search for
+// the lowest potential along the chord through the eclipser's reference
+// sphere. Almost all of those tests are far enough from the boundary that
+// their outcome follows from where the boundary is:
+//
+//   * fblink's first evaluation is the potential f at the chord's midpoint,
+//     the closest approach to the eclipser's centre; f <= pref answers "hidden"
+//     at once;
+//   * when the lowest potential on the chord exceeds pref, nothing that the
+//     search evaluates can reach it: "not hidden".
+//
+// edge_zone finds the root of f(phase) - pref by Newton's method and, with a
+// bound K on |f''| around it, certifies by Taylor's theorem an interval of
+// phases on either side of the root: hidden up to hid, not hidden from vis on
+// (vis allows for the depth of the potential's minimum below f). The
+// bisection takes the same midpoints as before; inside the certified
+// intervals a midpoint is compared instead of tested, and the few between hid
+// and vis (the eclipser's tide moves the minimum off the midpoint: about
+// twenty delta_phase wide on an M dwarf, far below one on a white dwarf) run
+// fblink. Every decision is fblink's, so the phases are the bisection's, bit
+// for bit. eval_edge alone answers the midpoints outside the intervals.
+//
+// All in FP64. Margins cover the rounding of both sides: positions to a few
+// ulps of the orbit's size, times the gradient, and the potential itself.
+#pragma once
+
+#include "roche.cuh"
+
+namespace lcg {
+
+enum { kEdgeFalse = 0, kEdgeTrue = 1, kEdgeUnsure = 2 };
+
+// Potential about the eclipser's centre (the shift moved into pref):
+//   f(u) = -me/|u| - mo/|u - (dx,0,0)| - ss/2 (ux^2 + uy^2) + k ux - pref
+struct EdgeStar {
+    double me, mo, dx, ss, k, pref, rref2, cosi, sini;
+};
+
+LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, double sini,
+                               double rref, double pref) {
+    EdgeStar s;
+    const double mu = q / (1 + q), comp = 1. - mu;
+    s.ss = spin * spin;
+    if (star == kStar1) {
+        s.me = comp; s.mo = mu; s.dx = 1.; s.k = mu;
+        s.pref = pref;
+    } else {
+        // rpot2 = ... - ss (1/2 + (x^2 + y^2) / 2 - x) - comp x with x = 1 + ux
+        s.me = mu; s.mo = comp; s.dx = -1.; s.k = -comp;
+        s.pref = pref + comp;
+    }
+    s.rref2 = rref * rref;
+    s.cosi = cosi;
+    s.sini = sini;
+    return s;
+}
+
+// One evaluation on the line of sight at a phase, a distance t beyond the
+// chord's midpoint: f, df/dphase (t held), slope g and curvature h along the
+// line; squared distances b2 (closest approach), r2 (of the point) from the
+// eclipser's centre and inverse distance io from the other star's; x, the way
+// to the midpoint, and its rate xp; main term ae = m_e / r^3; a bound tol on
+// the rounding of f.
+struct EdgeEval {
+    double f, fp, g, h, b2, r2, io, x, xp, ae, tol;
+    int ans;  // kEdge*: what fblink answers at this phase (t = 0)
+    bool on;  // the chord exists and f and the rest are set
+};
+
+LCG_HD double edge_rsqrt(double v) {
+#ifdef __CUDA_ARCH__
+    return rsqrt(v);
+#else
+    return 1. / sqrt(v);
+#endif
+}
+
+LCG_HD void edge_sincos(double phase, double &s, double &c) {
+#ifdef __CUDA_ARCH__
+    sincospi(2. * phase, &s, &c);
+#else
+    const double r = phase - rint(phase);
+    s = sin(kTwoPi * r);
+    c = cos(kTwoPi * r);
+#endif
+}
+
+// u0: the element relative to the eclipser's centre, u2 = |u0|^2; acc: fblink's
+// accuracy on the line parameter. An element inside the reference sphere (or
+// on it) is left to fblink, which answers "hidden" without a search.
+LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, double phase,
+                          double t) {
+    EdgeEval r;
+    r.on = false;
+    r.ans = kEdgeUnsure;
+    if (!(u2 > S.rref2 * (1. + 1e-9))) return r;
+    double sn, cs;
+    edge_sincos(phase, sn, cs);
+    const double ex = S.sini * cs, ey = -S.sini * sn, ez = S.cosi;
+    const double x = -fma(ex, u0.x, fma(ey, u0.y, ez * u0.z));
+    const double tiny = 1e-13 * (1. + u2);
+    if (x <= tiny) {
+        if (x < -tiny) r.ans = kEdgeFalse;  // the eclipser lies behind
+        return r;
+    }
+    const double b2 = u2 - x * x;
+    const double hc2 = S.rref2 - b2;  // squared half chord
+    const double a2 = 0.25 * acc * acc;
+    if (hc2 <= a2 * (1. + 1e-6) + tiny) {
+        // no chord, or one no longer than acc: fblink does not search
+        if (hc2 < a2 * (1. - 1e-6) - tiny) r.ans = kEdgeFalse;
+        return r;
+    }
+    const double lam = x + t;
+    const double ux = fma(lam, ex, u0.x), uy = fma(lam, ey, u0.y), uz = fma(lam, ez, u0.z);
+    const double vx = ux - S.dx;
+    const double rxy = fma(ux, ux, uy * uy), r2 = fma(uz, uz, rxy);
+    const double ie = edge_rsqrt(r2), io = edge_rsqrt(fma(vx, vx, fma(uy, uy, uz * uz)));
+    const double ie2 = ie * ie, io2 = io * io, pe = S.me * ie, po = S.mo * io;
+    const double ae = pe * ie2, ao = po * io2;
+    r.f = fma(S.k, ux, fma(-0.5 * S.ss, rxy, -(pe + po))) - S.pref;
+    const double as = ae + ao - S.ss;
+    const double gx = fma(as, ux, fma(-ao, S.dx, S.k)), gy = as * uy, gz = (ae + ao) * uz;
+    r.g = fma(gx, ex, fma(gy, ey, gz * ez));
+    const double ev = fma(-S.dx, ex, t);  // e.v; e.u = t
+    r.h = fma(ae, fma(-3. * t * t, ie2, 1.),
+              fma(ao, fma(-3. * ev * ev, io2, 1.), -S.ss * fma(ex, ex, ey * ey)));
+    const double px = kTwoPi * ey, py = -kTwoPi * ex;  // de/dphase
+    r.xp = -fma(px, u0.x, py * u0.y);
+    r.fp = fma(r.xp, r.g, lam * fma(gx, px, gy * py));
+    r.b2 = b2;
+    r.r2 = r2;
+    r.io = io;
+    r.x = x;
+    r.ae = ae;
+    r.tol = 1e-14 * (pe * ie + po * io + pe + po + 1.);
+    r.on = true;
+    if (r.f <= -r.tol) {
+        r.ans = kEdgeTrue;
+        return r;
+    }
+    // the minimum along the chord: at most tau = 2 |g| / h away, where the
+    // eclipser's curvature falls by at most 5 (tau / b)^2 of itself (tau <= b / 10)
+    // and the other star's changes by at most 6 mo / r^4 per length
+    if (r.f > r.tol && r.h > 0.) {
+        const double tau = 2. * fabs(r.g) / r.h, near = 1. / io - tau;
+        if (100. * tau * tau <= b2 && tau * tau <= hc2 && near > 0.1) {
+            const double c3 = 6. * S.mo / (near * near * near * near);
+            const double hmin = r.h - 5. * ae * tau * tau * ie2 - c3 * tau;
+            if (hmin > 0. && r.f - r.g * r.g / (2. * hmin) > r.tol) r.ans = kEdgeFalse;
+        }
+    }
+    return r;
+}
+
+// Roche::fblink's search with one evaluation of value and slope per point
+// (both square roots as reciprocals, shared), for the phases between the
+// certified intervals: the same chord, bracket check and dbrent
+// (dbrent.cpp:21-126) steps, so the same answer except where rounding could
+// decide it; there (a value within rounding of pref, a bracket that fails)
+// kEdgeUnsure hands the phase to fblink itself. Of the about 720 FP64
+// instructions of an fblink that searches, some 250 remain.
+LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double phase) {
+    double sn, cs;
+    edge_sincos(phase, sn, cs);
+    const double ex = S.sini * cs, ey = -S.sini * sn, ez = S.cosi;
+    const double B = fma(ex, u0.x, fma(ey, u0.y, ez * u0.z)), C = u2 - S.rref2;
+    const double fac = B * B - C, tiny = 1e-12 * (1. + u2);
+    if (!(B < -tiny && fac > tiny && C > tiny)) return kEdgeUnsure;
+    const double lam2 = sqrt(fac) - B, lam1 = C / lam2;
+    if (!(lam2 - lam1 > acc * (1. + 1e-9))) return kEdgeUnsure;
+    const double tol = 1e-14 * (S.me / S.rref2 * 4. + fabs(S.pref) + S.mo + 10.);
+    const double exy2 = fma(ex, ex, ey * ey), uxy = fma(ex, u0.x, ey * u0.y);
+    auto eval = [&](double l, double &f, double &d) {
+        const double ux = fma(l, ex, u0.x), uy = fma(l, ey, u0.y), uz = fma(l, ez, u0.z);
+        const double vx = ux - S.dx, yz = fma(uy, uy, uz * uz), eu = l + B;
+        const double ie = edge_rsqrt(fma(ux, ux, yz)), io = edge_rsqrt(fma(vx, vx, yz));
+        const double pe = S.me * ie, po = S.mo * io;
+        f = fma(S.k, ux, fma(-0.5 * S.ss, fma(ux, ux, uy * uy), -(pe + po))) - S.pref;
+        d = fma(pe * ie * ie, eu,
+                fma(po * io * io, fma(-S.dx, ex, eu), fma(-S.ss, fma(l, exy2, uxy), S.k * ex)));
+    };
+    double x = lam1 + (lam2 - lam1) / 2., fx, dx, f1, f2, t;
+    eval(x, fx, dx);
+    if (fabs(fx) <= tol) return kEdgeUnsure;
+    if (fx < 0.) return kEdgeTrue;
+    eval(lam1, f1, t);
+    eval(lam2, f2, t);
+    // the first level of fblink's subdivision brackets the minimum
+    if (!(fx < f1 - tol && fx < f2 - tol)) return kEdgeUnsure;
+    double a = lam1, b = lam2, w = x, v = x, fw = fx, fv = fx, dw = dx, dv = dx;
+    double e = 0., d = 0.;
+    const double tol1 = acc, tol2 = 2. * acc;
+#pragma unroll 1
+    for (int iter = 0; iter < 100; iter++) {
+        const double xm = 0.5 * (a + b);
+        if (fabs(x - xm) <= tol2 - 0.5 * (b - a)) return kEdgeFalse;
+        bool half = true;
+        if (fabs(e) > tol1) {
+            double d1 = 2. * (b - a), d2 = d1;
+            if (dw != dx) d1 = (w - x) * dx / (dx - dw);
+            if (dv != dx) d2 = (v - x) * dx / (dx - dv);
+            const double u1 = x + d1, u2_ = x + d2;
+            const bool ok1 = (a - u1) * (u1 - b) > 0. && dx * d1 <= 0.;
+            const bool ok2 = (a - u2_) * (u2_ - b) > 0. && dx * d2 <= 0.;
+            const double olde = e;
+            e = d;
+            if (ok1 || ok2) {
+                const double dn = ok1 && ok2 ? (fabs(d1) < fabs(d2) ? d1 : d2) : ok1 ? d1 : d2;
+                if (fabs(dn) <= fabs(0.5 * olde)) {
+                    const double u = x + dn;
+                    d = (u - a < tol2 || b - u < tol2) ? dsign(tol1, xm - x) : dn;
+                    half = false;
+                }
+            }
+        }
+        if (half) d = 0.5 * (e = (dx >= 0. ? a - x : b - x));
+        const bool far = fabs(d) >= tol1;
+        const double u = far ? x + d : x + dsign(tol1, d);
+        double fu, du;
+        eval(u, fu, du);
+        if (fabs(fu) <= tol) return kEdgeUnsure;
+        if (fu < 0.) return kEdgeTrue;
+        if (!far && fu > fx) return kEdgeFalse;
+        if (fu <= fx) {
+            if (u >= x) a = x; else b = x;
+            v = w; fv = fw; dv = dw;
+            w = x; fw = fx; dw = dx;
+            x = u; fx = fu; dx = du;
+        } else {
+            if (u < x) a = u; else b = u;
+            if (fu <= fw || w == x) {
+                v = w; fv = fw; dv = dw;
+                w = u; fw = fu; dw = du;
+            } else if (fu < fv || v == x || v == w) {
+                v = u; fv = fu; dv = du;
+            }
+        }
+    }
+    return kEdgeUnsure;
+}
+
+// Certified phases of one boundary; dir = +1 when the eclipse ends with growing
+// phase. fblink answers "hidden" for -hrad <= dir (phase - hc) <= hid and "not
+// hidden" for vis <= dir (phase - vc) <= vrad (a radius of 0: nothing).
+struct EdgeZone {
+    double hc, hrad, hid, vc, vrad, vis;
+};
+
+// Bounds within a phase radius rad of the point v was taken at, where the
+// point's distance r from the eclipser changes by at most a tenth of itself
+// and the one from the other star by no more (P the point on the line):
+//   |P'| <= 2 pi (lam + |t|), |P''| <= 4 pi^2 (2 lam + 2 |t| + 2.2 r),
+//   |f''| <= |P'|^2 |H| + |P''| |grad f| = K.
+// t1, t2 bound the gradient and the second derivatives of the other star's and
+// the rotation's terms.
+struct EdgeBound {
+    double K, t1, t2, rad;
+};
+LCG_HD EdgeBound edge_bound(const EdgeStar &S, const EdgeEval &v, double lam) {
+    EdgeBound B;
+    const double r = sqrt(v.r2);
+    const double ni = 1.12 * v.io, ni2 = ni * ni;
+    B.t1 = S.mo * ni2 + 1.1 * S.ss * r + fabs(S.k);
+    B.t2 = 2. * S.mo * ni2 * ni + S.ss;
+    const double two2 = kTwoPi * kTwoPi;
+    B.K = two2 * (lam * lam * (2.75 * v.ae + B.t2) + (2. * lam + 2.2 * r) * (1.24 * v.ae * r + B.t1));
+    const double reach = r * v.io < 1. ? r : 1. / v.io;
+    B.rad = 0.1 * reach / (kTwoPi * lam);
+    return B;
+}
+
+// The intervals of one boundary of ingress_egress's bracket: pin the phase
+// pot_min found hidden, pout where the line touches the reference sphere;
+// delta the bisection's accuracy (intervals that end within a twentieth of it
+// of the root are near enough).
+LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, double pin,
+                          double pout) {
+    EdgeZone z;
+    z.hc = z.vc = pout;
+    z.hrad = z.hid = z.vrad = z.vis = 0.;
+    const double u2 = norm2(u0);
+    if (!(u2 > S.rref2 * (1. + 1e-9))) return z;
+    const double dir = pout > pin ? 1. : -1., span = fabs(pout - pin), lam = 1.05 * sqrt(u2);
+    // Newton's method for f = 0 (stage 0, t = 0: the hidden side), then for the
+    // lowest potential on the line = 0 (stage 1, with t: the visible side). A
+    // chord of length acc or less answers "not hidden" untested: start inside.
+    double w = -0.02 * span, t = 0.;
+    int stage = 0;
+#pragma unroll 1
+    for (int it = 0; it < 12; it++) {
+        const EdgeEval v = eval_edge(S, u0, u2, acc, pout + dir * w, t);
+        const double fp = dir * v.fp;
+        if (!v.on || !(fp > 0.) || (stage && !(v.h > 0.))) return z;
+        const double dt = stage ? -v.g / v.h : 0.;
+        const double m = stage ? v.f + 0.5 * v.g * dt : v.f;  // to second order
+        const double s0 = m / fp;
+        if (fabs(s0) < 1e-3) {
+            const EdgeBound B = edge_bound(S, v, lam);
+            const double r = sqrt(v.r2);
+            double rad = B.rad, K = B.K, fl = fp, extra = 4. * v.tol;
+            bool ok = true;
+            if (stage) {
+                // curvature along the line keeps 0.6 h while the point moves by
+                // at most move (third derivatives of -m / r: 6 m / r^4); the
+                // minimum shifts by at most gp rad / hl, gp bounding dg/dphase:
+                // the eclipser's part of g is ae t for every phase
+                const double t3 = 9. * (v.ae / r + S.mo * v.io * v.io * v.io * v.io);
+                double move = 0.4 * v.h / t3;
+                if (move > 0.09 * r) move = 0.09 * r;
+                if (move * v.io > 0.09) move = 0.09 / v.io;
+                const double hl = 0.6 * v.h, tm = fabs(t) + move;
+                const double gp = kTwoPi * (4.2 * v.ae * tm / r * lam + 1.3 * (B.t2 * lam + B.t1));
+                K += gp * gp / hl;
+                const double rm = (move - fabs(dt)) / (1.2 * kTwoPi * lam + gp / hl);
+                if (rm < rad) rad = rm;
+                fl -= gp * fabs(v.g) / hl;
+                extra += v.g * v.g * (0.5 / hl - 0.5 / v.h);
+                ok = tm < 0.5 * lam && dt * dt < 0.25 * (S.rref2 - v.b2);
+            } else {
+                // inwards the chord only grows: d(b^2)/dw > 0 within rad
+                const double db2 = -2. * v.x * v.xp * dir;
+                const double rb = 0.5 * db2 / (kTwoPi * kTwoPi * (1.3 * v.b2 + u2));
+                if (rb < rad) rad = rb;
+            }
+            if (rad * K > 0.8 * fl) rad = 0.8 * fl / K;
+            // f (or the minimum) within the zone is f0 + fl w up to K w^2 / 2 and
+            // grows with w; past eta from the Newton root it has its sign
+            const double eta = (K * s0 * s0 + 2. * extra) / fl;
+            const double off = stage ? fabs(s0) * (fp / fl - 1.) + eta : eta;
+            if (ok && fl > 0.5 * fp && rad > 0. && K * (fabs(s0) + off) <= 0.2 * fl &&
+                fabs(s0) + off < rad && off <= 0.05 * delta) {
+                // 4e-15: the rounding of phases near 1
+                if (stage) {
+                    z.vc = pout + dir * w;
+                    z.vrad = rad;
+                    z.vis = -s0 + off + 4e-15;
+                    return z;
+                }
+                z.hc = pout + dir * w;
+                z.hrad = rad;
+                z.hid = -s0 - off - 4e-15;
+                stage = 1;
+                w -= s0;
+                if (v.h > 0.) t = -v.g / v.h;
+                if (!(v.h > 0. && 25. * t * t < v.b2)) return z;
+                continue;
+            }
+        }
+        w -= s0;
+        t += dt;
+        if (!(w < 0. && w > -span)) return z;
+    }
+    return z;
+}
+
+// What the zones say of a phase.
+LCG_HD int zone_test(const EdgeZone &z, double dir, double phase) {
+    const double wh = dir * (phase - z.hc), wv = dir * (phase - z.vc);
+    if (wh >= -z.hrad && wh <= z.hid && z.hrad > 0.) return kEdgeTrue;
+    if (wv <= z.vrad && wv >= z.vis && z.vrad > 0.) return kEdgeFalse;
+    return kEdgeUnsure;
+}
+
+// A phase beyond both intervals' inner ends: only the search tells.
+LCG_HD bool zone_between(const EdgeZone &z, double dir, double phase) {
+    return z.hrad > 0. && z.vrad > 0. && dir * (phase - z.hc) > z.hid &&
+           dir * (phase - z.vc) < z.vis;
+}
+
+}  // namespace lcg

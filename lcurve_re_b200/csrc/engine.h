@@ -7,7 +7,7 @@
 
 #include "roche.cuh"
 #include "disc.cuh"
-#include "ecl_screen.cuh"
+#include "ecl_root.cuh"
 
 namespace lcg {
 
@@ -52,16 +52,8 @@ struct EclParams {
     int32_t comp_star;   // the eclipsing star
     int32_t comp_roche;  // Roche-distorted eclipser (else a sphere of radius comp_r)
     double q, comp_spin, comp_rref, comp_pref, comp_r, cosi, sini, delta;
-    EclScreen scr;       // FP32 screen of the bisections' line-of-sight tests
+    EdgeStar edge;       // the eclipser for the boundary roots (ecl_root.cuh)
 };
-
-// The FP32 screen runs in mixed contexts when neither the eclipsed star
-// (radius r_face) nor the eclipser (reference sphere rref) is tiny: a white
-// dwarf's own eclipse boundaries, and eclipses by one, stay with FP64 alone.
-inline void set_ecl_screen(EclParams &ep, int mixed, double r_face) {
-    ep.scr = make_ecl_screen(ep.comp_star, ep.q, ep.comp_spin, ep.comp_rref, ep.comp_pref);
-    ep.scr.on = mixed && ep.comp_roche && r_face >= 0.01 && ep.comp_rref >= 0.05;
-}
 
 // Continuum of one star (set_star_continuum.cpp:26-297).
 struct ContParams {
@@ -221,9 +213,8 @@ struct BatchDev {
     ulonglong2 *runh;  // FlatDev::runh per slot, from flat0 / 64
     ulonglong2 *ecl;
     int64_t *n0;  // per slot
-    // eclipse candidates: those whose bisections the FP32 screen serves go to
-    // the front of queue, the others (FP64 alone) to the back, so that warps
-    // do not mix the two; counters: [0] candidates, [1]-[3] work counters of
+    // eclipse candidates: those behind a large star go to the front of queue,
+    // those behind a white dwarf to the back, so that warps do not mix the two; counters: [0] candidates, [1]-[3] work counters of
     // the passes, [4] back-of-queue candidates, [5] front-of-queue ones, [6]
     // candidates pot_min found eclipsed
     int32_t *blockcnt, *queue, *counters;

@@ -153,13 +153,13 @@ __global__ void k_ecl_pre(EclParams p, int32_t eclipse_on, GridDev g, int32_t *q
     queue_push(cand, (int32_t)i, queue, counters);
 }
 
-// Ingress/egress of the queued candidates. Up to warp_max candidates, one
-// warp bisects each face (ingress_egress_warp): few candidates leave most of
-// the GPU idle otherwise. Beyond that, k_ecl_potmin and k_ecl_bisect take
-// over (one thread per candidate, each warp taking 32 consecutive candidates
-// at a time so that neighbouring faces, with similar iteration counts, run in
-// lockstep) and this kernel returns at once. The count is read on the device,
-// so the choice needs no host round trip.
+// Ingress/egress of the queued candidates, one warp per face
+// (ingress_egress_warp), for calls that ask for it with at most warp_max
+// candidates: the plain bisection, which the tests compare the thread mode
+// with. Otherwise k_ecl_potmin and k_ecl_bisect do the work (one thread per
+// candidate, each warp taking 32 consecutive candidates at a time so that
+// neighbouring faces, with similar iteration counts, run in lockstep) and this
+// kernel is not launched, or returns at once: the count is read on the device.
 __global__ void __launch_bounds__(128, 4) k_ecl_roche(EclParams p, GridDev g,
                                                    const int32_t *__restrict__ queue,
                                                    int32_t *counters, DevStatus *st,
@@ -208,59 +208,64 @@ __device__ __forceinline__ void push_hits(bool hit, int k, int32_t *hits, int32_
     if (hit) hits[at + __popc(m & ((1u << lane) - 1u))] = k;
 }
 
-// One test of a bisection: the FP32 screen where p.scr allows it (it decides
-// only where the FP64 test's answer is certain, so the bisection takes the
-// same midpoints), else Roche::fblink in FP64. u0: the point relative to the
-// eclipser's centre, in FP32.
-__device__ __noinline__ int ecl_screen_test(const EclScreen scr, float cosi, float sini,
-                                            double pmid, float u0x, float u0y, float u0z,
-                                            float acc) {
-    const double ph = pmid - rint(pmid);  // |ph| <= 1/2 keeps the FP32 angle fine
-    float sn, cs;
-    sincospif(2.f * (float)ph, &sn, &cs);
-    return fblink_screen(scr, u0x, u0y, u0z, sini * cs, -sini * sn, cosi, acc);
-}
-
 // The bisection of ingress (side 0) or egress (side 1) of ingress_egress
 // (ingress_egress.cpp:61-86) from the pot_min state, for every lane of a warp
-// at once (all 32 lanes call it; lanes with live false only vote). Each lane
-// screens its midpoints in FP32 until one is unsure; when no live lane can go
-// on, the warp runs Roche::fblink in FP64 for all the lanes waiting on one, in
-// a single pass, and the screening resumes. The FP64 passes are thus packed
-// (one per test of the lane that needs the most, instead of one per step
-// whenever any lane needs one), and the lanes take the FP64 decisions at the
-// same midpoints as the plain loop. With the screen off it is the plain loop.
+// at once (all 32 lanes call it; lanes with live false only vote). The root of
+// the boundary comes first (edge_zone); then each lane takes the bisection's
+// midpoints, comparing those that the certified intervals decide, until one
+// needs a test. The tests run in passes for all lanes that wait for one:
+// eval_edge outside the intervals, fblink_edge between them, and Roche::fblink
+// itself where that is unsure, so the lanes take fblink's decisions at the
+// same midpoints as the plain loop. FP64 latency and issue bound it: some 4
+// evaluations for the root, 2.3 outside the intervals and 3.3 searches of 5
+// evaluations per boundary by an M dwarf, against 20 tests in FP32 with 6.4
+// fblinks of 8 to 12 evaluations before (a white dwarf's: 6 evaluations
+// against 20 fblinks). 256 models of 60-400 strips: 13.8 -> 5.4 ms; one curve
+// on 81/163 strips: 203 us with its warp mode -> 62. With the FP32 screen kept
+// for the tests outside the intervals it took 5.8 ms.
 __device__ __forceinline__ double ecl_bisect_warp(const EclParams &p, bool live, double pin,
                                                   double pout, double acc, V3 pos, int &s) {
-    // what the screening loop reads, in registers (p may be global memory;
-    // the FP64 test, a third of the steps, reads the rest from it)
-    const EclScreen scr = p.scr;
+    // what the passes read, in registers (p may be global memory)
+    const EdgeStar S = p.edge;
     const double delta = p.delta;
-    const float cif = (float)p.cosi, sif = (float)p.sini, accf = (float)acc;
-    const float u0x = (float)(pos.x - (p.comp_star == kStar1 ? 0. : 1.));
-    const float u0y = (float)pos.y, u0z = (float)pos.z;
+    const V3 u0 = v3(pos.x - (p.comp_star == kStar1 ? 0. : 1.), pos.y, pos.z);
+    const double u2 = norm2(u0), dir = pout > pin ? 1. : -1.;
+    EdgeZone z;
+    z.hrad = z.vrad = z.hid = z.vis = z.hc = z.vc = 0.;
+    if (live) z = edge_zone(S, u0, acc, delta, pin, pout);
     bool done = !live;
     int guard = 0;
     double pmid = 0.;
     for (;;) {
-        bool need = false;
+        int need = 0;  // 1: a test outside the intervals, 2: between them
         while (!done) {
             if (!(fabs(pin - pout) > delta)) { done = true; break; }
             if (++guard > 400) { s = kEclNoConverge; done = true; break; }
             pmid = (pin + pout) / 2.;
-            if (!scr.on) { need = true; break; }
-            const int d = ecl_screen_test(scr, cif, sif, pmid, u0x, u0y, u0z, accf);
-            if (d == kScreenUnsure) { need = true; break; }
-            if (d == kScreenTrue) pin = pmid;
+            const int d = zone_test(z, dir, pmid);
+            if (d == kEdgeUnsure) {
+                need = zone_between(z, dir, pmid) ? 2 : 1;
+                break;
+            }
+            if (d == kEdgeTrue) pin = pmid;
             else pout = pmid;
         }
-        if (!__any_sync(0xffffffffu, need)) break;
-        if (need) {
-            if (fblink(p.comp_star, p.q, p.comp_spin, acc, set_earth(p.cosi, p.sini, pmid), pos,
-                       p.comp_rref, p.comp_pref, s))
-                pin = pmid;
-            else
-                pout = pmid;
+        if (!__any_sync(0xffffffffu, need != 0)) break;
+        if (need == 1) {
+            const int d = eval_edge(S, u0, u2, acc, pmid, 0.).ans;
+            if (d == kEdgeTrue) pin = pmid;
+            else if (d == kEdgeFalse) pout = pmid;
+            else need = 2;
+        }
+        if (need == 2) {
+            int d = fblink_edge(S, u0, u2, acc, pmid);
+            if (d == kEdgeUnsure)
+                d = fblink(p.comp_star, p.q, p.comp_spin, acc, set_earth(p.cosi, p.sini, pmid),
+                           pos, p.comp_rref, p.comp_pref, s)
+                        ? kEdgeTrue
+                        : kEdgeFalse;
+            if (d == kEdgeTrue) pin = pmid;
+            else pout = pmid;
             if (s) done = true;
         }
     }
@@ -1078,6 +1083,12 @@ __global__ void __launch_bounds__(128) k_grid_b(BatchDev b) {
     }
 }
 
+// Eclipsers whose reference sphere is at least this large share the front of
+// the batch queue: their boundaries take a few searches each (ecl_root.cuh),
+// those of a white dwarf almost none, and a warp runs at its slowest lane's
+// pace.
+constexpr double kBigEclipser = 0.05;
+
 // Sphere pre-test of the geometry list's faces; candidates are queued by
 // their batch face index. Whole warps step together (queue_push votes).
 __global__ void k_ecl_pre_b(BatchDev b) {
@@ -1089,7 +1100,7 @@ __global__ void k_ecl_pre_b(BatchDev b) {
     for (int64_t u0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); u0 < total;
          u0 += stride) {
         const int64_t u = u0 + lane;
-        bool cand = false, scr = false;
+        bool cand = false, big = false;
         int32_t item = 0;
         if (u < total) {
             const int k = find_seg(b.geo_face, nk, u);
@@ -1097,17 +1108,18 @@ __global__ void k_ecl_pre_b(BatchDev b) {
             const int64_t i = u - b.geo_face[k];
             cand = ecl_pre_face(S.ep, S.eclipse_on, slot_grid(b.g, S.face0, S.nface, S.ntiled), i);
             item = (int32_t)(S.face0 + i);
-            scr = S.ep.scr.on;
+            big = S.ep.comp_rref >= kBigEclipser;
         }
-        // screened candidates to the front of the queue, the others to the back
-        const unsigned back = __ballot_sync(0xffffffffu, cand && !scr);
-        queue_push(cand && scr, item, b.queue, b.counters);
+        // eclipses by a large star to the front of the queue, by a white dwarf to
+        // the back
+        const unsigned back = __ballot_sync(0xffffffffu, cand && !big);
+        queue_push(cand && big, item, b.queue, b.counters);
         if (back) {
             const int leader = __ffs(back) - 1;
             int base = 0;
             if (lane == leader) base = atomicAdd(&b.counters[4], __popc(back));
             base = __shfl_sync(0xffffffffu, base, leader);
-            if (cand && !scr)
+            if (cand && !big)
                 b.queue[b.qcap - 1 - (base + __popc(back & ((1u << lane) - 1u)))] = item;
         }
     }
@@ -1130,24 +1142,16 @@ __device__ __forceinline__ int32_t queue_at(const BatchDev &b, int k) {
 
 // k_ecl_roche over the batch queue: each candidate finds its slot by its
 // face index.
-// Warp mode of the batched eclipse (few candidates): one warp per candidate.
-// With more candidates than warp_max, k_ecl_potmin_b and k_ecl_bisect_b do
-// the work and this kernel returns at once (the choice is made on the device).
-// Warp mode for this call: at most warp_max candidates and, when the mode is
-// chosen automatically, none that the FP32 screen serves (the front of the
-// queue): thread mode with the screen has the shorter latency even for few.
-__device__ __forceinline__ bool batch_warp_mode(const BatchDev &b, int32_t warp_max,
-                                                int32_t auto_mode) {
-    return b.counters[0] <= warp_max && !(auto_mode && b.counters[5] > 0);
+__device__ __forceinline__ bool batch_warp_mode(const BatchDev &b, int32_t warp_max) {
+    return b.counters[0] <= warp_max;
 }
 
-__global__ void __launch_bounds__(128, 4) k_ecl_roche_b(BatchDev b, int32_t warp_max,
-                                                     int32_t auto_mode) {
+__global__ void __launch_bounds__(128, 4) k_ecl_roche_b(BatchDev b, int32_t warp_max) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int total = b.counters[0];
     const GridDev g = b.g;
-    if (batch_warp_mode(b, warp_max, auto_mode)) {
+    if (batch_warp_mode(b, warp_max)) {
         for (;;) {
             int k = 0;
             if (lane == 0) k = atomicAdd(&b.counters[1], 1);
@@ -1182,12 +1186,11 @@ __global__ void __launch_bounds__(128, 4) k_ecl_roche_b(BatchDev b, int32_t warp
 // egress bisections (ingress_egress.cpp:61-86) on the two lanes of a pair.
 // Warps take consecutive candidates (similar iteration counts run together).
 // Same arithmetic and decisions as ingress_egress: identical results.
-__global__ void __launch_bounds__(128, 4) k_ecl_potmin_b(BatchDev b, int32_t warp_max,
-                                                      int32_t auto_mode) {
+__global__ void __launch_bounds__(128, 4) k_ecl_potmin_b(BatchDev b, int32_t warp_max) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int total = b.counters[0];
-    if (batch_warp_mode(b, warp_max, auto_mode)) return;
+    if (batch_warp_mode(b, warp_max)) return;
     const GridDev g = b.g;
     for (;;) {
         int base = 0;
@@ -1224,11 +1227,11 @@ __global__ void __launch_bounds__(128, 4) k_ecl_potmin_b(BatchDev b, int32_t war
 // warps hide the FP64 latency, fewer registers spill more)
 template <int NB>
 __global__ void __launch_bounds__(128, NB)
-    k_ecl_bisect_b(__grid_constant__ const BatchDev b, int32_t warp_max, int32_t auto_mode) {
+    k_ecl_bisect_b(__grid_constant__ const BatchDev b, int32_t warp_max) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int total = b.counters[0];
-    if (batch_warp_mode(b, warp_max, auto_mode)) return;
+    if (batch_warp_mode(b, warp_max)) return;
     const int64_t n2 = 2 * (int64_t)b.counters[6];
     for (;;) {
         int64_t base = 0;
@@ -1462,13 +1465,13 @@ void launch_eclipse(const EclParams &p, int32_t eclipse_on, GridDev g, int32_t *
         unsigned nb = (unsigned)nsm * 4u;
         const unsigned need = nblocks(g.n, 4);
         if (need < nb) nb = need;
-        const int32_t warps = (int32_t)nb * 4;
-        // auto: warp mode for few candidates, unless the FP32 screen serves them
-        // (thread mode with the screen has the shorter latency even then)
-        const int32_t warp_max =
-            warp_mode < 0 ? -1 : warp_mode > 0 ? warp_mode : (p.scr.on ? -1 : 2 * warps);
-        k_ecl_roche<<<nb, 128, 0, s>>>(p, g, queue, counters, st, warp_max);
-        count_launch();
+        // warp mode on request only: with the boundary's root found first, the
+        // thread mode has the shorter latency for any number of candidates
+        const int32_t warp_max = warp_mode > 0 ? warp_mode : -1;
+        if (warp_max > 0) {
+            k_ecl_roche<<<nb, 128, 0, s>>>(p, g, queue, counters, st, warp_max);
+            count_launch();
+        }
         k_ecl_potmin<<<nb, 128, 0, s>>>(p, g, queue, counters, es, hits, st, warp_max);
         count_launch();
         const int nbs = bisect_blocks_per_sm();
@@ -1598,17 +1601,17 @@ void launch_batch_eclipse(const BatchDev &b, int nsm, int32_t warp_mode, cudaStr
     count_launch();
     k_ecl_join_b<<<1, 32, 0, s>>>(b);
     count_launch();
-    const int32_t warps = nsm * 16;
-    const int32_t warp_max = warp_mode < 0 ? -1 : warp_mode > 0 ? warp_mode : 2 * warps;
-    const int32_t auto_mode = warp_mode == 0;
-    k_ecl_roche_b<<<nsm * 4, 128, 0, s>>>(b, warp_max, auto_mode);
-    count_launch();
-    k_ecl_potmin_b<<<nsm * 4, 128, 0, s>>>(b, warp_max, auto_mode);
+    const int32_t warp_max = warp_mode > 0 ? warp_mode : -1;
+    if (warp_max > 0) {
+        k_ecl_roche_b<<<nsm * 4, 128, 0, s>>>(b, warp_max);
+        count_launch();
+    }
+    k_ecl_potmin_b<<<nsm * 4, 128, 0, s>>>(b, warp_max);
     count_launch();
     if (bisect_blocks_per_sm() == 6)
-        k_ecl_bisect_b<6><<<nsm * 6, 128, 0, s>>>(b, warp_max, auto_mode);
+        k_ecl_bisect_b<6><<<nsm * 6, 128, 0, s>>>(b, warp_max);
     else
-        k_ecl_bisect_b<4><<<nsm * 4, 128, 0, s>>>(b, warp_max, auto_mode);
+        k_ecl_bisect_b<4><<<nsm * 4, 128, 0, s>>>(b, warp_max);
     count_launch();
 }
 

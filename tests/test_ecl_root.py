@@ -1,0 +1,66 @@
+"""The eclipse boundaries from their roots (ecl_root.cuh) on the CPU.
+
+The bisections of ingress and egress compare a midpoint with intervals
+certified around the boundary's root instead of testing it, where they can.
+Every answer must be Roche::fblink's (fblink.cpp:34-104): here each midpoint of
+both bisections of every face of real grids is answered by the intervals, by
+the single evaluation and by the fused search, and by fblink. On ordinary
+binaries the intervals must also decide most midpoints, or they are not worth
+finding.
+"""
+import os
+import shutil
+import struct
+import subprocess
+
+import numpy as np
+import pytest
+
+from lcurve_re_b200 import workloads as W
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SRC = os.path.join(HERE, "screen", "root_check.cpp")
+EXE = os.path.join(HERE, "screen", "_build", "root_check")
+
+
+@pytest.fixture(scope="module")
+def checker():
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not available")
+    os.makedirs(os.path.dirname(EXE), exist_ok=True)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", EXE, SRC])
+    return EXE
+
+
+def _run(exe, m, star, posn):
+    c = m.to_c()
+    ecl = 1 - star
+    ri = np.radians(c.iangle)
+    hdr = struct.pack("8d", c.q, np.cos(ri), np.sin(ri), c.delta_phase,
+                      c.spin2 if ecl == 1 else c.spin1, c.r2 if ecl == 1 else c.r1, 0.0,
+                      float(ecl))
+    blob = hdr + struct.pack("q", posn.shape[0]) + np.ascontiguousarray(posn).tobytes()
+    out = subprocess.run([exe], input=blob, capture_output=True, timeout=600)
+    vals = [int(v) for v in out.stdout.split()]
+    return out.returncode, dict(zip(("hits", "tests", "zone", "evals", "searches", "wrong"), vals))
+
+
+# most: the certified intervals decide at least this share of the midpoints
+@pytest.mark.parametrize("most,over", [
+    (0.6, {}), (0.6, dict(iangle=90.0)), (0.6, dict(r1=0.002, iangle=88.0)),
+    (0.3, dict(r1=0.005, q=0.1, iangle=80.0)),       # grazing
+    (0.5, dict(q=0.15, r1=0.012, r2=-1.0, iangle=84.0)),  # lobe-filling donor
+    (0.0, dict(q=0.8, r1=-1.0, r2=-1.0, iangle=75.0)),    # both lobes filled, in contact
+    (0.6, dict(q=3.0, r2=0.35)), (0.6, dict(spin1=0.0, spin2=0.0)),
+    (0.6, dict(spin1=20.0, spin2=1.8, r2=0.15)),
+    (0.6, dict(delta_phase="1e-9")), (0.3, dict(delta_phase="1e-4"))])
+def test_roots_keep_every_decision(checker, oracle, most, over):
+    m = W.model(nlat1f=16, nlat2f=36, **over)
+    tests = zone = 0
+    for star in (0, 1):
+        rc, r = _run(checker, m, star, oracle.star_grid(m, star)["posn"])
+        assert rc == 0 and r["wrong"] == 0, (star, r)
+        tests += r["tests"]
+        zone += r["zone"]
+    assert tests > 1000
+    assert zone >= most * tests, (zone, tests)
