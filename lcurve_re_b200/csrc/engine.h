@@ -82,6 +82,24 @@ struct DevStatus {
     int32_t face;
 };
 
+// What a warp of the fast mixed sweep can tell about a group of consecutive
+// faces without reading them. At a sub-phase entry e, with |e| = |(ex, ey)|,
+//   mu = ex nx + ey ny + cz <= ex ax + ey ay + |e| r + cmax
+//                           >= ex ax + ey ay - |e| r + cmin
+// for every face of the group (cmin, cmax carry a margin over FP32 rounding):
+// below zero at all the warp's entries the group adds exact zeros, above zero
+// no element needs its sign tested. On the circle of fixed-point phase every
+// eclipse range of the group lies inside [hull.x, hull.x + hull.y) (hull.y = 0:
+// no face has one; ~0: anywhere), and every face of the group is eclipsed
+// throughout [all.x, all.x + all.y) (all.y = 0: nowhere).
+struct RunRec {
+    float ax, ay, r, cmax, cmin, pad[3];
+    ulonglong2 hull, all;
+};
+constexpr int kRunRecs = 5;    // a run of 32 face pairs, then its four parts of 8
+constexpr int kRunFaces = 64;
+static_assert(sizeof(RunRec) == 64, "bulk copies and the chunk's shared memory count on it");
+
 // Flattened grid for the flux sweep (FlatGrid, comp_light_flat.cpp:26-65).
 // Faces [0,n0) are never eclipsed, [n0,n) have one eclipse range. The
 // mixed-precision view packs (nx,ny,nz,flux) as float4 and the eclipse range
@@ -100,15 +118,9 @@ struct FlatDev {
     // with cz = cos(i) nz and f_k = flux * p_k, so each float2 operand of the
     // packed FP32x2 arithmetic is an aligned register pair
     float *fp;
-    // per run of 32 pairs (64 faces) of fp: (ax, ay, R, C) bounding
-    // mu = ex nx + ey ny + cz <= ex ax + ey ay + |(ex, ey)| R + C for every face
-    // of the run (C includes a margin over FP32 rounding), so a warp can skip
-    // a run that faces away at all its phases
-    float4 *runb;
-    // per run: an arc (I, W) of fixed-point phase holding every eclipse range
-    // of the run's faces (W = ~0: test each face; (0, 0): none has a range), so
-    // a warp whose phases all lie outside it skips the run's eclipse tests
-    ulonglong2 *runh;
+    // bounds of every 64 consecutive faces of fp (a run) and of its four parts of
+    // 16: kRunRecs records per run, the run's first
+    RunRec *runs;
     // faces with two or more eclipse ranges (opaque discs) sit last, in
     // [*n1, n): their records above are zero (they add nothing to the main
     // sweeps); ridx is each one's face index in the grid, rr its rn ranges
@@ -209,8 +221,7 @@ struct BatchDev {
     int32_t nslots, nmodels;
     GridDev g;  // every face of the batch
     float *fp;  // fast sweep records (FlatDev::fp layout per slot)
-    float4 *runb;  // FlatDev::runb per slot, from flat0 / 64
-    ulonglong2 *runh;  // FlatDev::runh per slot, from flat0 / 64
+    RunRec *runs;  // FlatDev::runs per slot, from kRunRecs flat0 / 64
     ulonglong2 *ecl;
     int64_t *n0;  // per slot
     // eclipse candidates: those behind a large star go to the front of queue,
@@ -291,9 +302,9 @@ void launch_interp(const DatumRec *data, int32_t n, const int64_t *idx, int32_t 
                    const double *mc, double *calc, int32_t rdata, double *out, cudaStream_t s);
 
 void launch_pack_flat(FlatDev f, int64_t n0, int need_pos, cudaStream_t s);
-// run bounds of fast records: npairs pairs from fp, one float4 per 32 pairs
-void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, float4 *runb,
-                       ulonglong2 *runh, cudaStream_t s);
+// run records of npairs pairs of fast records (and their eclipse ranges)
+void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, RunRec *runs,
+                       cudaStream_t s);
 void launch_batch_run_bounds(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_pack_phases(PhaseDev ph, cudaStream_t s);
 

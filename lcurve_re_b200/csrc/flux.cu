@@ -255,18 +255,18 @@ void launch_ppt(int star, const FluxConsts &k, const FlatDev &f, const PhaseDev 
 // are bit-identical to evaluating them.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-// The warp's phase arc: every entry of the warp below nent lies in [A, A + L]
-// (mod 2^64), A its first lane's first entry. For time-ordered points it is a
-// short arc of the orbit; in any order it still holds every entry.
+// The warp's phase arc: every entry of the warp lies in [A, A + L] (mod 2^64),
+// A its first lane's first entry. For time-ordered points it is a short arc of
+// the orbit; in any order it still holds every entry.
 template <int PPT>
-__device__ __forceinline__ void warp_arc(const unsigned long long *pf, int64_t e0, int64_t nent,
-                                         unsigned long long &A, unsigned long long &L) {
+__device__ __forceinline__ void warp_arc(const unsigned long long *pf, unsigned long long &A,
+                                         unsigned long long &L) {
     A = __shfl_sync(0xffffffffu, pf[0], 0);
     unsigned long long l = 0ull;
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
         const unsigned long long d = pf[j] - A;
-        if (e0 + j < nent && d > l) l = d;
+        if (d > l) l = d;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -276,24 +276,80 @@ __device__ __forceinline__ void warp_arc(const unsigned long long *pf, int64_t e
     L = l;
 }
 
-// A run's eclipse-range hull (I, W) (FlatDev::runh) meets the arc [A, A + L]:
-// the hull starts inside the arc, or the arc starts inside the hull; W = ~0
-// means "test every face", W = 0 "no face of the run has a range". Exact on
-// the circle, so a run whose hull misses the arc has every face visible at
-// every entry of the warp.
-__device__ __forceinline__ bool hull_meets_arc(ulonglong2 H, unsigned long long A,
-                                               unsigned long long L) {
-    if (H.y == ~0ull) return true;
-    return H.y != 0ull && ((H.x - A) <= L || (A - H.x) < H.y);
+// What the warp knows of a group of faces: which of its entries could see it
+// and whether a range could hide it (warp-uniform).
+enum { kGroupDark = 0, kGroupBright = 1, kGroupSigns = 2, kGroupRanges = 3 };
+
+// Dark: every face turned away, or eclipsed, at all the warp's entries: exact
+// zeros. Bright: every face visible and none eclipsed: no sign or range to
+// test. Signs: signs to test, no range. Ranges: both.
+template <int PPT, bool ECL>
+__device__ __forceinline__ int group_class(const RunRec &R, const float2 *ex, const float2 *ey,
+                                           const float *exy, unsigned long long A,
+                                           unsigned long long L) {
+    bool some = false, every = true;
+    const float4 B = *reinterpret_cast<const float4 *>(&R);
+    const float cmin = R.cmin;
+#pragma unroll
+    for (int j = 0; j < PPT; j++) {
+        const float d = fmaf(ex[j].x, B.x, ey[j].x * B.y);
+        some = some || fmaf(exy[j], B.z, d + B.w) >= 0.f;
+        every = every && fmaf(-exy[j], B.z, d + cmin) > 0.f;
+    }
+    if (!__any_sync(0xffffffffu, some)) return kGroupDark;
+    bool ranges = false;
+    if constexpr (ECL) {
+        // the arc [A, A + L] of the warp's phases against the group's: exact on
+        // the circle
+        const ulonglong2 H = R.hull;
+        ranges = H.y == ~0ull || (H.y != 0ull && ((H.x - A) <= L || (A - H.x) < H.y));
+        if (ranges) {
+            const unsigned long long o = A - R.all.x;
+            if (o < R.all.y && L < R.all.y - o) return kGroupDark;
+            return kGroupRanges;
+        }
+    }
+    return __all_sync(0xffffffffu, every) ? kGroupBright : kGroupSigns;
 }
 
-// One fold block of cnt face pairs at rp (eclipse records at ep when ECL):
-// the PPT entries' FP32 sums of the block.
+// cnt face pairs at rp into the entries' FP32 sums; every element visible.
+// Nothing branches or votes, so the iterations overlap: 7 FFMA2 and 2 MUFU per
+// pair and entry. The loop alone takes 22.1 cycles of a scheduler per pair and
+// entry at PPT 4, of which the FFMA2 occupy 18 (2.6 each: three 64-bit operands
+// read from two register banks) and the MUFU 16 beside them; 23.1 at PPT 2.
+// Two pairs per trip help at PPT 4 only (1%); below it the longer code costs 3%
+// of a 256-model batch and 9% of 64 coarse models.
+template <int PPT, int LT>
+__device__ __forceinline__ void bright_pairs(const float4 *rp, int cnt, const float2 *ex,
+                                             const float2 *ey, float2 *s) {
+    constexpr int kTrip = PPT >= 4 ? 2 : 1;
+#pragma unroll kTrip
+    for (int i = 0; i < cnt; i++) {
+        const float4 P0 = rp[4 * i], P1 = rp[4 * i + 1], P2 = rp[4 * i + 2], P3 = rp[4 * i + 3];
+        const float2 nx = f2(P0.x, P0.y), ny = f2(P0.z, P0.w), cz = f2(P1.x, P1.y);
+        const float2 p0 = f2(P1.z, P1.w), p1 = f2(P2.x, P2.y), p2 = f2(P2.z, P2.w);
+        const float2 p3 = f2(P3.x, P3.y), p4 = f2(P3.z, P3.w);
+#pragma unroll
+        for (int j = 0; j < PPT; j++) {
+            const float2 m = __ffma2_rn(ex[j], nx, __ffma2_rn(ey[j], ny, cz));
+            float2 t;
+            if constexpr (LT == 1) t = f2(sqrt_approx(m.x), sqrt_approx(m.y));
+            else t = m;
+            const float2 fI =
+                __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, p4, p3), p2), p1), p0);
+            s[j] = __ffma2_rn(m, fI, s[j]);
+        }
+    }
+}
+
+// The same with the sign of mu tested per element, and the eclipse range (a
+// 64-bit subtract and compare) when ECL: a pair dark at every entry of the
+// warp skips its intensity after one vote.
 template <int PPT, int LT, bool ECL>
-__device__ __forceinline__ void fold_block(const float4 *rp, const ulonglong2 *ep, int cnt,
-                                           const float2 *ex, const float2 *ey,
-                                           const unsigned long long *pf, float2 *s) {
-#pragma unroll 2
+__device__ __forceinline__ void mixed_pairs(const float4 *rp, const ulonglong2 *ep, int cnt,
+                                            const float2 *ex, const float2 *ey,
+                                            const unsigned long long *pf, float2 *s) {
+#pragma unroll 1
     for (int i = 0; i < cnt; i++) {
         const float4 P0 = rp[4 * i], P1 = rp[4 * i + 1];
         const float2 nx = f2(P0.x, P0.y), ny = f2(P0.z, P0.w), cz = f2(P1.x, P1.y);
@@ -331,115 +387,130 @@ __device__ __forceinline__ void fold_block(const float4 *rp, const ulonglong2 *e
     }
 }
 
+// Face pairs [lo, hi) of a staged chunk whose first pair is q0, in FP32 sums of
+// up to kFold faces each added to acc. A fold is classified whole (by its run's
+// record, or the two when it straddles runs), and part by part where that
+// leaves signs or ranges to test. Every class gives the sums of testing every
+// element, bit for bit.
 template <int PPT, int LT, bool ECL>
-__device__ __forceinline__ void sweep_pairs(const float4 *sp, const ulonglong2 *se, int64_t q0,
-                                            int64_t lo, int64_t hi, const float2 *ex,
-                                            const float2 *ey, const float *exy,
+__device__ __forceinline__ void sweep_pairs(const float4 *sp, const ulonglong2 *se,
+                                            const RunRec *sr, int q0, int lo, int hi,
+                                            const float2 *ex, const float2 *ey, const float *exy,
                                             const unsigned long long *pf, unsigned long long A,
-                                            unsigned long long L,
-                                            const float4 *__restrict__ runb,
-                                            const ulonglong2 *__restrict__ runh, float *acc) {
-    constexpr int kFoldPairs = kFold / 2;
-    for (int64_t b = lo; b < hi; b += kFoldPairs) {
-        const int cnt = (int)((b + kFoldPairs < hi) ? kFoldPairs : hi - b);
-        {
-            // the run bound (or the two, when the fold run straddles stored runs):
-            // negative at every phase entry of the warp -> the whole run adds zero
-            const float4 B0 = runb[b >> 5], B1 = runb[(b + cnt - 1) >> 5];
-            bool vis = false;
-#pragma unroll
-            for (int j = 0; j < PPT; j++) {
-                const float e0 = fmaf(ex[j].x, B0.x, fmaf(ey[j].x, B0.y, fmaf(exy[j], B0.z, B0.w)));
-                const float e1 = fmaf(ex[j].x, B1.x, fmaf(ey[j].x, B1.y, fmaf(exy[j], B1.z, B1.w)));
-                vis = vis || e0 >= 0.f || e1 >= 0.f;
-            }
-            if (!__any_sync(0xffffffffu, vis)) continue;
+                                            unsigned long long L, float *acc) {
+    constexpr int kFoldPairs = kFold / 2, kPart = 8;
+    for (int b = lo; b < hi; b += kFoldPairs) {
+        const int end = b + kFoldPairs < hi ? b + kFoldPairs : hi;
+        const int r0 = (b - q0) >> 5, r1 = (end - 1 - q0) >> 5;
+        int c = group_class<PPT, ECL>(sr[kRunRecs * r0], ex, ey, exy, A, L);
+        if (r1 != r0) {
+            const int c1 = group_class<PPT, ECL>(sr[kRunRecs * r1], ex, ey, exy, A, L);
+            if (c != c1) c = kGroupSigns;
         }
-        const float4 *rp = sp + 4 * (b - q0);
-        const ulonglong2 *ep = se + 2 * (b - q0);
+        if (c == kGroupDark) continue;
         float2 s[PPT];
 #pragma unroll
         for (int j = 0; j < PPT; j++) s[j] = f2(0.f, 0.f);
-        // the per-entry eclipse tests only where a run's ranges can reach the
-        // warp's arc of phases (warp-uniform: the hulls and the arc are)
-        if (ECL && (hull_meets_arc(runh[b >> 5], A, L) ||
-                    hull_meets_arc(runh[(b + cnt - 1) >> 5], A, L)))
-            fold_block<PPT, LT, true>(rp, ep, cnt, ex, ey, pf, s);
-        else
-            fold_block<PPT, LT, false>(rp, ep, cnt, ex, ey, pf, s);
+        if (c == kGroupBright) {
+            bright_pairs<PPT, LT>(sp + 4 * (b - q0), end - b, ex, ey, s);
+        } else {
+#pragma unroll 1
+            for (int p = b; p < end;) {
+                const int k = (p - q0) >> 3;  // the part holding pair p
+                const int pe = q0 + kPart * (k + 1) < end ? q0 + kPart * (k + 1) : end;
+                const int cp = group_class<PPT, ECL>(sr[kRunRecs * (k >> 2) + 1 + (k & 3)], ex, ey,
+                                                     exy, A, L);
+                const float4 *rp = sp + 4 * (p - q0);
+                if (cp == kGroupBright) bright_pairs<PPT, LT>(rp, pe - p, ex, ey, s);
+                else if (cp == kGroupSigns)
+                    mixed_pairs<PPT, LT, false>(rp, nullptr, pe - p, ex, ey, pf, s);
+                else if (ECL && cp == kGroupRanges)
+                    mixed_pairs<PPT, LT, ECL>(rp, se + 2 * (p - q0), pe - p, ex, ey, pf, s);
+                p = pe;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < PPT; j++) acc[j] += s[j].x + s[j].y;
     }
 }
 
-// 3 CTAs per SM for PPT <= 4 (80 registers, no spills): 24 warps hide the
-// FFMA2 and MUFU latencies better than 16; larger PPT keeps 2
-// A thread's PPT consecutive phase entries of phase tile `tile`.
+// A thread's PPT consecutive phase entries of phase tile `tile`. Threads past
+// the last entry repeat it, so that they never widen their warp's view; what
+// they sum is not stored.
 template <int PPT>
-__device__ __forceinline__ void load_entries(const PhaseDev &ph, int64_t tile, int tid,
-                                             float2 *ex, float2 *ey, float *exy,
-                                             unsigned long long *pf) {
+__device__ __forceinline__ void load_entries(const float4 *ef, const unsigned long long *pfx,
+                                             int64_t nent, int64_t tile, int tid, float2 *ex,
+                                             float2 *ey, float *exy, unsigned long long *pf) {
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
-        const int64_t e = tile * (kThreads * PPT) + tid * PPT + j;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        unsigned long long p = 0ull;
-        if (e < ph.nent) {
-            v = ph.ef[e];
-            p = ph.pfx[e];
-        }
+        int64_t e = tile * (kThreads * PPT) + tid * PPT + j;
+        if (e >= nent) e = nent - 1;
+        const float4 v = ef[e];
         ex[j] = f2(v.x, v.x);
         ey[j] = f2(v.y, v.y);
         exy[j] = sqrtf(fmaf(v.x, v.x, v.y * v.y));
-        pf[j] = p;
+        pf[j] = pfx[e];
     }
 }
 
+// Bytes of shared memory and of bulk copies per face of a chunk: the record,
+// the eclipse range, its share of the run records.
+constexpr uint32_t kRecBytes = 32, kEclBytes = 16;
+constexpr uint32_t kRunBytes = kRunRecs * sizeof(RunRec) / kRunFaces;
+
+// The copies of one chunk of `chunk` faces, by one thread.
+__device__ __forceinline__ void stage_chunk(unsigned char *smem, const float *fp,
+                                            const ulonglong2 *ecl, const RunRec *runs,
+                                            uint32_t chunk, bool need_ecl, uint64_t *bar) {
+    mbar_arrive_expect_tx(bar, chunk * (kRecBytes + kRunBytes + (need_ecl ? kEclBytes : 0u)));
+    bulk_g2s(smem, fp, chunk * kRecBytes, bar);
+    if (need_ecl) bulk_g2s(smem + chunk * kRecBytes, ecl, chunk * kEclBytes, bar);
+    bulk_g2s(smem + chunk * (kRecBytes + kEclBytes), runs, chunk * kRunBytes, bar);
+}
+
 // One staged chunk [c0, cend): the pairs holding face n0 and those after it
-// take the eclipse test (a never-eclipsed face in that pair has an empty
-// range); faces past n in the last pair carry zero coefficients.
+// may be eclipsed (a never-eclipsed face in that pair has an empty range);
+// faces past n in the last pair carry zero coefficients. 3 CTAs per SM for PPT
+// <= 4 (80 registers): 24 warps hide the FFMA2 and MUFU latencies better than
+// 16.
 template <int PPT, int LT>
-__device__ __forceinline__ void sweep_chunk(const FlatDev &f, const float4 *sp,
-                                            const ulonglong2 *se, int64_t c0, int64_t cend,
-                                            int64_t n0, const float2 *ex, const float2 *ey,
-                                            const float *exy, const unsigned long long *pf,
-                                            unsigned long long A, unsigned long long L,
-                                            float *acc) {
-    const int64_t q0 = c0 >> 1, qend = (cend + 1) >> 1, qn0 = n0 >> 1;
-    const int64_t qa = qn0 < qend ? qn0 : qend;
-    sweep_pairs<PPT, LT, false>(sp, se, q0, q0, qa > q0 ? qa : q0, ex, ey, exy, pf, A, L, f.runb,
-                                f.runh, acc);
-    sweep_pairs<PPT, LT, true>(sp, se, q0, qa > q0 ? qa : q0, qend, ex, ey, exy, pf, A, L, f.runb,
-                               f.runh, acc);
+__device__ __forceinline__ void sweep_chunk(const unsigned char *smem, uint32_t chunk, int64_t c0,
+                                            int64_t cend, int64_t n0, const float2 *ex,
+                                            const float2 *ey, const float *exy,
+                                            const unsigned long long *pf, unsigned long long A,
+                                            unsigned long long L, float *acc) {
+    const float4 *sp = reinterpret_cast<const float4 *>(smem);
+    const ulonglong2 *se = reinterpret_cast<const ulonglong2 *>(smem + chunk * kRecBytes);
+    const RunRec *sr =
+        reinterpret_cast<const RunRec *>(smem + chunk * (kRecBytes + kEclBytes));
+    // pairs counted from the chunk's first
+    const int64_t q0 = c0 >> 1, qn0 = (n0 >> 1) - q0;
+    const int qend = (int)(((cend + 1) >> 1) - q0);
+    const int qa = qn0 < 0 ? 0 : qn0 < qend ? (int)qn0 : qend;
+    sweep_pairs<PPT, LT, false>(sp, se, sr, 0, 0, qa, ex, ey, exy, pf, A, L, acc);
+    sweep_pairs<PPT, LT, true>(sp, se, sr, 0, qa, qend, ex, ey, exy, pf, A, L, acc);
 }
 
 template <int PPT, int LT>
-__global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
-    k_flux_fast(FlatDev f, PhaseDev ph, int64_t chunk, int64_t ntile, double *part, int64_t ldp,
-                DevStatus *st) {
+__global__ void __launch_bounds__(kThreads, 3)
+    k_flux_fast(FlatDev f, PhaseDev ph, int64_t chunk, double *part, int64_t ldp, DevStatus *st) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
     const int tid = threadIdx.x;
     const int64_t c0 = (int64_t)blockIdx.y * chunk;
     const int64_t n = f.n, n0 = *f.n0;
     const int64_t cend = (c0 + chunk < n) ? c0 + chunk : n;
-    const bool need_ecl = cend > n0;
-    float4 *sp = reinterpret_cast<float4 *>(smem);
-    ulonglong2 *se = reinterpret_cast<ulonglong2 *>(smem + chunk * 32);
     if (tid == 0) mbar_init(&bar, 1);
     __syncthreads();
-    if (tid == 0) {
-        const uint32_t bytes = (uint32_t)(chunk * 32) + (need_ecl ? (uint32_t)(chunk * 16) : 0u);
-        mbar_arrive_expect_tx(&bar, bytes);
-        bulk_g2s(sp, f.fp + 8 * c0, (uint32_t)(chunk * 32), &bar);
-        if (need_ecl) bulk_g2s(se, f.ecl + c0, (uint32_t)(chunk * 16), &bar);
-    }
+    if (tid == 0)
+        stage_chunk(smem, f.fp + 8 * c0, f.ecl + c0, f.runs + kRunRecs * (c0 / kRunFaces),
+                    (uint32_t)chunk, cend > n0, &bar);
     float2 ex[PPT], ey[PPT];
     float exy[PPT];
     unsigned long long pf[PPT];
-    load_entries<PPT>(ph, (int64_t)blockIdx.x, tid, ex, ey, exy, pf);
+    load_entries<PPT>(ph.ef, ph.pfx, ph.nent, (int64_t)blockIdx.x, tid, ex, ey, exy, pf);
     unsigned long long A, L;
-    warp_arc<PPT>(pf, (int64_t)blockIdx.x * (kThreads * PPT) + tid * PPT, ph.nent, A, L);
+    warp_arc<PPT>(pf, A, L);
     // warp-uniform: a warp leaves together, so no lane is missing at the votes
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar, 0))) {
         if (tid == 0) {
@@ -453,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
     float acc[PPT];
 #pragma unroll
     for (int j = 0; j < PPT; j++) acc[j] = 0.f;
-    sweep_chunk<PPT, LT>(f, sp, se, c0, cend, n0, ex, ey, exy, pf, A, L, acc);
+    sweep_chunk<PPT, LT>(smem, (uint32_t)chunk, c0, cend, n0, ex, ey, exy, pf, A, L, acc);
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
         const int64_t e = (int64_t)blockIdx.x * (kThreads * PPT) + tid * PPT + j;
@@ -466,7 +537,7 @@ __global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
 // its limb-darkening law. Same per-element arithmetic and sums as
 // k_flux_fast.
 template <int PPT>
-__global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, 3)
     k_flux_batch(BatchDev b, BatchPhases ph, int64_t chunk, int64_t ntile, double *part,
                  int64_t ldp) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -480,40 +551,20 @@ __global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
     const int64_t n = S.nface, n0 = b.n0[s];
     const int64_t cend = (c0 + chunk < n) ? c0 + chunk : n;
     const int model = S.model, ltype = S.fc.ltype;
-    const bool need_ecl = cend > n0;
-    float4 *sp = reinterpret_cast<float4 *>(smem);
-    ulonglong2 *se = reinterpret_cast<ulonglong2 *>(smem + chunk * 32);
     if (tid == 0) mbar_init(&bar, 1);
     __syncthreads();
     if (tid == 0) {
-        const uint32_t bytes = (uint32_t)(chunk * 32) + (need_ecl ? (uint32_t)(chunk * 16) : 0u);
-        mbar_arrive_expect_tx(&bar, bytes);
-        bulk_g2s(sp, b.fp + 8 * (S.flat0 + c0), (uint32_t)(chunk * 32), &bar);
-        if (need_ecl) bulk_g2s(se, b.ecl + S.flat0 + c0, (uint32_t)(chunk * 16), &bar);
+        const int64_t f0 = S.flat0 + c0;
+        stage_chunk(smem, b.fp + 8 * f0, b.ecl + f0, b.runs + kRunRecs * (f0 / kRunFaces),
+                    (uint32_t)chunk, cend > n0, &bar);
     }
-    const float4 *ef = ph.ef + model * ph.ldp;
-    const unsigned long long *pfx = ph.pfx + model * ph.ldp;
-    const float4 *runb = b.runb + S.flat0 / 64;
-    const ulonglong2 *runh = b.runh + S.flat0 / 64;
     float2 ex[PPT], ey[PPT];
     float exy[PPT];
     unsigned long long pf[PPT];
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int64_t e = tile * (kThreads * PPT) + tid * PPT + j;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        unsigned long long p = 0ull;
-        if (e < ph.nent) {
-            v = ef[e];
-            p = pfx[e];
-        }
-        ex[j] = f2(v.x, v.x);
-        ey[j] = f2(v.y, v.y);
-        exy[j] = sqrtf(fmaf(v.x, v.x, v.y * v.y));
-        pf[j] = p;
-    }
+    load_entries<PPT>(ph.ef + model * ph.ldp, ph.pfx + model * ph.ldp, ph.nent, tile, tid, ex, ey,
+                      exy, pf);
     unsigned long long A, L;
-    warp_arc<PPT>(pf, tile * (kThreads * PPT) + tid * PPT, ph.nent, A, L);
+    warp_arc<PPT>(pf, A, L);
     // warp-uniform: a warp leaves together, so no lane is missing at the votes
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar, 0))) {
         if (tid == 0) {
@@ -525,16 +576,10 @@ __global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
     float acc[PPT];
 #pragma unroll
     for (int j = 0; j < PPT; j++) acc[j] = 0.f;
-    const int64_t q0 = c0 >> 1, qend = (cend + 1) >> 1, qn0 = n0 >> 1;
-    const int64_t qa = qn0 < qend ? qn0 : qend;
-    const int64_t qb = qa > q0 ? qa : q0;
-    if (ltype == 1) {
-        sweep_pairs<PPT, 1, false>(sp, se, q0, q0, qb, ex, ey, exy, pf, A, L, runb, runh, acc);
-        sweep_pairs<PPT, 1, true>(sp, se, q0, qb, qend, ex, ey, exy, pf, A, L, runb, runh, acc);
-    } else {
-        sweep_pairs<PPT, 0, false>(sp, se, q0, q0, qb, ex, ey, exy, pf, A, L, runb, runh, acc);
-        sweep_pairs<PPT, 0, true>(sp, se, q0, qb, qend, ex, ey, exy, pf, A, L, runb, runh, acc);
-    }
+    if (ltype == 1)
+        sweep_chunk<PPT, 1>(smem, (uint32_t)chunk, c0, cend, n0, ex, ey, exy, pf, A, L, acc);
+    else
+        sweep_chunk<PPT, 0>(smem, (uint32_t)chunk, c0, cend, n0, ex, ey, exy, pf, A, L, acc);
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
         const int64_t e = tile * (kThreads * PPT) + tid * PPT + j;
@@ -545,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, (PPT <= 4) ? 3 : 2)
 template <int PPT>
 void launch_batch_t(const BatchDev &b, const BatchPhases &ph, const FluxPlan &plan, double *part,
                     int64_t ldp, cudaStream_t s) {
-    const size_t smem = (size_t)plan.chunk * 48;  // 32 B records + 16 B eclipse ranges
+    const size_t smem = (size_t)plan.chunk * (kRecBytes + kEclBytes + kRunBytes);
     auto kern = k_flux_batch<PPT>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int64_t nblk = plan.nchunk * plan.ntile;
@@ -556,11 +601,11 @@ void launch_batch_t(const BatchDev &b, const BatchPhases &ph, const FluxPlan &pl
 template <int PPT, int LT>
 void launch_fast_t(const FlatDev &f, const PhaseDev &ph, const FluxPlan &plan, double *part,
                    int64_t ldp, DevStatus *st, cudaStream_t s) {
-    const size_t smem = (size_t)plan.chunk * 48;  // 32 B records + 16 B eclipse ranges
+    const size_t smem = (size_t)plan.chunk * (kRecBytes + kEclBytes + kRunBytes);
     auto kern = k_flux_fast<PPT, LT>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid((unsigned)plan.ntile, (unsigned)plan.nchunk);
-    kern<<<grid, kThreads, smem, s>>>(f, ph, plan.chunk, plan.ntile, part, ldp, st);
+    kern<<<grid, kThreads, smem, s>>>(f, ph, plan.chunk, part, ldp, st);
     count_launch();
 }
 
@@ -608,26 +653,37 @@ FluxPlan plan_flux(int mixed, int fast, int64_t nface, int64_t nent, int nsm) {
     FluxPlan p;
     p.fast = mixed && fast;
     if (p.fast) {
-        // entries per thread: the fewest idle lanes, weighed against the per-face
-        // shared-memory loads that a larger PPT amortises
+        // The chunk fixes how the FP32 sums are grouped, so its rule stands by
+        // itself: the largest that gives the SMs four CTAs each at the phase
+        // tiling with the fewest idle lanes, weighing c entries a thread 8 + 8 / c.
         p.threads = kThreads;
-        const int cand[] = {4, 2, 1};  // PPT 8 spills with the face loop unrolled by 2
-        double best = 1e300;
-        p.ppt = 1;
-        for (int c : cand) {
-            const int64_t nt = (nent + (int64_t)kThreads * c - 1) / ((int64_t)kThreads * c);
-            const double cost = (double)nt * kThreads * c * (8.0 + 8.0 / c) / (double)(nent > 0 ? nent : 1);
-            if (cost < best - 1e-9) {
-                best = cost;
-                p.ppt = c;
+        const int cand[] = {4, 2, 1};  // PPT 8 spills
+        const auto tiles = [&](int c) {
+            const int64_t t = (nent + (int64_t)kThreads * c - 1) / ((int64_t)kThreads * c);
+            return t < 1 ? (int64_t)1 : t;
+        };
+        const auto fewest = [&](double fixed, double per_face) {
+            double best = 1e300;
+            int pick = 1;
+            for (int c : cand) {
+                const double cost = (double)tiles(c) * kThreads * c * (fixed + per_face / c);
+                if (cost < best * (1. - 1e-12)) {
+                    best = cost;
+                    pick = c;
+                }
             }
-        }
-        p.ntile = (nent + (int64_t)kThreads * p.ppt - 1) / ((int64_t)kThreads * p.ppt);
-        if (p.ntile < 1) p.ntile = 1;
-        const int64_t want = ((int64_t)nsm * 4 + p.ntile - 1) / p.ntile;
-        int64_t chunk = 1024;  // 48 B per face: 48 KB of shared memory per CTA
+            return pick;
+        };
+        const int64_t nt = tiles(fewest(8., 8.));
+        const int64_t want = ((int64_t)nsm * 4 + nt - 1) / nt;
+        int64_t chunk = 1024;  // 53 B per face: 54 KB of shared memory per CTA
         while (chunk > 64 && (nface + chunk - 1) / chunk < want) chunk >>= 1;
         p.chunk = chunk;
+        // Entries per thread change no sum. Measured per element and thread: 22.1
+        // cycles at 4, 23.1 at 2 (and narrower warps, which see more groups whole),
+        // about 25 at 1; idle lanes of the last tile cost as much as busy ones.
+        p.ppt = fewest(21., 4.);
+        p.ntile = tiles(p.ppt);
     } else if (mixed) {
         p.threads = kThreads;
         p.ppt = nent >= 16384 ? 8 : (nent >= 2048 ? 4 : 1);
@@ -660,9 +716,6 @@ void launch_flux(int mixed, int star, const FluxConsts &k, const FlatDev &f,
     }
     if (plan.fast) {
         switch (plan.ppt) {
-        case 16: launch_fast_ppt<16>(k.ltype, f, ph, plan, part, ldp, st, s); break;
-        case 12: launch_fast_ppt<12>(k.ltype, f, ph, plan, part, ldp, st, s); break;
-        case 8: launch_fast_ppt<8>(k.ltype, f, ph, plan, part, ldp, st, s); break;
         case 4: launch_fast_ppt<4>(k.ltype, f, ph, plan, part, ldp, st, s); break;
         case 2: launch_fast_ppt<2>(k.ltype, f, ph, plan, part, ldp, st, s); break;
         default: launch_fast_ppt<1>(k.ltype, f, ph, plan, part, ldp, st, s); break;

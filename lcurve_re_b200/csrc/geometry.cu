@@ -879,101 +879,145 @@ __global__ void __launch_bounds__(1024) k_interp(const DatumRec *__restrict__ da
     }
 }
 
-// Bound of mu over one run of 32 face pairs of the fast records, one warp per
-// run (lane l reads pair l): with a = the mean of (nx, ny), R = the largest
-// |(nx, ny) - a| and C = the largest cz of the run's faces,
-//   mu = ex nx + ey ny + cz <= ex ax + ey ay + |(ex, ey)| R + C.
-// R and C are widened well past FP32 rounding (1e-6, 1e-5), so when the bound
-// is negative the computed mu of every face of the run is <= 0 and the run adds
-// exactly zero. All-zero records (padding) are left out; a run of padding only
-// gets C = -1.
-// With ecl, also the run's eclipse-range hull: an arc [I, I + W) holding every
-// nonempty range (I_f, W_f + 1) of the run's faces, as the record (I, W), or
-// W = ~0 for "test every face" (ranges a quarter orbit long or spread over
-// more than that), (0, 0) when no face of the run has a range.
+// Bounds of a group of consecutive lanes' faces (two per lane), W lanes a
+// group: the mean of (nx, ny), the largest distance r from it and the extremes
+// of cz. r and the extremes are widened well past FP32 rounding (1e-6, 1e-5).
+// All-zero records (padding, faces with several ranges) add zeros whatever is
+// concluded and are left out; a group of them alone gets cmax = -1.
+template <int W>
+__device__ __forceinline__ void group_mu(const float *nx, const float *ny, const float *cz,
+                                         const bool *use, RunRec &R) {
+    const unsigned full = 0xffffffffu;
+    float sx = 0.f, sy = 0.f, cnt = 0.f;
+    for (int k = 0; k < 2; k++)
+        if (use[k]) { sx += nx[k]; sy += ny[k]; cnt += 1.f; }
+    for (int o = W / 2; o > 0; o >>= 1) {
+        sx += __shfl_xor_sync(full, sx, o);
+        sy += __shfl_xor_sync(full, sy, o);
+        cnt += __shfl_xor_sync(full, cnt, o);
+    }
+    const float ax = cnt > 0.f ? sx / cnt : 0.f, ay = cnt > 0.f ? sy / cnt : 0.f;
+    float r = 0.f, hi = -2.f, lo = 2.f;
+    for (int k = 0; k < 2; k++)
+        if (use[k]) {
+            r = fmaxf(r, sqrtf((nx[k] - ax) * (nx[k] - ax) + (ny[k] - ay) * (ny[k] - ay)));
+            hi = fmaxf(hi, cz[k]);
+            lo = fminf(lo, cz[k]);
+        }
+    for (int o = W / 2; o > 0; o >>= 1) {
+        r = fmaxf(r, __shfl_xor_sync(full, r, o));
+        hi = fmaxf(hi, __shfl_xor_sync(full, hi, o));
+        lo = fminf(lo, __shfl_xor_sync(full, lo, o));
+    }
+    R.ax = ax;
+    R.ay = ay;
+    R.r = cnt > 0.f ? r * (1.f + 1e-6f) + 1e-6f : 0.f;
+    R.cmax = cnt > 0.f ? hi + 1e-5f : -1.f;
+    R.cmin = cnt > 0.f ? lo - 1e-5f : -1.f;
+}
+
+// The eclipse arcs of a group from its lanes' offsets off the reference phase
+// ref (signed distances on the circle): hull [lo, hi), common part [lo2, hi2).
+template <int W>
+__device__ __forceinline__ void group_arcs(long long &lo, long long &hi, long long &lo2,
+                                           long long &hi2, bool &whole, bool &bare) {
+    const unsigned full = 0xffffffffu;
+    for (int o = W / 2; o > 0; o >>= 1) {
+        const long long a = __shfl_xor_sync(full, lo, o), b = __shfl_xor_sync(full, hi, o);
+        const long long c = __shfl_xor_sync(full, lo2, o), d = __shfl_xor_sync(full, hi2, o);
+        lo = a < lo ? a : lo;
+        hi = b > hi ? b : hi;
+        lo2 = c > lo2 ? c : lo2;
+        hi2 = d < hi2 ? d : hi2;
+    }
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned mine = W == 32 ? full : ((1u << W) - 1u) << (lane & ~(W - 1));
+    whole = (__ballot_sync(full, whole) & mine) != 0u;
+    bare = (__ballot_sync(full, bare) & mine) != 0u;
+}
+
+__device__ __forceinline__ void set_arcs(RunRec &R, unsigned long long ref, long long lo,
+                                         long long hi, long long lo2, long long hi2, bool whole,
+                                         bool bare) {
+    R.hull = R.all = make_ulonglong2(0ull, 0ull);
+    if (whole) {
+        R.hull.y = ~0ull;
+    } else if (hi > lo) {
+        R.hull = make_ulonglong2(ref + (unsigned long long)lo,
+                                 (unsigned long long)hi - (unsigned long long)lo);
+        if (!bare && hi2 > lo2)
+            R.all = make_ulonglong2(ref + (unsigned long long)lo2,
+                                    (unsigned long long)hi2 - (unsigned long long)lo2);
+    }
+}
+
+// The records of one run (RunRec), one warp per run, lane l reading pair l:
+// the four parts of 8 lanes first, then the run.
 __device__ __forceinline__ void run_bound(const float *__restrict__ fp,
                                           const ulonglong2 *__restrict__ ecl, int64_t npairs,
-                                          int64_t run, float4 *out, ulonglong2 *hull) {
+                                          int64_t run, RunRec *out) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t q = run * 32 + lane;
     float nx[2] = {0.f, 0.f}, ny[2] = {0.f, 0.f}, cz[2] = {0.f, 0.f};
+    ulonglong2 E[2] = {make_ulonglong2(0ull, 0ull), make_ulonglong2(0ull, 0ull)};
     bool use[2] = {false, false};
     if (q < npairs) {
         const float4 P0 = reinterpret_cast<const float4 *>(fp)[4 * q];
         const float4 P1 = reinterpret_cast<const float4 *>(fp)[4 * q + 1];
         nx[0] = P0.x; nx[1] = P0.y; ny[0] = P0.z; ny[1] = P0.w; cz[0] = P1.x; cz[1] = P1.y;
         for (int k = 0; k < 2; k++) use[k] = nx[k] != 0.f || ny[k] != 0.f || cz[k] != 0.f;
-    }
-    float sx = 0.f, sy = 0.f, cnt = 0.f;
-    for (int k = 0; k < 2; k++)
-        if (use[k]) { sx += nx[k]; sy += ny[k]; cnt += 1.f; }
-    for (int o = 16; o > 0; o >>= 1) {
-        sx += __shfl_xor_sync(full, sx, o);
-        sy += __shfl_xor_sync(full, sy, o);
-        cnt += __shfl_xor_sync(full, cnt, o);
-    }
-    const float ax = cnt > 0.f ? sx / cnt : 0.f, ay = cnt > 0.f ? sy / cnt : 0.f;
-    float r = 0.f, c = -1.f;
-    for (int k = 0; k < 2; k++)
-        if (use[k]) {
-            r = fmaxf(r, sqrtf((nx[k] - ax) * (nx[k] - ax) + (ny[k] - ay) * (ny[k] - ay)));
-            c = fmaxf(c, cz[k]);
-        }
-    for (int o = 16; o > 0; o >>= 1) {
-        r = fmaxf(r, __shfl_xor_sync(full, r, o));
-        c = fmaxf(c, __shfl_xor_sync(full, c, o));
-    }
-    if (lane == 0)
-        *out = cnt > 0.f ? make_float4(ax, ay, r * (1.f + 1e-6f) + 1e-6f, c + 1e-5f)
-                         : make_float4(0.f, 0.f, 0.f, -1.f);
-    if (!ecl) return;
-    ulonglong2 E[2] = {make_ulonglong2(0ull, 0ull), make_ulonglong2(0ull, 0ull)};
-    if (q < npairs) {
         E[0] = ecl[2 * q];
         E[1] = ecl[2 * q + 1];
     }
+    RunRec part, whole_run;
+    group_mu<8>(nx, ny, cz, use, part);
+    group_mu<32>(nx, ny, cz, use, whole_run);
+    // offsets from one range's start, as signed 64-bit distances on the circle;
+    // ranges a quarter orbit long or further than that from it make the group's
+    // hull "anywhere"; a live face without a range leaves no common part
+    for (int k = 0; k < 2; k++)
+        if (!use[k]) E[k].y = 0ull;
     const unsigned m = __ballot_sync(full, E[0].y != 0ull || E[1].y != 0ull);
-    ulonglong2 H = make_ulonglong2(0ull, 0ull);
-    if (m) {
-        // offsets from one range's start, as signed 64-bit distances on the circle
-        const unsigned long long mine = E[0].y != 0ull ? E[0].x : E[1].x;
-        const unsigned long long ref = __shfl_sync(full, mine, __ffs(m) - 1);
-        constexpr long long kQuarter = 1ll << 62;
-        long long lo = LLONG_MAX, hi = LLONG_MIN;
-        bool whole = false;
-        for (int k = 0; k < 2; k++)
-            if (E[k].y != 0ull) {
-                const long long off = (long long)(E[k].x - ref);
-                if (E[k].y >= (unsigned long long)kQuarter || off >= kQuarter || off <= -kQuarter) {
-                    whole = true;
-                } else {
-                    lo = off < lo ? off : lo;
-                    const long long end = off + (long long)E[k].y;
-                    hi = end > hi ? end : hi;
-                }
-            }
-        for (int o = 16; o > 0; o >>= 1) {
-            const long long l2 = __shfl_xor_sync(full, lo, o), h2 = __shfl_xor_sync(full, hi, o);
-            lo = l2 < lo ? l2 : lo;
-            hi = h2 > hi ? h2 : hi;
+    const unsigned long long mine = E[0].y != 0ull ? E[0].x : E[1].x;
+    const unsigned long long ref = __shfl_sync(full, mine, m ? __ffs(m) - 1 : 0);
+    constexpr long long kQuarter = 1ll << 62;
+    long long lo = LLONG_MAX, hi = LLONG_MIN, lo2 = LLONG_MIN, hi2 = LLONG_MAX;
+    bool whole = false, bare = false;
+    for (int k = 0; k < 2; k++) {
+        if (E[k].y == 0ull) {
+            bare = bare || use[k];
+            continue;
         }
-        whole = __any_sync(full, whole);
-        H = whole ? make_ulonglong2(0ull, ~0ull)
-                  : make_ulonglong2(ref + (unsigned long long)lo,
-                                    (unsigned long long)hi - (unsigned long long)lo);
+        const long long off = (long long)(E[k].x - ref);
+        if (E[k].y >= (unsigned long long)kQuarter || off >= kQuarter || off <= -kQuarter) {
+            whole = true;
+            continue;
+        }
+        const long long end = off + (long long)E[k].y;
+        lo = off < lo ? off : lo;
+        hi = end > hi ? end : hi;
+        lo2 = off > lo2 ? off : lo2;
+        hi2 = end < hi2 ? end : hi2;
     }
-    if (lane == 0) *hull = H;
+    long long l = lo, h = hi, l2 = lo2, h2 = hi2;
+    bool w = whole, b = bare;
+    group_arcs<8>(l, h, l2, h2, w, b);
+    set_arcs(part, ref, l, h, l2, h2, w, b);
+    group_arcs<32>(lo, hi, lo2, hi2, whole, bare);
+    set_arcs(whole_run, ref, lo, hi, lo2, hi2, whole, bare);
+    if ((lane & 7) == 0) out[1 + (lane >> 3)] = part;
+    if (lane == 0) out[0] = whole_run;
 }
 
 __global__ void k_run_bounds(const float *__restrict__ fp, const ulonglong2 *__restrict__ ecl,
-                             int64_t npairs, float4 *runb, ulonglong2 *runh) {
+                             int64_t npairs, RunRec *runs) {
     const int64_t run = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (run >= (npairs + 31) / 32) return;  // whole warps
-    run_bound(fp, ecl, npairs, run, runb + run, runh + run);
+    run_bound(fp, ecl, npairs, run, runs + kRunRecs * run);
 }
 
-// Run bounds of the continuum list's slots (16 runs per 1024-face block).
+// Run records of the continuum list's slots (16 runs per 1024-face block).
 __global__ void k_run_bounds_b(BatchDev b) {
     const int nk = b.counts[1];
     if (nk <= 0) return;
@@ -986,7 +1030,7 @@ __global__ void k_run_bounds_b(BatchDev b) {
         const SlotDev &S = b.slots[b.cont_slot[k]];
         const int64_t run = (B - b.cont_blk[k]) * 16 + (w & 15);
         run_bound(b.fp + 8 * S.flat0, b.ecl + S.flat0, (S.nface + 1) / 2, run,
-                  b.runb + S.flat0 / 64 + run, b.runh + S.flat0 / 64 + run);
+                  b.runs + kRunRecs * (S.flat0 / kRunFaces + run));
     }
 }
 
@@ -1512,7 +1556,7 @@ void launch_flatten(GridDev g, FlatDev f, int32_t *blockcnt, int mixed, int need
     count_launch();
     k_flat_scatter<<<nb, kFlatBlock, 0, s>>>(g, f, blockcnt, mixed, need_pos, fc);
     count_launch();
-    if (mixed && fc.on) launch_run_bounds(f.fp, f.ecl, f.npad / 2, f.runb, f.runh, s);
+    if (mixed && fc.on) launch_run_bounds(f.fp, f.ecl, f.npad / 2, f.runs, s);
 }
 
 void launch_phases(const PhaseParams &p, const DatumRec *data, const int64_t *off, int32_t n,
@@ -1551,11 +1595,11 @@ void launch_interp(const DatumRec *data, int32_t n, const int64_t *idx, int32_t 
     count_launch();
 }
 
-void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, float4 *runb,
-                       ulonglong2 *runh, cudaStream_t s) {
+void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, RunRec *runs,
+                       cudaStream_t s) {
     const int64_t nruns = (npairs + 31) / 32;
     if (nruns <= 0) return;
-    k_run_bounds<<<nblocks(nruns * 32, 256), 256, 0, s>>>(fp, ecl, npairs, runb, runh);
+    k_run_bounds<<<nblocks(nruns * 32, 256), 256, 0, s>>>(fp, ecl, npairs, runs);
     count_launch();
 }
 
