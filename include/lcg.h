@@ -452,6 +452,19 @@ lcg_status lcg_mlp_backward_data(void *stream, int32_t m, int32_t depth, int32_t
                                  const void *g_out, const void *const *wt_bf16,
                                  const void *const *z, void *const *g, void *const *gt,
                                  int32_t ldt, int32_t *err);
+/* The weight and bias gradients of the same network from the chain's
+ * transposed gradients gt[l] and activations yt[l], in two launches: for layers
+ * l = 1..nl dw[l] = gt[l] yt[l - 1]^T on the tensor cores and db[l] the row sums
+ * of gt[l]; for the input layer dw[0] [width x kin] = gt[0] x and db[0]. gt[l]
+ * is [width x ldt] ([nout x ldt] for l = nl), yt[l] [width x ldt], x [rows x
+ * kin] FP32 (kin <= 16); rows and width multiples of 128, nout of 64, nl <= 5.
+ * With loss_acc, the sum of loss_rows is added to it in double.
+ * Slices of the batch may be added atomically: dw is reproducible to FP32
+ * rounding of the order. 16-byte aligned gt, yt and dw. */
+lcg_status lcg_mlp_grads(void *stream, int32_t rows, int32_t ldt, int32_t width, int32_t nl,
+                         int32_t nout, const void *const *gt, const void *const *yt,
+                         const float *x, int32_t kin, float *const *dw, float *const *db,
+                         const float *loss_rows, double *loss_acc, int32_t *err);
 /* Per row r of coef [m x ncoef]: the surrogate curve s(c) = mean + c * basis
  * (basis [ncoef x npts]) at the data points, or, with an anchor (exact curves
  * [m x npts] at the points coef_x [m x ncoef] describes), the anchored curve

@@ -129,6 +129,8 @@ PROTOTYPES = {
                                   C.c_int32, P, P, P, P, P, C.c_int32, P, P, P, P, P]),
     "lcg_mlp_backward_data": (C.c_int, [P, C.c_int32, C.c_int32, C.c_int32, P, P, P, P, P,
                                         C.c_int32, P]),
+    "lcg_mlp_grads": (C.c_int, [P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, P, P,
+                                P, C.c_int32, P, P, P, P, P]),
     "lcg_mlp_colsum": (C.c_int, [P, P, C.c_int32, C.c_int32, C.c_int32, P]),
     "lcg_mlp_input": (C.c_int, [P, P, C.c_int32, P, P, C.c_int32, C.c_int32, C.c_int32, P, P,
                                 P, C.c_int32]),

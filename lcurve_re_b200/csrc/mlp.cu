@@ -48,10 +48,12 @@ struct GemmOut {
     int32_t *err;
 };
 
+// One 128 x BN tile at (m0, n0) over K columns [k0, k0 + k); split: other
+// slices of K add into the same FP32 output, which is zero before.
 template <int BN, int EPI>
-__global__ void __launch_bounds__(128) k_gemm(const __grid_constant__ CUtensorMap ta,
-                                              const __grid_constant__ CUtensorMap tb, int32_t k,
-                                              GemmOut o) {
+__device__ __forceinline__ void gemm_tile(const CUtensorMap &ta, const CUtensorMap &tb, int32_t k,
+                                          int32_t k0, int m0, int n0, bool split,
+                                          const GemmOut &o) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem =
         reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -60,7 +62,6 @@ __global__ void __launch_bounds__(128) k_gemm(const __grid_constant__ CUtensorMa
     __shared__ uint32_t tmem_base;
     __shared__ int ok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
     unsigned char *sa0 = smem, *sb0 = smem + 2 * kABytes;
     if (tid == 0) {
         mbar_init(&full[0], 1);
@@ -80,8 +81,7 @@ __global__ void __launch_bounds__(128) k_gemm(const __grid_constant__ CUtensorMa
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const int nk = k / kBK;          // k: the K slice of this CTA
-    const int k0 = blockIdx.z * k;   // split-K: slices along grid z
+    const int nk = k / kBK;
     if (tid == 0) {
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                                ((uint32_t)(kBM >> 4) << 24);
@@ -188,10 +188,15 @@ __global__ void __launch_bounds__(128) k_gemm(const __grid_constant__ CUtensorMa
                         for (int i = 0; i < 16; i++) o.yt[(size_t)(nb + i) * o.ldt + m] = gb[i];
                     }
                 }
-            } else if (EPI == kEpiF32 && gridDim.z > 1) {
-                // split-K: slices add into the output the launcher zeroed
-                if (store) {
-                    float *op = o.out + (size_t)m * N + nb;
+            } else if (EPI == kEpiF32 && split) {
+                float *op = o.out + (size_t)m * N + nb;
+                if (store && ((uintptr_t)o.out & 15) == 0) {
+                    // four adds an instruction: a lane's row is a sector of its own
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        atomicAdd(reinterpret_cast<float4 *>(op) + i,
+                                  make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+                } else if (store) {
 #pragma unroll
                     for (int i = 0; i < 16; i++) atomicAdd(op + i, v[i]);
                 }
@@ -211,6 +216,148 @@ __global__ void __launch_bounds__(128) k_gemm(const __grid_constant__ CUtensorMa
         fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN)
                      : "memory");
+    }
+}
+
+template <int BN, int EPI>
+__global__ void __launch_bounds__(128) k_gemm(const __grid_constant__ CUtensorMap ta,
+                                              const __grid_constant__ CUtensorMap tb, int32_t k,
+                                              const __grid_constant__ GemmOut o) {
+    // split-K: slices along grid z
+    gemm_tile<BN, EPI>(ta, tb, k, (int32_t)blockIdx.z * k, blockIdx.y * kBM, blockIdx.x * BN,
+                       gridDim.z > 1, o);
+}
+
+// The weight gradients of every layer after the first in one launch:
+// dw[l] = gt[l] yt[l]^T over K = the batch. Four launches of 64 CTAs each, with a
+// memset before it, took 38 + 5 us for 4096 rows: each is the latency of one
+// tile (setup, its slice of K, atomics). Together they take that once.
+constexpr int kWgradMax = 5, kWgradBN = 64;
+struct WgradSet {
+    CUtensorMap a[kWgradMax], b[kWgradMax];
+    float *out[kWgradMax];
+    int32_t mvalid[kWgradMax], tile0[kWgradMax + 1];  // first 128 x 64 tile of each layer
+    int32_t nl, n, k;  // k: columns of K per slice
+    int32_t *err;
+};
+
+__global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ WgradSet w) {
+    int l = 0;
+    while (l + 1 < w.nl && (int)blockIdx.x >= w.tile0[l + 1]) l++;
+    const int t = (int)blockIdx.x - w.tile0[l], nt = w.n / kWgradBN;
+    GemmOut o{nullptr, nullptr, nullptr, nullptr, w.out[l], w.n, w.mvalid[l], 0, w.err};
+    gemm_tile<kWgradBN, kEpiF32>(w.a[l], w.b[l], w.k, (int32_t)blockIdx.y * w.k, (t / nt) * kBM,
+                                 (t % nt) * kWgradBN, gridDim.y > 1, o);
+}
+
+// What else a training step needs from the layers' gradients, in one launch (five
+// column sums, the input layer's gradient and four memsets were ten, 64 us for
+// 4096 rows, the column sums on 8 CTAs each): by CTA, in this order
+//   * the input layer: two units a CTA, four warps each over a quarter of the
+//     rows: dw0[u][k] = sum gt0[u][r] x[r][k], db[0][u] = sum gt0[u][r];
+//   * the other layers' bias gradients, one warp per unit along its row of gt;
+//   * zeros into the weight gradients, which k_wgrad's slices add into;
+//   * the loss rows added to *loss_acc in double.
+// Fixed order throughout: per lane, then a shuffle tree (deterministic).
+constexpr int kGradThreads = 256;
+struct GradSet {
+    const __nv_bfloat16 *gt[kWgradMax + 1];  // [units x ldt] of layers 0..nl
+    float *db[kWgradMax + 1], *dw[kWgradMax + 1];
+    int32_t units[kWgradMax + 1], cta0[kWgradMax + 2];
+    int64_t zero[kWgradMax + 1], zcta0[kWgradMax + 2];  // floats to clear in dw[1..nl]
+    const float *x, *loss_rows;
+    double *loss_acc;
+    int32_t nl, rows, ldt, kin, loss_cta;
+};
+constexpr int kZeroPerCta = kGradThreads * 16;
+
+__device__ __forceinline__ float warp_add(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__global__ void __launch_bounds__(kGradThreads) k_grads(const __grid_constant__ GradSet s) {
+    const int cta = blockIdx.x, t = threadIdx.x, w = t >> 5, lane = t & 31;
+    if (cta < s.cta0[1]) {
+        __shared__ float sh[8][17];
+        const int u = 2 * cta + (w >> 2), quarter = w & 3;
+        const int per = s.rows / 4, r0 = quarter * per;  // rows: a multiple of 128
+        const __nv_bfloat16 *g = s.gt[0] + (size_t)u * s.ldt;
+        float acc[17];
+#pragma unroll
+        for (int k = 0; k < 17; k++) acc[k] = 0.f;
+#pragma unroll 4
+        for (int r = r0 + lane; r < r0 + per; r += 32) {
+            const float gv = __bfloat162float(g[r]);
+            const float *xr = s.x + (size_t)r * s.kin;
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                if (k < s.kin) acc[k] = fmaf(gv, xr[k], acc[k]);
+            acc[16] += gv;
+        }
+#pragma unroll
+        for (int k = 0; k < 17; k++) {
+            const float v = warp_add(acc[k]);
+            if (lane == 0) sh[w][k] = v;
+        }
+        __syncthreads();
+        if (t < 64) {
+            const int uu = t >> 5, k = t & 31, W = 4 * uu;
+            if (k < 17) {
+                const float v = (sh[W][k] + sh[W + 1][k]) + (sh[W + 2][k] + sh[W + 3][k]);
+                if (k == 16) s.db[0][2 * cta + uu] = v;
+                else if (k < s.kin) s.dw[0][(size_t)(2 * cta + uu) * s.kin + k] = v;
+            }
+        }
+        return;
+    }
+    if (cta < s.cta0[s.nl + 1]) {
+        int l = 1;
+        while (cta >= s.cta0[l + 1]) l++;
+        const int u = (cta - s.cta0[l]) * 8 + w;
+        if (u >= s.units[l]) return;
+        // 8 columns a lane and trip: ldt and the rows are multiples of 8
+        const uint4 *g = reinterpret_cast<const uint4 *>(s.gt[l] + (size_t)u * s.ldt);
+        float acc = 0.f;
+        for (int c = lane; c < s.rows / 8; c += 32) {
+            const uint4 q = g[c];
+            const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&q);
+            float part = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 f = __bfloat1622float2(h[i]);
+                part += f.x + f.y;
+            }
+            acc += part;
+        }
+        acc = warp_add(acc);
+        if (lane == 0) s.db[l][u] = acc;
+        return;
+    }
+    if (cta < s.loss_cta) {
+        const int64_t c = cta - s.cta0[s.nl + 1];
+        int l = 1;
+        while (c >= s.zcta0[l + 1]) l++;
+        const int64_t base = (c - s.zcta0[l]) * kZeroPerCta;
+        for (int i = 0; i < 4; i++) {
+            const int64_t e = base + 4 * ((int64_t)i * kGradThreads + t);
+            if (e < s.zero[l])
+                *reinterpret_cast<float4 *>(s.dw[l] + e) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        return;
+    }
+    __shared__ double sd[8];
+    double v = 0.;
+    for (int r = t; r < s.rows; r += kGradThreads) v += (double)s.loss_rows[r];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) sd[w] = v;
+    __syncthreads();
+    if (t == 0) {
+        double sum = 0.;
+        for (int i = 0; i < 8; i++) sum += sd[i];
+        *s.loss_acc += sum;
     }
 }
 
@@ -467,10 +614,15 @@ EncodeFn encode_fn() {
 }  // namespace
 
 bool make_map(CUtensorMap *map, const void *base, int32_t rows, int32_t cols, int32_t box_rows) {
+    return make_map_ld(map, base, rows, cols, cols, box_rows);
+}
+
+bool make_map_ld(CUtensorMap *map, const void *base, int32_t rows, int32_t cols, int32_t ld,
+                 int32_t box_rows) {
     EncodeFn fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
     cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides,
@@ -594,6 +746,75 @@ lcg_status lcg_mlp_adam_all(void *stream, int32_t n, float *const *w, float *con
     }
     k_adam_all<<<(unsigned)((a.start[n] + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, sched,
                                                                                        step);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? LCG_OK : LCG_E_CUDA;
+}
+
+lcg_status lcg_mlp_grads(void *stream, int32_t rows, int32_t ldt, int32_t width, int32_t nl,
+                         int32_t nout, const void *const *gt, const void *const *yt,
+                         const float *x, int32_t kin, float *const *dw, float *const *db,
+                         const float *loss_rows, double *loss_acc, int32_t *err) {
+    if (!gt || !yt || !x || !dw || !db || rows <= 0 || rows % kBM || ldt < rows || ldt % 8 ||
+        width <= 0 || width % kBM || nl < 1 || nl > kWgradMax || nout <= 0 || nout % 64 ||
+        kin <= 0 || kin > 16 || (loss_acc && !loss_rows))
+        return LCG_E_INVALID;
+    GradSet g;
+    WgradSet w;
+    memset(&g, 0, sizeof(g));
+    memset(&w, 0, sizeof(w));
+    g.x = x;
+    g.loss_rows = loss_rows;
+    g.loss_acc = loss_acc;
+    g.nl = nl;
+    g.rows = rows;
+    g.ldt = ldt;
+    g.kin = kin;
+    g.cta0[1] = width / 2;
+    w.nl = nl;
+    w.n = width;
+    w.err = err;
+    for (int l = 0; l <= nl; l++) {
+        const int units = l == nl ? nout : width;
+        if (!gt[l] || !dw[l] || !db[l] || (((uintptr_t)gt[l] | (uintptr_t)dw[l]) & 15))
+            return LCG_E_INVALID;
+        g.gt[l] = (const __nv_bfloat16 *)gt[l];
+        g.dw[l] = dw[l];
+        g.db[l] = db[l];
+        g.units[l] = units;
+        if (l == 0) continue;
+        g.cta0[l + 1] = g.cta0[l] + (units + 7) / 8;
+        g.zero[l] = (int64_t)units * width;
+        g.zcta0[l + 1] = g.zcta0[l] + (g.zero[l] + kZeroPerCta - 1) / kZeroPerCta;
+        if (!yt[l - 1] || ((uintptr_t)yt[l - 1] & 15)) return LCG_E_INVALID;
+        // tiles of 128 rows: the copies fill what lies past the last unit with zeros
+        const int mtiles = (units + kBM - 1) / kBM;
+        if (!make_map_ld(&w.a[l - 1], gt[l], units, rows, ldt, kBM) ||
+            !make_map_ld(&w.b[l - 1], yt[l - 1], width, rows, ldt, kWgradBN))
+            return LCG_E_CUDA;
+        w.out[l - 1] = dw[l];
+        w.mvalid[l - 1] = units;
+        w.tile0[l] = w.tile0[l - 1] + mtiles * (width / kWgradBN);
+    }
+    int nsm = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // slices of K: the most that keep two CTAs an SM and four K-blocks a slice
+    // (4096 rows: 28 tiles x 8 slices)
+    const int tiles = w.tile0[nl];
+    int splits = 1;
+    while (tiles * splits * 2 <= 2 * nsm && (rows / kBK) % (splits * 2) == 0 &&
+           rows / (splits * 2) >= 4 * kBK)
+        splits *= 2;
+    w.k = rows / splits;
+    g.loss_cta = g.cta0[nl + 1] + (splits > 1 ? (int32_t)g.zcta0[nl + 1] : 0);
+    cudaStream_t s = (cudaStream_t)stream;
+    k_grads<<<(unsigned)(g.loss_cta + (loss_acc ? 1 : 0)), kGradThreads, 0, s>>>(g);
+    count_launch();
+    const size_t smem = 2 * (size_t)(kBM + kWgradBN) * kBK * 2 + 1024;
+    cudaError_t e =
+        cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return LCG_E_CUDA;
+    k_wgrad<<<dim3((unsigned)tiles, (unsigned)splits), 128, smem, s>>>(w);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? LCG_OK : LCG_E_CUDA;
 }

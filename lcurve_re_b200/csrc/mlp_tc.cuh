@@ -19,6 +19,9 @@ enum { kEpiGelu = 0, kEpiLinear = 1, kEpiDGelu = 2, kEpiF32 = 3 };
 // box_rows rows and 128-byte swizzle (host; false if the driver entry point
 // is missing or the encoding fails).
 bool make_map(CUtensorMap *map, const void *base, int32_t rows, int32_t cols, int32_t box_rows);
+// The same with rows ld elements apart (a multiple of 8).
+bool make_map_ld(CUtensorMap *map, const void *base, int32_t rows, int32_t cols, int32_t ld,
+                 int32_t box_rows);
 
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
     // start address >> 4, LBO 16 B (unused for swizzled K-major), SBO 1024 B

@@ -133,7 +133,11 @@ class MLP:
         self._bw_wt = _ptrs([self.Wt[l] for l in range(L, 0, -1)])
         self._bw_z = _ptrs([self.Z[l] for l in range(L - 1, -1, -1)])
         self._bw_g = _ptrs([self.G[l] for l in range(L - 1, -1, -1)])
-        self._bw_gt = _ptrs([self.Gt[l] for l in range(L - 1, 0, -1)] + [None])
+        self._bw_gt = _ptrs([self.Gt[l] for l in range(L - 1, -1, -1)])
+        self._gr_gt = _ptrs(self.Gt)
+        self._gr_yt = _ptrs(self.Yt)
+        self._gr_dw = _ptrs(self.dW)
+        self._gr_db = _ptrs(self.db)
         self._target_fused = False
         # graph-captured training steps: static batch, device-side schedule
         self.tgt = torch.zeros(B, nout, **f32)
@@ -210,11 +214,12 @@ class MLP:
                    out=self.out, mvalid=n)
         return self.out[:n]
 
-    def backward(self, target=None, sync=True):
+    def backward(self, target=None, sync=True, loss_acc=None):
         """Gradients of the mean squared error of the last forward (a full
         training batch) against target [B, nout], or against the target the
         forward already took. Returns the loss (sync=True) or None (no host
-        synchronisation)."""
+        synchronisation). loss_acc (a float64 device scalar): the batch's summed
+        squared error is added to it."""
         B, w, L = self.B, self.width, self.depth
         if not self._target_fused:
             if target is None:
@@ -229,16 +234,19 @@ class MLP:
                                                 self._bw_wt, self._bw_z, self._bw_g, self._bw_gt,
                                                 B, _p(self.err))
             self._ok(st, "lcg_mlp_backward_data")
-            for l in range(L, 0, -1):
-                self._gemm(EPI_F32, self.Gt[l].shape[0], w, B, self.Gt[l], self.Yt[l - 1],
-                           out=self.dW[l], mvalid=self.nout if l == L else w)
-                self._colsum(self.G[l], self.nout if l == L else w, self.db[l])
+            st = self.lib.lcg_mlp_grads(self._stream(), B, B, w, L, self.nout, self._gr_gt,
+                                        self._gr_yt, _p(self.x), self.nin, self._gr_dw,
+                                        self._gr_db, _p(self.loss_rows), _p(loss_acc),
+                                        _p(self.err))
+            self._ok(st, "lcg_mlp_grads")
         else:
             self._backward_layers()
-        st = self.lib.lcg_mlp_input_grad(self._stream(), _p(self.G[0]), _p(self.x), self.nin, B,
-                                         w, B, _p(self.dW[0]))
-        self._ok(st, "lcg_mlp_input_grad")
-        self._colsum(self.G[0], w, self.db[0])
+            st = self.lib.lcg_mlp_input_grad(self._stream(), _p(self.G[0]), _p(self.x), self.nin,
+                                             B, w, B, _p(self.dW[0]))
+            self._ok(st, "lcg_mlp_input_grad")
+            self._colsum(self.G[0], w, self.db[0])
+            if loss_acc is not None:
+                loss_acc.add_(self.loss_rows.sum(dtype=self.torch.float64))
         if sync:
             return float(self.loss_rows.sum().item()) / (B * self.nout)
         return None
@@ -288,16 +296,14 @@ class MLP:
         self.step_dev.zero_()
 
     def _train_ops(self):
-        torch = self.torch
         self.forward(self.x, train=True, target=self.tgt)
-        self.backward(sync=False)
+        self.backward(sync=False, loss_acc=self.loss_acc)
         n, w, m1, m2, g, wb, wt = self._adam
         st = self.lib.lcg_mlp_adam_all(self._stream(), n, w, m1, m2, g, self._adam_rows,
                                        self._adam_cols, wb, wt, _p(self.sched),
                                        _p(self.step_dev))
         self._ok(st, "lcg_mlp_adam_all")
         self.step_dev.add_(1)
-        self.loss_acc.add_(self.loss_rows.sum(dtype=torch.float64))
 
     def graph_step(self):
         """One training step on the batch in self.x / self.tgt: fused forward

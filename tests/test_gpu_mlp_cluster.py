@@ -64,3 +64,33 @@ def test_training_pass_is_the_same(nout, depth, batch):
         assert torch.equal(small.G[l], large.G[l][:batch]), l
     small.check()
     large.check()
+
+
+@pytest.mark.parametrize("nout,depth,batch", [(64, 4, 128), (64, 1, 384), (192, 2, 640),
+                                              (256, 5, 4096), (128, 3, 1152)])
+def test_gradients_in_two_launches(nout, depth, batch):
+    """lcg_mlp_grads against FP64 products of the same BF16 factors: the FP32
+    sums of K = batch products are within K 2^-24 of the summed magnitudes
+    (tensor-core adds truncate: twice that)."""
+    import torch
+    from lcurve_re_b200.mlp import MLP
+    net = MLP(nin=9, nout=nout, depth=depth, batch=batch, seed=1)
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    net.x.copy_(torch.rand(net.B, 9, generator=g, device="cuda") * 2 - 1)
+    t = torch.randn(net.B, nout, generator=g, device="cuda")
+    acc = torch.full((1,), 2.5, dtype=torch.float64, device="cuda")
+    for _ in range(2):  # the second pass starts from the first one's gradients
+        net.forward(net.x, train=True, target=t)
+        net.backward(sync=False, loss_acc=acc)
+    net.check()
+    tol = 2 * batch * 2.0 ** -24
+    for l in range(depth + 1):
+        n = net.W[l].shape[0]
+        G = net.G[l].double()
+        prev = net.x.double() if l == 0 else net.Yt[l - 1].double().T
+        ref, mag = G.T @ prev, G.abs().T @ prev.abs()
+        assert ((net.dW[l][:n].double() - ref).abs() <= tol * mag + 1e-30).all(), l
+        ref, mag = G.sum(0), G.abs().sum(0)
+        assert ((net.db[l].double() - ref).abs() <= tol * mag + 1e-30).all(), l
+    want = 2.5 + 2 * float(net.loss_rows.double().sum())
+    assert abs(float(acc) - want) <= 1e-12 * want
