@@ -27,47 +27,82 @@ __device__ __forceinline__ void report(DevStatus *st, int code, int idx) {
 // them from star faces.
 __device__ __forceinline__ int elem_tag(int i) { return -1 - i; }
 
-// The eclipses of one element: the opaque disc's (disc and rim only; the
-// spot gets none, set_bright_spot_grid.cpp:80-81), then star 1's, then star
-// 2's (set_disc_grid.cpp:99-113). trap1: a Roche_Error from star 1 becomes
-// the range (0, 1), as for the rim's upper elements (set_disc_grid.cpp:222-231).
-// One thread solves all of an element's eclipses: nearly every disc element is
-// a Roche candidate of the donor, and a warp per candidate (as for star grids
-// with few candidates) measured slower here.
-__device__ void elem_eclipses(const CompParams &p, V3 posn, bool opaque, bool trap1, ElemRec &r,
-                              DevStatus *st, int idx) {
+// The boundary `side` (0 ingress, 1 egress) of the eclipse of posn by star 1
+// or 2 (ingress_egress.cpp:35-97), by every lane of a warp at once: ecl whether
+// it is eclipsed at all, at the phase; s the failure of pot_min or of this side.
+__device__ __forceinline__ void elem_boundary(const CompParams &p, int star, int side, bool on,
+                                              V3 posn, bool &ecl, double &at, int &s) {
+    const EclParams &E = p.ecl[star];
+    double phi1 = 0., phi2 = 0., lam1, lam2, phi = 0., lam, acc = 0.;
+    ecl = false;
+    at = 0.;
+    s = 0;
+    bool live = false;
+    if (on) {
+        const V3 c = star == kStar1 ? v3(0., 0., 0.) : v3(1., 0., 0.);
+        const double rs = E.comp_roche ? E.comp_rref : E.comp_r;
+        ecl = sphere_eclipse_ph(E.cosi, E.sini, posn, c, rs, phi1, phi2, lam1, lam2);
+        if (ecl && E.comp_roche) {
+            acc = 2. * sqrt(2. * kTwoPi * (lam2 - lam1) * E.delta);
+            ecl = live = pot_min(star, E.q, E.comp_spin, E.cosi, E.sini, posn, phi1, phi2, lam1,
+                                 lam2, E.comp_rref, E.comp_pref, acc, phi, lam, s);
+        }
+    }
+    at = side ? phi2 : phi1;
+    const double v = bisect_warp(E, live, phi, at, acc, posn, s);
+    if (live) at = v - floor(v);
+}
+
+// The eclipses of one element from its four lanes (star 1 ingress, egress, star 2
+// ingress, egress): the opaque disc's (disc and rim only; the spot gets none,
+// set_bright_spot_grid.cpp:80-81), then star 1's, then star 2's
+// (set_disc_grid.cpp:99-113). trap1: a Roche_Error from star 1 becomes the
+// range (0, 1), as for the rim's upper elements (set_disc_grid.cpp:222-231).
+// Nearly every disc element is a candidate of the donor, and the solves are
+// serial FP64 chains: a lane per boundary runs the four side by side. 13,500
+// disc, rim and spot elements: 427 us with one thread solving all of an
+// element's eclipses by bisection -> 75 us.
+__device__ void elem_eclipses(const CompParams &p, V3 posn, bool in_range, bool opaque, bool trap1,
+                              ElemRec &r, DevStatus *st, int idx) {
+    const unsigned full = 0xffffffffu;
+    const int sub = threadIdx.x & 3;
+    bool ecl;
+    double at;
+    int s;
+    elem_boundary(p, sub >> 1, sub & 1, in_range && (sub < 2 ? p.eclipse1 : p.eclipse2), posn, ecl,
+                  at, s);
+    // lane 0 of the element collects (a failure of the ingress comes first)
+    bool necl[2];
+    double in[2], out[2];
+    int es[2];
+    for (int k = 0; k < 2; k++) {
+        const int src = (threadIdx.x & 28) + 2 * k;
+        necl[k] = __shfl_sync(full, ecl, src);
+        in[k] = __shfl_sync(full, at, src);
+        out[k] = __shfl_sync(full, at, src + 1);
+        const int s0 = __shfl_sync(full, s, src), s1 = __shfl_sync(full, s, src + 1);
+        es[k] = s0 ? s0 : s1;
+        if (p.ecl[k].comp_roche && out[k] < in[k]) out[k]++;
+    }
+    if (!in_range || sub != 0) return;
     r.nr = 0;  // an element whose eclipse failed is left with none
     for (int k = 0; k < kMaxRanges; k++) r.r[k] = make_double2(0., 0.);
     int nr = 0;
     double rin[kMaxRanges], rout[kMaxRanges];
-    int s = 0;
     if (opaque) {
-        disc_eclipse(p.dg, posn, nr, rin, rout, kMaxRanges, s);
-        if (s) { report(st, s, idx); return; }
+        int ds = 0;
+        disc_eclipse(p.dg, posn, nr, rin, rout, kMaxRanges, ds);
+        if (ds) { report(st, ds, idx); return; }
     }
-    for (int star = 0; star < 2; star++) {
-        if (!(star == 0 ? p.eclipse1 : p.eclipse2)) continue;
-        double in = 0., out = 0.;
-        bool ecl;
-        int es = 0;
-        if (star == 0 ? p.roche1 : p.roche2) {
-            ecl = ingress_egress(star == 0 ? kStar1 : kStar2, p.q, star == 0 ? p.spin1 : p.spin2,
-                                 p.cosi, p.sini, p.delta, posn, star == 0 ? p.rref1 : p.rref2,
-                                 star == 0 ? p.pref1 : p.pref2, in, out, es);
-        } else {
-            double l1, l2;
-            ecl = sphere_eclipse_ph(p.cosi, p.sini, posn,
-                                    star == 0 ? v3(0., 0., 0.) : v3(1., 0., 0.),
-                                    star == 0 ? p.r1 : p.r2, in, out, l1, l2);
+    for (int k = 0; k < 2; k++) {
+        if (es[k]) {
+            if (!(k == 0 && trap1 && es[k] == kEclRoche)) { report(st, es[k], idx); return; }
+            necl[k] = true;
+            in[k] = 0.;
+            out[k] = 1.;
         }
-        if (es) {
-            if (!(star == 0 && trap1 && es == kEclRoche)) { report(st, es, idx); return; }
-            ecl = true;
-            in = 0.;
-            out = 1.;
-        }
-        if (ecl) {
-            if (nr < kMaxRanges) { rin[nr] = in; rout[nr] = out; }
+        if (necl[k]) {
+            if (nr < kMaxRanges) { rin[nr] = in[k]; rout[nr] = out[k]; }
             nr++;
         }
     }
@@ -76,11 +111,14 @@ __device__ void elem_eclipses(const CompParams &p, V3 posn, bool opaque, bool tr
         r.r[k] = k < r.nr ? make_double2(rin[k], rout[k]) : make_double2(0., 0.);
 }
 
-__global__ void __launch_bounds__(kThreadsC) k_components(CompParams p, ElemRec *el, double4 *pos,
-                                                          DevStatus *st) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Four lanes per element (elem_eclipses); lanes past the last element repeat
+// it without storing, so that warps stay whole.
+__global__ void __launch_bounds__(kThreadsC)
+    k_components(__grid_constant__ const CompParams p, ElemRec *el, double4 *pos, DevStatus *st) {
     const int n = p.nd + p.ne + p.ns;
-    if (i >= n) return;
+    const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const bool in_range = u < n;
+    const int i = in_range ? u : n - 1;
     constexpr double EFAC = 1.0000001;
     V3 posn, dirn;
     double area, flux;
@@ -155,7 +193,8 @@ __global__ void __launch_bounds__(kThreadsC) k_components(CompParams p, ElemRec 
     r.dy = dirn.y;
     r.dz = dirn.z;
     r.flux = (float)flux;
-    elem_eclipses(p, posn, p.opaque && i < p.nd + p.ne, trap1, r, st, elem_tag(i));
+    elem_eclipses(p, posn, in_range, p.opaque && i < p.nd + p.ne, trap1, r, st, elem_tag(i));
+    if (!in_range || (threadIdx.x & 3) != 0) return;
     el[i] = r;
     pos[i] = make_double4(posn.x, posn.y, posn.z, (double)(float)area);
 }
@@ -397,7 +436,7 @@ void launch_components(const CompParams &p, ElemRec *el, double4 *pos, DevStatus
                        cudaStream_t s) {
     const int n = p.nd + p.ne + p.ns;
     if (n <= 0) return;
-    k_components<<<nblk(n, kThreadsC), kThreadsC, 0, s>>>(p, el, pos, st);
+    k_components<<<nblk(4 * (int64_t)n, kThreadsC), kThreadsC, 0, s>>>(p, el, pos, st);
     count_launch();
 }
 
@@ -675,6 +714,21 @@ bool comp_setup(const lcg_model &m, CompParams &p, std::vector<DiscRing> &rings,
         p.length = m.length_spot;
         p.nspot = m.nspot;
         p.ns = 2 * m.nspot;
+    }
+    for (int star = 0; star < 2; star++) {
+        EclParams &e = p.ecl[star];
+        const bool one = star == kStar1;
+        e.comp_star = star;
+        e.comp_roche = one ? p.roche1 : p.roche2;
+        e.q = p.q;
+        e.comp_spin = one ? p.spin1 : p.spin2;
+        e.comp_rref = one ? p.rref1 : p.rref2;
+        e.comp_pref = one ? p.pref1 : p.pref2;
+        e.comp_r = one ? p.r1 : p.r2;
+        e.cosi = p.cosi;
+        e.sini = p.sini;
+        e.delta = p.delta;
+        e.edge = make_edge_star(star, e.q, e.comp_spin, e.cosi, e.sini, e.comp_rref, e.comp_pref);
     }
     return true;
 }

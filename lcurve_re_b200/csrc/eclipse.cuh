@@ -2,8 +2,8 @@
 //
 // Device restatement of Roche::ingress_egress (ingress_egress.cpp:35-97)
 // with its helpers pot_min / linmin (pot_min.cpp:38-420), fblink
-// (fblink.cpp:34-104) and Subs::dbrent (dbrent.cpp:21-126), one thread per
-// surface element. FP64 throughout, same operation order (the file that
+// (fblink.cpp:34-104) and Subs::dbrent (dbrent.cpp:21-126): pot_min per
+// element, then bisect_warp per boundary. FP64 throughout, same operation order (the file that
 // includes this is compiled with --fmad=false), so the eclipse flags and
 // phases follow the reference decision for decision. Every loop that the
 // reference leaves unbounded carries an iteration cap; hitting one returns
@@ -13,6 +13,7 @@
 // inline in its two callers).
 #pragma once
 
+#include "ecl_root.cuh"
 #include "roche.cuh"
 
 namespace lcg {
@@ -353,47 +354,69 @@ __device__ __noinline__ bool fblink(int star, double q, double spin, double acc,
     return false;
 }
 
-// Roche::ingress_egress (ingress_egress.cpp:35-97) with the reference
-// sphere (rref, pref) precomputed. Returns true when eclipsed.
-__device__ bool ingress_egress(int star, double q, double spin, double cosi, double sini,
-                               double delta, V3 r, double rref, double pref, double &ingress,
-                               double &egress, int &st) {
-    const V3 cofm = star == kStar1 ? v3(0., 0., 0.) : v3(1., 0., 0.);
-    double phi1, phi2, lam1, lam2, phi, lam;
-    if (!sphere_eclipse_ph(cosi, sini, r, cofm, rref, phi1, phi2, lam1, lam2)) return false;
-    const double ACC = 2. * sqrt(2. * kTwoPi * (lam2 - lam1) * delta);
-    if (!pot_min(star, q, spin, cosi, sini, r, phi1, phi2, lam1, lam2, rref, pref, ACC, phi,
-                 lam, st))
-        return false;
-    double pin = phi, pout = phi1, pmid;
+// The bisection of ingress (side 0) or egress (side 1) of ingress_egress
+// (ingress_egress.cpp:61-86) from the pot_min state, for every lane of a warp
+// at once (all 32 lanes call it; lanes with live false only vote). The root of
+// the boundary comes first (edge_zone); then each lane takes the bisection's
+// midpoints, comparing those that the certified intervals decide, until one
+// needs a test. The tests run in passes for all lanes that wait for one:
+// eval_edge outside the intervals, fblink_edge between them, and Roche::fblink
+// itself where that is unsure, so the lanes take fblink's decisions at the
+// same midpoints as the plain loop (p: EclParams). FP64 latency and issue bound it: some 4
+// evaluations for the root, 2.3 outside the intervals and 3.3 searches of 5
+// evaluations per boundary by an M dwarf, against 20 tests in FP32 with 6.4
+// fblinks of 8 to 12 evaluations before (a white dwarf's: 6 evaluations
+// against 20 fblinks). 256 models of 60-400 strips: 13.8 -> 5.4 ms; one curve
+// on 81/163 strips: 203 us with its warp mode -> 62. With the FP32 screen kept
+// for the tests outside the intervals it took 5.8 ms.
+template <class Ecl>
+__device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pin, double pout,
+                                              double acc, V3 pos, int &s) {
+    // what the passes read, in registers (p may be global memory)
+    const EdgeStar S = p.edge;
+    const double delta = p.delta;
+    const V3 u0 = v3(pos.x - (p.comp_star == kStar1 ? 0. : 1.), pos.y, pos.z);
+    const double u2 = norm2(u0), dir = pout > pin ? 1. : -1.;
+    EdgeZone z;
+    z.hrad = z.vrad = z.hid = z.vis = z.hc = z.vc = 0.;
+    if (live) z = edge_zone(S, u0, acc, delta, pin, pout);
+    bool done = !live;
     int guard = 0;
-    while (fabs(pin - pout) > delta) {
-        if (++guard > 400) { st = kEclNoConverge; return false; }
-        pmid = (pin + pout) / 2.;
-        if (fblink(star, q, spin, ACC, set_earth(cosi, sini, pmid), r, rref, pref, st))
-            pin = pmid;
-        else
-            pout = pmid;
-        if (st) return false;
+    double pmid = 0.;
+    for (;;) {
+        int need = 0;  // 1: a test outside the intervals, 2: between them
+        while (!done) {
+            if (!(fabs(pin - pout) > delta)) { done = true; break; }
+            if (++guard > 400) { s = kEclNoConverge; done = true; break; }
+            pmid = (pin + pout) / 2.;
+            const int d = zone_test(z, dir, pmid);
+            if (d == kEdgeUnsure) {
+                need = zone_between(z, dir, pmid) ? 2 : 1;
+                break;
+            }
+            if (d == kEdgeTrue) pin = pmid;
+            else pout = pmid;
+        }
+        if (!__any_sync(0xffffffffu, need != 0)) break;
+        if (need == 1) {
+            const int d = eval_edge(S, u0, u2, acc, pmid, 0.).ans;
+            if (d == kEdgeTrue) pin = pmid;
+            else if (d == kEdgeFalse) pout = pmid;
+            else need = 2;
+        }
+        if (need == 2) {
+            int d = fblink_edge(S, u0, u2, acc, pmid);
+            if (d == kEdgeUnsure)
+                d = fblink(p.comp_star, p.q, p.comp_spin, acc, set_earth(p.cosi, p.sini, pmid),
+                           pos, p.comp_rref, p.comp_pref, s)
+                        ? kEdgeTrue
+                        : kEdgeFalse;
+            if (d == kEdgeTrue) pin = pmid;
+            else pout = pmid;
+            if (s) done = true;
+        }
     }
-    ingress = (pin + pout) / 2.;
-    ingress = ingress - floor(ingress);
-    pin = phi;
-    pout = phi2;
-    guard = 0;
-    while (fabs(pin - pout) > delta) {
-        if (++guard > 400) { st = kEclNoConverge; return false; }
-        pmid = (pin + pout) / 2.;
-        if (fblink(star, q, spin, ACC, set_earth(cosi, sini, pmid), r, rref, pref, st))
-            pin = pmid;
-        else
-            pout = pmid;
-        if (st) return false;
-    }
-    egress = (pin + pout) / 2.;
-    egress = egress - floor(egress);
-    if (egress < ingress) egress++;
-    return true;
+    return (pin + pout) / 2.;
 }
 
 }  // namespace

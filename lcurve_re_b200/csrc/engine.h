@@ -385,6 +385,7 @@ struct CompParams {
     int32_t nspot;
     int32_t opaque, eclipse1, eclipse2, roche1, roche2;  // star_eclipse
     double q, spin1, spin2, cosi, sini, delta, r1, r2, rref1, pref1, rref2, pref2;
+    EclParams ecl[2];  // eclipses of the elements by star 1 and by star 2
     DiscGeom dg;
 };
 // Elements into el (and (x, y, z, area) into pos); errors into *st.

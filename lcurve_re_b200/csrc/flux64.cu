@@ -86,14 +86,6 @@ __device__ __forceinline__ double elem_mu(double mu, double ex, double ey, doubl
     return (double)(mu > L.mucrit) * val;
 }
 
-template <int LT, bool BEAM, bool GLENS, int STAR>
-__device__ __forceinline__ double elem(double ex, double ey, double ez, double dx, double dy,
-                                       double dz, double px, double py, double pz, double flux,
-                                       const Consts64 &L) {
-    return elem_mu<LT, BEAM, GLENS, STAR>(mu_of(ex, ey, ez, dx, dy, dz), ex, ey, ez, dx, dy, px,
-                                          py, pz, flux, L);
-}
-
 template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
 __global__ void __launch_bounds__(kThreads64)
     k_flux64(FluxConsts k, FlatDev f, PhaseDev ph, double *part, int64_t ldp, DevStatus *st) {
@@ -225,12 +217,16 @@ __global__ void __launch_bounds__(kThreads64)
     const int64_t n = f.n, n1 = f.n1[0];
     const int64_t lo = b * blk, hi = (lo + blk < n) ? lo + blk : n;
     const int64_t c0 = lo > n1 ? lo : n1;
-    const int64_t e = blockIdx.x * (int64_t)kThreads64 + threadIdx.x;
-    if (c0 >= hi || e >= ph.nent) return;
+    if (c0 >= hi) return;
+    // threads past the last entry repeat it without storing: warps stay whole
+    // for the votes
+    const int64_t e1 = blockIdx.x * (int64_t)kThreads64 + threadIdx.x;
+    const int64_t e = e1 < ph.nent ? e1 : ph.nent - 1;
     const Consts64 L{k.c[0], k.c[1], k.c[2], k.c[3], k.base, k.mucrit,
                      k.beam, k.spin, k.vfac, k.xcofm, k.rlens1};
     const double ex = ph.ex[e], ey = ph.ey[e], ez = ph.ez[e], pn = ph.phin[e];
     double acc = part[b * ldp + e];
+    const double zb = zero_below<BEAM>(L);
     for (int64_t i = c0; i < hi; i++) {
         const int64_t r = i - n1;
         const int32_t fi = f.ridx[r];
@@ -240,11 +236,15 @@ __global__ void __launch_bounds__(kThreads64)
             const double2 R = f.rr[kRagRanges * r + q];
             if ((pn >= R.x && pn <= R.y) || pn <= R.y - 1.0) { ecl = true; break; }
         }
+        // at or below zero_below, or eclipsed, at every entry of the warp: exact zeros
+        const double dx = g.nx[fi], dy = g.ny[fi], dz = g.nz[fi];
+        const double mu = mu_of(ex, ey, ez, dx, dy, dz);
+        if (!__any_sync(0xffffffffu, !ecl && mu > zb)) continue;
         if (!ecl)
-            acc += elem<LT, BEAM, GLENS, STAR>(ex, ey, ez, g.nx[fi], g.ny[fi], g.nz[fi], g.px[fi],
-                                               g.py[fi], g.pz[fi], (double)g.flux[fi], L);
+            acc += elem_mu<LT, BEAM, GLENS, STAR>(mu, ex, ey, ez, dx, dy, g.px[fi], g.py[fi],
+                                                  g.pz[fi], (double)g.flux[fi], L);
     }
-    part[b * ldp + e] = acc;
+    if (e1 < ph.nent) part[b * ldp + e] = acc;
 }
 
 template <int LT, bool BEAM, bool GLENS, int STAR>

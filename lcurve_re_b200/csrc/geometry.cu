@@ -208,70 +208,6 @@ __device__ __forceinline__ void push_hits(bool hit, int k, int32_t *hits, int32_
     if (hit) hits[at + __popc(m & ((1u << lane) - 1u))] = k;
 }
 
-// The bisection of ingress (side 0) or egress (side 1) of ingress_egress
-// (ingress_egress.cpp:61-86) from the pot_min state, for every lane of a warp
-// at once (all 32 lanes call it; lanes with live false only vote). The root of
-// the boundary comes first (edge_zone); then each lane takes the bisection's
-// midpoints, comparing those that the certified intervals decide, until one
-// needs a test. The tests run in passes for all lanes that wait for one:
-// eval_edge outside the intervals, fblink_edge between them, and Roche::fblink
-// itself where that is unsure, so the lanes take fblink's decisions at the
-// same midpoints as the plain loop. FP64 latency and issue bound it: some 4
-// evaluations for the root, 2.3 outside the intervals and 3.3 searches of 5
-// evaluations per boundary by an M dwarf, against 20 tests in FP32 with 6.4
-// fblinks of 8 to 12 evaluations before (a white dwarf's: 6 evaluations
-// against 20 fblinks). 256 models of 60-400 strips: 13.8 -> 5.4 ms; one curve
-// on 81/163 strips: 203 us with its warp mode -> 62. With the FP32 screen kept
-// for the tests outside the intervals it took 5.8 ms.
-__device__ __forceinline__ double ecl_bisect_warp(const EclParams &p, bool live, double pin,
-                                                  double pout, double acc, V3 pos, int &s) {
-    // what the passes read, in registers (p may be global memory)
-    const EdgeStar S = p.edge;
-    const double delta = p.delta;
-    const V3 u0 = v3(pos.x - (p.comp_star == kStar1 ? 0. : 1.), pos.y, pos.z);
-    const double u2 = norm2(u0), dir = pout > pin ? 1. : -1.;
-    EdgeZone z;
-    z.hrad = z.vrad = z.hid = z.vis = z.hc = z.vc = 0.;
-    if (live) z = edge_zone(S, u0, acc, delta, pin, pout);
-    bool done = !live;
-    int guard = 0;
-    double pmid = 0.;
-    for (;;) {
-        int need = 0;  // 1: a test outside the intervals, 2: between them
-        while (!done) {
-            if (!(fabs(pin - pout) > delta)) { done = true; break; }
-            if (++guard > 400) { s = kEclNoConverge; done = true; break; }
-            pmid = (pin + pout) / 2.;
-            const int d = zone_test(z, dir, pmid);
-            if (d == kEdgeUnsure) {
-                need = zone_between(z, dir, pmid) ? 2 : 1;
-                break;
-            }
-            if (d == kEdgeTrue) pin = pmid;
-            else pout = pmid;
-        }
-        if (!__any_sync(0xffffffffu, need != 0)) break;
-        if (need == 1) {
-            const int d = eval_edge(S, u0, u2, acc, pmid, 0.).ans;
-            if (d == kEdgeTrue) pin = pmid;
-            else if (d == kEdgeFalse) pout = pmid;
-            else need = 2;
-        }
-        if (need == 2) {
-            int d = fblink_edge(S, u0, u2, acc, pmid);
-            if (d == kEdgeUnsure)
-                d = fblink(p.comp_star, p.q, p.comp_spin, acc, set_earth(p.cosi, p.sini, pmid),
-                           pos, p.comp_rref, p.comp_pref, s)
-                        ? kEdgeTrue
-                        : kEdgeFalse;
-            if (d == kEdgeTrue) pin = pmid;
-            else pout = pmid;
-            if (s) done = true;
-        }
-    }
-    return (pin + pout) / 2.;
-}
-
 // Thread mode (more candidates than warp_max), in two passes with a small code
 // footprint each, as for the batch (k_ecl_potmin_b / k_ecl_bisect_b): the
 // sphere test and pot_min per candidate, then ingress and egress on the two
@@ -329,7 +265,7 @@ __global__ void __launch_bounds__(128, NB)
         if (lane == 0) base = atomicAdd(&counters[3], 32);
         base = __shfl_sync(full, base, 0);
         if (base >= n2) break;
-        // every lane stays here (ecl_bisect_warp votes over the warp); both
+        // every lane stays here (bisect_warp votes over the warp); both
         // lanes of a pair agree on live
         const int64_t u = base + lane;
         const int side = (int)(u & 1);
@@ -339,7 +275,7 @@ __global__ void __launch_bounds__(128, NB)
         const double4 E = live ? es[k] : make_double4(0., 0., 0., 0.);
         const V3 pos = live ? v3(g.px[i], g.py[i], g.pz[i]) : v3(0., 0., 0.);
         int s = 0;
-        double v = ecl_bisect_warp(p, live, E.x, side ? E.z : E.y, E.w, pos, s);
+        double v = bisect_warp(p, live, E.x, side ? E.z : E.y, E.w, pos, s);
         v = v - floor(v);
         const double other = __shfl_xor_sync(full, v, 1);
         const int os = __shfl_xor_sync(full, s, 1);
@@ -1291,7 +1227,7 @@ __global__ void __launch_bounds__(128, NB)
         const double4 E = live ? b.es[k] : make_double4(0., 0., 0., 0.);
         const V3 pos = live ? v3(b.g.px[i], b.g.py[i], b.g.pz[i]) : v3(0., 0., 0.);
         int s = 0;
-        double v = ecl_bisect_warp(b.slots[sl].ep, live, E.x, side ? E.z : E.y, E.w, pos, s);
+        double v = bisect_warp(b.slots[sl].ep, live, E.x, side ? E.z : E.y, E.w, pos, s);
         v = v - floor(v);
         const double other = __shfl_xor_sync(full, v, 1);
         const int os = __shfl_xor_sync(full, s, 1);
