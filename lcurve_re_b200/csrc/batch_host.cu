@@ -161,10 +161,10 @@ struct BatchState {
     size_t tab_bytes = 0;
     DBuf<unsigned char> d_tab;
     size_t o_slots = 0, o_models = 0, o_face0 = 0, o_chunk = 0, o_counts = 0, o_geo_slot = 0,
-           o_geo_half = 0, o_geo_face = 0, o_cont_slot = 0, o_cont_face = 0, o_cont_blk = 0;
+           o_geo_half = 0, o_geo_face = 0, o_geo_blk = 0, o_cont_slot = 0, o_cont_blk = 0;
     // device arrays
     DBuf<double> px, py, pz, nx, ny, nz, ein, eout;
-    DBuf<float> area, grav, flux, fp;
+    DBuf<float> area, grav, fp;
     DBuf<uint8_t> necl;
     DBuf<ulonglong2> ecl;
     DBuf<int64_t> n0;
@@ -201,7 +201,7 @@ struct BatchState {
         DBuf<double> *d[] = {&px, &py, &pz, &nx, &ny, &nz, &ein, &eout,
                              &w1, &w2, &part, &osum, &calc, &sfac, &out};
         for (auto *b : d) b->release();
-        area.release(); grav.release(); flux.release(); fp.release(); necl.release();
+        area.release(); grav.release(); fp.release(); necl.release();
         ecl.release(); n0.release(); blockcnt.release(); queue.release(); counters.release();
         st.release(); ef.release(); pfx.release(); runs.release(); rings.release(); es.release(); hits.release(); d_tab.release();
         rows.release(); gathered.release(); tune_pre.release();
@@ -223,7 +223,7 @@ struct BatchState {
         b.rings = rings.p;
         b.nslots = nslots;
         b.nmodels = nmodels;
-        b.g = GridDev{px.p, py.p, pz.p, nx.p, ny.p, nz.p, area.p, grav.p, flux.p,
+        b.g = GridDev{px.p, py.p, pz.p, nx.p, ny.p, nz.p, area.p, grav.p, nullptr,
                       necl.p, ein.p, eout.p, nfaces};
         b.fp = fp.p;
         b.runs = runs.p;
@@ -240,8 +240,8 @@ struct BatchState {
         b.geo_slot = reinterpret_cast<const int32_t *>(d + o_geo_slot);
         b.geo_half = reinterpret_cast<const int64_t *>(d + o_geo_half);
         b.geo_face = reinterpret_cast<const int64_t *>(d + o_geo_face);
+        b.geo_blk = reinterpret_cast<const int64_t *>(d + o_geo_blk);
         b.cont_slot = reinterpret_cast<const int32_t *>(d + o_cont_slot);
-        b.cont_face = reinterpret_cast<const int64_t *>(d + o_cont_face);
         b.cont_blk = reinterpret_cast<const int64_t *>(d + o_cont_blk);
         return b;
     }
@@ -350,8 +350,8 @@ lcg_status relayout(lcg_ctx *c, BatchState &B, const lcg_model *models, int32_t 
     B.o_geo_slot = sect(ns * 4);
     B.o_geo_half = sect((ns + 1) * 8);
     B.o_geo_face = sect((ns + 1) * 8);
+    B.o_geo_blk = sect((ns + 1) * 8);
     B.o_cont_slot = sect(ns * 4);
-    B.o_cont_face = sect((ns + 1) * 8);
     B.o_cont_blk = sect((ns + 1) * 8);
     B.tab_bytes = o;
     if (B.h_tab) cudaFreeHost(B.h_tab);
@@ -381,7 +381,7 @@ lcg_status relayout(lcg_ctx *c, BatchState &B, const lcg_model *models, int32_t 
     DBuf<double> *d[] = {&B.px, &B.py, &B.pz, &B.nx, &B.ny, &B.nz, &B.ein, &B.eout};
     for (auto *b : d)
         if ((e = b->ensure(nf))) return c->cuda_fail(e, "batch grids");
-    if ((e = B.area.ensure(nf)) || (e = B.grav.ensure(nf)) || (e = B.flux.ensure(nf)) ||
+    if ((e = B.area.ensure(nf)) || (e = B.grav.ensure(nf)) ||
         (e = B.necl.ensure(nf)) || (e = B.queue.ensure(nf)) ||
         (e = B.fp.ensure(8 * (size_t)B.nflat)) || (e = B.ecl.ensure((size_t)B.nflat)) ||
         (e = B.runs.ensure(kRunRecs * (size_t)B.nflat / kRunFaces)) ||
@@ -567,8 +567,8 @@ void enqueue(lcg_ctx *c, BatchState &B, bool timed, int part = 0) {
         cudaMemsetAsync(B.st.p, 0, (size_t)B.nmodels * sizeof(DevStatus), s);
         stage(LCG_STAGE_GRID, [&] { launch_batch_grid(b, c->nsm, s); });
         stage(LCG_STAGE_ECLIPSE, [&] { launch_batch_eclipse(b, c->nsm, c->eclipse_warp, s); });
+        stage(LCG_STAGE_FLATTEN, [&] { launch_batch_partition(b, c->nsm, s); });
         stage(LCG_STAGE_CONTINUUM, [&] { launch_batch_continuum(b, c->nsm, s); });
-        stage(LCG_STAGE_FLATTEN, [&] { launch_batch_flatten(b, c->nsm, s); });
         stage(LCG_STAGE_PHASES, [&] { launch_batch_phases(b, c->data.p, c->off.p, B.n, ph, s); });
     }
     if (part == 1) return;
@@ -693,6 +693,7 @@ extern "C" lcg_status lcg_light_curve_batch_resident(lcg_ctx *c, const lcg_model
                     gp.acc = M.delta_phase / 10.;
                     gp.gref = su.gref;
                     gp.rad_sphere = star == kStar1 ? su.r1 : su.r2;
+                    gp.own = make_edge_star(star, gp.q, gp.spin, 0., 0., gp.rref, gp.pref);
                     EclParams &ep = X.ep;
                     ep.comp_star = star == kStar1 ? kStar2 : kStar1;
                     ep.comp_roche = star == kStar1 ? M.roche2 : M.roche1;
@@ -737,24 +738,26 @@ extern "C" lcg_status lcg_light_curve_batch_resident(lcg_ctx *c, const lcg_model
         int32_t *counts = B.tab<int32_t>(B.o_counts);
         int32_t *gs = B.tab<int32_t>(B.o_geo_slot), *cs = B.tab<int32_t>(B.o_cont_slot);
         int64_t *gh = B.tab<int64_t>(B.o_geo_half), *gf = B.tab<int64_t>(B.o_geo_face);
-        int64_t *cf = B.tab<int64_t>(B.o_cont_face), *cb = B.tab<int64_t>(B.o_cont_blk);
+        int64_t *gb = B.tab<int64_t>(B.o_geo_blk), *cb = B.tab<int64_t>(B.o_cont_blk);
         int32_t ng = 0, nc = 0;
-        gh[0] = gf[0] = cf[0] = cb[0] = 0;
+        gh[0] = gf[0] = gb[0] = cb[0] = 0;
         for (int32_t m = 0; m < nmodels; m++) {
             if (!md[m].live) continue;
             for (int star = 0; star < 2; star++) {
                 const int s = 2 * m + star;
                 const RingSet &R = B.slot_rings[s];
+                const int64_t nblk = (R.nface + kSlotAlign - 1) / kSlotAlign;
+                slots[s].fresh = geo[m];
                 if (geo[m]) {
                     gs[ng] = s;
+                    gb[ng + 1] = gb[ng] + nblk;
                     gh[ng + 1] = gh[ng] + R.nhalf;
                     gf[ng + 1] = gf[ng] + R.nface;
                     ng++;
                 }
                 if (cont[m]) {
                     cs[nc] = s;
-                    cf[nc + 1] = cf[nc] + R.nface;
-                    cb[nc + 1] = cb[nc] + (R.nface + kSlotAlign - 1) / kSlotAlign;
+                    cb[nc + 1] = cb[nc] + nblk;
                     nc++;
                 }
             }

@@ -372,4 +372,81 @@ LCG_HD bool zone_between(const EdgeZone &z, double dir, double phase) {
            dir * (phase - z.vc) < z.vis;
 }
 
+// ---- the surface radius along a ray ------------------------------------------------
+
+// face_chop (roche.cuh) halves and bisects the radius at which the potential
+// along a ray reaches pref: about 27 evaluations of a square root and two
+// divisions. Along the ray the potential is, about the star's centre,
+//   f(r) = -me / r - mo / d - ss/2 (dx^2 + dy^2) r^2 + k dx r - pref,
+//   d^2 = r^2 + 1 - 2 S.dx dx r,
+// and concave while 2 me / r^3 > mo / (1 - r)^3 (checked at rref, where the left
+// side is least). With f'(rref) > 0 it then increases on (0, rref], so its root
+// decides every comparison of face_chop: Newton's method from rref lands left
+// of the root once and climbs (a concave function lies under its tangents), and
+// a value e <= 0 at r encloses it in [r - e / f'(r), r - e / f'(rref)], f' being
+// between the two from there on. The radius is face_chop's, bit for bit: the
+// same midpoints, those inside the enclosure (1e-13 wide, far below acc) by
+// chop_pot itself. 4-5 evaluations replace 27; where a condition fails (the
+// ray through L1 of a lobe-filling star), face_chop runs as it is.
+LCG_HD int face_chop_root(const EdgeStar &S, int star, double q, double spin, double dx, double dy,
+                          double rref, double pref, double acc, double &rad) {
+    const double dxy2 = dx * dx + dy * dy, sd = S.dx * dx, kd = S.k * dx;
+    double tol = 0.;
+    auto eval = [&](double r, double &f, double &d1) {
+        const double ir = 1. / r, io = edge_rsqrt(fma(r, r - 2. * sd, 1.));
+        const double pe = S.me * ir, po = S.mo * io;
+        f = fma(kd, r, fma(-0.5 * S.ss * dxy2, r * r, -(pe + po))) - S.pref;
+        d1 = fma(pe, ir, fma(po * io * io, r - sd, fma(-S.ss * dxy2, r, kd)));
+        tol = 1e-14 * (pe + po + 2.);
+    };
+    const double gap = 1. - rref;
+    double f, d1;
+    eval(rref, f, d1);
+    const double dmin = d1;
+    bool ok = gap > 0.1 && 2. * S.me * gap * gap * gap > S.mo * rref * rref * rref && dmin > 0. &&
+              f > 4. * tol;
+    double lo = 0., hi = 0.;
+    if (ok) {
+        double r = rref;
+        ok = false;
+#pragma unroll 1
+        for (int it = 0; it < 12; it++) {
+            r -= f / d1;
+            if (!(r > 0.)) break;
+            eval(r, f, d1);
+            if (!(d1 > 0.)) break;
+            if (f <= tol && (tol - f) < 1e-2 * acc * dmin) {
+                // f is at most 0 up to rounding: both ends with 2 tol to spare
+                const double e = f < 0. ? -f : 0.;
+                lo = r + (e - 2. * tol) / d1 - 2. * tol / dmin;
+                hi = r + (e + 4. * tol) / dmin;
+                ok = true;
+                break;
+            }
+        }
+    }
+    if (!ok) return face_chop(star, q, spin, dx, dy, rref, pref, acc, rad);
+    // face_chop's walk; pot(r) < pref left of lo, > pref right of hi
+    double r1 = rref / 2, r2 = rref;
+    bool above = true;
+    for (int it = 0; it < 30 && above; it++) {
+        r1 = r2 / 2;
+        above = r1 < lo ? false : r1 > hi ? true : chop_pot(star, q, spin, dx, dy, r1) > pref;
+        if (above) r2 = r1;
+    }
+    int fail = above ? 2 : 0;
+    if (!fail) {
+        for (int nchop = 0; nchop < 100 && r2 - r1 > acc; nchop++) {
+            const double r = (r1 + r2) / 2.;
+            const bool below =
+                r < lo ? true : r > hi ? false : chop_pot(star, q, spin, dx, dy, r) < pref;
+            if (below) r1 = r;
+            else r2 = r;
+        }
+        if (r2 - r1 > acc) fail = 3;
+    }
+    rad = (r1 + r2) / 2.;
+    return fail;
+}
+
 }  // namespace lcg

@@ -436,6 +436,7 @@ lcg_status build_geometry(lcg_ctx *c, const lcg_model &m, int star, int fine, Gr
     gp.acc = m.delta_phase / 10.;
     gp.gref = s.gref;
     gp.rad_sphere = star == kStar1 ? s.r1 : s.r2;
+    gp.own = make_edge_star(star, gp.q, gp.spin, 0., 0., gp.rref, gp.pref);
     {
         StageScope t(c, LCG_STAGE_GRID);
         launch_grid(gp, g.rings.p, g.dev(), c->status.p, st);

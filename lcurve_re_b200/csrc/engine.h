@@ -45,6 +45,7 @@ struct GridParams {
     int32_t star, roche, npole, nrings;
     int64_t nhalf;  // total half-faces (sum over rings of (nphi+1)/2)
     double q, spin, rref, pref, acc, gref, rad_sphere;
+    EdgeStar own;  // the star itself, for the surface radii (face_chop_root)
 };
 
 // Eclipse of one star's faces by its companion (set_star_grid.cpp:372-386).
@@ -202,6 +203,7 @@ struct SlotDev {
     int64_t blk0;   // first 1024-face partition block
     int32_t ring0;  // first ring of the slot's table in the ring pool
     int32_t model, eclipse_on, live;
+    int32_t fresh;  // its geometry is rebuilt in this call
 };
 
 struct ModelDev {
@@ -240,9 +242,9 @@ struct BatchDev {
     // list has its slots and prefix sums (count + 1 entries) of its units
     const int32_t *counts;
     const int32_t *geo_slot;
-    const int64_t *geo_half, *geo_face;
+    const int64_t *geo_half, *geo_face, *geo_blk;
     const int32_t *cont_slot;
-    const int64_t *cont_face, *cont_blk;
+    const int64_t *cont_blk;
 };
 
 // k such that pre[k] <= u < pre[k + 1], over count entries.
@@ -308,14 +310,15 @@ void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, R
 void launch_batch_run_bounds(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_pack_phases(PhaseDev ph, cudaStream_t s);
 
-// batched stages (geometry.cu): grid + eclipse of the geometry list;
-// continuum + partition of the continuum list; phases; reduction, scatter and
+// batched stages (geometry.cu): grid, eclipse and partition offsets of the
+// geometry list; continuum and sweep records of the continuum list; phases;
+// reduction, scatter and
 // scale / chi**2 of every model. Grids are fixed by the layout (persistent
 // loops over device-side counts), so a captured graph replays any work lists.
 void launch_batch_grid(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_batch_eclipse(const BatchDev &b, int nsm, int32_t warp_mode, cudaStream_t s);
+void launch_batch_partition(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_batch_continuum(const BatchDev &b, int nsm, cudaStream_t s);
-void launch_batch_flatten(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_batch_phases(const BatchDev &b, const DatumRec *data, const int64_t *off, int32_t n,
                          const BatchPhases &ph, cudaStream_t s);
 void launch_batch_reduce(const BatchDev &b, const BatchPhases &ph, const double *part,

@@ -64,3 +64,25 @@ def test_roots_keep_every_decision(checker, oracle, most, over):
         zone += r["zone"]
     assert tests > 1000
     assert zone >= most * tests, (zone, tests)
+
+
+@pytest.mark.parametrize("q,spin,radius", [
+    (0.25, 1.0, 0.015), (0.25, 1.0, 0.2), (0.05, 1.0, 0.2), (0.15, 1.0, -1.0), (0.8, 1.0, -1.0),
+    (3.0, 1.0, 0.35), (0.25, 0.0, 0.25), (0.25, 3.0, 0.1), (0.01, 1.0, 0.002), (0.9, 1.5, 0.3)])
+@pytest.mark.parametrize("acc", [1e-8, 1e-5, 1e-12])
+def test_radii_are_the_plain_walks(q, spin, radius, acc):
+    """face_chop_root against face_chop, bit for bit, both stars."""
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not available")
+    exe = os.path.join(HERE, "screen", "_build", "chop_check")
+    src = os.path.join(HERE, "screen", "chop_check.cpp")
+    hdr = os.path.join(HERE, "..", "lcurve_re_b200", "csrc", "ecl_root.cuh")
+    os.makedirs(os.path.dirname(exe), exist_ok=True)
+    if not os.path.exists(exe) or os.path.getmtime(exe) < max(os.path.getmtime(src),
+                                                              os.path.getmtime(hdr)):
+        subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe, src])
+    for star in (0, 1):
+        out = subprocess.run([exe] + [repr(v) for v in (q, spin, radius, star, acc, 1500)],
+                             capture_output=True, timeout=300)
+        n, bad = (int(v) for v in out.stdout.split())
+        assert n > 30000 and bad == 0 and out.returncode == 0, (star, bad)
