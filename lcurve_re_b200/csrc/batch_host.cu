@@ -882,8 +882,8 @@ extern "C" lcg_status lcg_light_curve_batch_resident(lcg_ctx *c, const lcg_model
     for (int k = 0; k < nw; k++)
         if (c->worker_data_version[k] != c->data_version) {
             lcg_status rc = lcg_set_data(c->workers[k],
-                                         reinterpret_cast<const lcg_datum *>(c->h_data.data()),
-                                         (int32_t)c->h_data.size());
+                                         reinterpret_cast<const lcg_datum *>(c->h_data()),
+                                         c->h_data_n);
             if (rc) return c->fail(rc, "resident points of a batch worker");
             c->worker_data_version[k] = c->data_version;
         }

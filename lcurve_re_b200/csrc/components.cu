@@ -199,17 +199,28 @@ __global__ void __launch_bounds__(kThreadsC)
     pos[i] = make_double4(posn.x, posn.y, posn.z, (double)(float)area);
 }
 
-__global__ void k_disc_faces(DiscGeom dg, GridDev g, uint8_t *ndx, double2 *xr, DevStatus *st) {
+// The disc's ranges of each face, and the partition counts with them: one-range
+// and several-range faces per CTA of 256 (k_flat_scatter).
+__global__ void __launch_bounds__(256) k_disc_faces(DiscGeom dg, GridDev g, uint8_t *ndx,
+                                                    double2 *xr, int32_t *cnt, DevStatus *st) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= g.n) return;
-    int nr = 0, s = 0;
-    double rin[kDiscRanges], rout[kDiscRanges];
-    disc_eclipse(dg, v3(g.px[i], g.py[i], g.pz[i]), nr, rin, rout, kDiscRanges, s);
-    if (s) report(st, s, (int)i);
-    nr = s ? 0 : (nr < kDiscRanges ? nr : kDiscRanges);
-    ndx[i] = (uint8_t)nr;
-    for (int k = 0; k < kDiscRanges; k++)
-        xr[kDiscRanges * i + k] = k < nr ? make_double2(rin[k], rout[k]) : make_double2(0., 0.);
+    int ranges = 0;
+    if (i < g.n) {
+        int nr = 0, s = 0;
+        double rin[kDiscRanges], rout[kDiscRanges];
+        disc_eclipse(dg, v3(g.px[i], g.py[i], g.pz[i]), nr, rin, rout, kDiscRanges, s);
+        if (s) report(st, s, (int)i);
+        nr = s ? 0 : (nr < kDiscRanges ? nr : kDiscRanges);
+        ndx[i] = (uint8_t)nr;
+        for (int k = 0; k < kDiscRanges; k++)
+            xr[kDiscRanges * i + k] = k < nr ? make_double2(rin[k], rout[k]) : make_double2(0., 0.);
+        ranges = g.necl[i] + nr;
+    }
+    const int c1 = __syncthreads_count(ranges == 1), c2 = __syncthreads_count(ranges > 1);
+    if (threadIdx.x == 0) {
+        cnt[blockIdx.x] = c1;
+        cnt[gridDim.x + blockIdx.x] = c2;
+    }
 }
 
 // One CTA per (tile of phase entries, chunk of kElemChunk elements): each
@@ -441,9 +452,9 @@ void launch_components(const CompParams &p, ElemRec *el, double4 *pos, DevStatus
 }
 
 void launch_disc_faces(const DiscGeom &dg, const GridDev &g, uint8_t *ndx, double2 *xr,
-                       DevStatus *st, cudaStream_t s) {
+                       int32_t *cnt, DevStatus *st, cudaStream_t s) {
     if (g.n <= 0) return;
-    k_disc_faces<<<nblk(g.n, 256), 256, 0, s>>>(dg, g, ndx, xr, st);
+    k_disc_faces<<<nblk(g.n, 256), 256, 0, s>>>(dg, g, ndx, xr, cnt, st);
     count_launch();
 }
 

@@ -37,6 +37,29 @@ struct DBuf {
     }
 };
 
+// Pinned host memory that grows; its contents do not survive growth.
+struct HBuf {
+    unsigned char *p = nullptr;
+    size_t cap = 0;
+    cudaError_t ensure(size_t bytes) {
+        if (bytes <= cap) return cudaSuccess;
+        release();
+        bytes += bytes / 2;  // a fit's light curves come in a few sizes
+        cudaError_t e = cudaHostAlloc((void **)&p, bytes, cudaHostAllocDefault);
+        if (e != cudaSuccess) {
+            p = nullptr;
+            return e;
+        }
+        cap = bytes;
+        return cudaSuccess;
+    }
+    void release() {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        cap = 0;
+    }
+};
+
 struct StarSetup {
     double r1, r2, rl1, rl2, ffac1, ffac2, rref1, pref1, rref2, pref2, gref;
     int infill, nlat, nlatfill, nlngfill, eclipse;
@@ -60,6 +83,9 @@ struct Grid {
     DBuf<int32_t> queue, counters;  // eclipse candidates of this grid
     DBuf<double4> es;               // and their state between the two passes
     DBuf<int32_t> hits;
+    DBuf<int32_t> cnt;   // partition counts (k_continuum, k_disc_faces)
+    DBuf<double> dsum;   // diagnostic sums (k_continuum)
+    int32_t ring_nlat = 0;  // the strips whose ring table is on the device (no infill)
     // flat
     DBuf<int64_t> n0;
     DBuf<float4> geo, pos;
@@ -84,7 +110,8 @@ struct Grid {
         for (auto *b : d)
             if ((e = b->ensure(nf)) != cudaSuccess) return e;
         if ((e = area.ensure(nf)) || (e = grav.ensure(nf)) || (e = flux.ensure(nf)) ||
-            (e = necl.ensure(nf)))
+            (e = necl.ensure(nf)) || (e = cnt.ensure(2 * cont_blocks(nf))) ||
+            (e = dsum.ensure(4 * cont_blocks(nf))))
             return e;
         return cudaSuccess;
     }
@@ -127,6 +154,7 @@ struct Grid {
         for (auto *b : d) b->release();
         area.release(); grav.release(); flux.release(); necl.release(); rings.release();
         queue.release(); counters.release(); es.release(); hits.release();
+        cnt.release(); dsum.release();
         n0.release(); geo.release(); pos.release(); ecl.release(); fp.release();
         runs.release(); ndx.release(); rn.release(); xr.release(); rr.release(); ridx.release();
         disc = false;
@@ -170,15 +198,22 @@ struct lcg_ctx {
     // copy of the resident points (h_data, from lcg_set_data)
     std::vector<lcg_ctx *> workers;
     std::vector<int64_t> worker_data_version;
-    std::vector<DatumRec> h_data;
+    // the points and their entry offsets as last given, pinned: what the copies to
+    // the device read, and what the workers copy
+    lcg::eng::HBuf h_in;
+    int32_t h_data_n = 0;
+    const DatumRec *h_data() const { return reinterpret_cast<const DatumRec *>(h_in.p); }
+    // a call's results: a TailOut, then the curve; read back with one copy into
+    // pinned memory
+    DBuf<double> res;
+    lcg::eng::HBuf h_res;
+    lcg::TailOut *tail() const { return reinterpret_cast<lcg::TailOut *>(res.p); }
+    double *calc() const { return res.p + sizeof(lcg::TailOut) / sizeof(double); }
     // work buffers
     DBuf<DevStatus> status;
-    DBuf<int32_t> queue, counters, blockcnt;
-    DBuf<int32_t> blockcnt2;  // star 2's partition scratch when it flattens on side[0]
     DBuf<DatumRec> data;
     DBuf<int64_t> off;
-    DBuf<double> pex, pey, pez, pphin, pw1, pw2, part1f, part1c, part2f, part2c, calc, scratch,
-        sfac, out, diag, osum;
+    DBuf<double> pex, pey, pez, pphin, pw1, pw2, part1f, part1c, part2f, part2c, osum;
     DBuf<float4> pef;
     DBuf<unsigned long long> ppfx;
     DBuf<uint8_t> ptype;
@@ -197,8 +232,6 @@ struct lcg_ctx {
     // the SMs that star 2's latency-bound geometry leaves idle.
     cudaStream_t side[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr}, ev_phases = nullptr;
-    std::vector<int64_t> h_off;
-    std::vector<double> h_diag;
     // resident light-curve points (lcg_set_data)
     // light_curve_comp_fast: all points, sample indices, interpolated curve
     DBuf<DatumRec> fdata;
@@ -288,7 +321,7 @@ lcg_status check_model(lcg_ctx *c, const lcg_model *m);
 // reference error.
 bool comp_setup(const lcg_model &m, CompParams &p, std::vector<DiscRing> &rings, Fail &f);
 bool bright_spot_position(double q, double rad, double *pos, Fail &f);
-lcg_status finish_status(lcg_ctx *c);
+lcg_status finish_status(lcg_ctx *c, const DevStatus *got = nullptr);
 
 }  // namespace eng
 }  // namespace lcg

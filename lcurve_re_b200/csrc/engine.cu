@@ -415,14 +415,29 @@ FluxConsts flux_consts(const lcg_model &m, int star, double spin, double rlens1)
 lcg_status build_geometry(lcg_ctx *c, const lcg_model &m, int star, int fine, Grid &g,
                           cudaStream_t st) {
     Fail f{0, ""};
-    if (!prepare_star(m, star, fine, g.setup, f)) return c->fail(f.code, "%s", f.msg.c_str());
-    const StarSetup &s = g.setup;
+    // A grid without infill has the ring table of its strip count, the one on the
+    // device if it had as many strips before.
+    StarSetup &s = g.setup;
+    const int32_t nlat = star == kStar1 ? (fine ? m.nlat1f : m.nlat1c) : (fine ? m.nlat2f : m.nlat2c);
+    const bool plain = star == kStar1 || !fine || !m.npole ||
+                       (m.nlatfill <= 0 && m.nlngfill <= 0);
+    const bool rings_on = plain && g.ring_nlat == nlat && nlat > 0;
+    const int nface = s.nface;
+    if (!prepare_star(m, star, fine, s, f, !rings_on)) {
+        g.ring_nlat = 0;
+        return c->fail(f.code, "%s", f.msg.c_str());
+    }
+    if (rings_on) s.nface = nface;
     cudaError_t e;
     if ((e = g.alloc_points(s.nface)) != cudaSuccess) return c->cuda_fail(e, "grid allocation");
     g.ntiled = s.ntiled;
-    if ((e = g.rings.ensure(s.rings.size())) != cudaSuccess) return c->cuda_fail(e, "rings");
-    cudaMemcpyAsync(g.rings.p, s.rings.data(), s.rings.size() * sizeof(RingRec),
-                    cudaMemcpyHostToDevice, st);
+    if (!rings_on) {
+        g.ring_nlat = 0;
+        if ((e = g.rings.ensure(s.rings.size())) != cudaSuccess) return c->cuda_fail(e, "rings");
+        cudaMemcpyAsync(g.rings.p, s.rings.data(), s.rings.size() * sizeof(RingRec),
+                        cudaMemcpyHostToDevice, st);
+        if (plain) g.ring_nlat = nlat;
+    }
     GridParams gp{};
     gp.star = star;
     gp.roche = star == kStar1 ? m.roche1 : m.roche2;
@@ -437,13 +452,13 @@ lcg_status build_geometry(lcg_ctx *c, const lcg_model &m, int star, int fine, Gr
     gp.gref = s.gref;
     gp.rad_sphere = star == kStar1 ? s.r1 : s.r2;
     gp.own = make_edge_star(star, gp.q, gp.spin, 0., 0., gp.rref, gp.pref);
-    {
-        StageScope t(c, LCG_STAGE_GRID);
-        launch_grid(gp, g.rings.p, g.dev(), c->status.p, st);
-    }
     if ((e = g.queue.ensure(s.nface)) || (e = g.counters.ensure(8)) ||
         (e = g.es.ensure(s.nface)) || (e = g.hits.ensure(s.nface)))
         return c->cuda_fail(e, "queue");
+    {
+        StageScope t(c, LCG_STAGE_GRID);
+        launch_grid(gp, g.rings.p, g.dev(), g.counters.p, c->status.p, st);
+    }
     EclParams ep{};
     ep.comp_star = star == kStar1 ? kStar2 : kStar1;
     ep.comp_roche = star == kStar1 ? m.roche2 : m.roche1;
@@ -489,19 +504,16 @@ FastCoef fast_coef(const lcg_model &m, int star, int mixed) {
     return f;
 }
 
-// side: run on side[0] with its own partition scratch (star 2, concurrent
-// order); otherwise on the context's stream.
+// side: run on side[0] (star 2, concurrent order); otherwise on the context's
+// stream.
 lcg_status flatten(lcg_ctx *c, Grid &g, int need_pos, const FastCoef &fc, bool side = false) {
     const int mixed = c->precision == LCG_PREC_MIXED;
     cudaError_t e;
     if ((e = g.alloc_flat(mixed, need_pos, fc.on)) != cudaSuccess)
         return c->cuda_fail(e, "flat grid");
     g.fast = fc.on;
-    DBuf<int32_t> &bc = side ? c->blockcnt2 : c->blockcnt;
-    if ((e = bc.ensure(2 * ((g.n + 1023) / 1024) + 1)) != cudaSuccess)
-        return c->cuda_fail(e, "partition");
     StageScope t(c, LCG_STAGE_FLATTEN);
-    launch_flatten(g.dev(), g.flat(), bc.p, mixed, need_pos, fc, c->status.p,
+    launch_flatten(g.dev(), g.flat(), g.cnt.p, mixed, need_pos, fc,
                    side ? c->side[0] : c->stream);
     return LCG_OK;
 }
@@ -595,7 +607,10 @@ lcg_status check_model(lcg_ctx *c, const lcg_model *m) {
     return LCG_OK;
 }
 
-lcg_status finish_status(lcg_ctx *c) {
+// Waits for the context's stream; an error of the launches, of the stream or of the
+// device status word becomes the call's. got: where the status arrives on the
+// host with the call's results; NULL: read it here.
+lcg_status finish_status(lcg_ctx *c, const DevStatus *got) {
     cudaError_t le = cudaGetLastError();
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (le != cudaSuccess) {
@@ -606,8 +621,12 @@ lcg_status finish_status(lcg_ctx *c) {
     c->collect_timers();
     if (e != cudaSuccess) return c->cuda_fail(e, "stream");
     DevStatus st{};
-    e = cudaMemcpy(&st, c->status.p, sizeof st, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return c->cuda_fail(e, "status");
+    if (got) {
+        st = *got;
+    } else {
+        e = cudaMemcpy(&st, c->status.p, sizeof st, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return c->cuda_fail(e, "status");
+    }
     if (st.code) {
         c->has_geom = c->has_cont = false;
         if (st.face < 0)  // a disc, rim or spot element (components.cu)
@@ -713,8 +732,7 @@ lcg_status lcg_create(lcg_ctx **out, const lcg_options *opt) {
         (e = cudaEventCreateWithFlags(&c->ev_join[0], cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&c->ev_join[1], cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&c->ev_phases, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = c->status.ensure(1)) != cudaSuccess || (e = c->counters.ensure(2)) != cudaSuccess ||
-        (e = c->sfac.ensure(8)) != cudaSuccess || (e = c->out.ensure(4)) != cudaSuccess) {
+        (e = c->status.ensure(1)) != cudaSuccess) {
         g_create_error = cudaGetErrorString(e);
         delete c;
         return LCG_E_CUDA;
@@ -740,11 +758,9 @@ void lcg_destroy(lcg_ctx *c) {
     Grid *gs[] = {&c->g1f, &c->g2f, &c->g1c, &c->g2c};
     for (Grid *g : gs) g->release();
     DBuf<double> *d[] = {&c->pex, &c->pey, &c->pez, &c->pphin, &c->pw1, &c->pw2, &c->part1f,
-                         &c->part1c, &c->part2f, &c->part2c, &c->calc, &c->scratch, &c->sfac,
-                         &c->out, &c->diag, &c->osum};
+                         &c->part1c, &c->part2f, &c->part2c, &c->res, &c->osum};
     for (auto *b : d) b->release();
-    c->status.release(); c->queue.release(); c->counters.release(); c->blockcnt.release();
-    c->blockcnt2.release();
+    c->status.release(); c->h_in.release(); c->h_res.release();
     c->data.release(); c->off.release(); c->pef.release(); c->ppfx.release(); c->ptype.release();
     c->fdata.release(); c->fidx.release(); c->fcalc.release(); c->fout.release();
     c->elem.release(); c->epos.release(); c->drings.release(); c->csum.release();
@@ -802,9 +818,18 @@ lcg_status lcg_set_data(lcg_ctx *c, const lcg_datum *data, int32_t n) {
     if (n < 1) return c->fail(LCG_E_INVALID, "light_curve_comp: no data points");
     cudaSetDevice(c->device);
     // per-point offsets of the sub-exposure entries and the time range used
-    // by the polynomial factor (light_curve_comp.cpp:351-356)
-    std::vector<int64_t> &off = c->h_off;
-    off.resize((size_t)n + 1);
+    // by the polynomial factor (light_curve_comp.cpp:351-356). Points and offsets go
+    // to pinned memory first, so that the copies run on while the host goes on;
+    // the last ones out of it are done once the stream is.
+    cudaError_t e;
+    if (c->h_data_n && (e = cudaStreamSynchronize(c->stream))) return c->cuda_fail(e, "stream");
+    c->h_data_n = 0;
+    const size_t dbytes = (size_t)n * sizeof(DatumRec), obytes = ((size_t)n + 1) * sizeof(int64_t);
+    if ((e = c->h_in.ensure(dbytes + obytes)) || (e = c->data.ensure(n)) ||
+        (e = c->off.ensure(n + 1)))
+        return c->cuda_fail(e, "data buffers");
+    memcpy(c->h_in.p, data, dbytes);
+    int64_t *off = reinterpret_cast<int64_t *>(c->h_in.p + dbytes);
     off[0] = 0;
     double xmin = data[0].time, xmax = data[0].time;
     for (int i = 0; i < n; i++) {
@@ -814,15 +839,9 @@ lcg_status lcg_set_data(lcg_ctx *c, const lcg_datum *data, int32_t n) {
             xmax = data[i].time < xmax ? xmax : data[i].time;
         }
     }
-    cudaError_t e;
-    if ((e = c->data.ensure(n)) || (e = c->off.ensure(n + 1)))
-        return c->cuda_fail(e, "data buffers");
-    cudaMemcpyAsync(c->data.p, data, (size_t)n * sizeof(DatumRec), cudaMemcpyHostToDevice,
-                    c->stream);
-    c->h_data.assign(reinterpret_cast<const DatumRec *>(data),
-                     reinterpret_cast<const DatumRec *>(data) + n);
-    cudaMemcpyAsync(c->off.p, off.data(), (size_t)(n + 1) * sizeof(int64_t),
-                    cudaMemcpyHostToDevice, c->stream);
+    cudaMemcpyAsync(c->data.p, c->h_in.p, dbytes, cudaMemcpyHostToDevice, c->stream);
+    cudaMemcpyAsync(c->off.p, off, obytes, cudaMemcpyHostToDevice, c->stream);
+    c->h_data_n = n;
     c->data_n = n;
     c->data_version++;
     c->data_nent = off[n];
@@ -842,7 +861,7 @@ lcg_status lcg_light_curve(lcg_ctx *c, const lcg_model *mp, const lcg_datum *dat
     return lcg_light_curve_resident(c, mp, flags, sfac, calc, scalars);
 }
 
-const double *lcg_device_calc(lcg_ctx *c) { return c ? c->calc.p : nullptr; }
+const double *lcg_device_calc(lcg_ctx *c) { return c && c->res.p ? c->calc() : nullptr; }
 
 lcg_status lcg_light_curve_fast(lcg_ctx *c, const lcg_model *mp, const lcg_datum *data,
                                 int32_t n, int32_t flags, int32_t max_model_points, double *sfac,
@@ -874,7 +893,7 @@ lcg_status lcg_light_curve_fast(lcg_ctx *c, const lcg_model *mp, const lcg_datum
     cudaMemcpyAsync(c->fidx.p, idx.data(), (size_t)m * sizeof(int64_t), cudaMemcpyHostToDevice,
                     c->stream);
     const int32_t rdata = (flags & LCG_FLAG_RDATA) != 0;
-    launch_interp(c->fdata.p, n, c->fidx.p, m, c->calc.p, c->fcalc.p, rdata, c->fout.p,
+    launch_interp(c->fdata.p, n, c->fidx.p, m, c->calc(), c->fcalc.p, rdata, c->fout.p,
                   c->stream);
     double out[2] = {0., 0.};
     cudaMemcpyAsync(calc, c->fcalc.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost,
@@ -928,6 +947,42 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
     const bool iscale = m.iscale != 0;
     cudaMemsetAsync(c->status.p, 0, sizeof(DevStatus), c->stream);
     cudaEventRecord(c->ev_fork, c->stream);  // side-stream work starts here
+
+    // phase entries (light_curve_comp.cpp:358-455) over the resident points, with
+    // diagnostics one more: comp_star1_flat at phase 0.5 (:504-508)
+    const int64_t nent = c->data_nent;
+    const double xmin = c->data_xmin, xmax = c->data_xmax;
+    const bool diag = (flags & LCG_FLAG_DIAGNOSTICS) != 0;
+    const int64_t nall = nent + (diag ? 1 : 0);
+    const int64_t ldp = ((nall + 3) / 4) * 4;
+    if ((e = c->pex.ensure(nall)) || (e = c->pey.ensure(nall)) || (e = c->pez.ensure(nall)) ||
+        (e = c->pphin.ensure(nall)) || (e = c->pw1.ensure(nall)) || (e = c->pw2.ensure(nall)) ||
+        (e = c->pef.ensure(nall)) || (e = c->ppfx.ensure(nall)) || (e = c->ptype.ensure(nall)) ||
+        (e = c->res.ensure(sizeof(TailOut) / sizeof(double) + (size_t)n)) ||
+        (e = c->h_res.ensure(sizeof(TailOut) + (size_t)n * sizeof(double))))
+        return c->cuda_fail(e, "phase and result buffers");
+    PhaseDev ph{c->pex.p, c->pey.p, c->pez.p, c->pphin.p, c->pw1.p, c->pw2.p,
+                c->pef.p, c->ptype.p, nall, c->ppfx.p};
+    const double ri = deg2rad(m.iangle);
+    const double cosi = cos(ri), sini = sin(ri);
+    PhaseParams pp{};
+    pp.t0 = m.t0; pp.period = m.period; pp.pdot = m.pdot; pp.deltat = m.deltat;
+    pp.slope = m.slope; pp.quad = m.quad; pp.cube = m.cube;
+    pp.middle = (xmin + xmax) / 2.;
+    pp.range = (xmax - xmin) / 2.;
+    pp.cosi = cosi; pp.sini = sini;
+    auto phases = [&](const Ginterp &gi) {
+        pp.gi = gi;
+        StageScope t(c, LCG_STAGE_PHASES);
+        launch_phases(pp, c->data.p, c->off.p, n, ph, diag, set_earth(cosi, sini, 0.5), 0.5,
+                      c->stream);
+    };
+    // Only the coarse grids' scales (Ginterp) make the phases wait for the
+    // geometry; with fine grids alone they run while the host sets the stars up.
+    const bool fine_only = m.nlat1f == m.nlat1c && m.nlat2f == m.nlat2c &&
+                           (!m.npole || r1 >= r2 || (m.nlatfill == 0 && m.nlngfill == 0));
+    const Ginterp unit{m.phase1, m.phase2, 1., 1., 1., 1.};
+    if (fine_only) phases(unit);
 
     // geometry (GeomKey)
     const bool geom_hit = c->has_geom && !(flags & LCG_FLAG_NO_CACHE) && same_geometry(c->key, m);
@@ -1003,7 +1058,8 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
             const bool on_side = conc && k == 1;  // star 2's fine grid
             {
                 StageScope t(c, LCG_STAGE_CONTINUUM);
-                launch_continuum(cp, gl[k]->dev(), on_side ? c->side[0] : c->stream);
+                launch_continuum(cp, gl[k]->dev(), gl[k]->cnt.p, gl[k]->dsum.p,
+                                 on_side ? c->side[0] : c->stream);
             }
             // (with an opaque disc the grids are flattened below, after the
             // disc's ranges; first without them when the Ginterp scales need it)
@@ -1013,7 +1069,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
                                   on_side)))
                     return rc;
         }
-        c->gi = Ginterp{m.phase1, m.phase2, 1., 1., 1., 1.};
+        c->gi = unit;
         if (!c->copy1 || !c->copy2) {
             if ((rc = ginterp_scales(c, m, rlens1))) return rc;
         }
@@ -1034,7 +1090,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
                     return c->cuda_fail(e, "disc eclipses");
                 {
                     StageScope t(c, LCG_STAGE_ECLIPSE);
-                    launch_disc_faces(dg, g.dev(), g.ndx.p, g.xr.p, c->status.p, c->stream);
+                    launch_disc_faces(dg, g.dev(), g.ndx.p, g.xr.p, g.cnt.p, c->status.p, c->stream);
                 }
                 g.disc = true;
                 if ((rc = flatten(c, g, need_pos,
@@ -1045,46 +1101,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
         c->cached_mixed_pos = (int)need_pos;
     }
 
-    // phase entries (light_curve_comp.cpp:358-455) over the resident points
-    const int64_t nent = c->data_nent;
-    const double xmin = c->data_xmin, xmax = c->data_xmax;
-    const bool diag = (flags & LCG_FLAG_DIAGNOSTICS) != 0;
-    const int64_t nall = nent + (diag ? 1 : 0);  // + the phase-0.5 entry of wdwarf
-    const int64_t ldp = ((nall + 3) / 4) * 4;
-    if ((e = c->pex.ensure(nall)) || (e = c->pey.ensure(nall)) || (e = c->pez.ensure(nall)) ||
-        (e = c->pphin.ensure(nall)) || (e = c->pw1.ensure(nall)) || (e = c->pw2.ensure(nall)) ||
-        (e = c->pef.ensure(nall)) || (e = c->ppfx.ensure(nall)) || (e = c->ptype.ensure(nall)) || (e = c->calc.ensure(n)) ||
-        (e = c->scratch.ensure(3 * (size_t)n)))
-        return c->cuda_fail(e, "phase buffers");
-    PhaseDev ph{c->pex.p, c->pey.p, c->pez.p, c->pphin.p, c->pw1.p, c->pw2.p,
-                c->pef.p, c->ptype.p, nall, c->ppfx.p};
-    const double ri = deg2rad(m.iangle);
-    const double cosi = cos(ri), sini = sin(ri);
-    PhaseParams pp{};
-    pp.t0 = m.t0; pp.period = m.period; pp.pdot = m.pdot; pp.deltat = m.deltat;
-    pp.slope = m.slope; pp.quad = m.quad; pp.cube = m.cube;
-    pp.middle = (xmin + xmax) / 2.;
-    pp.range = (xmax - xmin) / 2.;
-    pp.cosi = cosi; pp.sini = sini;
-    pp.gi = c->gi;
-    {
-        StageScope t(c, LCG_STAGE_PHASES);
-        launch_phases(pp, c->data.p, c->off.p, n, ph, c->stream);
-        if (diag) {
-            // comp_star1_flat at phase 0.5 (light_curve_comp.cpp:504-508)
-            const V3 ew = set_earth(cosi, sini, 0.5);
-            double v[4] = {ew.x, ew.y, ew.z, 0.5};
-            cudaMemcpyAsync(c->pex.p + nent, &v[0], 8, cudaMemcpyHostToDevice, c->stream);
-            cudaMemcpyAsync(c->pey.p + nent, &v[1], 8, cudaMemcpyHostToDevice, c->stream);
-            cudaMemcpyAsync(c->pez.p + nent, &v[2], 8, cudaMemcpyHostToDevice, c->stream);
-            cudaMemcpyAsync(c->pphin.p + nent, &v[3], 8, cudaMemcpyHostToDevice, c->stream);
-            PhaseDev one = ph;
-            one.ex += nent; one.ey += nent; one.ez += nent; one.phin += nent; one.ef += nent;
-            one.pfx += nent;
-            one.nent = 1;
-            launch_pack_phases(one, c->stream);
-        }
-    }
+    if (!fine_only) phases(c->gi);
     if (conc) {
         cudaEventRecord(c->ev_phases, c->stream);
         cudaStreamWaitEvent(c->side[0], c->ev_phases, 0);
@@ -1141,6 +1158,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
     }
 
     // scatter, third light, scale, chi**2
+    const bool fine_half = c->copy1 || gi_type(c->gi, 0.5) == 1;
     {
         ScatterParams sp{};
         sp.copy1 = c->copy1;
@@ -1164,57 +1182,55 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
             rp.osum[k] = c->osum.p + k * ldp;
         }
         StageScope t(c, LCG_STAGE_REDUCE);
-        launch_scatter(sp, rp, ph, c->data.p, c->off.p, n, c->calc.p, c->stream);
-        cudaMemcpyAsync(c->sfac.p, sfac, 5 * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-        if (iscale)
+        launch_scatter(sp, rp, ph, c->data.p, c->off.p, n, c->calc(), c->stream);
+        TailOut *tail = c->tail();
+        TailIn ti{};
+        ti.status = c->status.p;
+        if (diag) {
+            ti.dsum[0] = g1f.dsum.p;
+            ti.dsum[1] = g2f.dsum.p;
+            ti.nb[0] = cont_blocks(g1f.n);
+            ti.nb[1] = cont_blocks(g2f.n);
+            // star1c aliases star1f when copy1 (light_curve_comp.cpp:192-195)
+            ti.wsum = c->osum.p + (fine_half ? 0 : 1) * ldp + nent;
+        }
+        if (iscale) {
+            cudaMemcpyAsync(tail->sfac, sfac, 5 * sizeof(double), cudaMemcpyHostToDevice,
+                            c->stream);
             launch_iscale(flags & 3, m.t2 > 0 ? 5 : 4, c->data.p, n, c->fcomp.p, c->iwork.p,
-                          c->calc.p, c->sfac.p, c->out.p, c->stream);
-        else
-            launch_finalize(flags & 3, c->data.p, n, c->calc.p, c->sfac.p, c->out.p, c->stream);
+                          c->calc(), tail->sfac, tail->out, c->stream);
+            launch_tail(ti, tail, c->stream);
+        } else {
+            launch_finalize(flags & 3, c->data.p, n, c->calc(), sfac[0], ti, tail, c->stream);
+        }
     }
-    double hout[4] = {0, 0, 0, 0};
-    if (calc)
-        cudaMemcpyAsync(calc, c->calc.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost,
-                        c->stream);
-    cudaMemcpyAsync(sfac, c->sfac.p, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(hout, c->out.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-
-    // diagnostics: wdwarf's phase-0.5 sum, logg / rv block sums
-    double wsum = 0.;
-    if (diag) {
-        // star1c aliases star1f when copy1 (light_curve_comp.cpp:192-195)
-        const bool fine = c->copy1 || gi_type(c->gi, 0.5) == 1;
-        cudaMemcpyAsync(&wsum, c->osum.p + (fine ? 0 : 1) * ldp + nent, sizeof(double),
-                        cudaMemcpyDeviceToHost, c->stream);
-        const int64_t nb1 = diag_blocks(g1f.n), nb2 = diag_blocks(g2f.n);
-        if ((e = c->diag.ensure(4 * (size_t)(nb1 + nb2))))
-            return c->cuda_fail(e, "diagnostics");
-        launch_diagnostics(g1f.dev(), g2f.dev(), c->diag.p, c->stream);
-        c->h_diag.resize(4 * (size_t)(nb1 + nb2));
-        cudaMemcpyAsync(c->h_diag.data(), c->diag.p, c->h_diag.size() * sizeof(double),
-                        cudaMemcpyDeviceToHost, c->stream);
-    }
-    if ((rc = finish_status(c))) return rc;
+    // one copy for everything the call returns, through pinned memory
+    cudaMemcpyAsync(c->h_res.p, c->res.p,
+                    sizeof(TailOut) + (calc ? (size_t)n * sizeof(double) : 0),
+                    cudaMemcpyDeviceToHost, c->stream);
+    const TailOut &T = *reinterpret_cast<const TailOut *>(c->h_res.p);
+    if ((rc = finish_status(c, &T.status))) return rc;
+    if (calc) memcpy(calc, c->h_res.p + sizeof(TailOut), (size_t)n * sizeof(double));
+    if (iscale || (flags & LCG_FLAG_SCALE)) memcpy(sfac, T.sfac, sizeof T.sfac);
+    double wsum = T.wsum;
     c->key = m;
     c->has_geom = c->has_cont = true;
     if (diag && m.beam_factor1 != 0. && m.spin1 != 1.0 && !iscale) {
         // wdwarf is comp_star1_flat at phase 0.5, which beams with spin 1
         // (light_curve_comp.cpp:504-508); the sweeps above used spin1
-        const bool fine = c->copy1 || gi_type(c->gi, 0.5) == 1;
-        if ((rc = sweep_one(c, m, fine ? g1f : g1c, kStar1, 0.5, cosi, sini, rlens1, wsum)))
+        if ((rc = sweep_one(c, m, fine_half ? g1f : g1c, kStar1, 0.5, cosi, sini, rlens1, wsum)))
             return rc;
     }
 
-    if (hout[2] != 0.) {
-        scalars[LCG_OUT_CHISQ] = hout[0];
-        scalars[LCG_OUT_WNOK] = hout[1];
+    if (T.out[2] != 0.) {
+        scalars[LCG_OUT_CHISQ] = T.out[0];
+        scalars[LCG_OUT_WNOK] = T.out[1];
     }
     const double sc = sfac[0];
     if (diag) {
         double wd = 1.0 * gi_scale1(c->gi, 0.5) * wsum;
         scalars[LCG_OUT_WDWARF] = wd / 1 * sc;
         // comp_gravity1/2 (comp_gravity.cpp:20-155), comp_radius1/2 (comp_radius.cpp)
-        const int64_t nb1 = diag_blocks(g1f.n), nb2 = diag_blocks(g2f.n);
         double gm = pow(1000. * m.velocity_scale, 3) * m.tperiod * kDay / kTwoPi;
         double a = pow(gm / sq(kTwoPi / kDay / m.tperiod), 1. / 3.);
         double gscale = 100 * gm / sq(a);
@@ -1224,15 +1240,8 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
         if (m.r2 < 0) rr2 = rlb2;
         const double ACC = m.delta_phase / 10.;
         for (int star = 0; star < 2; star++) {
-            const double *b = c->h_diag.data() + (star == 0 ? 0 : 4 * nb1);
-            const int64_t nb = star == 0 ? nb1 : nb2;
-            double sumfg = 0., sumf = 0, sumsa = 0., sumvol = 0.;
-            for (int64_t k = 0; k < nb; k++) {
-                sumfg += b[4 * k];
-                sumf += b[4 * k + 1];
-                sumsa += b[4 * k + 2];
-                sumvol += b[4 * k + 3];
-            }
+            const double sumfg = T.diag[star][0], sumf = T.diag[star][1];
+            const double sumsa = T.diag[star][2], sumvol = T.diag[star][3];
             double gref;
             const bool roche = star == 0 ? m.roche1 : m.roche2;
             if (roche) {
@@ -1354,7 +1363,7 @@ lcg_status lcg_star_grid(lcg_ctx *c, const lcg_model *m, int32_t star, int32_t f
         return c->fail(LCG_E_INVALID, "nface = %d but the grid has %lld faces", nface,
                        (long long)g.n);
     ContParams cp = continuum_params(*m, star);
-    launch_continuum(cp, g.dev(), c->stream);
+    launch_continuum(cp, g.dev(), nullptr, nullptr, c->stream);
     std::vector<double> px(nface), py(nface), pz(nface), nx(nface), ny(nface), nz(nface);
     std::vector<uint8_t> ne(nface);
     const size_t d8 = (size_t)nface * sizeof(double), f4 = (size_t)nface * sizeof(float);

@@ -267,39 +267,57 @@ struct BatchPhases {
     unsigned long long *pfx;  // PhaseDev::pfx, ldp per model
 };
 
+// What a single-model call brings back besides its curve (one copy).
+struct TailIn {
+    const double *dsum[2];  // k_continuum's diagnostic sums of each star, or NULL
+    int64_t nb[2];          // and how many CTAs wrote them
+    const double *wsum;     // the phase-0.5 sum of wdwarf, or NULL
+    const DevStatus *status;
+};
+struct TailOut {
+    double out[3];      // chisq, wnok, 1 when they were computed
+    double sfac[5];
+    double diag[2][4];  // per star: sum f g, sum f, sum solid angle, sum volume
+    double wsum;
+    DevStatus status;
+    double pad_[6];
+};
+static_assert(sizeof(TailOut) == 24 * sizeof(double), "the curve follows it in the result block");
+
 // ---- launchers (geometry.cu) ------------------------------------------------
-void launch_grid(const GridParams &p, const RingRec *rings, GridDev g, DevStatus *st,
-                 cudaStream_t s);
+// counters: the eclipse stage's eight work counters, cleared here
+void launch_grid(const GridParams &p, const RingRec *rings, GridDev g, int32_t *counters,
+                 DevStatus *st, cudaStream_t s);
 // queue: one int per face; counters: 8 (candidates, work counters, hits);
 // es / hits: per-candidate state between the thread mode's two passes and the
 // compacted list of the eclipsed candidates (one per face each).
 void launch_eclipse(const EclParams &p, int32_t eclipse_on, GridDev g, int32_t *queue,
                     int32_t *counters, double4 *es, int32_t *hits, DevStatus *st, int nsm,
                     int32_t warp_mode, cudaStream_t s);
-void launch_continuum(const ContParams &p, GridDev g, cudaStream_t s);
-void launch_flatten(GridDev g, FlatDev f, int32_t *blockcnt, int mixed, int need_pos,
-                    const FastCoef &fc, DevStatus *st, cudaStream_t s);
+// cnt: 2 cont_blocks(n) partition counts; dsum: 4 cont_blocks(n) diagnostic sums
+// (either may be NULL)
+int64_t cont_blocks(int64_t n);
+void launch_continuum(const ContParams &p, GridDev g, int32_t *cnt, double *dsum,
+                      cudaStream_t s);
+void launch_flatten(GridDev g, FlatDev f, const int32_t *cnt, int mixed, int need_pos,
+                    const FastCoef &fc, cudaStream_t s);
+// extra: one more entry after the last point's, with earth vector ew and phase phw
 void launch_phases(const PhaseParams &p, const DatumRec *data, const int64_t *off, int32_t n,
-                   PhaseDev ph, cudaStream_t s);
+                   PhaseDev ph, bool extra, V3 ew, double phw, cudaStream_t s);
 void launch_scatter(const ScatterParams &p, const ReduceParams &r, const PhaseDev &ph,
                     const DatumRec *data, const int64_t *off, int32_t n, double *calc,
                     cudaStream_t s);
-// finalize: scale / chi**2 (re_scale.cpp:16-42, light_curve_comp.cpp:557-585).
-// out[0] = chisq, out[1] = wnok, out[2] = 1 when they were computed.
-void launch_finalize(int32_t flags, const DatumRec *data, int32_t n, double *calc,
-                     double *sfac_io, double *out, cudaStream_t s);
-// flux-weighted gravity / volume-averaged radius sums (comp_gravity.cpp,
-// comp_radius.cpp) of the two stars' grids: per block of kDiagBlock faces, star
-// 1's diag_blocks(g1.n) blocks first, four partial sums (f*g, f, solid angle,
-// volume) to out
-constexpr int64_t kDiagBlock = 2048;
-inline int64_t diag_blocks(int64_t n) { return (n + kDiagBlock - 1) / kDiagBlock; }
-void launch_diagnostics(const GridDev &g1, const GridDev &g2, double *out, cudaStream_t s);
-// light_curve_comp_fast interpolation of the model at sampled points mc
-// (sample indices idx, m of them) to all n points; chi**2, wnok -> out[0..1].
+// finalize: scale / chi**2 (re_scale.cpp:16-42, light_curve_comp.cpp:557-585)
+// from the given scale sfac0 (used unless the scale is fitted), with the rest of
+// the call's results beside it; tail: those alone.
+void launch_finalize(int32_t flags, const DatumRec *data, int32_t n, double *calc, double sfac0,
+                     const TailIn &in, TailOut *out, cudaStream_t s);
+void launch_tail(const TailIn &in, TailOut *out, cudaStream_t s);
 // dst row r = src row rows[r] (count rows of n doubles)
 void launch_gather_rows(const double *src, int32_t n, const int32_t *rows, int32_t count,
                         double *dst, cudaStream_t s);
+// light_curve_comp_fast interpolation of the model at sampled points mc
+// (sample indices idx, m of them) to all n points; chi**2, wnok -> out[0..1].
 void launch_interp(const DatumRec *data, int32_t n, const int64_t *idx, int32_t m,
                    const double *mc, double *calc, int32_t rdata, double *out, cudaStream_t s);
 
@@ -396,7 +414,7 @@ void launch_components(const CompParams &p, ElemRec *el, double4 *pos, DevStatus
                        cudaStream_t s);
 // The ranges an opaque disc adds to each face of a star grid.
 void launch_disc_faces(const DiscGeom &dg, const GridDev &g, uint8_t *ndx, double2 *xr,
-                       DevStatus *st, cudaStream_t s);
+                       int32_t *cnt, DevStatus *st, cudaStream_t s);
 // Per phase entry, the disc, rim and spot element sums (comp_light.cpp:323-408)
 // into rows 0, 1, 2 of out (row stride ldc); part holds comp_sums_scratch
 // doubles (per-chunk partial sums, added in chunk order).

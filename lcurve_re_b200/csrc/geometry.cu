@@ -91,9 +91,11 @@ __device__ __forceinline__ void grid_half(const GridParams &p, const RingRec *__
     }
 }
 
+// Also clears the eclipse stage's eight work counters.
 __global__ void k_grid(GridParams p, const RingRec *__restrict__ rings, GridDev g,
-                       DevStatus *st) {
+                       int32_t *counters, DevStatus *st) {
     const int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (h < 8) counters[h] = 0;
     if (h < p.nhalf) grid_half(p, rings, g, h, st);
 }
 
@@ -396,11 +398,7 @@ __device__ __forceinline__ float continuum_flux(const ContParams &p, const GridD
     return f;
 }
 
-__global__ void k_continuum(ContParams p, GridDev g) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < g.n) g.flux[i] = continuum_flux(p, g, i);
-}
-
+constexpr int kContBlock = 256;  // faces per CTA of k_continuum and of the partition counts
 constexpr int kFlatBlock = 1024;
 
 // Eclipse class of face i for the FlatGrid partition (comp_light_flat.cpp:26-65):
@@ -411,16 +409,48 @@ __device__ __forceinline__ int flat_class(const GridDev &g, int64_t i) {
     return k < 2 ? k : 2;
 }
 
-// Per 1024-face block: the one-range count in blockcnt[b], the several-range
-// count in blockcnt[nb + b].
-__global__ void k_flat_count(GridDev g, int32_t *blockcnt) {
-    const int64_t i = blockIdx.x * (int64_t)kFlatBlock + threadIdx.x;
-    const int cls = i < g.n ? flat_class(g, i) : 0;
-    const int c1 = __syncthreads_count(cls == 1);
-    const int c2 = g.ndx ? __syncthreads_count(cls == 2) : 0;
-    if (threadIdx.x == 0) {
-        blockcnt[blockIdx.x] = c1;
-        blockcnt[gridDim.x + blockIdx.x] = c2;
+// Face fluxes, and while the face is in registers what later stages would read
+// it again for: per CTA of 256 faces the number of one-range faces (cnt, for
+// k_flat_scatter; an opaque disc's ranges replace the counts, k_disc_faces) and
+// the sums behind log g and the volume-averaged radius (comp_gravity.cpp:20-155,
+// comp_radius.cpp:16-86: f g, f, solid angle, volume) as four doubles (dsum), a
+// fixed tree. Either may be null. A pass of its own over the faces took 8 us on
+// 10,300 faces and 25 us on 865,000; here they add 0.6 and 7.
+__global__ void __launch_bounds__(kContBlock) k_continuum(ContParams p, GridDev g, int32_t *cnt,
+                                                          double *dsum) {
+    const int64_t i = blockIdx.x * (int64_t)kContBlock + threadIdx.x;
+    const bool in = i < g.n;
+    double v[4] = {0., 0., 0., 0.};
+    if (in) {
+        const float f = continuum_flux(p, g, i);
+        g.flux[i] = f;
+        v[0] = (double)(f * g.grav[i]);
+        v[1] = (double)f;
+        const V3 vec = v3(g.px[i] - (p.star == kStar1 ? 0. : 1.), g.py[i], g.pz[i]);
+        const double r = len(vec);
+        v[3] = g.area[i] * dot(v3(g.nx[i], g.ny[i], g.nz[i]), vec);
+        v[2] = v[3] / (r * r * r);
+    }
+    if (cnt) {
+        const int c = __syncthreads_count(in && g.necl[i] == 1);
+        if (threadIdx.x == 0) {
+            cnt[blockIdx.x] = c;
+            cnt[gridDim.x + blockIdx.x] = 0;
+        }
+    }
+    if (!dsum) return;
+    __shared__ double sh[kContBlock / 32][4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        if (lane == 0) sh[w][k] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double s = 0.;
+        for (int k = 0; k < kContBlock / 32; k++) s += sh[k][threadIdx.x];
+        dsum[4 * (int64_t)blockIdx.x + threadIdx.x] = s;
     }
 }
 
@@ -452,19 +482,6 @@ __device__ __forceinline__ void scan_blocks(int32_t *blockcnt, int32_t nb, int64
     __syncthreads();
 }
 
-// Both counts scanned: n0 = faces never eclipsed, n1 = n0 + one-range faces
-// (n0[0] and n0[1]).
-__global__ void k_flat_scan(int32_t *blockcnt, int32_t nb, int64_t n, int64_t *n0) {
-    __shared__ int64_t c2;
-    int64_t t2 = 0;
-    scan_blocks(blockcnt + nb, nb, n, n0);  // n0[0] = n - (several-range faces)
-    if (threadIdx.x == 0) c2 = n - n0[0];
-    __syncthreads();
-    t2 = c2;
-    scan_blocks(blockcnt, nb, n - t2, n0);  // n0[0] = n - several - one-range
-    if (threadIdx.x == 0) n0[1] = n - t2;
-}
-
 // Face i's record of the fast mixed sweep at flat position dest (pairs of
 // faces interleaved, FlatDev::fp).
 __device__ __forceinline__ void fast_record(float *fp, int64_t dest, GridDev g, int64_t i,
@@ -483,13 +500,35 @@ __device__ __forceinline__ void fast_record(float *fp, int64_t dest, GridDev g, 
 
 // Stable three-way partition [never | one range | several]. Several-range
 // faces get all-zero records (they add exact zeros to the main sweeps) and
-// their face index and ranges in FlatGrid order; k_flux_ragged adds them.
-__global__ void k_flat_scatter(GridDev g, FlatDev f, const int32_t *__restrict__ blockoff,
-                               int mixed, int need_pos, FastCoef fc) {
-    __shared__ int32_t warp_tot[2][32];
+// their face index and ranges in FlatGrid order; k_flux_ragged adds them. Each
+// CTA adds up the counts before its block itself (at most a few thousand, 16 KB
+// from L2), which spares the two launches that counted and scanned; CTA 0
+// stores n0 and n1. CTAs past the last face zero the fast records up to npad.
+__global__ void __launch_bounds__(kFlatBlock) k_flat_scatter(GridDev g, FlatDev f,
+                                                             const int32_t *__restrict__ cnt,
+                                                             int32_t ncnt, int mixed, int need_pos,
+                                                             FastCoef fc) {
+    __shared__ int32_t warp_tot[2][32], red[32][4];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int64_t i = blockIdx.x * (int64_t)kFlatBlock + t;
     const bool in = i < g.n;
+    // one- and several-range faces before this block, and of the grid
+    const int mine = (int)blockIdx.x * (kFlatBlock / kContBlock);
+    int sum[4] = {0, 0, 0, 0};
+    for (int k = t; k < ncnt; k += kFlatBlock) {
+        const int c1 = cnt[k], c2 = cnt[ncnt + k];
+        sum[2] += c1;
+        sum[3] += c2;
+        if (k < mine) {
+            sum[0] += c1;
+            sum[1] += c2;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_down_sync(0xffffffffu, sum[q], o);
+        if (lane == 0) red[w][q] = sum[q];
+    }
     const int cls = in ? flat_class(g, i) : 0;
     const unsigned m1 = __ballot_sync(0xffffffffu, cls == 1);
     const unsigned m2 = __ballot_sync(0xffffffffu, cls == 2);
@@ -498,6 +537,19 @@ __global__ void k_flat_scatter(GridDev g, FlatDev f, const int32_t *__restrict__
         warp_tot[1][w] = __popc(m2);
     }
     __syncthreads();
+    // every warp adds the 32 partial sums the same way
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        int v = red[lane][q];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        sum[q] = v;
+    }
+    const int64_t boff1 = sum[0], boff2 = sum[1];
+    const int64_t n1 = g.n - sum[3], n0 = n1 - sum[2];
+    if (blockIdx.x == 0 && t == 0) {
+        f.n0[0] = n0;
+        f.n0[1] = n1;
+    }
     int b1 = 0, b2 = 0;
     for (int k = 0; k < w; k++) {
         b1 += warp_tot[0][k];
@@ -505,9 +557,13 @@ __global__ void k_flat_scatter(GridDev g, FlatDev f, const int32_t *__restrict__
     }
     const unsigned below = (1u << lane) - 1u;
     const int rank1 = b1 + __popc(m1 & below), rank2 = b2 + __popc(m2 & below);
-    if (!in) return;
-    const int64_t n0 = f.n0[0], n1 = f.n0[1];
-    const int64_t boff1 = blockoff[blockIdx.x], boff2 = blockoff[gridDim.x + blockIdx.x];
+    if (!in) {
+        if (mixed && fc.on && i < f.npad) {  // padding adds nothing
+            float *r = f.fp + 16 * (i >> 1) + (i & 1);
+            for (int q = 0; q < 16; q += 2) r[q] = 0.f;
+        }
+        return;
+    }
     const int64_t dest = cls == 1   ? n0 + boff1 + rank1
                          : cls == 2 ? n1 + boff2 + rank2
                                     : blockIdx.x * (int64_t)kFlatBlock - boff1 - boff2 +
@@ -581,9 +637,22 @@ __device__ __forceinline__ void sub_exposure(double phase, double expose, int nd
     }
 }
 
+// The point's sub-exposure entries; with extra, one more entry after the last
+// point's (the phase-0.5 entry of wdwarf, light_curve_comp.cpp:504-508: its earth
+// vector and phase are given, its weights unused).
 __global__ void k_phases(PhaseParams p, const DatumRec *__restrict__ data,
-                         const int64_t *__restrict__ off, int32_t n, PhaseDev ph) {
+                         const int64_t *__restrict__ off, int32_t n, PhaseDev ph, int32_t extra,
+                         V3 ew, double phw) {
     const int np = blockIdx.x * blockDim.x + threadIdx.x;
+    if (np == n && extra) {
+        const int64_t e = off[n];
+        ph.ex[e] = ew.x;
+        ph.ey[e] = ew.y;
+        ph.ez[e] = ew.z;
+        ph.phin[e] = phw;
+        ph.ef[e] = make_float4((float)ew.x, (float)ew.y, (float)ew.z, 0.f);
+        ph.pfx[e] = phase_fx64(phw);
+    }
     if (np >= n) return;
     const DatumRec d = data[np];
     double phase, slfac;
@@ -609,6 +678,29 @@ __global__ void k_phases(PhaseParams p, const DatumRec *__restrict__ data,
     }
 }
 
+// v[0] + v[ldp] + ... over nc rows in order, 32 loads in flight: a thread's sum
+// is bound by their latency (100 rows: 7.6 us with 8, 4.6 with 32).
+__device__ __forceinline__ double sum_rows(const double *__restrict__ v, int64_t nc, int64_t ldp) {
+    double o = 0.0;
+    int64_t c = 0;
+    for (; c + 32 <= nc; c += 32) {
+        double x[32];
+#pragma unroll
+        for (int u = 0; u < 32; u++) x[u] = v[(c + u) * ldp];
+#pragma unroll
+        for (int u = 0; u < 32; u++) o += x[u];
+    }
+    for (; c + 4 <= nc; c += 4) {
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = v[(c + u) * ldp];
+#pragma unroll
+        for (int u = 0; u < 4; u++) o += x[u];
+    }
+    for (; c < nc; c++) o += v[c * ldp];
+    return o;
+}
+
 // Sum of the chunk partials of every phase entry, chunks in order (for the
 // FP64 sweep: the reference's block order). One thread per (sweep, entry);
 // consecutive threads read consecutive entries of a chunk row.
@@ -618,17 +710,7 @@ __global__ void k_reduce_chunks(ReduceParams p) {
     const double *__restrict__ part = p.part[s];
     if (!part || e >= p.nent[s]) return;
     const int64_t nc = p.nchunk[s], ldp = p.ldp;
-    double o = 0.0;
-    int64_t c = 0;
-    for (; c + 8 <= nc; c += 8) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = part[(c + u) * ldp + e];
-#pragma unroll
-        for (int u = 0; u < 8; u++) o += v[u];
-    }
-    for (; c < nc; c++) o += part[c * ldp + e];
-    p.osum[s][e] = o;
+    p.osum[s][e] = sum_rows(part + e, nc, ldp);
 }
 
 // Per data point: weighted sub-exposure sums of the four sweeps in the
@@ -692,19 +774,27 @@ __global__ void k_scatter(ScatterParams p, const double *__restrict__ o1f,
     calc[np] = c + p.third;
 }
 
-// Fixed-shape tree over the 1024 threads of the block: deterministic.
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-    const int t = threadIdx.x;
-    sh[t] = v;
-    __syncthreads();
-    for (int w = 512; w > 0; w >>= 1) {
-        if (t < w) sh[t] += sh[t + w];
-        __syncthreads();
+// Sums of K values over the 1024 threads of the block, in every thread: shuffles
+// within the warps, then the 32 warps' sums the same way in each warp
+// (deterministic; two barriers, where a tree in shared memory took ten for
+// each value).
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double *sh) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) sh[32 * k + w] = v[k];
     }
-    const double r = sh[0];
     __syncthreads();
-    return r;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        v[k] = sh[32 * k + lane];
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    __syncthreads();
 }
+constexpr int kBlockSums = 32 * 4;  // doubles of shared memory for up to four values
 
 // One block of 1024 threads: thread t takes points t, t+1024, ... in order,
 // the block sums them in a fixed tree.
@@ -724,7 +814,9 @@ __device__ __forceinline__ void finalize_block(int32_t flags, const DatumRec *__
                 w += d.weight;
             }
         }
-        const double sdy = block_sum(a, sh), syy = block_sum(b, sh), wnok = block_sum(w, sh);
+        double s3[3] = {a, b, w};
+        block_sums(s3, sh);
+        const double sdy = s3[0], syy = s3[1], wnok = s3[2];
         const bool ok = wnok > 0.0;
         const double sc = ok ? sdy / syy : 1.;
         if (t == 0) {
@@ -755,19 +847,52 @@ __device__ __forceinline__ void finalize_block(int32_t flags, const DatumRec *__
             w += d.weight;
         }
     }
-    const double chisq = block_sum(cs, sh), wnok = block_sum(w, sh);
+    double s2[2] = {cs, w};
+    block_sums(s2, sh);
     if (t == 0) {
-        out[0] = chisq;
-        if (!scale) out[1] = wnok;
+        out[0] = s2[0];
+        if (!scale) out[1] = s2[1];
         out[2] = 1.;
     }
 }
 
+// What a call reads back besides the curve, gathered beside the finalize block:
+// the diagnostic sums of the two stars' CTAs (k_continuum), the phase-0.5 sum of
+// wdwarf and the device status.
+__device__ __forceinline__ void tail_block(const TailIn &in, TailOut *out, double *sh) {
+    const int t = threadIdx.x;
+    for (int star = 0; star < 2; star++) {
+        double v[4] = {0., 0., 0., 0.};
+        const double *p = in.dsum[star];
+        if (p)
+            for (int64_t b = t; b < in.nb[star]; b += 1024)
+#pragma unroll
+                for (int k = 0; k < 4; k++) v[k] += p[4 * b + k];
+        block_sums(v, sh);
+        if (t < 4) out->diag[star][t] = t == 0 ? v[0] : t == 1 ? v[1] : t == 2 ? v[2] : v[3];
+    }
+    if (t == 0) {
+        out->wsum = in.wsum ? *in.wsum : 0.;
+        out->status = *in.status;
+    }
+}
+
 __global__ void __launch_bounds__(1024) k_finalize(int32_t flags, const DatumRec *__restrict__ data,
-                                                   int32_t n, double *calc, double *sfac_io,
-                                                   double *out) {
-    __shared__ double sh[1024];
-    finalize_block(flags, data, n, calc, sfac_io, out, sh);
+                                                   int32_t n, double *calc, double sfac0,
+                                                   TailIn in, TailOut *out) {
+    __shared__ double sh[kBlockSums];
+    if (blockIdx.x == 1) {
+        tail_block(in, out, sh);
+        return;
+    }
+    if (threadIdx.x == 0) out->sfac[0] = sfac0;
+    __syncthreads();
+    finalize_block(flags, data, n, calc, out->sfac, out->out, sh);
+}
+
+__global__ void __launch_bounds__(1024) k_tail(TailIn in, TailOut *out) {
+    __shared__ double sh[kBlockSums];
+    tail_block(in, out, sh);
 }
 
 // light_curve_comp_fast's interpolation (light_curve_comp_fast.cpp:46-83):
@@ -778,7 +903,7 @@ __global__ void __launch_bounds__(1024) k_interp(const DatumRec *__restrict__ da
                                                  const int64_t *__restrict__ idx, int32_t m,
                                                  const double *__restrict__ mc, double *calc,
                                                  int32_t rdata, double *out) {
-    __shared__ double sh[1024];
+    __shared__ double sh[kBlockSums];
     const int t = threadIdx.x;
     double cs = 0., w = 0.;
     for (int i = t; i < n; i += 1024) {
@@ -806,10 +931,11 @@ __global__ void __launch_bounds__(1024) k_interp(const DatumRec *__restrict__ da
         }
     }
     if (!rdata) return;
-    const double chisq = block_sum(cs, sh), wnok = block_sum(w, sh);
+    double s2[2] = {cs, w};
+    block_sums(s2, sh);
     if (t == 0) {
-        out[0] = chisq;
-        out[1] = wnok;
+        out[0] = s2[0];
+        out[1] = s2[1];
     }
 }
 
@@ -981,50 +1107,6 @@ __global__ void k_gather_rows(const double *__restrict__ src, int32_t n,
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     dst[(int64_t)blockIdx.y * n + i] = src[(int64_t)rows[blockIdx.y] * n + i];
-}
-
-// comp_gravity / comp_radius sums (flux-weighted gravity, flux, solid angle,
-// volume) of both stars in one launch: CTA b takes kDiagBlock consecutive
-// faces of star 1, then of star 2; 256 threads stride over them (coalesced)
-// and a fixed-shape tree adds the threads, the host adds the CTAs in order
-// (deterministic, and a shorter rounding chain than one sum over the faces).
-// Each face costs a square root, a division and 80 B read, so the kernel is
-// bound by HBM on fine grids and by one load latency on small ones. One thread
-// per 8192 faces, serial, took 6.58 ms on 10,300 faces and 13.8 ms on 865,000
-// (one dependent division chain per face on two SMs); this split with 2048
-// faces a CTA puts at least 8 faces on every thread and 423 CTAs on the chip
-// at 865,000.
-__global__ void __launch_bounds__(256) k_diag(GridDev g1, GridDev g2, int32_t nb1, double *blk) {
-    const bool one = (int)blockIdx.x < nb1;
-    const GridDev &g = one ? g1 : g2;
-    const double cx = one ? 0. : 1.;
-    const int64_t lo = (int64_t)(one ? blockIdx.x : blockIdx.x - nb1) * kDiagBlock;
-    const int64_t hi = (g.n < lo + kDiagBlock) ? g.n : lo + kDiagBlock;
-    double v[4] = {0., 0., 0., 0.};
-    for (int64_t i = lo + threadIdx.x; i < hi; i += 256) {
-        const float f = g.flux[i];
-        v[0] += (double)(f * g.grav[i]);
-        v[1] += (double)f;
-        const V3 vec = v3(g.px[i] - cx, g.py[i], g.pz[i]);
-        const double r = len(vec);
-        const double rcosa = dot(v3(g.nx[i], g.ny[i], g.nz[i]), vec);
-        const double a = g.area[i] * rcosa;
-        v[2] += a / (r * r * r);
-        v[3] += a;
-    }
-    __shared__ double sh[8][4];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        if (lane == 0) sh[w][k] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-        double s = 0.;
-        for (int k = 0; k < 8; k++) s += sh[k][threadIdx.x];
-        blk[4 * (int64_t)blockIdx.x + threadIdx.x] = s;
-    }
 }
 
 // FP64 FlatGrid columns -> the packed mixed-precision view (used when a
@@ -1409,17 +1491,7 @@ __global__ void k_reduce_b(BatchDev b, const double *__restrict__ part, int64_t 
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= nent || !b.slots[s].live) return;
     const int64_t c0 = b.chunk_pre[s], c1 = b.chunk_pre[s + 1];
-    double o = 0.0;
-    int64_t c = c0;
-    for (; c + 8 <= c1; c += 8) {
-        double v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = part[(c + u) * ldp + e];
-#pragma unroll
-        for (int u = 0; u < 8; u++) o += v[u];
-    }
-    for (; c < c1; c++) o += part[c * ldp + e];
-    osum[s * ldp + e] = o;
+    osum[s * ldp + e] = sum_rows(part + c0 * ldp + e, c1 - c0, ldp);
 }
 
 // Per model and point: star 1 then star 2 sub-exposure sums, third light.
@@ -1442,7 +1514,7 @@ __global__ void __launch_bounds__(1024) k_finalize_b(BatchDev b, int32_t flags,
                                                      const DatumRec *__restrict__ data,
                                                      int32_t n, double *calc, double *sfac,
                                                      double *out) {
-    __shared__ double sh[1024];
+    __shared__ double sh[kBlockSums];
     const int m = blockIdx.x;
     if (!b.models[m].live) return;  // keeps the previous call's results
     double *sf = sfac + 5 * (int64_t)m;
@@ -1466,10 +1538,10 @@ void launch_pack_phases(PhaseDev ph, cudaStream_t s) {
     count_launch();
 }
 
-void launch_grid(const GridParams &p, const RingRec *rings, GridDev g, DevStatus *st,
-                 cudaStream_t s) {
+void launch_grid(const GridParams &p, const RingRec *rings, GridDev g, int32_t *counters,
+                 DevStatus *st, cudaStream_t s) {
     if (p.nhalf <= 0) return;
-    k_grid<<<nblocks(p.nhalf, 128), 128, 0, s>>>(p, rings, g, st);
+    k_grid<<<nblocks(p.nhalf, 128), 128, 0, s>>>(p, rings, g, counters, st);
     count_launch();
 }
 
@@ -1489,7 +1561,6 @@ void launch_eclipse(const EclParams &p, int32_t eclipse_on, GridDev g, int32_t *
                     int32_t *counters, double4 *es, int32_t *hits, DevStatus *st, int nsm,
                     int32_t warp_mode, cudaStream_t s) {
     if (g.n <= 0) return;
-    cudaMemsetAsync(counters, 0, 8 * sizeof(int32_t), s);
     k_ecl_pre<<<nblocks(g.n, 256), 256, 0, s>>>(p, eclipse_on, g, queue, counters);
     count_launch();
     if (eclipse_on && p.comp_roche) {
@@ -1517,40 +1588,32 @@ void launch_eclipse(const EclParams &p, int32_t eclipse_on, GridDev g, int32_t *
     }
 }
 
-void launch_continuum(const ContParams &p, GridDev g, cudaStream_t s) {
+int64_t cont_blocks(int64_t n) { return (n + kContBlock - 1) / kContBlock; }
+
+void launch_continuum(const ContParams &p, GridDev g, int32_t *cnt, double *dsum,
+                      cudaStream_t s) {
     if (g.n <= 0) return;
-    k_continuum<<<nblocks(g.n, 256), 256, 0, s>>>(p, g);
+    k_continuum<<<(unsigned)cont_blocks(g.n), kContBlock, 0, s>>>(p, g, cnt, dsum);
     count_launch();
 }
 
-void launch_flatten(GridDev g, FlatDev f, int32_t *blockcnt, int mixed, int need_pos,
-                    const FastCoef &fc, DevStatus *st, cudaStream_t s) {
-    (void)st;
-    const unsigned nb = nblocks(g.n, kFlatBlock);
-    if (nb == 0) {
+void launch_flatten(GridDev g, FlatDev f, const int32_t *cnt, int mixed, int need_pos,
+                    const FastCoef &fc, cudaStream_t s) {
+    if (g.n <= 0) {
         cudaMemsetAsync(f.n0, 0, 2 * sizeof(int64_t), s);
         return;
     }
-    if (mixed && fc.on && f.npad > g.n) {
-        // padding faces must add nothing: zero from the pair holding face n
-        // (records interleave the two faces of a pair; the scatter below
-        // rewrites face n-1's half when n is odd)
-        const int64_t z0 = 16 * (g.n >> 1);
-        cudaMemsetAsync(f.fp + z0, 0, (size_t)(8 * f.npad - z0) * sizeof(float), s);
-    }
-    k_flat_count<<<nb, kFlatBlock, 0, s>>>(g, blockcnt);
-    count_launch();
-    k_flat_scan<<<1, 1024, 0, s>>>(blockcnt, (int32_t)nb, g.n, f.n0);
-    count_launch();
-    k_flat_scatter<<<nb, kFlatBlock, 0, s>>>(g, f, blockcnt, mixed, need_pos, fc);
+    const int64_t cover = mixed && fc.on ? f.npad : g.n;
+    k_flat_scatter<<<nblocks(cover, kFlatBlock), kFlatBlock, 0, s>>>(
+        g, f, cnt, (int32_t)cont_blocks(g.n), mixed, need_pos, fc);
     count_launch();
     if (mixed && fc.on) launch_run_bounds(f.fp, f.ecl, f.npad / 2, f.runs, s);
 }
 
 void launch_phases(const PhaseParams &p, const DatumRec *data, const int64_t *off, int32_t n,
-                   PhaseDev ph, cudaStream_t s) {
+                   PhaseDev ph, bool extra, V3 ew, double phw, cudaStream_t s) {
     if (n <= 0) return;
-    k_phases<<<nblocks(n, 128), 128, 0, s>>>(p, data, off, n, ph);
+    k_phases<<<nblocks(n + (extra ? 1 : 0), 128), 128, 0, s>>>(p, data, off, n, ph, extra, ew, phw);
     count_launch();
 }
 
@@ -1570,9 +1633,14 @@ void launch_scatter(const ScatterParams &p, const ReduceParams &r, const PhaseDe
     count_launch();
 }
 
-void launch_finalize(int32_t flags, const DatumRec *data, int32_t n, double *calc,
-                     double *sfac_io, double *out, cudaStream_t s) {
-    k_finalize<<<1, 1024, 0, s>>>(flags, data, n, calc, sfac_io, out);
+void launch_finalize(int32_t flags, const DatumRec *data, int32_t n, double *calc, double sfac0,
+                     const TailIn &in, TailOut *out, cudaStream_t s) {
+    k_finalize<<<2, 1024, 0, s>>>(flags, data, n, calc, sfac0, in, out);
+    count_launch();
+}
+
+void launch_tail(const TailIn &in, TailOut *out, cudaStream_t s) {
+    k_tail<<<1, 1024, 0, s>>>(in, out);
     count_launch();
 }
 
@@ -1600,13 +1668,6 @@ void launch_gather_rows(const double *src, int32_t n, const int32_t *rows, int32
                         double *dst, cudaStream_t s) {
     if (n <= 0 || count <= 0) return;
     k_gather_rows<<<dim3(nblocks(n, 256), (unsigned)count), 256, 0, s>>>(src, n, rows, dst);
-    count_launch();
-}
-
-void launch_diagnostics(const GridDev &g1, const GridDev &g2, double *out, cudaStream_t s) {
-    const int64_t nb1 = diag_blocks(g1.n), nb = nb1 + diag_blocks(g2.n);
-    if (nb <= 0) return;
-    k_diag<<<(unsigned)nb, 256, 0, s>>>(g1, g2, (int32_t)nb1, out);
     count_launch();
 }
 
