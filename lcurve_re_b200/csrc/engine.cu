@@ -1175,6 +1175,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
         if ((e = c->osum.ensure(4 * (size_t)ldp))) return c->cuda_fail(e, "entry sums");
         ReduceParams rp{};
         rp.ldp = ldp;
+        rp.in_order = !mixed;
         for (int k = 0; k < 4; k++) {
             rp.part[k] = use_sw[k] ? sw[k].part->p : nullptr;
             rp.nchunk[k] = use_sw[k] ? sw[k].plan.nchunk : 0;

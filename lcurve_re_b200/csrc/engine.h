@@ -183,6 +183,7 @@ struct ReduceParams {
     int64_t nchunk[4], nent[4];
     int64_t ldp;  // row stride of the partials
     double *osum[4];
+    int32_t in_order;  // add the chunks strictly in order (FP64 sweeps)
 };
 
 // ---- batched evaluation -----------------------------------------------------

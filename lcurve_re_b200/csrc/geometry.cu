@@ -296,6 +296,50 @@ __global__ void __launch_bounds__(128, NB)
     }
 }
 
+// The whole eclipse stage of a grid small enough that two lanes per face fit the
+// GPU at once: sphere test, pot_min (both lanes of a pair, in step) and the
+// boundaries, one lane each. The three kernels and the candidate queue of larger
+// grids keep warps full, which nothing is gained by here: 8,152 faces 36 us in
+// three launches -> 24 in one.
+__global__ void __launch_bounds__(128, 4)
+    k_ecl_small(__grid_constant__ const EclParams p, int32_t eclipse_on,
+                __grid_constant__ const GridDev g, DevStatus *st) {
+    const unsigned full = 0xffffffffu;
+    const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = u >> 1;
+    const int side = (int)(u & 1);
+    // lane 0 of a pair writes the face's defaults and says whether it is a candidate
+    bool cand = side == 0 && i < g.n && ecl_pre_face(p, eclipse_on, g, i);
+    cand = __shfl_sync(full, cand, threadIdx.x & 30);
+    if (!__any_sync(full, cand)) return;
+    const V3 cofm = p.comp_star == kStar1 ? v3(0., 0., 0.) : v3(1., 0., 0.);
+    const V3 pos = cand ? v3(g.px[i], g.py[i], g.pz[i]) : v3(0., 0., 0.);
+    double phi1 = 0., phi2 = 0., lam1 = 0., lam2 = 0., phi = 0., lam = 0., acc = 0.;
+    bool live = false;
+    int s = 0;
+    if (cand &&
+        sphere_eclipse_ph(p.cosi, p.sini, pos, cofm, p.comp_rref, phi1, phi2, lam1, lam2)) {
+        acc = 2. * sqrt(2. * kTwoPi * (lam2 - lam1) * p.delta);
+        live = pot_min(p.comp_star, p.q, p.comp_spin, p.cosi, p.sini, pos, phi1, phi2, lam1, lam2,
+                       p.comp_rref, p.comp_pref, acc, phi, lam, s);
+        if (s) live = false;
+    }
+    double v = bisect_warp(p, live, phi, side ? phi2 : phi1, acc, pos, s);
+    v = v - floor(v);
+    const double other = __shfl_xor_sync(full, v, 1);
+    const int os = __shfl_xor_sync(full, s, 1);
+    if (!cand || side) return;
+    if (s || os) {
+        set_status(st, s ? s : os, i);
+    } else if (live) {
+        double egr = other;
+        if (egr < v) egr++;
+        g.necl[i] = 1;
+        g.ein[i] = v;
+        g.eout[i] = egr;
+    }
+}
+
 // The flux of face i (set_star_continuum.cpp:26-297).
 __device__ __forceinline__ float continuum_flux(const ContParams &p, const GridDev &g, int64_t i) {
     if (i >= g.ntiled) return 0.f;  // default Point: zero area, zero flux
@@ -701,16 +745,36 @@ __device__ __forceinline__ double sum_rows(const double *__restrict__ v, int64_t
     return o;
 }
 
-// Sum of the chunk partials of every phase entry, chunks in order (for the
-// FP64 sweep: the reference's block order). One thread per (sweep, entry);
-// consecutive threads read consecutive entries of a chunk row.
-__global__ void k_reduce_chunks(ReduceParams p) {
+// Sum of the chunk partials of every phase entry. G = 1: chunks in order (for the
+// FP64 sweep: the reference's block order), one thread per (sweep, entry);
+// consecutive threads read consecutive entries of a chunk row. G = 8 (mixed
+// sweeps): eight warps take eighths of the rows and their sums are added in
+// order, eight times the loads in flight: 796 rows of 25,000 entries 72 -> 38 us,
+// 130 rows of 500 7.4 -> 2.8.
+template <int G>
+__global__ void __launch_bounds__(256) k_reduce_chunks(ReduceParams p) {
+    constexpr int W = 256 / G;  // entries per CTA
     const int s = blockIdx.y;
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int x = threadIdx.x % W, y = threadIdx.x / W;
+    const int64_t e = blockIdx.x * (int64_t)W + x;
     const double *__restrict__ part = p.part[s];
-    if (!part || e >= p.nent[s]) return;
+    if (!part) return;
+    const bool in = e < p.nent[s];
     const int64_t nc = p.nchunk[s], ldp = p.ldp;
-    p.osum[s][e] = sum_rows(part + e, nc, ldp);
+    if constexpr (G == 1) {
+        if (in) p.osum[s][e] = sum_rows(part + e, nc, ldp);
+    } else {
+        __shared__ double sh[G][W];
+        const int64_t c0 = nc * y / G, c1 = nc * (y + 1) / G;
+        sh[y][x] = in ? sum_rows(part + c0 * ldp + e, c1 - c0, ldp) : 0.;
+        __syncthreads();
+        if (y == 0 && in) {
+            double o = sh[0][x];
+#pragma unroll
+            for (int k = 1; k < G; k++) o += sh[k][x];
+            p.osum[s][e] = o;
+        }
+    }
 }
 
 // Per data point: weighted sub-exposure sums of the four sweeps in the
@@ -1561,6 +1625,12 @@ void launch_eclipse(const EclParams &p, int32_t eclipse_on, GridDev g, int32_t *
                     int32_t *counters, double4 *es, int32_t *hits, DevStatus *st, int nsm,
                     int32_t warp_mode, cudaStream_t s) {
     if (g.n <= 0) return;
+    // two lanes per face at four CTAs of 128 per SM
+    if (eclipse_on && p.comp_roche && warp_mode <= 0 && g.n <= (int64_t)nsm * 256) {
+        k_ecl_small<<<nblocks(2 * g.n, 128), 128, 0, s>>>(p, eclipse_on, g, st);
+        count_launch();
+        return;
+    }
     k_ecl_pre<<<nblocks(g.n, 256), 256, 0, s>>>(p, eclipse_on, g, queue, counters);
     count_launch();
     if (eclipse_on && p.comp_roche) {
@@ -1625,7 +1695,8 @@ void launch_scatter(const ScatterParams &p, const ReduceParams &r, const PhaseDe
     for (int k = 0; k < 4; k++)
         if (r.part[k] && r.nent[k] > nmax) nmax = r.nent[k];
     if (nmax > 0) {
-        k_reduce_chunks<<<dim3(nblocks(nmax, 256), 4), 256, 0, s>>>(r);
+        if (r.in_order) k_reduce_chunks<1><<<dim3(nblocks(nmax, 256), 4), 256, 0, s>>>(r);
+        else k_reduce_chunks<8><<<dim3(nblocks(nmax, 32), 4), 256, 0, s>>>(r);
         count_launch();
     }
     k_scatter<<<nblocks(n, 128), 128, 0, s>>>(p, r.osum[0], r.osum[1], r.osum[2], r.osum[3], ph,
