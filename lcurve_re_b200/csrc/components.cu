@@ -491,71 +491,96 @@ namespace eng {
 
 namespace {
 
-// Restricted three-body acceleration in the rotating frame (rocacc.cpp).
-void stream_deriv(double q, const double *y, double *dy) {
-    const double f1 = 1.0 / (1.0 + q), f2 = f1 * q;
-    const double yzsq = sq(y[1]) + sq(y[2]);
-    const double r1sq = sq(y[0]) + yzsq, r2sq = sq(y[0] - 1.0) + yzsq;
-    const double fm1 = f1 / (r1sq * sqrt(r1sq)), fm2 = f2 / (r2sq * sqrt(r2sq)), fm3 = fm1 + fm2;
-    dy[0] = y[3]; dy[1] = y[4]; dy[2] = y[5];
-    dy[3] = -fm3 * y[0] + fm2 + 2.0 * y[4] + y[0] - f2;
-    dy[4] = -fm3 * y[1] - 2.0 * y[3] + y[1];
-    dy[5] = -fm3 * y[2];
-}
+// The gas stream's motion (rocacc.cpp: the restricted three-body problem in the
+// rotating frame, in the orbital plane, where the stream starts at rest in z)
+// by Taylor series (e.g. Jorba & Zou 2005): with p_i = r_i^-3 the equations
+//   x'' =  2 y' + x - f2 - f1 p1 x - f2 p2 (x - 1)
+//   y'' = -2 x' + y - f1 p1 y - f2 p2 y
+// give the next coefficients of x and y from the lower ones, those of p_i
+// following from r_i^2 by the recurrence of a power. Order kOrder with steps at
+// which the last terms are 1e-16 of the coordinates: some 20 steps, where a
+// fifth-order Runge-Kutta pair at 1e-13 took 5000.
+constexpr int kOrder = 26;
+struct StreamSeries {
+    double x[kOrder + 1], y[kOrder + 1];
 
-// One Dormand-Prince 5(4) step (Dormand & Prince 1980); returns the scaled
-// error estimate of the embedded pair.
-double dp5_step(double q, const double *y, double h, double *yo) {
-    static const double A[6][5] = {{1. / 5},
-                                   {3. / 40, 9. / 40},
-                                   {44. / 45, -56. / 15, 32. / 9},
-                                   {19372. / 6561, -25360. / 2187, 64448. / 6561, -212. / 729},
-                                   {9017. / 3168, -355. / 33, 46732. / 5247, 49. / 176,
-                                    -5103. / 18656},
-                                   {35. / 384, 0., 500. / 1113, 125. / 192, -2187. / 6784}};
-    static const double B6 = 11. / 84;
-    static const double E[7] = {71. / 57600, 0., -71. / 16695, 71. / 1920, -17253. / 339200,
-                                22. / 525, -1. / 40};
-    double k[7][6], t[6];
-    stream_deriv(q, y, k[0]);
-    for (int s = 1; s <= 5; s++) {
-        for (int i = 0; i < 6; i++) {
-            double a = 0.;
-            for (int j = 0; j < s; j++) a += A[s - 1][j] * k[j][i];
-            t[i] = y[i] + h * a;
+    void expand(double q, const double *s) {  // s = x, y, x', y'
+        const double f1 = 1. / (1. + q), f2 = f1 * q;
+        double s1[kOrder], s2[kOrder], p1[kOrder], p2[kOrder];
+        x[0] = s[0]; x[1] = s[2];
+        y[0] = s[1]; y[1] = s[3];
+        for (int n = 0; n + 2 <= kOrder; n++) {
+            // r^2 about either star (x - 1 differs from x in its first coefficient)
+            double xx = 0., yy = 0.;
+            for (int k = 0; k <= n; k++) {
+                xx += x[k] * x[n - k];
+                yy += y[k] * y[n - k];
+            }
+            s1[n] = xx + yy;
+            s2[n] = s1[n] - 2. * x[n] + (n == 0 ? 1. : 0.);
+            if (n == 0) {
+                p1[0] = 1. / (s1[0] * sqrt(s1[0]));
+                p2[0] = 1. / (s2[0] * sqrt(s2[0]));
+            } else {
+                double a1 = 0., a2 = 0.;
+                for (int k = 0; k < n; k++) {
+                    const double c = -1.5 * (n - k) - k;
+                    a1 += c * s1[n - k] * p1[k];
+                    a2 += c * s2[n - k] * p2[k];
+                }
+                p1[n] = a1 / (n * s1[0]);
+                p2[n] = a2 / (n * s2[0]);
+            }
+            double px1 = 0., px2 = 0., py = 0.;
+            for (int k = 0; k <= n; k++) {
+                px1 += p1[k] * x[n - k];
+                px2 += p2[k] * x[n - k];
+                py += (f1 * p1[k] + f2 * p2[k]) * y[n - k];
+            }
+            px2 -= p2[n];
+            const double d = (n + 1.) * (n + 2.);
+            x[n + 2] = (2. * (n + 1) * y[n + 1] + x[n] - (n == 0 ? f2 : 0.) - f1 * px1 - f2 * px2) / d;
+            y[n + 2] = (-2. * (n + 1) * x[n + 1] + y[n] - py) / d;
         }
-        stream_deriv(q, t, k[s]);
     }
-    for (int i = 0; i < 6; i++) {
-        double a = 0.;
-        for (int j = 0; j < 5; j++) a += A[5][j] * k[j][i];
-        yo[i] = y[i] + h * (a + B6 * k[5][i]);
+    // the step whose last two terms stay below 1e-16 of the start's coordinates
+    double step() const {
+        const double scale = 1e-16 * std::max(fabs(x[0]), fabs(y[0]));
+        double h = 1.;
+        for (int n = kOrder - 1; n <= kOrder; n++) {
+            const double c = std::max(fabs(x[n]), fabs(y[n]));
+            if (c > 0.) h = std::min(h, pow(scale / c, 1. / n));
+        }
+        return h;
     }
-    stream_deriv(q, yo, k[6]);
-    double err = 0.;
-    for (int i = 0; i < 6; i++) {
-        double ei = 0.;
-        for (int j = 0; j < 7; j++) ei += E[j] * k[j][i];
-        ei *= h;
-        const double sc = 1e-14 + 1e-13 * std::max(fabs(y[i]), fabs(yo[i]));
-        err = std::max(err, fabs(ei) / sc);
+    void at(double t, double *s) const {
+        double a = 0., b = 0., da = 0., db = 0.;
+        for (int n = kOrder; n >= 1; n--) {
+            da = da * t + n * x[n];
+            db = db * t + n * y[n];
+            a = (a + x[n]) * t;
+            b = (b + y[n]) * t;
+        }
+        s[0] = a + x[0];
+        s[1] = b + y[0];
+        s[2] = da;
+        s[3] = db;
     }
-    return err;
-}
+};
 
-double radius(const double *y) { return sqrt(sq(y[0]) + sq(y[1]) + sq(y[2])); }
+double radius(const double *s) { return sqrt(sq(s[0]) + sq(s[1])); }
+double outward(const double *s) { return s[0] * s[2] + s[1] * s[3]; }  // r dr/dt
 
 }  // namespace
 
 // Where the gas stream from L1 first reaches distance rad from star 1:
 // Roche::strinit's start (strining.cpp:14-33) and the motion of rocacc.cpp,
-// integrated with Dormand-Prince 5(4) under a tight tolerance, the crossing
-// bisected in time to 1e-10 in radius (the accuracy stradv.cpp:27-80 asks
-// for). The reference integrates with a Bulirsch-Stoer stepper whose first
-// step size is kept in a static between calls, so the two agree to their
-// integration error (about 1e-11 in position), not bit for bit.
+// integrated by Taylor series, the crossing bisected in time to the last bits.
+// The reference integrates with a Bulirsch-Stoer stepper whose first step size
+// is kept in a static between calls (stradv.cpp:35), to 1e-10 in radius, so the
+// two agree to its error, not bit for bit.
 bool bright_spot_position(double q, double rad, double *pos, Fail &f) {
-    const double SMALL = 1.e-5, ACC = 1.e-10, SMAX = 1.e-3, TMAX = 10.;
+    const double SMALL = 1.e-5, TMAX = 10.;
     const double rl1 = xl1(q);
     if (rl1 < 0) {
         f = {LCG_E_NOCONVERGE, "Roche::xl1(double): exceeded maximum iterations"};
@@ -565,48 +590,60 @@ bool bright_spot_position(double q, double rad, double *pos, Fail &f) {
     const double a = (1.0 - mu) / pow(rl1, 3) + mu / pow((1. - rl1), 3);
     const double lambda1 = sqrt(((a - 2.0) + sqrt(a * (9.0 * a - 8.0))) / 2.0);
     const double m1 = (lambda1 * lambda1 - 2.0 * a - 1.0) / 2.0 / lambda1;
-    double y[6] = {rl1 - SMALL, -m1 * SMALL, 0., -lambda1 * SMALL, -lambda1 * m1 * SMALL, 0.};
-    double yo[6], ylo[6], h = 1e-4, t = 0.;
-    const double rinit = radius(y);
+    double s[4] = {rl1 - SMALL, -m1 * SMALL, -lambda1 * SMALL, -lambda1 * m1 * SMALL};
+    const double rinit = radius(s);
     auto before = [&](double r) { return (rinit > rad && r > rad) || (rinit < rad && r < rad); };
-    double rnow = rinit;
-    for (int guard = 0; before(rnow); guard++) {
-        if (guard > 1000000 || t > TMAX) {
+    double t = 0.;
+    for (int guard = 0; before(radius(s)); guard++) {
+        if (guard > 100000 || t > TMAX) {
             f = {LCG_E_ROCHE, "Roche::stradv: taken too long without crossing radius"};
             return false;
         }
-        h = std::min(h, SMAX);
-        const double err = dp5_step(q, y, h, yo);
-        if (err > 1.) {
-            h *= std::max(0.2, 0.9 * pow(err, -0.2));
-            continue;
-        }
-        std::copy(y, y + 6, ylo);
-        std::copy(yo, yo + 6, y);
-        t += h;
-        rnow = radius(y);
-        const double hstep = h;
-        h *= err > 0. ? std::min(5., 0.9 * pow(err, -0.2)) : 5.;
-        if (!before(rnow)) {
-            double lo = 0., hi = hstep, rlo = radius(ylo), rhi = rnow;
-            for (int g2 = 0; fabs(rhi - rlo) > ACC && g2 < 200; g2++) {
-                const double tt = (lo + hi) / 2.;
-                dp5_step(q, ylo, tt, y);
-                rnow = radius(y);
-                if ((rhi > rad && rnow > rad) || (rhi < rad && rnow < rad)) {
-                    rhi = rnow;
-                    hi = tt;
-                } else {
-                    rlo = rnow;
-                    lo = tt;
+        StreamSeries S;
+        S.expand(q, s);
+        const double h = S.step();
+        // the radius within the step: at 16 times, and at a turning point between
+        // two of them, where it may cross and come back
+        double lo = 0., slo[4] = {s[0], s[1], s[2], s[3]}, shi[4];
+        bool crossed = false;
+        for (int k = 1; k <= 16 && !crossed; k++) {
+            double hi = h * k / 16;
+            S.at(hi, shi);
+            if (before(radius(shi)) && (outward(slo) > 0.) != (outward(shi) > 0.)) {
+                double ta = lo, tb = hi, sm[4];
+                const bool up = outward(slo) > 0.;
+                for (int i = 0; i < 60; i++) {
+                    const double tm = (ta + tb) / 2.;
+                    S.at(tm, sm);
+                    if ((outward(sm) > 0.) == up) ta = tm;
+                    else tb = tm;
+                }
+                if (!before(radius(sm))) {
+                    hi = (ta + tb) / 2.;
+                    S.at(hi, shi);
                 }
             }
-            break;
+            if (!before(radius(shi))) {
+                for (int i = 0; i < 60; i++) {
+                    const double tm = (lo + hi) / 2.;
+                    double sm[4];
+                    S.at(tm, sm);
+                    if (before(radius(sm))) lo = tm;
+                    else hi = tm;
+                }
+                S.at(hi, shi);
+                crossed = true;
+            }
+            lo = hi;
+            std::copy(shi, shi + 4, slo);
         }
+        std::copy(slo, slo + 4, s);
+        t += h;
+        if (crossed) break;
     }
-    pos[0] = y[0];
-    pos[1] = y[1];
-    pos[2] = y[2];
+    pos[0] = s[0];
+    pos[1] = s[1];
+    pos[2] = 0.;
     return true;
 }
 
