@@ -247,21 +247,23 @@ __global__ void __launch_bounds__(kThreadsC) k_comp_sums(const ElemRec *__restri
         for (int t = 0; t < m; t++) {
             const int i = base + t;
             const ElemRec &r = tile[t];
+            // turned away or hidden at every entry of the warp: exact zeros
+            const double mu = ex * r.dx + ey * r.dy + ez * r.dz;
+            if (!__any_sync(0xffffffffu, mu > 0.0)) continue;
             // Point::visible (lcurve.h:81-89)
             bool vis = true;
             const int nr = r.nr < kMaxRanges ? r.nr : kMaxRanges;
             for (int k = 0; k < nr; k++) {
                 const double in = r.r[k].x, o = r.r[k].y;
-                if ((phi >= in && phi <= o) || phi <= o - 1.0) { vis = false; break; }
+                vis = vis && !((phi >= in && phi <= o) || phi <= o - 1.0);
             }
+            if (!__any_sync(0xffffffffu, vis && mu > 0.0)) continue;
             double v = 0.0;
-            if (vis) {
-                const double mu = ex * r.dx + ey * r.dy + ez * r.dz;
-                if (i >= nd + ne) {
-                    v = (mu > 0.0) ? mu * (double)r.flux : 0.0;  // spot_elem
-                } else if (mu > 0.0) {                          // disc_elem
+            if (vis && mu > 0.0) {
+                v = mu * (double)r.flux;  // spot_elem
+                if (i < nd + ne) {        // disc_elem
                     const double om = 1.0 - mu;
-                    v = mu * (double)r.flux * (1.0 - om * (lin + quad * om));
+                    v = v * (1.0 - om * (lin + quad * om));
                 }
             }
             const int c = i < nd ? 0 : (i < nd + ne ? 1 : 2);

@@ -226,10 +226,11 @@ struct lcg_ctx {
     // side streams: star 2's grids (side[0]) and the component elements
     // (side[1]) run beside star 1's; their eclipse solves are latency-bound,
     // so they overlap well. Created by the first call.
-    // With fine grids only (no coarse ones, no opaque disc), star 2's continuum,
-    // partition and flux sweep also stay on side[0], which waits for the phase
-    // entries (ev_phases) and joins before the scatter: star 1's sweep fills
-    // the SMs that star 2's latency-bound geometry leaves idle.
+    // With fine grids only (no coarse ones), star 2's continuum, an opaque disc's
+    // ranges, partition and flux sweeps also stay on side[0], and the components'
+    // sums on side[1]; both wait for the phase entries (ev_phases) and join before
+    // the scatter: star 1's sweep fills the SMs that their latency-bound geometry
+    // leaves idle.
     cudaStream_t side[2] = {nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr}, ev_phases = nullptr;
     // resident light-curve points (lcg_set_data)

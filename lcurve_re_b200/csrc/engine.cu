@@ -982,7 +982,10 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
     const bool fine_only = m.nlat1f == m.nlat1c && m.nlat2f == m.nlat2c &&
                            (!m.npole || r1 >= r2 || (m.nlatfill == 0 && m.nlngfill == 0));
     const Ginterp unit{m.phase1, m.phase2, 1., 1., 1., 1.};
-    if (fine_only) phases(unit);
+    if (fine_only) {
+        phases(unit);
+        cudaEventRecord(c->ev_phases, c->stream);
+    }
 
     // geometry (GeomKey)
     const bool geom_hit = c->has_geom && !(flags & LCG_FLAG_NO_CACHE) && same_geometry(c->key, m);
@@ -999,8 +1002,9 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
         if (!c->copy2 && (rc = build_geometry(c, m, kStar2, 0, c->g2c, c->side[0]))) return rc;
     }
     // concurrent order (see lcg_ctx::side): star 2 stays on side[0] up to its
-    // sweep; otherwise the streams join here
-    const bool conc = c->copy1 && c->copy2 && !opaque && !c->profiling;
+    // sweep, the components on side[1] up to their sums; otherwise the streams
+    // join here
+    const bool conc = fine_only && !c->profiling;
     if (conc) {
         cudaStreamWaitEvent(c->side[0], c->ev_fork, 0);  // also when the grids were reused
     } else if (!geom_hit) {
@@ -1036,7 +1040,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
                             cudaMemcpyHostToDevice, c->side[1]);
         c->comp.rings = c->drings.p;
         launch_components(c->comp, c->elem.p, c->epos.p, c->status.p, c->side[1]);
-        cudaEventRecord(c->ev_join[1], c->side[1]);
+        if (!conc) cudaEventRecord(c->ev_join[1], c->side[1]);
         if ((flags & LCG_FLAG_INFO) && m.add_disc)
             fprintf(stderr, "Number of points for the disc = %d\n", c->comp.nd);
     }
@@ -1088,13 +1092,16 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
                 Grid &g = *gl[k];
                 if ((e = g.ndx.ensure(g.n)) || (e = g.xr.ensure(kDiscRanges * g.n)))
                     return c->cuda_fail(e, "disc eclipses");
+                const bool on_side = conc && k == 1;
                 {
                     StageScope t(c, LCG_STAGE_ECLIPSE);
-                    launch_disc_faces(dg, g.dev(), g.ndx.p, g.xr.p, g.cnt.p, c->status.p, c->stream);
+                    launch_disc_faces(dg, g.dev(), g.ndx.p, g.xr.p, g.cnt.p, c->status.p,
+                                      on_side ? c->side[0] : c->stream);
                 }
                 g.disc = true;
                 if ((rc = flatten(c, g, need_pos,
-                                  fast_coef(m, stars[k], c->precision == LCG_PREC_MIXED))))
+                                  fast_coef(m, stars[k], c->precision == LCG_PREC_MIXED),
+                                  on_side)))
                     return rc;
             }
         }
@@ -1102,10 +1109,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
     }
 
     if (!fine_only) phases(c->gi);
-    if (conc) {
-        cudaEventRecord(c->ev_phases, c->stream);
-        cudaStreamWaitEvent(c->side[0], c->ev_phases, 0);
-    }
+    if (conc) cudaStreamWaitEvent(c->side[0], c->ev_phases, 0);
 
     // flux sweeps (light_curve_comp.cpp:457-473)
     struct Sweep {
@@ -1151,10 +1155,22 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
             return c->cuda_fail(e, "component sums");
         PhaseDev phc = ph;
         phc.nent = nent;
-        cudaStreamWaitEvent(c->stream, c->ev_join[1], 0);
-        StageScope t(c, LCG_STAGE_FLUX);
-        launch_comp_sums(c->elem.p, c->comp.nd, c->comp.ne, ncomp, m.lin_limb_disc,
-                         m.quad_limb_disc, phc, c->csum.p + 3 * ldp, c->csum.p, ldp, c->stream);
+        cudaStream_t cs = c->stream;
+        if (conc) {
+            cs = c->side[1];
+            cudaStreamWaitEvent(cs, c->ev_phases, 0);
+        } else {
+            cudaStreamWaitEvent(cs, c->ev_join[1], 0);
+        }
+        {
+            StageScope t(c, LCG_STAGE_FLUX);
+            launch_comp_sums(c->elem.p, c->comp.nd, c->comp.ne, ncomp, m.lin_limb_disc,
+                             m.quad_limb_disc, phc, c->csum.p + 3 * ldp, c->csum.p, ldp, cs);
+        }
+        if (conc) {
+            cudaEventRecord(c->ev_join[1], cs);
+            cudaStreamWaitEvent(c->stream, c->ev_join[1], 0);
+        }
     }
 
     // scatter, third light, scale, chi**2
