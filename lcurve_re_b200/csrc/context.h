@@ -124,9 +124,9 @@ struct Grid {
             return e;
         if (mixed) {
             if ((e = ecl.ensure(npad))) return e;
+            if ((e = runs.ensure(kRunRecs * npad / kRunFaces))) return e;
             if (fast_on) {
-                if ((e = fp.ensure(8 * npad)) || (e = runs.ensure(kRunRecs * npad / kRunFaces)))
-                    return e;
+                if ((e = fp.ensure(8 * npad))) return e;
             } else if ((e = geo.ensure(npad))) {
                 return e;
             }

@@ -1431,7 +1431,8 @@ lcg_status lcg_sum_star_multi(lcg_ctx *c, int32_t star, int64_t n, int64_t n0, c
         if ((e = b->ensure(g.npad))) return c->cuda_fail(e, "flat columns");
     if ((e = g.n0.ensure(1))) return c->cuda_fail(e, "n0");
     if (mixed && ((e = g.geo.ensure(g.npad)) || (e = g.ecl.ensure(g.npad)) ||
-                  (e = g.pos.ensure(g.npad))))
+                  (e = g.pos.ensure(g.npad)) ||
+                  (e = g.runs.ensure(kRunRecs * g.npad / kRunFaces))))
         return c->cuda_fail(e, "packed grid");
     const double *src[] = {dx, dy, dz, px, py, pz, flux};
     for (int k = 0; k < 7; k++)
@@ -1443,7 +1444,10 @@ lcg_status lcg_sum_star_multi(lcg_ctx *c, int32_t star, int64_t n, int64_t n0, c
         cudaMemcpyAsync(g.fout.p + n0, out1, (size_t)(n - n0) * 8, cudaMemcpyHostToDevice, c->stream);
     }
     cudaMemcpyAsync(g.n0.p, &n0, sizeof(int64_t), cudaMemcpyHostToDevice, c->stream);
-    if (mixed) launch_pack_flat(g.flat(), n0, need_pos, c->stream);
+    if (mixed) {
+        launch_pack_flat(g.flat(), n0, need_pos, c->stream);
+        launch_run_bounds_geo(g.flat(), c->stream);
+    }
     if ((e = c->pex.ensure(nent)) || (e = c->pey.ensure(nent)) || (e = c->pez.ensure(nent)) ||
         (e = c->pphin.ensure(nent)) || (e = c->pef.ensure(nent)) || (e = c->ppfx.ensure(nent)))
         return c->cuda_fail(e, "phases");

@@ -119,8 +119,8 @@ struct FlatDev {
     // with cz = cos(i) nz and f_k = flux * p_k, so each float2 operand of the
     // packed FP32x2 arithmetic is an aligned register pair
     float *fp;
-    // bounds of every 64 consecutive faces of fp (a run) and of its four parts of
-    // 16: kRunRecs records per run, the run's first
+    // bounds of every 64 consecutive faces of fp (of geo with nz for the z term)
+    // and of their four parts of 16: kRunRecs records per run, the run's first
     RunRec *runs;
     // faces with two or more eclipse ranges (opaque discs) sit last, in
     // [*n1, n): their records above are zero (they add nothing to the main
@@ -326,6 +326,8 @@ void launch_pack_flat(FlatDev f, int64_t n0, int need_pos, cudaStream_t s);
 // run records of npairs pairs of fast records (and their eclipse ranges)
 void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, RunRec *runs,
                        cudaStream_t s);
+// run records of f.n faces of general records (cmin, cmax: the extremes of nz)
+void launch_run_bounds_geo(const FlatDev &f, cudaStream_t s);
 void launch_batch_run_bounds(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_pack_phases(PhaseDev ph, cudaStream_t s);
 

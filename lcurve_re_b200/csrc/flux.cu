@@ -59,28 +59,80 @@ __device__ __forceinline__ float magnification(float4 s, float ex, float ey, flo
     return (float)(pd * pd / (pd - ph) / ph / 4.0);
 }
 
+// The warp's phase arc: every entry of the warp lies in [A, A + L] (mod 2^64),
+// A its first lane's first entry. For time-ordered points it is a short arc of
+// the orbit; in any order it still holds every entry.
+template <int PPT>
+__device__ __forceinline__ void warp_arc(const unsigned long long *pf, unsigned long long &A,
+                                         unsigned long long &L) {
+    A = __shfl_sync(0xffffffffu, pf[0], 0);
+    unsigned long long l = 0ull;
+#pragma unroll
+    for (int j = 0; j < PPT; j++) {
+        const unsigned long long d = pf[j] - A;
+        if (d > l) l = d;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, l, o);
+        l = t > l ? t : l;
+    }
+    L = l;
+}
+
+// What the warp knows of a group of faces: which of its entries could see it
+// and whether a range could hide it (warp-uniform).
+enum { kGroupDark = 0, kGroupBright = 1, kGroupSigns = 2, kGroupRanges = 3 };
+
+// The arc [A, A + L] of the warp's phases against a group's ranges, exact on the
+// circle: all faces hidden throughout it, some range meeting it, or none.
+__device__ __forceinline__ int arc_class(const RunRec &R, unsigned long long A,
+                                         unsigned long long L) {
+    const ulonglong2 H = R.hull;
+    if (!(H.y == ~0ull || (H.y != 0ull && ((H.x - A) <= L || (A - H.x) < H.y))))
+        return kGroupSigns;
+    const unsigned long long o = A - R.all.x;
+    return o < R.all.y && L < R.all.y - o ? kGroupDark : kGroupRanges;
+}
+
 struct FaceConsts {
     float c1, c2, c3, c4, base, cut, mucrit, vfac, spin, xcofm, beam;
     double rlens1;
 };
 
-// Sums faces [lo, hi) of the staged chunk (first face c0) into acc, in FP32
-// runs of kFold faces folded into FP64.
-template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
-__device__ __forceinline__ void sweep(const float4 *sgeo, const ulonglong2 *secl,
-                                      const float4 *spos, int64_t c0, int64_t lo, int64_t hi,
-                                      const float *ex, const float *ey, const float *ez,
-                                      const unsigned long long *pf,
-                                      const FaceConsts &k, double *acc) {
-    constexpr bool need_pos = BEAM || GLENS;
-    for (int64_t b = lo; b < hi; b += kFold) {
-        const int cnt = (int)((b + kFold < hi) ? kFold : hi - b);
-        const float4 *gp = sgeo + (b - c0);
-        const ulonglong2 *ep = secl + (b - c0);
-        const float4 *pp4 = spos + (b - c0);
-        float s[PPT];
+// What a run of faces is to a warp's entries in the general sweep (group_class
+// for the fast one): kGroupDark when mu cannot exceed the threshold at any of
+// them or all of its faces are eclipsed, else whether ranges need testing. The
+// record bounds nz, each entry has its own ez; 2e-6 covers the rounding of both
+// sides.
+template <int PPT, bool ECL>
+__device__ __forceinline__ int run_class(const RunRec &R, float cut, const float *ex,
+                                         const float *ey, const float *ez,
+                                         unsigned long long A, unsigned long long L) {
+    const float4 B = *reinterpret_cast<const float4 *>(&R);
+    const float zmin = R.cmin;
+    bool some = false;
 #pragma unroll
-        for (int j = 0; j < PPT; j++) s[j] = 0.f;
+    for (int j = 0; j < PPT; j++) {
+        const float e = sqrtf(fmaf(ex[j], ex[j], ey[j] * ey[j]));
+        const float z = fmaxf(ez[j] * B.w, ez[j] * zmin);
+        some = some ||
+               fmaf(ex[j], B.x, fmaf(ey[j], B.y, fmaf(e, B.z, z))) + 2e-6f >= cut;
+    }
+    if (!__any_sync(0xffffffffu, some)) return kGroupDark;
+    if constexpr (ECL) return arc_class(R, A, L);
+    return kGroupSigns;
+}
+
+// One fold of cnt faces into the entries' FP32 sums, element by element.
+template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
+__device__ __forceinline__ void fold_faces(const float4 *gp, const ulonglong2 *ep,
+                                           const float4 *pp4, int cnt, const float *ex,
+                                           const float *ey, const float *ez,
+                                           const unsigned long long *pf, const FaceConsts &k,
+                                           float *s) {
+    constexpr bool need_pos = BEAM || GLENS;
+    {
 #pragma unroll 4
         for (int i = 0; i < cnt; i++) {
             const float4 g = gp[i];
@@ -115,6 +167,40 @@ __device__ __forceinline__ void sweep(const float4 *sgeo, const ulonglong2 *secl
                 s[j] = vis ? fmaf(v, g.w, s[j]) : s[j];
             }
         }
+    }
+}
+
+// Sums faces [lo, hi) of the staged chunk (first face c0) into acc, in FP32
+// runs of kFold faces folded into FP64. A warp skips a fold whose run (or two
+// runs, where it straddles them) is dark to it, and tests ranges only where they
+// reach its arc of phases; what it leaves out are exact zeros.
+template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
+__device__ __forceinline__ void sweep(const float4 *sgeo, const ulonglong2 *secl,
+                                      const float4 *spos, const RunRec *__restrict__ runs,
+                                      int64_t c0, int64_t lo, int64_t hi, const float *ex,
+                                      const float *ey, const float *ez,
+                                      const unsigned long long *pf, unsigned long long A,
+                                      unsigned long long L, const FaceConsts &k, double *acc) {
+    const float cut = BEAM ? k.mucrit : k.cut;
+    for (int64_t b = lo; b < hi; b += kFold) {
+        const int cnt = (int)((b + kFold < hi) ? kFold : hi - b);
+        const int64_t r0 = b / kRunFaces, r1 = (b + cnt - 1) / kRunFaces;
+        int c = run_class<PPT, ECL>(runs[kRunRecs * r0], cut, ex, ey, ez, A, L);
+        if (r1 != r0) {
+            const int c1 = run_class<PPT, ECL>(runs[kRunRecs * r1], cut, ex, ey, ez, A, L);
+            // one of the two may be dark for its ranges: test each face's
+            if (c != c1) c = ECL ? kGroupRanges : kGroupSigns;
+        }
+        if (c == kGroupDark) continue;
+        const float4 *gp = sgeo + (b - c0), *pp4 = spos + (b - c0);
+        const ulonglong2 *ep = secl + (b - c0);
+        float s[PPT];
+#pragma unroll
+        for (int j = 0; j < PPT; j++) s[j] = 0.f;
+        if (ECL && c == kGroupRanges)
+            fold_faces<PPT, LT, BEAM, GLENS, STAR, ECL>(gp, ep, pp4, cnt, ex, ey, ez, pf, k, s);
+        else
+            fold_faces<PPT, LT, BEAM, GLENS, STAR, false>(gp, ep, pp4, cnt, ex, ey, ez, pf, k, s);
 #pragma unroll
         for (int j = 0; j < PPT; j++) acc[j] += (double)s[j];
     }
@@ -147,24 +233,22 @@ __global__ void __launch_bounds__(kThreads)
         if (need_pos) bulk_g2s(spos, f.pos + c0, (uint32_t)(chunk * 16), &bar);
     }
 
-    // phase entries of this thread, loaded while the faces stream in
+    // phase entries of this thread, loaded while the faces stream in: PPT
+    // consecutive ones, so that a warp holds a narrow arc; threads past the last
+    // entry repeat it
     float ex[PPT], ey[PPT], ez[PPT];
-    unsigned long long pf[PPT];
-    const int64_t ebase = (int64_t)blockIdx.x * kThreads * PPT + tid;
+    unsigned long long pf[PPT], A, L;
+    const int64_t ebase = ((int64_t)blockIdx.x * kThreads + tid) * PPT;
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
-        const int64_t e = ebase + (int64_t)j * kThreads;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        unsigned long long p = 0ull;
-        if (e < ph.nent) {
-            v = ph.ef[e];
-            p = ph.pfx[e];
-        }
+        const int64_t e = ebase + j < ph.nent ? ebase + j : ph.nent - 1;
+        const float4 v = ph.ef[e];
         ex[j] = v.x;
         ey[j] = v.y;
         ez[j] = v.z;
-        pf[j] = p;
+        pf[j] = ph.pfx[e];
     }
+    warp_arc<PPT>(pf, A, L);
     const float c1 = (float)k.c[0], c2 = (float)k.c[1], c3 = (float)k.c[2], c4 = (float)k.c[3];
     const float base = (float)k.base;
     const float cut = (float)(k.mucrit > 0. ? k.mucrit : 0.);
@@ -186,13 +270,13 @@ __global__ void __launch_bounds__(kThreads)
     const FaceConsts fc{c1, c2, c3, c4, base, cut, (float)k.mucrit, vfac, spin, xcofm, beam,
                         k.rlens1};
     // plain faces [c0, min(n0,cend)), then one-range faces [max(n0,c0), cend)
-    sweep<PPT, LT, BEAM, GLENS, STAR, false>(sgeo, secl, spos, c0, c0, n0 < cend ? n0 : cend,
-                                            ex, ey, ez, pf, fc, acc);
-    sweep<PPT, LT, BEAM, GLENS, STAR, true>(sgeo, secl, spos, c0, n0 > c0 ? n0 : c0, cend, ex,
-                                           ey, ez, pf, fc, acc);
+    sweep<PPT, LT, BEAM, GLENS, STAR, false>(sgeo, secl, spos, f.runs, c0, c0,
+                                            n0 < cend ? n0 : cend, ex, ey, ez, pf, A, L, fc, acc);
+    sweep<PPT, LT, BEAM, GLENS, STAR, true>(sgeo, secl, spos, f.runs, c0, n0 > c0 ? n0 : c0, cend,
+                                           ex, ey, ez, pf, A, L, fc, acc);
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
-        const int64_t e = ebase + (int64_t)j * kThreads;
+        const int64_t e = ebase + j;
         if (e < ph.nent) part[(int64_t)blockIdx.y * ldp + e] = acc[j];
     }
 }
@@ -255,31 +339,6 @@ void launch_ppt(int star, const FluxConsts &k, const FlatDev &f, const PhaseDev 
 // are bit-identical to evaluating them.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
-// The warp's phase arc: every entry of the warp lies in [A, A + L] (mod 2^64),
-// A its first lane's first entry. For time-ordered points it is a short arc of
-// the orbit; in any order it still holds every entry.
-template <int PPT>
-__device__ __forceinline__ void warp_arc(const unsigned long long *pf, unsigned long long &A,
-                                         unsigned long long &L) {
-    A = __shfl_sync(0xffffffffu, pf[0], 0);
-    unsigned long long l = 0ull;
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const unsigned long long d = pf[j] - A;
-        if (d > l) l = d;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, l, o);
-        l = t > l ? t : l;
-    }
-    L = l;
-}
-
-// What the warp knows of a group of faces: which of its entries could see it
-// and whether a range could hide it (warp-uniform).
-enum { kGroupDark = 0, kGroupBright = 1, kGroupSigns = 2, kGroupRanges = 3 };
-
 // Dark: every face turned away, or eclipsed, at all the warp's entries: exact
 // zeros. Bright: every face visible and none eclipsed: no sign or range to
 // test. Signs: signs to test, no range. Ranges: both.
@@ -297,17 +356,9 @@ __device__ __forceinline__ int group_class(const RunRec &R, const float2 *ex, co
         every = every && fmaf(-exy[j], B.z, d + cmin) > 0.f;
     }
     if (!__any_sync(0xffffffffu, some)) return kGroupDark;
-    bool ranges = false;
     if constexpr (ECL) {
-        // the arc [A, A + L] of the warp's phases against the group's: exact on
-        // the circle
-        const ulonglong2 H = R.hull;
-        ranges = H.y == ~0ull || (H.y != 0ull && ((H.x - A) <= L || (A - H.x) < H.y));
-        if (ranges) {
-            const unsigned long long o = A - R.all.x;
-            if (o < R.all.y && L < R.all.y - o) return kGroupDark;
-            return kGroupRanges;
-        }
+        const int c = arc_class(R, A, L);
+        if (c != kGroupSigns) return c;
     }
     return __all_sync(0xffffffffu, every) ? kGroupBright : kGroupSigns;
 }

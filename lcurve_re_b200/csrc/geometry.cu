@@ -1075,25 +1075,13 @@ __device__ __forceinline__ void set_arcs(RunRec &R, unsigned long long ref, long
     }
 }
 
-// The records of one run (RunRec), one warp per run, lane l reading pair l:
-// the four parts of 8 lanes first, then the run.
-__device__ __forceinline__ void run_bound(const float *__restrict__ fp,
-                                          const ulonglong2 *__restrict__ ecl, int64_t npairs,
-                                          int64_t run, RunRec *out) {
+// The records of one run (RunRec), one warp per run, lane l holding pair l
+// (normals, the z term cz, eclipse ranges): the four parts of 8 lanes first, then
+// the run.
+__device__ __forceinline__ void run_records(const float *nx, const float *ny, const float *cz,
+                                            const bool *use, ulonglong2 *E, RunRec *out) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int64_t q = run * 32 + lane;
-    float nx[2] = {0.f, 0.f}, ny[2] = {0.f, 0.f}, cz[2] = {0.f, 0.f};
-    ulonglong2 E[2] = {make_ulonglong2(0ull, 0ull), make_ulonglong2(0ull, 0ull)};
-    bool use[2] = {false, false};
-    if (q < npairs) {
-        const float4 P0 = reinterpret_cast<const float4 *>(fp)[4 * q];
-        const float4 P1 = reinterpret_cast<const float4 *>(fp)[4 * q + 1];
-        nx[0] = P0.x; nx[1] = P0.y; ny[0] = P0.z; ny[1] = P0.w; cz[0] = P1.x; cz[1] = P1.y;
-        for (int k = 0; k < 2; k++) use[k] = nx[k] != 0.f || ny[k] != 0.f || cz[k] != 0.f;
-        E[0] = ecl[2 * q];
-        E[1] = ecl[2 * q + 1];
-    }
     RunRec part, whole_run;
     group_mu<8>(nx, ny, cz, use, part);
     group_mu<32>(nx, ny, cz, use, whole_run);
@@ -1139,6 +1127,45 @@ __device__ __forceinline__ void run_bound(const float *__restrict__ fp,
     set_arcs(whole_run, ref, lo, hi, lo2, hi2, whole, bare);
     if ((lane & 7) == 0) out[1 + (lane >> 3)] = part;
     if (lane == 0) out[0] = whole_run;
+}
+
+// From the fast records: cz = cos(i) nz.
+__device__ __forceinline__ void run_bound(const float *__restrict__ fp,
+                                          const ulonglong2 *__restrict__ ecl, int64_t npairs,
+                                          int64_t run, RunRec *out) {
+    const int64_t q = run * 32 + (threadIdx.x & 31);
+    float nx[2] = {0.f, 0.f}, ny[2] = {0.f, 0.f}, cz[2] = {0.f, 0.f};
+    ulonglong2 E[2] = {make_ulonglong2(0ull, 0ull), make_ulonglong2(0ull, 0ull)};
+    bool use[2] = {false, false};
+    if (q < npairs) {
+        const float4 P0 = reinterpret_cast<const float4 *>(fp)[4 * q];
+        const float4 P1 = reinterpret_cast<const float4 *>(fp)[4 * q + 1];
+        nx[0] = P0.x; nx[1] = P0.y; ny[0] = P0.z; ny[1] = P0.w; cz[0] = P1.x; cz[1] = P1.y;
+        for (int k = 0; k < 2; k++) use[k] = nx[k] != 0.f || ny[k] != 0.f || cz[k] != 0.f;
+        E[0] = ecl[2 * q];
+        E[1] = ecl[2 * q + 1];
+    }
+    run_records(nx, ny, cz, use, E, out);
+}
+
+// From the general records (nx, ny, nz, flux) of n faces: cz = nz, the sweep
+// multiplies by each entry's ez.
+__global__ void k_run_bounds_geo(const float4 *__restrict__ geo,
+                                 const ulonglong2 *__restrict__ ecl, int64_t n, RunRec *runs) {
+    const int64_t run = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (run >= (n + kRunFaces - 1) / kRunFaces) return;  // whole warps
+    const int64_t i = run * kRunFaces + 2 * (threadIdx.x & 31);
+    float nx[2] = {0.f, 0.f}, ny[2] = {0.f, 0.f}, cz[2] = {0.f, 0.f};
+    ulonglong2 E[2] = {make_ulonglong2(0ull, 0ull), make_ulonglong2(0ull, 0ull)};
+    bool use[2] = {false, false};
+    for (int k = 0; k < 2; k++) {
+        if (i + k >= n) continue;
+        const float4 g = geo[i + k];
+        nx[k] = g.x; ny[k] = g.y; cz[k] = g.z;
+        use[k] = g.x != 0.f || g.y != 0.f || g.z != 0.f;
+        E[k] = ecl[i + k];
+    }
+    run_records(nx, ny, cz, use, E, runs + kRunRecs * run);
 }
 
 __global__ void k_run_bounds(const float *__restrict__ fp, const ulonglong2 *__restrict__ ecl,
@@ -1678,6 +1705,7 @@ void launch_flatten(GridDev g, FlatDev f, const int32_t *cnt, int mixed, int nee
         g, f, cnt, (int32_t)cont_blocks(g.n), mixed, need_pos, fc);
     count_launch();
     if (mixed && fc.on) launch_run_bounds(f.fp, f.ecl, f.npad / 2, f.runs, s);
+    else if (mixed) launch_run_bounds_geo(f, s);
 }
 
 void launch_phases(const PhaseParams &p, const DatumRec *data, const int64_t *off, int32_t n,
@@ -1727,6 +1755,13 @@ void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, R
     const int64_t nruns = (npairs + 31) / 32;
     if (nruns <= 0) return;
     k_run_bounds<<<nblocks(nruns * 32, 256), 256, 0, s>>>(fp, ecl, npairs, runs);
+    count_launch();
+}
+
+void launch_run_bounds_geo(const FlatDev &f, cudaStream_t s) {
+    const int64_t nruns = (f.n + kRunFaces - 1) / kRunFaces;
+    if (nruns <= 0) return;
+    k_run_bounds_geo<<<nblocks(nruns * 32, 256), 256, 0, s>>>(f.geo, f.ecl, f.n, f.runs);
     count_launch();
 }
 

@@ -48,3 +48,21 @@ def test_opaque_disc_sums_do_not_depend_on_the_warp():
         a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
         b = e.light_curve_comp(m, d[perm], scale=False, rdata=False, diagnostics=False)[0]
     np.testing.assert_array_equal(a[perm], b)
+
+
+# the general sweep: beaming, a limb cut-off, lensing, both laws
+@pytest.mark.parametrize("over,npts", [
+    (dict(nlat1f=20, nlat2f=41, beam_factor1=1.3, beam_factor2=1.6), 1000),
+    (dict(nlat1f=33, nlat2f=90, beam_factor1=1.3, limb2="Poly"), 2500),
+    (dict(nlat1f=60, nlat2f=30, mucrit1=0.1, mucrit2=0.2), 700),
+    (dict(nlat1f=30, nlat2f=40, glens1=1, roche1=0, eclipse2=0, beam_factor1=1.0), 400),
+    (dict(nlat1f=25, nlat2f=31, beam_factor1=1.3, mucrit1=-0.5), 17)])
+@pytest.mark.parametrize("span", [{}, ECLIPSE])
+def test_general_sums_do_not_depend_on_the_warp(over, npts, span):
+    m = W.model(**over)
+    d = W.data(npts, **span)
+    perm = np.random.default_rng(npts).permutation(npts)
+    with Engine(precision="mixed") as e:
+        a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
+        b = e.light_curve_comp(m, d[perm], scale=False, rdata=False, diagnostics=False)[0]
+    np.testing.assert_array_equal(a[perm], b)
