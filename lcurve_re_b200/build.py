@@ -37,7 +37,7 @@ SOURCES = {
     "walk.cu": ["--fmad=false"],
 }
 HEADERS = ["roche.cuh", "eclipse.cuh", "disc.cuh", "ecl_root.cuh", "engine.h", "tma.cuh",
-           "context.h", "fixed_phase.cuh", "mlp_tc.cuh"]
+           "context.h", "fixed_phase.cuh", "flux_groups.cuh", "mlp_tc.cuh"]
 
 
 def nvcc():

@@ -122,9 +122,9 @@ struct Grid {
         if (e) return e;
         if (disc && ((e = ridx.ensure(n)) || (e = rn.ensure(n)) || (e = rr.ensure(kRagRanges * n))))
             return e;
+        if ((e = runs.ensure(kRunRecs * npad / kRunFaces))) return e;
         if (mixed) {
             if ((e = ecl.ensure(npad))) return e;
-            if ((e = runs.ensure(kRunRecs * npad / kRunFaces))) return e;
             if (fast_on) {
                 if ((e = fp.ensure(8 * npad))) return e;
             } else if ((e = geo.ensure(npad))) {

@@ -535,7 +535,7 @@ lcg_status sweep_one(lcg_ctx *c, const lcg_model &m, Grid &g, int star, double p
     PhaseDev ph{c->pex.p, c->pey.p, c->pez.p, c->pphin.p, nullptr, nullptr, c->pef.p, nullptr, 1,
                 c->ppfx.p};
     const int mixed = c->precision == LCG_PREC_MIXED;
-    if (mixed) launch_pack_phases(ph, c->stream);
+    launch_pack_phases(ph, c->stream);
     FluxPlan plan = plan_flux(mixed, g.fast, g.n, 1, c->nsm);
     if ((err = c->part1f.ensure((size_t)std::max<int64_t>(plan.nchunk, 1) * 4)))
         return c->cuda_fail(err, "partials");
@@ -1430,9 +1430,9 @@ lcg_status lcg_sum_star_multi(lcg_ctx *c, int32_t star, int64_t n, int64_t n0, c
     for (auto *b : cols)
         if ((e = b->ensure(g.npad))) return c->cuda_fail(e, "flat columns");
     if ((e = g.n0.ensure(1))) return c->cuda_fail(e, "n0");
+    if ((e = g.runs.ensure(kRunRecs * g.npad / kRunFaces))) return c->cuda_fail(e, "run records");
     if (mixed && ((e = g.geo.ensure(g.npad)) || (e = g.ecl.ensure(g.npad)) ||
-                  (e = g.pos.ensure(g.npad)) ||
-                  (e = g.runs.ensure(kRunRecs * g.npad / kRunFaces))))
+                  (e = g.pos.ensure(g.npad))))
         return c->cuda_fail(e, "packed grid");
     const double *src[] = {dx, dy, dz, px, py, pz, flux};
     for (int k = 0; k < 7; k++)
@@ -1447,6 +1447,8 @@ lcg_status lcg_sum_star_multi(lcg_ctx *c, int32_t star, int64_t n, int64_t n0, c
     if (mixed) {
         launch_pack_flat(g.flat(), n0, need_pos, c->stream);
         launch_run_bounds_geo(g.flat(), c->stream);
+    } else {
+        launch_run_bounds64(g.flat(), c->stream);
     }
     if ((e = c->pex.ensure(nent)) || (e = c->pey.ensure(nent)) || (e = c->pez.ensure(nent)) ||
         (e = c->pphin.ensure(nent)) || (e = c->pef.ensure(nent)) || (e = c->ppfx.ensure(nent)))
@@ -1459,7 +1461,7 @@ lcg_status lcg_sum_star_multi(lcg_ctx *c, int32_t star, int64_t n, int64_t n0, c
     }
     PhaseDev ph{c->pex.p, c->pey.p, c->pez.p, c->pphin.p, nullptr, nullptr, c->pef.p, nullptr, nent,
                 c->ppfx.p};
-    if (mixed) launch_pack_phases(ph, c->stream);
+    launch_pack_phases(ph, c->stream);
     FluxConsts k{};
     for (int i = 0; i < 4; i++) k.c[i] = ldc[i];
     k.base = 1.0 - (ldc[0] + ldc[1] + ldc[2] + ldc[3]);

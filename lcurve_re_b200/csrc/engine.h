@@ -328,6 +328,8 @@ void launch_run_bounds(const float *fp, const ulonglong2 *ecl, int64_t npairs, R
                        cudaStream_t s);
 // run records of f.n faces of general records (cmin, cmax: the extremes of nz)
 void launch_run_bounds_geo(const FlatDev &f, cudaStream_t s);
+// the same of the FP64 columns
+void launch_run_bounds64(const FlatDev &f, cudaStream_t s);
 void launch_batch_run_bounds(const BatchDev &b, int nsm, cudaStream_t s);
 void launch_pack_phases(PhaseDev ph, cudaStream_t s);
 

@@ -19,6 +19,7 @@
 //    mod 2^64 >= width + 1 (ecl_fx64, geometry.cu), the reference's double
 //    comparisons decision for decision.
 #include "engine.h"
+#include "flux_groups.cuh"
 #include "tma.cuh"
 
 namespace lcg {
@@ -57,42 +58,6 @@ __device__ __forceinline__ float magnification(float4 s, float ex, float ey, flo
     const double ph = 0.5 * p, rd = rlens1 * d;
     const double pd = (ph * ph > 25.0 * rd) ? p + rd / p : ph + sqrt(ph * ph + rd);
     return (float)(pd * pd / (pd - ph) / ph / 4.0);
-}
-
-// The warp's phase arc: every entry of the warp lies in [A, A + L] (mod 2^64),
-// A its first lane's first entry. For time-ordered points it is a short arc of
-// the orbit; in any order it still holds every entry.
-template <int PPT>
-__device__ __forceinline__ void warp_arc(const unsigned long long *pf, unsigned long long &A,
-                                         unsigned long long &L) {
-    A = __shfl_sync(0xffffffffu, pf[0], 0);
-    unsigned long long l = 0ull;
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const unsigned long long d = pf[j] - A;
-        if (d > l) l = d;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, l, o);
-        l = t > l ? t : l;
-    }
-    L = l;
-}
-
-// What the warp knows of a group of faces: which of its entries could see it
-// and whether a range could hide it (warp-uniform).
-enum { kGroupDark = 0, kGroupBright = 1, kGroupSigns = 2, kGroupRanges = 3 };
-
-// The arc [A, A + L] of the warp's phases against a group's ranges, exact on the
-// circle: all faces hidden throughout it, some range meeting it, or none.
-__device__ __forceinline__ int arc_class(const RunRec &R, unsigned long long A,
-                                         unsigned long long L) {
-    const ulonglong2 H = R.hull;
-    if (!(H.y == ~0ull || (H.y != 0ull && ((H.x - A) <= L || (A - H.x) < H.y))))
-        return kGroupSigns;
-    const unsigned long long o = A - R.all.x;
-    return o < R.all.y && L < R.all.y - o ? kGroupDark : kGroupRanges;
 }
 
 struct FaceConsts {

@@ -11,6 +11,7 @@
 // A CTA owns one 1024-face block and a tile of phase entries; the block's
 // SoA columns are staged into shared memory by bulk TMA copies.
 #include "engine.h"
+#include "flux_groups.cuh"
 #include "tma.cuh"
 
 namespace lcg {
@@ -86,6 +87,151 @@ __device__ __forceinline__ double elem_mu(double mu, double ex, double ey, doubl
     return (double)(mu > L.mucrit) * val;
 }
 
+// A warp's entries for the group tests: earth vectors in FP32 with the length of
+// their xy part, and the phase arc.
+template <int PPT>
+struct Arc64 {
+    float ex[PPT], ey[PPT], ez[PPT], exy[PPT];
+    unsigned long long A, L;
+};
+
+// What a group of faces is to a warp's entries (flux_groups.cuh): dark when mu is
+// at or below zb, or every face eclipsed, at all of them; bright when mu lies
+// above zb for every face and entry and no range reaches the warp's arc. The
+// bounds are FP32; 2e-6 covers the rounding for vectors of length one. Longer
+// ones and NaN come as NaN, which is neither dark nor bright.
+template <int PPT, bool ECL>
+__device__ __forceinline__ int group64(const RunRec &R, float zb, const Arc64<PPT> &W) {
+    bool some = false, every = true;
+#pragma unroll
+    for (int j = 0; j < PPT; j++) {
+        const float d = W.ex[j] * R.ax + W.ey[j] * R.ay, q = W.exy[j] * R.r;
+        const float z0 = W.ez[j] * R.cmin, z1 = W.ez[j] * R.cmax;
+        some |= !(q + d + fmaxf(z0, z1) + 2e-6f < zb);
+        every &= d - q + fminf(z0, z1) - 2e-6f > zb;
+    }
+    if (!__any_sync(0xffffffffu, some)) return kGroupDark;
+    if constexpr (ECL) {
+        const int c = arc_class(R, W.A, W.L);
+        if (c != kGroupSigns) return c;
+    }
+    return __all_sync(0xffffffffu, every) ? kGroupBright : kGroupSigns;
+}
+
+struct Cols64 {  // a staged block's columns
+    const double *dx, *dy, *dz, *fl, *in, *out, *px, *py, *pz;
+};
+
+// Faces [t0, t1) of the block, every one visible at every entry (no beaming, no
+// lensing): s1_elem / s2_elem without the factors that are one there, (mu > 0)
+// and (mu > mucrit).
+template <int PPT, int LT>
+__device__ __forceinline__ void bright64(const Cols64 &C, int t0, int t1, const double *ex,
+                                         const double *ey, const double *ez, const Consts64 &L,
+                                         double *br) {
+    for (int t = t0; t < t1; t++) {
+        const double dx = C.dx[t], dy = C.dy[t], dz = C.dz[t], fl = C.fl[t];
+#pragma unroll
+        for (int j = 0; j < PPT; j++) {
+            const double mu = mu_of(ex[j], ey[j], ez[j], dx, dy, dz);
+            const double m = (1.0 < mu) ? 1.0 : mu;
+            double im;
+            if constexpr (LT == 0) {
+                const double om = 1.0 - m;
+                im = 1.0 - om * (L.c1 + om * (L.c2 + om * (L.c3 + om * L.c4)));
+            } else {
+                const double msq = sqrt(m);
+                im = L.base + msq * (L.c1 + msq * (L.c2 + msq * (L.c3 + msq * L.c4)));
+            }
+            br[j] += mu * fl * im;
+        }
+    }
+}
+
+// The same faces with every factor, and the range when ECL. Per face, one vote
+// of the warp: at or below zb (exactly zero) or eclipsed at every entry of the
+// warp, its elements would add exact zeros, and the warp moves on.
+template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
+__device__ __forceinline__ void faces64(const Cols64 &C, int t0, int t1,
+                                        const double *ex, const double *ey, const double *ez,
+                                        const double *pn, double zb, const Consts64 &L,
+                                        double *br) {
+    constexpr bool need_pos = BEAM || GLENS;
+    for (int t = t0; t < t1; t++) {
+        const double dx = C.dx[t], dy = C.dy[t], dz = C.dz[t];
+        double ein = 0., eout = 0.;
+        if constexpr (ECL) { ein = C.in[t]; eout = C.out[t]; }
+        double mu[PPT];
+        bool ecl[PPT], live = false;
+#pragma unroll
+        for (int j = 0; j < PPT; j++) {
+            mu[j] = mu_of(ex[j], ey[j], ez[j], dx, dy, dz);
+            ecl[j] = ECL && ((pn[j] >= ein && pn[j] <= eout) || pn[j] <= eout - 1.0);
+            live |= (mu[j] > zb) && !ecl[j];
+        }
+        if (!__any_sync(0xffffffffu, live)) continue;
+        const double fl = C.fl[t];
+        double px = 0., py = 0., pz = 0.;
+        if constexpr (need_pos) { px = C.px[t]; py = C.py[t]; pz = C.pz[t]; }
+#pragma unroll
+        for (int j = 0; j < PPT; j++) {
+            const double v = elem_mu<LT, BEAM, GLENS, STAR>(mu[j], ex[j], ey[j], ez[j], dx, dy,
+                                                            px, py, pz, fl, L);
+            br[j] += ecl[j] ? 0.0 : v;
+        }
+    }
+}
+
+// Faces [t0, t1) of the block by groups: a run of 64, and its parts of 16 where
+// the run is neither dark nor bright.
+template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
+__device__ __forceinline__ void segment64(const Cols64 &C, const RunRec *sr, int t0,
+                                          int t1, const double *ex, const double *ey,
+                                          const double *ez, const double *pn,
+                                          const Arc64<PPT> &W, double zb, const Consts64 &L,
+                                          double *br) {
+    constexpr bool plain = !BEAM && !GLENS;
+    for (int t = t0; t < t1;) {
+        const int run = t / kRunFaces;
+        const int re = (run + 1) * kRunFaces < t1 ? (run + 1) * kRunFaces : t1;
+        const int c = group64<PPT, ECL>(sr[kRunRecs * run], (float)zb, W);
+        if (c == kGroupDark) {
+            t = re;
+            continue;
+        }
+        if constexpr (plain) {
+            if (c == kGroupBright) {
+                bright64<PPT, LT>(C, t, re, ex, ey, ez, L, br);
+                t = re;
+                continue;
+            }
+        }
+#pragma unroll 1
+        while (t < re) {
+            const int part = t / 16, pe = (part + 1) * 16 < re ? (part + 1) * 16 : re;
+            const int cp = group64<PPT, ECL>(sr[kRunRecs * run + 1 + (part & 3)], (float)zb, W);
+            bool done = cp == kGroupDark;
+            if constexpr (plain) {
+                if (cp == kGroupBright) {
+                    bright64<PPT, LT>(C, t, pe, ex, ey, ez, L, br);
+                    done = true;
+                }
+            }
+            if (!done) {
+                if (ECL && cp == kGroupRanges)
+                    faces64<PPT, LT, BEAM, GLENS, STAR, ECL>(C, t, pe, ex, ey, ez, pn, zb, L, br);
+                else
+                    faces64<PPT, LT, BEAM, GLENS, STAR, false>(C, t, pe, ex, ey, ez, pn, zb, L, br);
+            }
+            t = pe;
+        }
+    }
+}
+
+// Skipped or not, classified or not, every sum is bit-identical: what is left
+// out are exact zeros and factors of one, and the faces keep their order. FP64
+// issue bounds it (some 35 instructions for a visible element, 12 of them the
+// square root): star 2 of 100/200 strips over 15,000 entries 1.75 -> 1.49 ms.
 template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
 __global__ void __launch_bounds__(kThreads64)
     k_flux64(FluxConsts k, FlatDev f, PhaseDev ph, double *part, int64_t ldp, DevStatus *st) {
@@ -96,20 +242,20 @@ __global__ void __launch_bounds__(kThreads64)
     const int64_t lo = (int64_t)blockIdx.y * kBlock;
     const int64_t n = f.n, n0 = *f.n0;
     const int64_t hi = (lo + kBlock < n) ? lo + kBlock : n;
-    const int64_t a1 = hi < n0 ? hi : n0;  // plain segment [lo, a1)
-    const int64_t b0 = lo > n0 ? lo : n0;  // one-range segment [b0, hi)
     const bool need_ecl = hi > n0;
-    double *s_dx = reinterpret_cast<double *>(smem);
+    constexpr uint32_t col = kBlock * 8, rec = kBlock / kRunFaces * kRunRecs * sizeof(RunRec);
+    RunRec *sr = reinterpret_cast<RunRec *>(smem);
+    double *s_dx = reinterpret_cast<double *>(smem + rec);
     double *s_dy = s_dx + kBlock, *s_dz = s_dy + kBlock, *s_fl = s_dz + kBlock;
     double *s_in = s_fl + kBlock, *s_out = s_in + kBlock;
     double *s_px = s_out + kBlock, *s_py = s_px + kBlock, *s_pz = s_py + kBlock;
-    constexpr uint32_t col = kBlock * 8;
 
     if (tid == 0) mbar_init(&bar, 1);
     __syncthreads();
     if (tid == 0) {
-        uint32_t bytes = 4 * col + (need_ecl ? 2 * col : 0u) + (need_pos ? 3 * col : 0u);
+        uint32_t bytes = rec + 4 * col + (need_ecl ? 2 * col : 0u) + (need_pos ? 3 * col : 0u);
         mbar_arrive_expect_tx(&bar, bytes);
+        bulk_g2s(sr, f.runs + kRunRecs * (lo / kRunFaces), rec, &bar);
         bulk_g2s(s_dx, f.dx + lo, col, &bar);
         bulk_g2s(s_dy, f.dy + lo, col, &bar);
         bulk_g2s(s_dz, f.dz + lo, col, &bar);
@@ -124,18 +270,29 @@ __global__ void __launch_bounds__(kThreads64)
             bulk_g2s(s_pz, f.pz + lo, col, &bar);
         }
     }
+    // PPT consecutive entries a thread, so that a warp holds a narrow arc; threads
+    // past the last entry repeat it
     double ex[PPT], ey[PPT], ez[PPT], pn[PPT], br[PPT];
-    const int64_t ebase = (int64_t)blockIdx.x * kThreads64 * PPT + tid;
+    Arc64<PPT> W;
+    unsigned long long pf[PPT];
+    const int64_t ebase = ((int64_t)blockIdx.x * kThreads64 + tid) * PPT;
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
-        const int64_t e = ebase + (int64_t)j * kThreads64;
-        const bool ok = e < ph.nent;
-        ex[j] = ok ? ph.ex[e] : 0.;
-        ey[j] = ok ? ph.ey[e] : 0.;
-        ez[j] = ok ? ph.ez[e] : 0.;
-        pn[j] = ok ? ph.phin[e] : 0.;
+        const int64_t e = ebase + j < ph.nent ? ebase + j : ph.nent - 1;
+        ex[j] = ph.ex[e];
+        ey[j] = ph.ey[e];
+        ez[j] = ph.ez[e];
+        pn[j] = ph.phin[e];
+        pf[j] = ph.pfx[e];
+        W.ex[j] = (float)ex[j];
+        W.ey[j] = (float)ey[j];
+        W.ez[j] = (float)ez[j];
+        if (!(ex[j] * ex[j] + ey[j] * ey[j] + ez[j] * ez[j] < 1.000001))
+            W.ex[j] = nanf("");
+        W.exy[j] = sqrtf(W.ex[j] * W.ex[j] + W.ey[j] * W.ey[j]);
         br[j] = 0.0;
     }
+    warp_arc<PPT>(pf, W.A, W.L);
     const Consts64 L{k.c[0], k.c[1], k.c[2], k.c[3], k.base, k.mucrit,
                      k.beam, k.spin, k.vfac, k.xcofm, k.rlens1};
     // a warp leaves together whether its copies arrived or the wait gave up,
@@ -148,58 +305,16 @@ __global__ void __launch_bounds__(kThreads64)
         mbar_wait_bounded(&bar, 0);
         return;
     }
-    // Per face, one vote of the warp: when the face is at or below zero_below
-    // (exactly zero) or eclipsed at every entry of the warp, its elements
-    // would add exact zeros, and the warp moves on. The warp's entries are
-    // 32 consecutive sub-phases per j, so a face's visibility is shared by
-    // nearly all of them. Skipped or not, every sum is bit-identical.
     const double zb = zero_below<BEAM>(L);
-    for (int64_t i = lo; i < a1; i++) {
-        const int t = (int)(i - lo);
-        const double dx = s_dx[t], dy = s_dy[t], dz = s_dz[t];
-        double mu[PPT];
-        bool live = false;
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            mu[j] = mu_of(ex[j], ey[j], ez[j], dx, dy, dz);
-            live |= mu[j] > zb;
-        }
-        if (!__any_sync(0xffffffffu, live)) continue;
-        const double fl = s_fl[t];
-        double px = 0., py = 0., pz = 0.;
-        if constexpr (need_pos) { px = s_px[t]; py = s_py[t]; pz = s_pz[t]; }
-#pragma unroll
-        for (int j = 0; j < PPT; j++)
-            br[j] += elem_mu<LT, BEAM, GLENS, STAR>(mu[j], ex[j], ey[j], ez[j], dx, dy, px, py,
-                                                    pz, fl, L);
-    }
-    for (int64_t i = b0; i < hi; i++) {
-        const int t = (int)(i - lo);
-        const double dx = s_dx[t], dy = s_dy[t], dz = s_dz[t];
-        const double ein = s_in[t], eout = s_out[t];
-        double mu[PPT];
-        bool ecl[PPT];
-        bool live = false;
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            mu[j] = mu_of(ex[j], ey[j], ez[j], dx, dy, dz);
-            ecl[j] = (pn[j] >= ein && pn[j] <= eout) || pn[j] <= eout - 1.0;
-            live |= (mu[j] > zb) && !ecl[j];
-        }
-        if (!__any_sync(0xffffffffu, live)) continue;
-        const double fl = s_fl[t];
-        double px = 0., py = 0., pz = 0.;
-        if constexpr (need_pos) { px = s_px[t]; py = s_py[t]; pz = s_pz[t]; }
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            const double v = elem_mu<LT, BEAM, GLENS, STAR>(mu[j], ex[j], ey[j], ez[j], dx, dy,
-                                                            px, py, pz, fl, L);
-            br[j] += ecl[j] ? 0.0 : v;
-        }
-    }
+    const Cols64 C{s_dx, s_dy, s_dz, s_fl, s_in, s_out, s_px, s_py, s_pz};
+    // plain segment, then one-range segment, counted from the block's first face
+    const int64_t q0 = n0 - lo;
+    const int end = (int)(hi - lo), q = q0 < 0 ? 0 : q0 < end ? (int)q0 : end;
+    segment64<PPT, LT, BEAM, GLENS, STAR, false>(C, sr, 0, q, ex, ey, ez, pn, W, zb, L, br);
+    segment64<PPT, LT, BEAM, GLENS, STAR, true>(C, sr, q, end, ex, ey, ez, pn, W, zb, L, br);
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
-        const int64_t e = ebase + (int64_t)j * kThreads64;
+        const int64_t e = ebase + j;
         if (e < ph.nent) part[(int64_t)blockIdx.y * ldp + e] = br[j];
     }
 }
@@ -311,7 +426,8 @@ template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
 void launch_t(const FluxConsts &k, const FlatDev &f, const PhaseDev &ph, const FluxPlan &plan,
               double *part, int64_t ldp, DevStatus *st, cudaStream_t s) {
     constexpr bool need_pos = BEAM || GLENS;
-    const size_t smem = (size_t)kBlock * 8 * (need_pos ? 9 : 6);
+    const size_t smem = (size_t)kBlock * 8 * (need_pos ? 9 : 6) +
+                        kBlock / kRunFaces * kRunRecs * sizeof(RunRec);
     auto kern = k_flux64<PPT, LT, BEAM, GLENS, STAR>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid((unsigned)plan.ntile, (unsigned)plan.nchunk);

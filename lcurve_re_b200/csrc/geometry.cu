@@ -1168,6 +1168,48 @@ __global__ void k_run_bounds_geo(const float4 *__restrict__ geo,
     run_records(nx, ny, cz, use, E, runs + kRunRecs * run);
 }
 
+// From the FP64 columns: cz = nz; the arcs are drawn in (all) and out (hull) by
+// two units, so that a phase is only ever decided by them where the sweep's
+// double comparisons decide it alike.
+__global__ void k_run_bounds64(FlatDev f) {
+    const int64_t run = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (run >= (f.n + kRunFaces - 1) / kRunFaces) return;  // whole warps
+    const int64_t i = run * kRunFaces + 2 * (threadIdx.x & 31), n0 = *f.n0;
+    float nx[2] = {0.f, 0.f}, ny[2] = {0.f, 0.f}, cz[2] = {0.f, 0.f};
+    ulonglong2 E[2] = {make_ulonglong2(0ull, 0ull), make_ulonglong2(0ull, 0ull)};
+    bool use[2] = {false, false};
+    for (int k = 0; k < 2; k++) {
+        if (i + k >= f.n) continue;
+        const double x = f.dx[i + k], y = f.dy[i + k], z = f.dz[i + k];
+        use[k] = x != 0. || y != 0. || z != 0.;
+        // vectors longer than one, or NaN, spoil their groups' bounds
+        nx[k] = x * x + y * y + z * z < 1.000001 ? (float)x : nanf("");
+        ny[k] = (float)y;
+        cz[k] = (float)z;
+        if (i + k < n0) continue;
+        const double in = f.in1[i + k], out = f.out1[i + k];
+        // ranges that a turn does not hold as they are: tested face by face
+        E[k] = in >= 0. && in < 1. && out >= in ? ecl_fx64(in, out) : make_ulonglong2(0ull, ~0ull);
+    }
+    RunRec *out = f.runs + kRunRecs * run;
+    run_records(nx, ny, cz, use, E, out);
+    __syncwarp();
+    const int r = threadIdx.x & 31;
+    if (r < kRunRecs) {
+        RunRec &R = out[r];
+        if (R.hull.y != 0ull && R.hull.y != ~0ull) {
+            R.hull.x -= 2ull;
+            R.hull.y += 4ull;
+        }
+        if (R.all.y > 4ull) {
+            R.all.x += 2ull;
+            R.all.y -= 4ull;
+        } else {
+            R.all.y = 0ull;
+        }
+    }
+}
+
 __global__ void k_run_bounds(const float *__restrict__ fp, const ulonglong2 *__restrict__ ecl,
                              int64_t npairs, RunRec *runs) {
     const int64_t run = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -1706,6 +1748,7 @@ void launch_flatten(GridDev g, FlatDev f, const int32_t *cnt, int mixed, int nee
     count_launch();
     if (mixed && fc.on) launch_run_bounds(f.fp, f.ecl, f.npad / 2, f.runs, s);
     else if (mixed) launch_run_bounds_geo(f, s);
+    else launch_run_bounds64(f, s);
 }
 
 void launch_phases(const PhaseParams &p, const DatumRec *data, const int64_t *off, int32_t n,
@@ -1762,6 +1805,13 @@ void launch_run_bounds_geo(const FlatDev &f, cudaStream_t s) {
     const int64_t nruns = (f.n + kRunFaces - 1) / kRunFaces;
     if (nruns <= 0) return;
     k_run_bounds_geo<<<nblocks(nruns * 32, 256), 256, 0, s>>>(f.geo, f.ecl, f.n, f.runs);
+    count_launch();
+}
+
+void launch_run_bounds64(const FlatDev &f, cudaStream_t s) {
+    const int64_t nruns = (f.n + kRunFaces - 1) / kRunFaces;
+    if (nruns <= 0) return;
+    k_run_bounds64<<<nblocks(nruns * 32, 256), 256, 0, s>>>(f);
     count_launch();
 }
 

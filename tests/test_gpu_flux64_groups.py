@@ -1,0 +1,56 @@
+"""The double-precision flux sweep's groups of faces against the oracle, bit for bit.
+
+Groups of 64 and 16 faces are dark, bright or tested face by face by bounds that
+the warp holds against its entries; what is skipped must be exact zeros. The
+faces lie on a spiral, so that groups are narrow; sizes fall at the edges of
+parts, runs and blocks of 1024; ranges and normals include forms that the
+bounds cannot hold (ranges outside one turn, normals longer than one).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def flat_grid(n, n0, odd):
+    rng = np.random.default_rng(n)
+    z = np.linspace(0.999, -0.999, n)
+    az = 0.1 * np.sqrt(n) * np.arange(n) / n * 2 * np.pi
+    r = np.sqrt(1 - z * z)
+    d = np.stack([r * np.cos(az), r * np.sin(az), z])
+    ingress = rng.uniform(0.80, 0.999) + 0.01 * rng.random(n)
+    ingress = np.where(ingress >= 1, ingress - 1, ingress)
+    egress = ingress + rng.uniform(0.02, 0.3) + 0.01 * rng.random(n)
+    if odd:
+        d[:, rng.random(n) < 0.02] *= 1.5
+        k = rng.random(n)
+        ingress = np.where(k < 0.02, ingress - 1, np.where(k < 0.04, ingress + 1, ingress))
+        egress = np.where(k > 0.98, ingress - 0.1, np.where(k > 0.96, ingress + 1.0, egress))
+    p = 0.1 * d * (1 + 0.05 * rng.random(n))
+    return dict(dx=d[0], dy=d[1], dz=d[2], px=p[0], py=p[1], pz=p[2],
+                flux=rng.uniform(0.5, 1.5, n), n0=n0, in1=ingress[n0:], out1=egress[n0:])
+
+
+@pytest.mark.parametrize("n,n0,nent,order", [
+    (1, 0, 1, "time"), (15, 15, 33, "time"), (63, 16, 1000, "time"), (65, 64, 1023, "shuffled"),
+    (1024, 1000, 1024, "time"), (1025, 17, 1300, "shuffled"), (2049, 1024, 8192, "time"),
+    (3100, 0, 8300, "time"), (3100, 3100, 2500, "time"), (1500, 700, 130, "one phase")])
+@pytest.mark.parametrize("odd", [False, True])
+def test_group_classes_leave_the_sums_alone(engine_fp64, oracle, n, n0, nent, order, odd):
+    flat = flat_grid(n, n0, odd)
+    rng = np.random.default_rng(nent)
+    ph = np.linspace(0, 1, nent, endpoint=False) if order != "one phase" else np.full(nent, 0.95)
+    if order == "shuffled":
+        ph = rng.permutation(ph)
+    if order == "time":
+        ph[-1] = 1.0  # what a phase just below a whole one is rounded to
+    si, ci = np.sin(np.radians(85.0)), np.cos(np.radians(85.0))
+    phases = dict(ex=si * np.cos(2 * np.pi * ph), ey=-si * np.sin(2 * np.pi * ph),
+                  ez=np.full(nent, ci), phin=ph)
+    for star, ltype, kw in ((0, 1, {}), (1, 0, dict(mucrit=0.2)), (0, 0, dict(beam=1.4, mucrit=-0.5)),
+                            (1, 1, dict(beam=0.7, glens1=True, rlens1=2e-6)),
+                            (1, 1, dict(glens1=True, rlens1=2e-6, mucrit=-0.1))):
+        kw = dict(ldc=[0.4, 0.1, 0.05, 0.02], ltype=ltype, spin=1.1, vfac=1e-3, xcofm=0.2, **kw)
+        a = oracle.sum_star_multi(star, flat, phases, **kw)
+        b = engine_fp64.sum_star_multi(star, flat, phases, **kw)
+        np.testing.assert_array_equal(a, b)
