@@ -712,9 +712,8 @@ FluxPlan plan_flux(int mixed, int fast, int64_t nface, int64_t nent, int nsm) {
         while (chunk > 64 && (nface + chunk - 1) / chunk < want) chunk >>= 1;
         p.chunk = chunk;
     } else {
-        p.threads = 128;
-        p.ppt = nent >= 8192 ? 4 : (nent >= 1024 ? 2 : 1);
-        p.ntile = (nent + (int64_t)p.threads * p.ppt - 1) / ((int64_t)p.threads * p.ppt);
+        p.threads = 256;  // kThreads64, an entry each
+        p.ntile = (nent + p.threads - 1) / p.threads;
         if (p.ntile < 1) p.ntile = 1;
         p.chunk = 1024;  // FACE_BLOCK of comp_light_flat.cpp:239
     }

@@ -18,7 +18,8 @@ namespace lcg {
 
 namespace {
 
-constexpr int kThreads64 = 128;
+constexpr int kThreads64 = 256;
+constexpr int kThreadsRag = 128;  // several-range faces
 constexpr int kBlock = 1024;
 
 struct Consts64 {
@@ -87,11 +88,10 @@ __device__ __forceinline__ double elem_mu(double mu, double ex, double ey, doubl
     return (double)(mu > L.mucrit) * val;
 }
 
-// A warp's entries for the group tests: earth vectors in FP32 with the length of
-// their xy part, and the phase arc.
-template <int PPT>
+// A thread's entry, in FP32 for the group tests: earth vector, the length of its
+// xy part, and the phase arc of its warp.
 struct Arc64 {
-    float ex[PPT], ey[PPT], ez[PPT], exy[PPT];
+    float ex, ey, ez, exy;
     unsigned long long A, L;
 };
 
@@ -100,128 +100,100 @@ struct Arc64 {
 // above zb for every face and entry and no range reaches the warp's arc. The
 // bounds are FP32; 2e-6 covers the rounding for vectors of length one. Longer
 // ones and NaN come as NaN, which is neither dark nor bright.
-template <int PPT, bool ECL>
-__device__ __forceinline__ int group64(const RunRec &R, float zb, const Arc64<PPT> &W) {
-    bool some = false, every = true;
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const float d = W.ex[j] * R.ax + W.ey[j] * R.ay, q = W.exy[j] * R.r;
-        const float z0 = W.ez[j] * R.cmin, z1 = W.ez[j] * R.cmax;
-        some |= !(q + d + fmaxf(z0, z1) + 2e-6f < zb);
-        every &= d - q + fminf(z0, z1) - 2e-6f > zb;
-    }
-    if (!__any_sync(0xffffffffu, some)) return kGroupDark;
+template <bool ECL>
+__device__ __forceinline__ int group64(const RunRec &R, float zb, const Arc64 &W) {
+    const float d = W.ex * R.ax + W.ey * R.ay, q = W.exy * R.r;
+    const float z0 = W.ez * R.cmin, z1 = W.ez * R.cmax;
+    if (!__any_sync(0xffffffffu, !(q + d + fmaxf(z0, z1) + 2e-6f < zb))) return kGroupDark;
     if constexpr (ECL) {
         const int c = arc_class(R, W.A, W.L);
         if (c != kGroupSigns) return c;
     }
-    return __all_sync(0xffffffffu, every) ? kGroupBright : kGroupSigns;
+    return __all_sync(0xffffffffu, d - q + fminf(z0, z1) - 2e-6f > zb) ? kGroupBright
+                                                                       : kGroupSigns;
 }
 
 struct Cols64 {  // a staged block's columns
     const double *dx, *dy, *dz, *fl, *in, *out, *px, *py, *pz;
 };
 
+struct Entry64 {
+    double ex, ey, ez, pn;
+};
+
 // Faces [t0, t1) of the block, every one visible at every entry (no beaming, no
 // lensing): s1_elem / s2_elem without the factors that are one there, (mu > 0)
 // and (mu > mucrit).
-template <int PPT, int LT>
-__device__ __forceinline__ void bright64(const Cols64 &C, int t0, int t1, const double *ex,
-                                         const double *ey, const double *ez, const Consts64 &L,
-                                         double *br) {
+template <int LT>
+__device__ __forceinline__ void bright64(const Cols64 &C, int t0, int t1, const Entry64 &E,
+                                         const Consts64 &L, double &br) {
+#pragma unroll 4
     for (int t = t0; t < t1; t++) {
-        const double dx = C.dx[t], dy = C.dy[t], dz = C.dz[t], fl = C.fl[t];
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            const double mu = mu_of(ex[j], ey[j], ez[j], dx, dy, dz);
-            const double m = (1.0 < mu) ? 1.0 : mu;
-            double im;
-            if constexpr (LT == 0) {
-                const double om = 1.0 - m;
-                im = 1.0 - om * (L.c1 + om * (L.c2 + om * (L.c3 + om * L.c4)));
-            } else {
-                const double msq = sqrt(m);
-                im = L.base + msq * (L.c1 + msq * (L.c2 + msq * (L.c3 + msq * L.c4)));
-            }
-            br[j] += mu * fl * im;
+        const double mu = mu_of(E.ex, E.ey, E.ez, C.dx[t], C.dy[t], C.dz[t]);
+        const double m = (1.0 < mu) ? 1.0 : mu;
+        double im;
+        if constexpr (LT == 0) {
+            const double om = 1.0 - m;
+            im = 1.0 - om * (L.c1 + om * (L.c2 + om * (L.c3 + om * L.c4)));
+        } else {
+            const double msq = sqrt(m);
+            im = L.base + msq * (L.c1 + msq * (L.c2 + msq * (L.c3 + msq * L.c4)));
         }
+        br += mu * C.fl[t] * im;
     }
 }
 
 // The same faces with every factor, and the range when ECL. Per face, one vote
 // of the warp: at or below zb (exactly zero) or eclipsed at every entry of the
 // warp, its elements would add exact zeros, and the warp moves on.
-template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
-__device__ __forceinline__ void faces64(const Cols64 &C, int t0, int t1,
-                                        const double *ex, const double *ey, const double *ez,
-                                        const double *pn, double zb, const Consts64 &L,
-                                        double *br) {
+template <int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
+__device__ __forceinline__ void faces64(const Cols64 &C, int t0, int t1, const Entry64 &E,
+                                        double zb, const Consts64 &L, double &br) {
     constexpr bool need_pos = BEAM || GLENS;
+#pragma unroll 1
     for (int t = t0; t < t1; t++) {
         const double dx = C.dx[t], dy = C.dy[t], dz = C.dz[t];
         double ein = 0., eout = 0.;
         if constexpr (ECL) { ein = C.in[t]; eout = C.out[t]; }
-        double mu[PPT];
-        bool ecl[PPT], live = false;
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            mu[j] = mu_of(ex[j], ey[j], ez[j], dx, dy, dz);
-            ecl[j] = ECL && ((pn[j] >= ein && pn[j] <= eout) || pn[j] <= eout - 1.0);
-            live |= (mu[j] > zb) && !ecl[j];
-        }
-        if (!__any_sync(0xffffffffu, live)) continue;
-        const double fl = C.fl[t];
+        const double mu = mu_of(E.ex, E.ey, E.ez, dx, dy, dz);
+        const bool ecl = ECL && ((E.pn >= ein && E.pn <= eout) || E.pn <= eout - 1.0);
+        if (!__any_sync(0xffffffffu, (mu > zb) && !ecl)) continue;
         double px = 0., py = 0., pz = 0.;
         if constexpr (need_pos) { px = C.px[t]; py = C.py[t]; pz = C.pz[t]; }
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            const double v = elem_mu<LT, BEAM, GLENS, STAR>(mu[j], ex[j], ey[j], ez[j], dx, dy,
-                                                            px, py, pz, fl, L);
-            br[j] += ecl[j] ? 0.0 : v;
-        }
+        const double v = elem_mu<LT, BEAM, GLENS, STAR>(mu, E.ex, E.ey, E.ez, dx, dy, px, py, pz,
+                                                        C.fl[t], L);
+        br += ecl ? 0.0 : v;
     }
 }
 
 // Faces [t0, t1) of the block by groups: a run of 64, and its parts of 16 where
 // the run is neither dark nor bright.
-template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
-__device__ __forceinline__ void segment64(const Cols64 &C, const RunRec *sr, int t0,
-                                          int t1, const double *ex, const double *ey,
-                                          const double *ez, const double *pn,
-                                          const Arc64<PPT> &W, double zb, const Consts64 &L,
-                                          double *br) {
+template <int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
+__device__ __forceinline__ void segment64(const Cols64 &C, const RunRec *sr, int t0, int t1,
+                                          const Entry64 &E, const Arc64 &W, double zb,
+                                          const Consts64 &L, double &br) {
     constexpr bool plain = !BEAM && !GLENS;
+#pragma unroll 1
     for (int t = t0; t < t1;) {
         const int run = t / kRunFaces;
         const int re = (run + 1) * kRunFaces < t1 ? (run + 1) * kRunFaces : t1;
-        const int c = group64<PPT, ECL>(sr[kRunRecs * run], (float)zb, W);
-        if (c == kGroupDark) {
-            t = re;
-            continue;
-        }
-        if constexpr (plain) {
-            if (c == kGroupBright) {
-                bright64<PPT, LT>(C, t, re, ex, ey, ez, L, br);
-                t = re;
-                continue;
-            }
-        }
+        int c = group64<ECL>(sr[kRunRecs * run], (float)zb, W);
+        const bool whole = c == kGroupDark || (plain && c == kGroupBright);
 #pragma unroll 1
         while (t < re) {
-            const int part = t / 16, pe = (part + 1) * 16 < re ? (part + 1) * 16 : re;
-            const int cp = group64<PPT, ECL>(sr[kRunRecs * run + 1 + (part & 3)], (float)zb, W);
-            bool done = cp == kGroupDark;
-            if constexpr (plain) {
-                if (cp == kGroupBright) {
-                    bright64<PPT, LT>(C, t, pe, ex, ey, ez, L, br);
-                    done = true;
-                }
+            int pe = re;
+            if (!whole) {
+                const int part = t / 16;
+                pe = (part + 1) * 16 < re ? (part + 1) * 16 : re;
+                c = group64<ECL>(sr[kRunRecs * run + 1 + (part & 3)], (float)zb, W);
             }
-            if (!done) {
-                if (ECL && cp == kGroupRanges)
-                    faces64<PPT, LT, BEAM, GLENS, STAR, ECL>(C, t, pe, ex, ey, ez, pn, zb, L, br);
-                else
-                    faces64<PPT, LT, BEAM, GLENS, STAR, false>(C, t, pe, ex, ey, ez, pn, zb, L, br);
+            if (c == kGroupDark) {
+            } else if (plain && c == kGroupBright) {
+                bright64<LT>(C, t, pe, E, L, br);
+            } else if (ECL && c == kGroupRanges) {
+                faces64<LT, BEAM, GLENS, STAR, ECL>(C, t, pe, E, zb, L, br);
+            } else {
+                faces64<LT, BEAM, GLENS, STAR, false>(C, t, pe, E, zb, L, br);
             }
             t = pe;
         }
@@ -231,9 +203,14 @@ __device__ __forceinline__ void segment64(const Cols64 &C, const RunRec *sr, int
 // Skipped or not, classified or not, every sum is bit-identical: what is left
 // out are exact zeros and factors of one, and the faces keep their order. FP64
 // issue bounds it (some 35 instructions for a visible element, 12 of them the
-// square root): star 2 of 100/200 strips over 15,000 entries 1.75 -> 1.49 ms.
-template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
-__global__ void __launch_bounds__(kThreads64)
+// square root). One entry a thread: the columns come from shared memory either
+// way, a warp's arc is as narrow as it gets, and 32 warps an SM hide an element's
+// chain; dark CTAs leave early, so smaller tiles also share the bright ones out.
+// Curve of 100/200 strips and 15,000 entries, both stars at once, faces tested one
+// by one at 4 entries and 128 threads 1.98 ms; by groups 1.75; 2 and 128 1.49,
+// 1 and 128 1.51, 1 and 512 1.38, 1 and 256 1.34.
+template <int LT, bool BEAM, bool GLENS, int STAR>
+__global__ void __launch_bounds__(kThreads64, 4)
     k_flux64(FluxConsts k, FlatDev f, PhaseDev ph, double *part, int64_t ldp, DevStatus *st) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
@@ -270,29 +247,17 @@ __global__ void __launch_bounds__(kThreads64)
             bulk_g2s(s_pz, f.pz + lo, col, &bar);
         }
     }
-    // PPT consecutive entries a thread, so that a warp holds a narrow arc; threads
-    // past the last entry repeat it
-    double ex[PPT], ey[PPT], ez[PPT], pn[PPT], br[PPT];
-    Arc64<PPT> W;
-    unsigned long long pf[PPT];
-    const int64_t ebase = ((int64_t)blockIdx.x * kThreads64 + tid) * PPT;
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int64_t e = ebase + j < ph.nent ? ebase + j : ph.nent - 1;
-        ex[j] = ph.ex[e];
-        ey[j] = ph.ey[e];
-        ez[j] = ph.ez[e];
-        pn[j] = ph.phin[e];
-        pf[j] = ph.pfx[e];
-        W.ex[j] = (float)ex[j];
-        W.ey[j] = (float)ey[j];
-        W.ez[j] = (float)ez[j];
-        if (!(ex[j] * ex[j] + ey[j] * ey[j] + ez[j] * ez[j] < 1.000001))
-            W.ex[j] = nanf("");
-        W.exy[j] = sqrtf(W.ex[j] * W.ex[j] + W.ey[j] * W.ey[j]);
-        br[j] = 0.0;
-    }
-    warp_arc<PPT>(pf, W.A, W.L);
+    const int64_t entry = (int64_t)blockIdx.x * kThreads64 + tid;
+    // whole warps past the last entry leave (never the first, which waits for the
+    // copies); threads past it in the last warp repeat it
+    if ((entry & ~31ll) >= ph.nent) return;
+    const int64_t e = entry < ph.nent ? entry : ph.nent - 1;
+    const Entry64 E{ph.ex[e], ph.ey[e], ph.ez[e], ph.phin[e]};
+    Arc64 W{(float)E.ex, (float)E.ey, (float)E.ez, 0.f, 0ull, 0ull};
+    if (!(E.ex * E.ex + E.ey * E.ey + E.ez * E.ez < 1.000001)) W.ex = nanf("");
+    W.exy = sqrtf(W.ex * W.ex + W.ey * W.ey);
+    const unsigned long long pf = ph.pfx[e];
+    warp_arc<1>(&pf, W.A, W.L);
     const Consts64 L{k.c[0], k.c[1], k.c[2], k.c[3], k.base, k.mucrit,
                      k.beam, k.spin, k.vfac, k.xcofm, k.rlens1};
     // a warp leaves together whether its copies arrived or the wait gave up,
@@ -310,13 +275,10 @@ __global__ void __launch_bounds__(kThreads64)
     // plain segment, then one-range segment, counted from the block's first face
     const int64_t q0 = n0 - lo;
     const int end = (int)(hi - lo), q = q0 < 0 ? 0 : q0 < end ? (int)q0 : end;
-    segment64<PPT, LT, BEAM, GLENS, STAR, false>(C, sr, 0, q, ex, ey, ez, pn, W, zb, L, br);
-    segment64<PPT, LT, BEAM, GLENS, STAR, true>(C, sr, q, end, ex, ey, ez, pn, W, zb, L, br);
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int64_t e = ebase + j;
-        if (e < ph.nent) part[(int64_t)blockIdx.y * ldp + e] = br[j];
-    }
+    double br = 0.0;
+    segment64<LT, BEAM, GLENS, STAR, false>(C, sr, 0, q, E, W, zb, L, br);
+    segment64<LT, BEAM, GLENS, STAR, true>(C, sr, q, end, E, W, zb, L, br);
+    if (entry < ph.nent) part[(int64_t)blockIdx.y * ldp + entry] = br;
 }
 
 // Several-range faces (the ragged segment of comp_light_flat.cpp:306-316):
@@ -337,7 +299,7 @@ struct RagFace {
 };
 
 template <int LT, bool BEAM, bool GLENS, int STAR>
-__global__ void __launch_bounds__(kThreads64)
+__global__ void __launch_bounds__(kThreadsRag)
     k_flux_ragged(FluxConsts k, FlatDev f, GridDev g, PhaseDev ph, int64_t blk, double *part,
                   int64_t ldp) {
     constexpr bool POS = BEAM || GLENS;
@@ -349,7 +311,7 @@ __global__ void __launch_bounds__(kThreads64)
     if (c0 >= hi) return;
     // threads past the last entry repeat it without storing: warps stay whole
     // for the votes
-    const int64_t e1 = blockIdx.x * (int64_t)kThreads64 + threadIdx.x;
+    const int64_t e1 = blockIdx.x * (int64_t)kThreadsRag + threadIdx.x;
     const int64_t e = e1 < ph.nent ? e1 : ph.nent - 1;
     const Consts64 L{k.c[0], k.c[1], k.c[2], k.c[3], k.base, k.mucrit,
                      k.beam, k.spin, k.vfac, k.xcofm, k.rlens1};
@@ -400,8 +362,8 @@ __global__ void __launch_bounds__(kThreads64)
 template <int LT, bool BEAM, bool GLENS, int STAR>
 void launch_rag_t(const FluxConsts &k, const FlatDev &f, const GridDev &g, const PhaseDev &ph,
                   int64_t blk, int64_t nblk, double *part, int64_t ldp, cudaStream_t s) {
-    dim3 grid((unsigned)((ph.nent + kThreads64 - 1) / kThreads64), (unsigned)nblk);
-    k_flux_ragged<LT, BEAM, GLENS, STAR><<<grid, kThreads64, 0, s>>>(k, f, g, ph, blk, part, ldp);
+    dim3 grid((unsigned)((ph.nent + kThreadsRag - 1) / kThreadsRag), (unsigned)nblk);
+    k_flux_ragged<LT, BEAM, GLENS, STAR><<<grid, kThreadsRag, 0, s>>>(k, f, g, ph, blk, part, ldp);
     count_launch();
 }
 
@@ -422,40 +384,33 @@ void launch_rag_lt(int star, const FluxConsts &k, const FlatDev &f, const GridDe
     }
 }
 
-template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
+template <int LT, bool BEAM, bool GLENS, int STAR>
 void launch_t(const FluxConsts &k, const FlatDev &f, const PhaseDev &ph, const FluxPlan &plan,
               double *part, int64_t ldp, DevStatus *st, cudaStream_t s) {
     constexpr bool need_pos = BEAM || GLENS;
     const size_t smem = (size_t)kBlock * 8 * (need_pos ? 9 : 6) +
                         kBlock / kRunFaces * kRunRecs * sizeof(RunRec);
-    auto kern = k_flux64<PPT, LT, BEAM, GLENS, STAR>;
+    auto kern = k_flux64<LT, BEAM, GLENS, STAR>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid((unsigned)plan.ntile, (unsigned)plan.nchunk);
     kern<<<grid, kThreads64, smem, s>>>(k, f, ph, part, ldp, st);
     count_launch();
 }
 
-template <int PPT, int LT>
+template <int LT>
 void launch_lt(int star, const FluxConsts &k, const FlatDev &f, const PhaseDev &ph,
                const FluxPlan &plan, double *part, int64_t ldp, DevStatus *st, cudaStream_t s) {
     const bool beam = k.beam_on != 0, glens = (star == 1) && k.glens;
     if (star == 0) {
-        if (beam) launch_t<PPT, LT, true, false, 0>(k, f, ph, plan, part, ldp, st, s);
-        else launch_t<PPT, LT, false, false, 0>(k, f, ph, plan, part, ldp, st, s);
+        if (beam) launch_t<LT, true, false, 0>(k, f, ph, plan, part, ldp, st, s);
+        else launch_t<LT, false, false, 0>(k, f, ph, plan, part, ldp, st, s);
     } else if (glens) {
-        if (beam) launch_t<PPT, LT, true, true, 1>(k, f, ph, plan, part, ldp, st, s);
-        else launch_t<PPT, LT, false, true, 1>(k, f, ph, plan, part, ldp, st, s);
+        if (beam) launch_t<LT, true, true, 1>(k, f, ph, plan, part, ldp, st, s);
+        else launch_t<LT, false, true, 1>(k, f, ph, plan, part, ldp, st, s);
     } else {
-        if (beam) launch_t<PPT, LT, true, false, 1>(k, f, ph, plan, part, ldp, st, s);
-        else launch_t<PPT, LT, false, false, 1>(k, f, ph, plan, part, ldp, st, s);
+        if (beam) launch_t<LT, true, false, 1>(k, f, ph, plan, part, ldp, st, s);
+        else launch_t<LT, false, false, 1>(k, f, ph, plan, part, ldp, st, s);
     }
-}
-
-template <int PPT>
-void launch_ppt(int star, const FluxConsts &k, const FlatDev &f, const PhaseDev &ph,
-                const FluxPlan &plan, double *part, int64_t ldp, DevStatus *st, cudaStream_t s) {
-    if (k.ltype == 1) launch_lt<PPT, 1>(star, k, f, ph, plan, part, ldp, st, s);
-    else launch_lt<PPT, 0>(star, k, f, ph, plan, part, ldp, st, s);
 }
 
 // 8 independent DFMA chains per thread keep the FP64 pipe full.
@@ -492,11 +447,8 @@ void launch_flux_ragged(int star, const FluxConsts &k, const FlatDev &f, const G
 void launch_flux64(int star, const FluxConsts &k, const FlatDev &f, const PhaseDev &ph,
                    const FluxPlan &plan, double *part, int64_t ldp, DevStatus *st,
                    cudaStream_t s) {
-    switch (plan.ppt) {
-    case 4: launch_ppt<4>(star, k, f, ph, plan, part, ldp, st, s); break;
-    case 2: launch_ppt<2>(star, k, f, ph, plan, part, ldp, st, s); break;
-    default: launch_ppt<1>(star, k, f, ph, plan, part, ldp, st, s); break;
-    }
+    if (k.ltype == 1) launch_lt<1>(star, k, f, ph, plan, part, ldp, st, s);
+    else launch_lt<0>(star, k, f, ph, plan, part, ldp, st, s);
 }
 
 }  // namespace lcg
