@@ -11,7 +11,8 @@
 //     the closest approach to the eclipser's centre; f <= pref answers "hidden"
 //     at once;
 //   * when the lowest potential on the chord exceeds pref, nothing that the
-//     search evaluates can reach it: "not hidden".
+//     search evaluates can reach it: "not hidden";
+//   * in between, the search's second step answers nearly always (narrow_zone).
 //
 // edge_zone finds the root of f(phase) - pref by Newton's method and, with a
 // bound K on |f''| around it, certifies by Taylor's theorem an interval of
@@ -19,10 +20,11 @@
 // (vis allows for the depth of the potential's minimum below f). The
 // bisection takes the same midpoints as before; inside the certified
 // intervals a midpoint is compared instead of tested, and the few between hid
-// and vis (the eclipser's tide moves the minimum off the midpoint: about
-// twenty delta_phase wide on an M dwarf, far below one on a white dwarf) run
-// fblink. Every decision is fblink's, so the phases are the bisection's, bit
-// for bit. eval_edge alone answers the midpoints outside the intervals.
+// and vis run fblink. (The eclipser's tide moves the minimum off the midpoint,
+// which puts hid and vis about twenty delta_phase apart on an M dwarf before
+// narrow_zone, far below one on a white dwarf.) Every decision is fblink's, so
+// the phases are the bisection's, bit for bit. eval_edge alone answers the
+// midpoints outside the intervals.
 //
 // All in FP64. Margins cover the rounding of both sides: positions to a few
 // ulps of the orbit's size, times the gradient, and the potential itself.
@@ -274,10 +276,113 @@ LCG_HD EdgeBound edge_bound(const EdgeStar &S, const EdgeEval &v, double lam) {
     return B;
 }
 
+// What is known at the visible end of a boundary (edge_zone's stage 1), for
+// narrow_zone.
+struct EdgeEnd {
+    double t, dt, tol;           // offset of the minimum, its last step; rounding of f
+    double s0, off, fp, fl, K, rad;  // the Newton root of the minimum, its error, bounds
+    double gp, move, t3, vis0;   // bounds; where f(midpoint) > 0 from on, from hc
+    double r, h, ae, io, b2;     // EdgeEval's
+};
+
+// Between hid and vis fblink searches: f > pref at the midpoint x, the minimum
+// below. Its dbrent starts at x with slope -g and tries, first, half way to the
+// chord's end (u1, always higher: f rises); second, u2 = x + max(d1, acc), d1 the
+// secant step from the slopes at x and u1, to within err of the minimum; and third,
+// acc to one side of u2. So
+//   * u2 = x + acc, f(u2) > f(x) (the minimum is nearer to x than acc / 2): dbrent
+//     stops there, "not hidden" wherever f(x) > pref;
+//   * u2 = x + acc, f(u2) about f(x) or below: "hidden" where either is below pref;
+//     where neither is, dbrent stops there or, after u2 + acc, with the bracket closed;
+//   * u2 further, err below about acc / 2: "hidden" where f(u2) < pref, else not. The
+//     secant step from u2 is shorter than acc: dbrent moves acc instead and, finding
+//     f higher, stops; or, where that ends within 2 acc of x, it tries u2 + acc and if
+//     need be u2 - acc, both higher, and the bracket is closed;
+//   * otherwise f(u2) <= minimum + 0.7 h err^2, and "hidden" where that is below pref.
+// In all but the last the answer turns at the root of f, at x or at u2, and the gap
+// between hid and vis shrinks to the error of that root. Over the gap's width om all of
+// this moves by bounded amounts; what the bounds leave open is searched as before.
+// M-dwarf boundaries on 60-400 strips: 3.3 -> 0.003 searches each.
+LCG_HD void narrow_zone(const EdgeStar &S, V3 u0, double acc, double dir, double lam,
+                        const EdgeEnd &E, const EdgeBound &B, EdgeZone &z) {
+    const double om = 1.05 * (dir * (z.vc - z.hc) - z.hid + fabs(E.s0) + E.off);
+    const double hc2 = S.rref2 - E.b2, db = 2. * kTwoPi * lam * lam * om;  // of b^2 and hc^2
+    if (!(om > 0. && om < 0.5 * E.rad && om < 0.5 * z.hrad && db < 0.2 * hc2 && hc2 < 0.6 * E.b2))
+        return;
+    const double hc = sqrt(hc2), dhc = 0.6 * db / hc;
+    if (!(hc * E.io < 0.3 && hc > 5. * acc)) return;
+    // along the chord the slope grows by rise per length at least, so f has one
+    // minimum there, no further than g / rise from the midpoint
+    const double ni = E.io / (1. - 1.1 * hc * E.io), ir = edge_rsqrt(S.rref2);
+    const double t2 = 2. * S.mo * ni * ni * ni + S.ss, rise = S.me * ir * ir * ir - t2;
+    if (!(rise > 0.3 * t2)) return;
+    double sn, cs;
+    edge_sincos(z.vc, sn, cs);
+    const double ex = S.sini * cs, ey = -S.sini * sn, ez = S.cosi;
+    const double x = -fma(ex, u0.x, fma(ey, u0.y, ez * u0.z));
+    const double tm = fabs(E.t + E.dt), sg = E.t + E.dt > 0. ? 1. : -1.;
+    // slopes towards the minimum at x (g), u1 (g1) and u2; the value at u2 (f2)
+    double g = 0., g1 = 0., d1 = 0., den = 1., step = 0., f2 = 0.;
+#pragma unroll 1
+    for (int i = 0; i < 3; i++) {
+        const double t = i == 0 ? 0. : i == 1 ? 0.5 * sg * hc : sg * step, l = x + t;
+        const double ux = fma(l, ex, u0.x), uy = fma(l, ey, u0.y), uz = fma(l, ez, u0.z);
+        const double vx = ux - S.dx, yz = fma(uy, uy, uz * uz);
+        const double ie = edge_rsqrt(fma(ux, ux, yz)), io = edge_rsqrt(fma(vx, vx, yz));
+        const double pe = S.me * ie, po = S.mo * io;
+        const double d = sg * fma(pe * ie * ie, t,
+                                  fma(po * io * io, fma(-S.dx, ex, t),
+                                      fma(-S.ss, fma(ux, ex, uy * ey), S.k * ex)));
+        if (i == 0) {
+            g = -d;
+        } else if (i == 1) {
+            g1 = d;
+            den = g + g1;
+            d1 = 0.5 * hc * g / den;
+            step = d1 > acc ? d1 : acc;
+        } else {
+            f2 = fma(S.k, ux, fma(-0.5 * S.ss, fma(ux, ux, uy * uy), -(pe + po))) - S.pref;
+        }
+    }
+    const double dg = E.gp * om, gmax = g + dg, up = gmax / rise;
+    // the slope at u1 moves with the phase and with u1
+    const double gp1 = kTwoPi * (2.1 * E.ae * hc / E.r * lam + 2. * (B.t2 * lam + B.t1));
+    const double dw = gp1 * om + 0.6 * dhc * (1.3 * E.ae + B.t2);
+    if (!(g > 3. * dg && den > 0.25 * rise * hc && 20. * up * up < E.b2 && hc > 5. * up)) return;
+    const double rel = dhc / hc + dg / g + (dg + dw) / den;
+    if (!(rel < 0.2 && 0.45 * hc - 1.3 * d1 > 2.2 * acc && hc > 4.8 * step)) return;
+    const double et = fabs(E.dt) + dg / (0.6 * E.h), du = 1.3 * d1 * rel;
+    const double err = fabs(step - tm) + du + et;
+    const bool near = acc + tm + et < E.move, one = d1 + du < acc * (1. - 1e-9);
+    const double hmin = E.h - E.t3 * (acc + tm + et), far = acc - err;
+    const double dh = E.t3 * (1.5 * acc + et), vis0 = dir * (z.hc - z.vc) + E.vis0 + 4e-15;
+    if (near && one && 0.5 * hmin * acc > gmax * (1. + 1e-6) + 1e-9) {
+        if (vis0 < z.vis) z.vis = vis0;
+    } else if (near && (one ? err < 0.6 * acc
+                            : err < 0.4 * tm && err < 0.5 * acc &&
+                                  far * far * (E.h - dh) > 1.01 * err * err * (E.h + dh))) {
+        // df(u2)/dphase: fp at the minimum; the way from there to u2, u2's own motion, K om
+        const double e = E.gp * err + 1.4 * E.h * err * du / om + E.K * om;
+        const double s2 = f2 / E.fp, off = (fabs(s2) * e + 8. * E.tol) / (E.fp - e) + 8e-15;
+        if (!(e < 0.5 * E.fp && fabs(s2) + off < om)) return;
+        const double to = dir * (z.vc - z.hc) - s2 - off;
+        const double vis = one && vis0 > off - s2 ? vis0 : off - s2;
+        if (to > z.hid) z.hid = to;
+        if (vis < z.vis) z.vis = vis;
+    } else if (err + et < 0.5 * E.move) {
+        // f(u2) < pref where the minimum is this deep
+        const double del = 1.3 * (E.off + (0.7 * E.h * err * err + 8. * E.tol) / E.fl);
+        const double to = dir * (z.vc - z.hc) - E.s0 - del - 8e-15;
+        if (E.K * (fabs(E.s0) + del) <= 0.2 * E.fl && fabs(E.s0) + del < E.rad && to > z.hid)
+            z.hid = to;
+    }
+}
+
 // The intervals of one boundary of ingress_egress's bracket: pin the phase
 // pot_min found hidden, pout where the line touches the reference sphere;
-// delta the bisection's accuracy (intervals that end within a twentieth of it
-// of the root are near enough).
+// delta the bisection's accuracy: intervals that end within a twentieth of it of
+// the root are near enough, but narrow_zone's error grows with the distance from the
+// minimum's, which one more of Newton's steps makes nothing.
 LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, double pin,
                           double pout) {
     EdgeZone z;
@@ -289,7 +394,7 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
     // Newton's method for f = 0 (stage 0, t = 0: the hidden side), then for the
     // lowest potential on the line = 0 (stage 1, with t: the visible side). A
     // chord of length acc or less answers "not hidden" untested: start inside.
-    double w = -0.02 * span, t = 0.;
+    double w = -0.02 * span, t = 0., vis0 = 0.;
     int stage = 0;
 #pragma unroll 1
     for (int it = 0; it < 12; it++) {
@@ -299,22 +404,25 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
         const double dt = stage ? -v.g / v.h : 0.;
         const double m = stage ? v.f + 0.5 * v.g * dt : v.f;  // to second order
         const double s0 = m / fp;
-        if (fabs(s0) < 1e-3) {
+        const double fine = stage ? 5e-4 : 0.05;
+        // near enough for the bounds to hold (off below is K s0^2 / fl at least)
+        if (s0 * s0 * (kTwoPi * kTwoPi * 2.75) * lam * lam * v.ae <= fine * delta * fp) {
             const EdgeBound B = edge_bound(S, v, lam);
             const double r = sqrt(v.r2);
             double rad = B.rad, K = B.K, fl = fp, extra = 4. * v.tol;
+            double gp = 0., move = 0., t3 = 0.;
             bool ok = true;
             if (stage) {
                 // curvature along the line keeps 0.6 h while the point moves by
                 // at most move (third derivatives of -m / r: 6 m / r^4); the
                 // minimum shifts by at most gp rad / hl, gp bounding dg/dphase:
                 // the eclipser's part of g is ae t for every phase
-                const double t3 = 9. * (v.ae / r + S.mo * v.io * v.io * v.io * v.io);
-                double move = 0.4 * v.h / t3;
+                t3 = 9. * (v.ae / r + S.mo * v.io * v.io * v.io * v.io);
+                move = 0.4 * v.h / t3;
                 if (move > 0.09 * r) move = 0.09 * r;
                 if (move * v.io > 0.09) move = 0.09 / v.io;
                 const double hl = 0.6 * v.h, tm = fabs(t) + move;
-                const double gp = kTwoPi * (4.2 * v.ae * tm / r * lam + 1.3 * (B.t2 * lam + B.t1));
+                gp = kTwoPi * (4.2 * v.ae * tm / r * lam + 1.3 * (B.t2 * lam + B.t1));
                 K += gp * gp / hl;
                 const double rm = (move - fabs(dt)) / (1.2 * kTwoPi * lam + gp / hl);
                 if (rm < rad) rad = rm;
@@ -333,17 +441,21 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
             const double eta = (K * s0 * s0 + 2. * extra) / fl;
             const double off = stage ? fabs(s0) * (fp / fl - 1.) + eta : eta;
             if (ok && fl > 0.5 * fp && rad > 0. && K * (fabs(s0) + off) <= 0.2 * fl &&
-                fabs(s0) + off < rad && off <= 0.05 * delta) {
+                fabs(s0) + off < rad && off <= fine * delta) {
                 // 4e-15: the rounding of phases near 1
                 if (stage) {
                     z.vc = pout + dir * w;
                     z.vrad = rad;
                     z.vis = -s0 + off + 4e-15;
+                    const EdgeEnd E{t, dt, v.tol, s0, off, fp, fl, K, rad, gp, move, t3, vis0,
+                                    r, v.h, v.ae, v.io, v.b2};
+                    narrow_zone(S, u0, acc, dir, lam, E, B, z);
                     return z;
                 }
                 z.hc = pout + dir * w;
                 z.hrad = rad;
                 z.hid = -s0 - off - 4e-15;
+                vis0 = -s0 + off + 4e-15;
                 stage = 1;
                 w -= s0;
                 if (v.h > 0.) t = -v.g / v.h;
@@ -358,18 +470,45 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
     return z;
 }
 
-// What the zones say of a phase.
-LCG_HD int zone_test(const EdgeZone &z, double dir, double phase) {
-    const double wh = dir * (phase - z.hc), wv = dir * (phase - z.vc);
-    if (wh >= -z.hrad && wh <= z.hid && z.hrad > 0.) return kEdgeTrue;
-    if (wv <= z.vrad && wv >= z.vis && z.vrad > 0.) return kEdgeFalse;
+// The zones as phases: hidden on [h0, h1], not hidden on [v0, v1] (h0 > h1, v0 > v1:
+// nothing), each drawn in by the rounding of its ends.
+struct EdgeSpan {
+    double h0, h1, v0, v1;
+};
+
+LCG_HD EdgeSpan edge_span(const EdgeZone &z, double dir) {
+    constexpr double kRound = 2e-15;
+    const double ha = z.hc - dir * z.hrad, hb = z.hc + dir * z.hid;
+    const double va = z.vc + dir * z.vis, vb = z.vc + dir * z.vrad;
+    EdgeSpan e;
+    e.h0 = (dir > 0. ? ha : hb) + kRound;
+    e.h1 = (dir > 0. ? hb : ha) - kRound;
+    e.v0 = (dir > 0. ? va : vb) + kRound;
+    e.v1 = (dir > 0. ? vb : va) - kRound;
+    if (!(z.hrad > 0.)) { e.h0 = 10.; e.h1 = -10.; }
+    if (!(z.vrad > 0.)) { e.v0 = 10.; e.v1 = -10.; }
+    return e;
+}
+
+LCG_HD int span_test(const EdgeSpan &e, double phase) {
+    if (phase >= e.h0 && phase <= e.h1) return kEdgeTrue;
+    if (phase >= e.v0 && phase <= e.v1) return kEdgeFalse;
     return kEdgeUnsure;
 }
 
 // A phase beyond both intervals' inner ends: only the search tells.
+LCG_HD bool span_between(const EdgeSpan &e, double phase) {
+    return (phase > e.h1 && phase < e.v0 && e.h0 <= e.h1 && e.v0 <= e.v1) ||
+           (phase > e.v1 && phase < e.h0 && e.h0 <= e.h1 && e.v0 <= e.v1);
+}
+
+// What the zones say of a phase.
+LCG_HD int zone_test(const EdgeZone &z, double dir, double phase) {
+    return span_test(edge_span(z, dir), phase);
+}
+
 LCG_HD bool zone_between(const EdgeZone &z, double dir, double phase) {
-    return z.hrad > 0. && z.vrad > 0. && dir * (phase - z.hc) > z.hid &&
-           dir * (phase - z.vc) < z.vis;
+    return span_between(edge_span(z, dir), phase);
 }
 
 // ---- the surface radius along a ray ------------------------------------------------

@@ -362,13 +362,14 @@ __device__ __noinline__ bool fblink(int star, double q, double spin, double acc,
 // needs a test. The tests run in passes for all lanes that wait for one:
 // eval_edge outside the intervals, fblink_edge between them, and Roche::fblink
 // itself where that is unsure, so the lanes take fblink's decisions at the
-// same midpoints as the plain loop (p: EclParams). FP64 latency and issue bound it: some 4
-// evaluations for the root, 2.3 outside the intervals and 3.3 searches of 5
-// evaluations per boundary by an M dwarf, against 20 tests in FP32 with 6.4
-// fblinks of 8 to 12 evaluations before (a white dwarf's: 6 evaluations
-// against 20 fblinks). 256 models of 60-400 strips: 13.8 -> 5.4 ms; one curve
-// on 81/163 strips: 203 us with its warp mode -> 62. With the FP32 screen kept
-// for the tests outside the intervals it took 5.8 ms.
+// same midpoints as the plain loop (p: EclParams). FP64 latency and issue bound it:
+// some 5 evaluations for the root, 3 half ones for the search's steps and 2.3 outside
+// the intervals per boundary, against 20 tests in FP32 with 6.4 fblinks of 8 to 12
+// evaluations before (a white dwarf's: 6 evaluations against 20 fblinks). 256 models
+// of 60-400 strips: 13.8 ms; with the intervals of edge_zone alone, and 3.3 searches
+// per M-dwarf boundary for what they leave, 5.4; with narrow_zone 3.8. One curve on
+// 400/200 strips: 103 -> 60 us a star by narrow_zone. With the FP32 screen kept for
+// the tests outside the intervals the batch took 0.4 ms more.
 template <class Ecl>
 __device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pin, double pout,
                                               double acc, V3 pos, int &s) {
@@ -377,9 +378,8 @@ __device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pi
     const double delta = p.delta;
     const V3 u0 = v3(pos.x - (p.comp_star == kStar1 ? 0. : 1.), pos.y, pos.z);
     const double u2 = norm2(u0), dir = pout > pin ? 1. : -1.;
-    EdgeZone z;
-    z.hrad = z.vrad = z.hid = z.vis = z.hc = z.vc = 0.;
-    if (live) z = edge_zone(S, u0, acc, delta, pin, pout);
+    EdgeSpan z{10., -10., 10., -10.};
+    if (live) z = edge_span(edge_zone(S, u0, acc, delta, pin, pout), dir);
     bool done = !live;
     int guard = 0;
     double pmid = 0.;
@@ -389,9 +389,9 @@ __device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pi
             if (!(fabs(pin - pout) > delta)) { done = true; break; }
             if (++guard > 400) { s = kEclNoConverge; done = true; break; }
             pmid = (pin + pout) / 2.;
-            const int d = zone_test(z, dir, pmid);
+            const int d = span_test(z, pmid);
             if (d == kEdgeUnsure) {
-                need = zone_between(z, dir, pmid) ? 2 : 1;
+                need = span_between(z, pmid) ? 2 : 1;
                 break;
             }
             if (d == kEdgeTrue) pin = pmid;

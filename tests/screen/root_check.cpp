@@ -83,6 +83,12 @@ int main() {
                     const int a = zone_test(z, dir, p);
                     wrong += a != kEdgeUnsure && a != truth(p);
                 }
+                const double at[2] = {z.hc + dir * (z.hid - 30. * delta * w4),
+                                      z.vc + dir * (z.vis + 30. * delta * w4)};
+                for (double p : at) {
+                    const int a = zone_test(z, dir, p);
+                    wrong += a != kEdgeUnsure && a != truth(p);
+                }
             }
         }
     }

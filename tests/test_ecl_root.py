@@ -66,6 +66,18 @@ def test_roots_keep_every_decision(checker, oracle, most, over):
     assert zone >= most * tests, (zone, tests)
 
 
+# the search's second step from less than half of its accuracy to several times it:
+# smaller and larger eclipsers, finer and coarser bisections
+@pytest.mark.parametrize("r2", [0.08, 0.13, 0.17, 0.19, 0.205, 0.22, 0.235])
+@pytest.mark.parametrize("delta", ["1e-6", "1e-7", "1e-8"])
+def test_narrowed_gaps_keep_every_decision(checker, oracle, r2, delta):
+    m = W.model(nlat1f=14, nlat2f=20, r2=r2, delta_phase=delta, iangle=87.0)
+    rc, r = _run(checker, m, 0, oracle.star_grid(m, 0)["posn"])
+    assert rc == 0 and r["wrong"] == 0, r
+    if delta == "1e-7":
+        assert r["searches"] <= 0.01 * r["tests"], r
+
+
 @pytest.mark.parametrize("q,spin,radius", [
     (0.25, 1.0, 0.015), (0.25, 1.0, 0.2), (0.05, 1.0, 0.2), (0.15, 1.0, -1.0), (0.8, 1.0, -1.0),
     (3.0, 1.0, 0.35), (0.25, 0.0, 0.25), (0.25, 3.0, 0.1), (0.01, 1.0, 0.002), (0.9, 1.5, 0.3)])
