@@ -23,15 +23,29 @@ __device__ __forceinline__ void set_status(DevStatus *st, int code, int64_t face
     if (atomicCAS(&st->code, 0, code) == 0) st->face = (int32_t)face;
 }
 
-// One half-face h of a grid and its mirror partner.
-__device__ __forceinline__ void grid_half(const GridParams &p, const RingRec *__restrict__ rings,
-                                          GridDev g, int64_t h, DevStatus *st) {
-    int lo = 0, hi = p.nrings - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (rings[mid].hoff <= h) lo = mid;
-        else hi = mid - 1;
+// The largest k < n with at(k) <= u, at(0) <= u, for a whole warp at once: 32 entries
+// a step, so two dependent loads for a thousand entries instead of a binary
+// search's ten. The faces of 256 models of 60-400 strips: 1.21 -> 1.05 ms, their
+// sphere tests 0.36 -> 0.32; the queued candidates of the eclipse stage, whose lanes
+// do not follow one another, lose 2% by it and keep find_seg.
+template <class At>
+__device__ __forceinline__ int warp_search(int n, int64_t u, const At &at) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0;
+    while (n > 1) {
+        const int step = (n + 31) >> 5, o = lane * step;
+        const unsigned m = __ballot_sync(0xffffffffu, o < n && at(lo + o) <= u);
+        const int j = (31 - __clz(m)) * step;
+        lo += j;
+        n = n - j < step ? n - j : step;
     }
+    return lo;
+}
+
+// One half-face h of a grid and its mirror partner; lo: its ring or an earlier one.
+__device__ __forceinline__ void grid_half(const GridParams &p, const RingRec *__restrict__ rings,
+                                          GridDev g, int64_t h, int lo, DevStatus *st) {
+    while (lo + 1 < p.nrings && rings[lo + 1].hoff <= h) lo++;
     const RingRec R = rings[lo];
     const int np = (int)(h - R.hoff);
     const double phi = R.phi1 + R.span * (np + 0.5) / R.nphi;
@@ -96,11 +110,16 @@ __global__ void k_grid(GridParams p, const RingRec *__restrict__ rings, GridDev 
                        int32_t *counters, DevStatus *st) {
     const int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (h < 8) counters[h] = 0;
-    if (h < p.nhalf) grid_half(p, rings, g, h, st);
+    const int64_t h0 = h & ~31ll;
+    if (h0 >= p.nhalf) return;  // whole warps
+    const int lo = warp_search(p.nrings, h0, [&](int i) { return (int64_t)rings[i].hoff; });
+    if (h < p.nhalf) grid_half(p, rings, g, h, lo, st);
 }
 
 // Sphere test of face i: a spherical eclipser sets the range directly; a
-// Roche eclipser makes the face a candidate.
+// Roche eclipser makes the face a candidate. kZero: the range of a face that is
+// never eclipsed is written as zeros (grids that callers read).
+template <bool kZero>
 __device__ __forceinline__ bool ecl_pre_face(const EclParams &p, int32_t eclipse_on, GridDev g,
                                              int64_t i) {
     bool cand = false;
@@ -114,8 +133,10 @@ __device__ __forceinline__ bool ecl_pre_face(const EclParams &p, int32_t eclipse
         g.ein[i] = g.eout[i] = 0.;
     } else {
         g.necl[i] = 0;
-        g.ein[i] = 0.;
-        g.eout[i] = 0.;
+        if constexpr (kZero) {
+            g.ein[i] = 0.;
+            g.eout[i] = 0.;
+        }
         if (eclipse_on) {
             const V3 pos = v3(g.px[i], g.py[i], g.pz[i]);
             const V3 cofm = p.comp_star == kStar1 ? v3(0., 0., 0.) : v3(1., 0., 0.);
@@ -152,7 +173,7 @@ __device__ __forceinline__ void queue_push(bool cand, int32_t item, int32_t *que
 __global__ void k_ecl_pre(EclParams p, int32_t eclipse_on, GridDev g, int32_t *queue,
                           int32_t *counters) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const bool cand = i < g.n && ecl_pre_face(p, eclipse_on, g, i);
+    const bool cand = i < g.n && ecl_pre_face<true>(p, eclipse_on, g, i);
     queue_push(cand, (int32_t)i, queue, counters);
 }
 
@@ -309,7 +330,7 @@ __global__ void __launch_bounds__(128, 4)
     const int64_t i = u >> 1;
     const int side = (int)(u & 1);
     // lane 0 of a pair writes the face's defaults and says whether it is a candidate
-    bool cand = side == 0 && i < g.n && ecl_pre_face(p, eclipse_on, g, i);
+    bool cand = side == 0 && i < g.n && ecl_pre_face<true>(p, eclipse_on, g, i);
     cand = __shfl_sync(full, cand, threadIdx.x & 30);
     if (!__any_sync(full, cand)) return;
     const V3 cofm = p.comp_star == kStar1 ? v3(0., 0., 0.) : v3(1., 0., 0.);
@@ -1275,11 +1296,23 @@ __global__ void __launch_bounds__(128) k_grid_b(BatchDev b) {
     if (nk <= 0) return;
     const int64_t total = b.geo_half[nk];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < total; u += stride) {
-        const int k = find_seg(b.geo_half, nk, u);
+    const int lane = threadIdx.x & 31;
+    for (int64_t u0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); u0 < total;
+         u0 += stride) {
+        int k = warp_search(nk, u0, [&](int i) { return b.geo_half[i]; });
+        const SlotDev &S0 = b.slots[b.geo_slot[k]];
+        const RingRec *rings = b.rings + S0.ring0;
+        int lo = warp_search(S0.gp.nrings, u0 - b.geo_half[k],
+                             [&](int i) { return (int64_t)rings[i].hoff; });
+        const int64_t u = u0 + lane;
+        if (u >= total) continue;
+        while (u >= b.geo_half[k + 1]) {  // the warp reaches into the next slot: its first rings
+            k++;
+            lo = 0;
+        }
         const SlotDev &S = b.slots[b.geo_slot[k]];
-        grid_half(S.gp, b.rings + S.ring0, slot_grid(b.g, S.face0, S.nface, S.ntiled), u - b.geo_half[k],
-                  b.st + S.model);
+        grid_half(S.gp, b.rings + S.ring0, slot_grid(b.g, S.face0, S.nface, S.ntiled),
+                  u - b.geo_half[k], lo, b.st + S.model);
     }
 }
 
@@ -1302,11 +1335,12 @@ __global__ void k_ecl_pre_b(BatchDev b) {
         const int64_t u = u0 + lane;
         bool cand = false, big = false;
         int32_t item = 0;
+        int k = warp_search(nk, u0, [&](int i) { return b.geo_face[i]; });
         if (u < total) {
-            const int k = find_seg(b.geo_face, nk, u);
+            while (u >= b.geo_face[k + 1]) k++;
             const SlotDev &S = b.slots[b.geo_slot[k]];
             const int64_t i = u - b.geo_face[k];
-            cand = ecl_pre_face(S.ep, S.eclipse_on, slot_grid(b.g, S.face0, S.nface, S.ntiled), i);
+            cand = ecl_pre_face<false>(S.ep, S.eclipse_on, slot_grid(b.g, S.face0, S.nface, S.ntiled), i);
             item = (int32_t)(S.face0 + i);
             big = S.ep.comp_rref >= kBigEclipser;
         }
