@@ -288,7 +288,9 @@ __global__ void __launch_bounds__(kThreads64, 4)
 // same doubles): 64 faces at a time are gathered into shared memory, a thread
 // each, so that the serial walk over them meets no chain of global loads (its
 // index, then the face: 92 us for 10,000 faces and 2,000 entries, latency all
-// of it; 31 staged).
+// of it; 31 staged). Then 32 faces at a time, a lane each, are held against all of
+// the warp's entries; those left are summed two at a time without a
+// vote: both stars of an opaque-disc model on 100/200 strips 96 -> 77 us.
 constexpr int kRagTile = 64;
 template <bool POS>
 struct RagFace {
@@ -316,6 +318,16 @@ __global__ void __launch_bounds__(kThreadsRag)
     const Consts64 L{k.c[0], k.c[1], k.c[2], k.c[3], k.base, k.mucrit,
                      k.beam, k.spin, k.vfac, k.xcofm, k.rlens1};
     const double ex = ph.ex[e], ey = ph.ey[e], ez = ph.ez[e], pn = ph.phin[e];
+    const unsigned long long pf = ph.pfx[e];
+    unsigned long long A, La;
+    warp_arc<1>(&pf, A, La);
+    const int lane = threadIdx.x & 31;
+    // every entry of the warp lies within wide of the middle lane's
+    const double cx = __shfl_sync(0xffffffffu, ex, 16), cy = __shfl_sync(0xffffffffu, ey, 16),
+                 cz = __shfl_sync(0xffffffffu, ez, 16);
+    double wide = sqrt((ex - cx) * (ex - cx) + (ey - cy) * (ey - cy) + (ez - cz) * (ez - cz));
+    for (int o = 16; o > 0; o >>= 1) wide = fmax(wide, __shfl_xor_sync(0xffffffffu, wide, o));
+    wide = 1.0001 * wide + 1e-9;
     double acc = part[b * ldp + e];
     const double zb = zero_below<BEAM>(L);
     for (int64_t i0 = c0; i0 < hi; i0 += kRagTile) {
@@ -330,7 +342,8 @@ __global__ void __launch_bounds__(kThreadsRag)
             F.dz = g.nz[fi];
             F.flux = (double)g.flux[fi];
             F.nr = f.rn[r];
-            for (int q = 0; q < kRagRanges; q++) F.r[q] = f.rr[kRagRanges * r + q];
+            for (int q = 0; q < kRagRanges; q++)  // past the last: hides nothing
+                F.r[q] = q < F.nr ? f.rr[kRagRanges * r + q] : make_double2(10., -10.);
             if constexpr (POS) {
                 F.p[0] = g.px[fi];
                 F.p[1] = g.py[fi];
@@ -338,22 +351,43 @@ __global__ void __launch_bounds__(kThreadsRag)
             }
         }
         __syncthreads();
-        for (int t = 0; t < m; t++) {
-            const RagFace<POS> &F = face[t];
-            // at or below zero_below at every entry of the warp: exact zeros
-            const double mu = mu_of(ex, ey, ez, F.dx, F.dy, F.dz);
-            if (!__any_sync(0xffffffffu, mu > zb)) continue;
-            bool ecl = false;
-            for (int q = 0; q < F.nr; q++) {
-                const double2 R = F.r[q];
-                ecl = ecl || (pn >= R.x && pn <= R.y) || pn <= R.y - 1.0;
+        for (int t0 = 0; t0 < m; t0 += 32) {
+            // 32 faces, a lane each: turned away from, or hidden at, all of the warp's
+            // entries; ranges that meet them
+            int c = kGroupDark;
+            if (t0 + lane < m) {
+                const RagFace<POS> &F = face[t0 + lane];
+                if (mu_of(cx, cy, cz, F.dx, F.dy, F.dz) + wide > zb)
+                    c = ranges_class(F.r, F.nr, A, La);
             }
-            if (!__any_sync(0xffffffffu, !ecl && mu > zb)) continue;
-            double px = 0., py = 0., pz = 0.;
-            if constexpr (POS) { px = F.p[0]; py = F.p[1]; pz = F.p[2]; }
-            const double v = elem_mu<LT, BEAM, GLENS, STAR>(mu, ex, ey, ez, F.dx, F.dy, px, py, pz,
-                                                            F.flux, L);
-            if (!ecl) acc += v;
+            unsigned todo = __ballot_sync(0xffffffffu, c != kGroupDark);
+            const unsigned ranged = __ballot_sync(0xffffffffu, c == kGroupRanges);
+            auto value = [&](int t) {
+                const RagFace<POS> &F = face[t0 + t];
+                const double mu = mu_of(ex, ey, ez, F.dx, F.dy, F.dz);
+                bool ecl = false;
+                if ((ranged >> t) & 1u) {
+#pragma unroll
+                    for (int q = 0; q < kRagRanges; q++) {
+                        const double2 R = F.r[q];
+                        ecl = ecl || (pn >= R.x && pn <= R.y) || pn <= R.y - 1.0;
+                    }
+                }
+                double px = 0., py = 0., pz = 0.;
+                if constexpr (POS) { px = F.p[0]; py = F.p[1]; pz = F.p[2]; }
+                const double v = elem_mu<LT, BEAM, GLENS, STAR>(mu, ex, ey, ez, F.dx, F.dy, px, py,
+                                                                pz, F.flux, L);
+                return ecl ? 0.0 : v;
+            };
+            while (todo) {  // two at a time, added in order
+                const int i = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const int j = todo ? __ffs(todo) - 1 : i;
+                const double v = value(i), w = value(j);
+                acc += v;
+                if (todo) acc += w;
+                todo &= todo - 1u;
+            }
         }
     }
     if (e1 < ph.nent) part[b * ldp + e] = acc;

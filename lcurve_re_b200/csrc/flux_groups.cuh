@@ -4,6 +4,7 @@
 #pragma once
 
 #include "engine.h"
+#include "fixed_phase.cuh"
 
 namespace lcg {
 namespace {
@@ -42,6 +43,33 @@ __device__ __forceinline__ int arc_class(const RunRec &R, unsigned long long A,
         return kGroupSigns;
     const unsigned long long o = A - R.all.x;
     return o < R.all.y && L < R.all.y - o ? kGroupDark : kGroupRanges;
+}
+
+// One range [in, out], as the double-precision sweeps test it, against the arc: hidden
+// throughout (kGroupDark), met (kGroupRanges) or not (kGroupSigns). Its ends are drawn
+// in or out by two units; a range that a turn does not hold as it is counts as met.
+__device__ __forceinline__ int range_class(double in, double out, unsigned long long A,
+                                           unsigned long long L) {
+    if (!(in >= 0. && in < 1. && out >= in)) return kGroupRanges;
+    if (out - 1.0 >= in) return kGroupDark;
+    const ulonglong2 E = ecl_fx64(in, out);
+    if (E.y >= ~0ull - 4ull) return kGroupRanges;
+    const unsigned long long x = E.x - 2ull;
+    if (x - A > L && A - x >= E.y + 4ull) return kGroupSigns;
+    const unsigned long long o = A - (E.x + 2ull), y = E.y > 4ull ? E.y - 4ull : 0ull;
+    return o < y && L < y - o ? kGroupDark : kGroupRanges;
+}
+
+// An element's ranges together.
+__device__ __forceinline__ int ranges_class(const double2 *r, int nr, unsigned long long A,
+                                            unsigned long long L) {
+    int c = kGroupSigns;
+    for (int k = 0; k < nr; k++) {
+        const int q = range_class(r[k].x, r[k].y, A, L);
+        if (q == kGroupDark) return q;
+        if (q == kGroupRanges) c = q;
+    }
+    return c;
 }
 
 }  // namespace

@@ -54,3 +54,21 @@ def test_group_classes_leave_the_sums_alone(engine_fp64, oracle, n, n0, nent, or
         a = oracle.sum_star_multi(star, flat, phases, **kw)
         b = engine_fp64.sum_star_multi(star, flat, phases, **kw)
         np.testing.assert_array_equal(a, b)
+
+
+# the several-range faces and the disc's elements: points in any order share a warp
+# with other ranges and horizons
+@pytest.mark.parametrize("npts", [1, 31, 33, 500])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("over", [{}, dict(beam_factor1=1.4, beam_factor2=1.2, mucrit1=-0.3),
+                                  dict(iangle=79.0, limb2="Poly")])
+def test_disc_sums_do_not_depend_on_the_warp(npts, precision, over):
+    from lcurve_re_b200 import workloads as W
+    from lcurve_re_b200.engine import Engine
+    m = W.cv_disc(nlat1f=30, nlat2f=35, nrad=12, nspot=9, **over)
+    d = W.data(npts)
+    perm = np.random.default_rng(npts).permutation(npts)
+    with Engine(precision=precision) as e:
+        a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
+        b = e.light_curve_comp(m, d[perm], scale=False, rdata=False, diagnostics=False)[0]
+    np.testing.assert_array_equal(a[perm], b)
