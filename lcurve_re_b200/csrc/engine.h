@@ -355,6 +355,7 @@ struct FluxPlan {
     int ppt;        // phase entries per thread
     int threads;    // threads per CTA
     int64_t chunk;  // faces per CTA
+    int64_t group;  // general mixed sweep: its FP32 folds count from multiples of this
     int64_t nchunk;
     int64_t ntile;  // phase tiles
 };

@@ -89,7 +89,7 @@ __device__ __forceinline__ int run_class(const RunRec &R, float cut, const float
     return kGroupSigns;
 }
 
-// One fold of cnt faces into the entries' FP32 sums, element by element.
+// cnt faces of a fold into the entries' FP32 sums, element by element.
 template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
 __device__ __forceinline__ void fold_faces(const float4 *gp, const ulonglong2 *ep,
                                            const float4 *pp4, int cnt, const float *ex,
@@ -135,37 +135,47 @@ __device__ __forceinline__ void fold_faces(const float4 *gp, const ulonglong2 *e
     }
 }
 
-// Sums faces [lo, hi) of the staged chunk (first face c0) into acc, in FP32
-// runs of kFold faces folded into FP64. A warp skips a fold whose run (or two
-// runs, where it straddles them) is dark to it, and tests ranges only where they
-// reach its arc of phases; what it leaves out are exact zeros.
+// Sums the faces of [lo, hi) in the staged chunk (first face c0) into acc, in FP32
+// runs of kFold faces from lo on folded into FP64, those that start before stop. A warp skips a fold whose run is dark to it,
+// and in the others the parts of 16 faces that are (64 faces of a 121-strip grid span
+// a quarter of the horizon, and half of what the run's bounds let through is turned
+// away); ranges are tested only in parts where they reach its arc of phases. What it
+// leaves out are exact zeros.
 template <int PPT, int LT, bool BEAM, bool GLENS, int STAR, bool ECL>
 __device__ __forceinline__ void sweep(const float4 *sgeo, const ulonglong2 *secl,
                                       const float4 *spos, const RunRec *__restrict__ runs,
-                                      int64_t c0, int64_t lo, int64_t hi, const float *ex,
-                                      const float *ey, const float *ez,
+                                      int64_t c0, int64_t lo, int64_t stop, int64_t hi,
+                                      const float *ex, const float *ey, const float *ez,
                                       const unsigned long long *pf, unsigned long long A,
                                       unsigned long long L, const FaceConsts &k, double *acc) {
+    constexpr int kPart = 16;
     const float cut = BEAM ? k.mucrit : k.cut;
-    for (int64_t b = lo; b < hi; b += kFold) {
-        const int cnt = (int)((b + kFold < hi) ? kFold : hi - b);
-        const int64_t r0 = b / kRunFaces, r1 = (b + cnt - 1) / kRunFaces;
-        int c = run_class<PPT, ECL>(runs[kRunRecs * r0], cut, ex, ey, ez, A, L);
-        if (r1 != r0) {
-            const int c1 = run_class<PPT, ECL>(runs[kRunRecs * r1], cut, ex, ey, ez, A, L);
-            // one of the two may be dark for its ranges: test each face's
-            if (c != c1) c = ECL ? kGroupRanges : kGroupSigns;
-        }
-        if (c == kGroupDark) continue;
-        const float4 *gp = sgeo + (b - c0), *pp4 = spos + (b - c0);
-        const ulonglong2 *ep = secl + (b - c0);
+    for (int64_t b = lo; b < stop && b < hi; b += kFold) {
+        const int64_t end = b + kFold < hi ? b + kFold : hi;
+        const int64_t r0 = b / kRunFaces, r1 = (end - 1) / kRunFaces;
+        if (r0 == r1 &&
+            run_class<PPT, ECL>(runs[kRunRecs * r0], cut, ex, ey, ez, A, L) == kGroupDark)
+            continue;
         float s[PPT];
 #pragma unroll
         for (int j = 0; j < PPT; j++) s[j] = 0.f;
-        if (ECL && c == kGroupRanges)
-            fold_faces<PPT, LT, BEAM, GLENS, STAR, ECL>(gp, ep, pp4, cnt, ex, ey, ez, pf, k, s);
-        else
-            fold_faces<PPT, LT, BEAM, GLENS, STAR, false>(gp, ep, pp4, cnt, ex, ey, ez, pf, k, s);
+#pragma unroll 1
+        for (int64_t p = b; p < end;) {
+            const int64_t q = p / kPart, pe = kPart * (q + 1) < end ? kPart * (q + 1) : end;
+            const int c = run_class<PPT, ECL>(runs[kRunRecs * (q >> 2) + 1 + (q & 3)], cut, ex, ey,
+                                              ez, A, L);
+            const float4 *gp = sgeo + (p - c0), *pp4 = spos + (p - c0);
+            const int cnt = (int)(pe - p);
+            if (c == kGroupDark) {
+            } else if (ECL && c == kGroupRanges) {
+                fold_faces<PPT, LT, BEAM, GLENS, STAR, ECL>(gp, secl + (p - c0), pp4, cnt, ex, ey,
+                                                            ez, pf, k, s);
+            } else {
+                fold_faces<PPT, LT, BEAM, GLENS, STAR, false>(gp, nullptr, pp4, cnt, ex, ey, ez,
+                                                              pf, k, s);
+            }
+            p = pe;
+        }
 #pragma unroll
         for (int j = 0; j < PPT; j++) acc[j] += (double)s[j];
     }
@@ -173,29 +183,32 @@ __device__ __forceinline__ void sweep(const float4 *sgeo, const ulonglong2 *secl
 
 template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
 __global__ void __launch_bounds__(kThreads)
-    k_flux_mixed(FluxConsts k, FlatDev f, PhaseDev ph, int64_t chunk, double *part,
+    k_flux_mixed(FluxConsts k, FlatDev f, PhaseDev ph, int64_t chunk, int64_t group, double *part,
                  int64_t ldp, DevStatus *st) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
     const int tid = threadIdx.x;
     const int64_t c0 = (int64_t)blockIdx.y * chunk;
     const int64_t n = f.n, n0 = *f.n0;
-    const int64_t cend = (c0 + chunk < n) ? c0 + chunk : n;
+    // The FP32 folds count from the group's first face, and from n0 within it: this CTA
+    // takes those that start in its chunk, the last of which may reach past it
+    const int64_t g0 = c0 / group * group, gend = g0 + group < n ? g0 + group : n;
+    const int64_t cend = c0 + chunk < gend ? c0 + chunk : gend;
+    const int64_t rows = c0 + chunk + kFold < g0 + group ? chunk + kFold : g0 + group - c0;
     const bool need_ecl = cend > n0;
     constexpr bool need_pos = BEAM || GLENS;
     float4 *sgeo = reinterpret_cast<float4 *>(smem);
-    ulonglong2 *secl = reinterpret_cast<ulonglong2 *>(smem + chunk * 16);
-    float4 *spos = reinterpret_cast<float4 *>(smem + chunk * 32);
+    ulonglong2 *secl = reinterpret_cast<ulonglong2 *>(smem + rows * 16);
+    float4 *spos = reinterpret_cast<float4 *>(smem + rows * 32);
 
     if (tid == 0) mbar_init(&bar, 1);
     __syncthreads();
     if (tid == 0) {
-        uint32_t bytes = (uint32_t)(chunk * 16) + (need_ecl ? (uint32_t)(chunk * 16) : 0u) +
-                         (need_pos ? (uint32_t)(chunk * 16) : 0u);
-        mbar_arrive_expect_tx(&bar, bytes);
-        bulk_g2s(sgeo, f.geo + c0, (uint32_t)(chunk * 16), &bar);
-        if (need_ecl) bulk_g2s(secl, f.ecl + c0, (uint32_t)(chunk * 16), &bar);
-        if (need_pos) bulk_g2s(spos, f.pos + c0, (uint32_t)(chunk * 16), &bar);
+        const uint32_t col = (uint32_t)(rows * 16);
+        mbar_arrive_expect_tx(&bar, col + (need_ecl ? col : 0u) + (need_pos ? col : 0u));
+        bulk_g2s(sgeo, f.geo + c0, col, &bar);
+        if (need_ecl) bulk_g2s(secl, f.ecl + c0, col, &bar);
+        if (need_pos) bulk_g2s(spos, f.pos + c0, col, &bar);
     }
 
     // phase entries of this thread, loaded while the faces stream in: PPT
@@ -234,11 +247,14 @@ __global__ void __launch_bounds__(kThreads)
     for (int j = 0; j < PPT; j++) acc[j] = 0.0;
     const FaceConsts fc{c1, c2, c3, c4, base, cut, (float)k.mucrit, vfac, spin, xcofm, beam,
                         k.rlens1};
-    // plain faces [c0, min(n0,cend)), then one-range faces [max(n0,c0), cend)
-    sweep<PPT, LT, BEAM, GLENS, STAR, false>(sgeo, secl, spos, f.runs, c0, c0,
+    // plain faces [c0, min(n0, cend)), then one-range faces in folds of 64 from the
+    // group's first one on
+    sweep<PPT, LT, BEAM, GLENS, STAR, false>(sgeo, secl, spos, f.runs, c0, c0, cend,
                                             n0 < cend ? n0 : cend, ex, ey, ez, pf, A, L, fc, acc);
-    sweep<PPT, LT, BEAM, GLENS, STAR, true>(sgeo, secl, spos, f.runs, c0, n0 > c0 ? n0 : c0, cend,
-                                           ex, ey, ez, pf, A, L, fc, acc);
+    const int64_t o0 = n0 > g0 ? n0 : g0;
+    const int64_t lo = o0 >= c0 ? o0 : o0 + (c0 - o0 + kFold - 1) / kFold * kFold;
+    sweep<PPT, LT, BEAM, GLENS, STAR, true>(sgeo, secl, spos, f.runs, c0, lo, cend, gend, ex, ey,
+                                           ez, pf, A, L, fc, acc);
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
         const int64_t e = ebase + j;
@@ -249,12 +265,13 @@ __global__ void __launch_bounds__(kThreads)
 template <int PPT, int LT, bool BEAM, bool GLENS, int STAR>
 void launch_t(const FluxConsts &k, const FlatDev &f, const PhaseDev &ph, const FluxPlan &plan,
               double *part, int64_t ldp, DevStatus *st, cudaStream_t s) {
-    const size_t smem = (size_t)plan.chunk * ((BEAM || GLENS) ? 48 : 32);
+    const int64_t rows = plan.chunk + kFold < plan.group ? plan.chunk + kFold : plan.group;
+    const size_t smem = (size_t)rows * ((BEAM || GLENS) ? 48 : 32);
     auto kern = k_flux_mixed<PPT, LT, BEAM, GLENS, STAR>;
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid((unsigned)plan.ntile, (unsigned)plan.nchunk);
-    kern<<<grid, kThreads, smem, s>>>(k, f, ph, plan.chunk, part, ldp, st);
+    kern<<<grid, kThreads, smem, s>>>(k, f, ph, plan.chunk, plan.group, part, ldp, st);
     count_launch();
 }
 
@@ -705,12 +722,25 @@ FluxPlan plan_flux(int mixed, int fast, int64_t nface, int64_t nent, int nsm) {
         p.ppt = nent >= 16384 ? 8 : (nent >= 2048 ? 4 : 1);
         p.ntile = (nent + (int64_t)kThreads * p.ppt - 1) / ((int64_t)kThreads * p.ppt);
         if (p.ntile < 1) p.ntile = 1;
-        // enough CTAs to fill the SMs a few times over; chunk a power of two
-        // in [64, 4096] so that chunks tile the 4096-padded face arrays
+        // The group fixes where the FP32 folds of one-range faces start: four CTAs' worth
+        // for each SM, a power of two in [64, 4096], which tile the padded arrays.
         const int64_t want = ((int64_t)nsm * 4 + p.ntile - 1) / p.ntile;
-        int64_t chunk = 4096;
-        while (chunk > 64 && (nface + chunk - 1) / chunk < want) chunk >>= 1;
-        p.chunk = chunk;
+        p.group = 4096;
+        while (p.group > 64 && (nface + p.group - 1) / p.group < want) p.group >>= 1;
+        // The chunk only regroups FP64 sums: the one whose whole waves, three CTAs an SM
+        // (80 registers), cost least, a CTA's faces plus some 32 faces' worth of loading
+        // and ending. 9,003 entries and 18,600 faces: 256 faces fill 1.5 waves, 136 us;
+        // 128 three, 111. Above 1024 the shared memory would turn CTAs away.
+        const int64_t slots = 3 * (int64_t)nsm;
+        int64_t best = INT64_MAX;
+        for (int64_t chunk = p.group < 1024 ? p.group : 1024; chunk >= 64; chunk >>= 1) {
+            const int64_t ctas = (nface + chunk - 1) / chunk * p.ntile;
+            const int64_t cost = (ctas + slots - 1) / slots * (chunk + 32);
+            if (cost < best) {
+                best = cost;
+                p.chunk = chunk;
+            }
+        }
     } else {
         p.threads = 256;  // kThreads64, an entry each
         p.ntile = (nent + p.threads - 1) / p.threads;
