@@ -352,9 +352,8 @@ void launch_ppt(int star, const FluxConsts &k, const FlatDev &f, const PhaseDev 
 //   fI  = flux * I(t), Horner on per-face coefficients 4 FFMA2
 //   s  += m * fI                                       1 FFMA2
 // one-range faces add the fixed-point eclipse test (a 64-bit subtract and
-// compare, and a select, per face), skipped for a run of 32 pairs whose
-// ranges' hull misses the warp's arc of phases (an exact test on the circle,
-// once per run).
+// compare, and a select, per face). Groups of faces that are dark, or bright, to
+// all of a warp's entries need neither the max nor the test (group_class).
 // Each thread holds PPT consecutive phase entries, so a warp covers 32 * PPT
 // consecutive entries: a narrow arc of the orbit for time-ordered points.
 // A face pair that faces away (mu <= 0) or is eclipsed at every entry of the

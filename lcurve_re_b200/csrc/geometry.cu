@@ -1,14 +1,15 @@
 // geometry.cu — the FP64 stages of one light curve, compiled with
 // --fmad=false so that every product and sum rounds as in the reference:
 //   k_grid       face radius solve, normal, gravity, area (set_star_grid.cpp:226-523)
-//   k_ecl_pre    sphere pre-test + compaction of Roche eclipse candidates
-//   k_ecl_roche  ingress/egress of the candidates from a work queue
-//   k_continuum  gravity darkening, irradiation, black body (set_star_continuum.cpp)
+//   k_ecl_*      sphere pre-test, Roche eclipse candidates, their ingress and egress
+//   k_continuum  gravity darkening, irradiation, black body (set_star_continuum.cpp),
+//                sums behind logg and the volume-averaged radius (comp_gravity.cpp,
+//                comp_radius.cpp)
 //   k_flat_*     stable partition into FlatGrid order (comp_light_flat.cpp:26-65)
 //   k_phases     per-point phase and sub-exposure entries (light_curve_comp.cpp:350-455)
 //   k_scatter    merge of the flux partials into the light curve (:457-498)
+//   k_run_bounds* the sweeps' records of face groups
 //   k_finalize   scale factor and chi**2 (re_scale.cpp:16-42, light_curve_comp.cpp:557-585)
-//   k_diag       sums behind logg and the volume-averaged radius (comp_gravity.cpp, comp_radius.cpp)
 #include <stdlib.h>
 
 #include "eclipse.cuh"
