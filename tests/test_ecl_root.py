@@ -24,7 +24,7 @@ EXE = os.path.join(HERE, "screen", "_build", "root_check")
 
 
 @pytest.fixture(scope="module")
-def checker():
+def root_check():
     if shutil.which("g++") is None:
         pytest.skip("g++ not available")
     os.makedirs(os.path.dirname(EXE), exist_ok=True)
@@ -54,11 +54,11 @@ def _run(exe, m, star, posn):
     (0.6, dict(q=3.0, r2=0.35)), (0.6, dict(spin1=0.0, spin2=0.0)),
     (0.6, dict(spin1=20.0, spin2=1.8, r2=0.15)),
     (0.6, dict(delta_phase="1e-9")), (0.3, dict(delta_phase="1e-4"))])
-def test_roots_keep_every_decision(checker, oracle, most, over):
+def test_roots_keep_every_decision(root_check, oracle, most, over):
     m = W.model(nlat1f=16, nlat2f=36, **over)
     tests = zone = 0
     for star in (0, 1):
-        rc, r = _run(checker, m, star, oracle.star_grid(m, star)["posn"])
+        rc, r = _run(root_check, m, star, oracle.star_grid(m, star)["posn"])
         assert rc == 0 and r["wrong"] == 0, (star, r)
         tests += r["tests"]
         zone += r["zone"]
@@ -70,9 +70,9 @@ def test_roots_keep_every_decision(checker, oracle, most, over):
 # smaller and larger eclipsers, finer and coarser bisections
 @pytest.mark.parametrize("r2", [0.08, 0.13, 0.17, 0.19, 0.205, 0.22, 0.235])
 @pytest.mark.parametrize("delta", ["1e-6", "1e-7", "1e-8"])
-def test_narrowed_gaps_keep_every_decision(checker, oracle, r2, delta):
+def test_narrowed_gaps_keep_every_decision(root_check, oracle, r2, delta):
     m = W.model(nlat1f=14, nlat2f=20, r2=r2, delta_phase=delta, iangle=87.0)
-    rc, r = _run(checker, m, 0, oracle.star_grid(m, 0)["posn"])
+    rc, r = _run(root_check, m, 0, oracle.star_grid(m, 0)["posn"])
     assert rc == 0 and r["wrong"] == 0, r
     if delta == "1e-7":
         assert r["searches"] <= 0.01 * r["tests"], r
