@@ -1318,9 +1318,9 @@ __global__ void __launch_bounds__(128) k_grid_b(BatchDev b) {
 }
 
 // Eclipsers whose reference sphere is at least this large share the front of
-// the batch queue: their boundaries take a few searches each (ecl_root.cuh),
-// those of a white dwarf almost none, and a warp runs at its slowest lane's
-// pace.
+// the batch queue: a warp runs at its slowest lane's pace, and the boundaries of a
+// white dwarf and of a larger star take different steps (ecl_root.cuh: the former
+// have no gap to narrow). 256 models: bisections 3.84 ms so, 4.43 in queue order.
 constexpr double kBigEclipser = 0.05;
 
 // Sphere pre-test of the geometry list's faces; candidates are queued by
