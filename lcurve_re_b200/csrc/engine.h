@@ -119,7 +119,8 @@ struct FlatDev {
     // with cz = cos(i) nz and f_k = flux * p_k, so each float2 operand of the
     // packed FP32x2 arithmetic is an aligned register pair
     float *fp;
-    // bounds of every 64 consecutive faces of fp (of geo with nz for the z term)
+    // bounds of every 64 consecutive faces of fp (of geo or the FP64 columns, with nz
+    // for the z term)
     // and of their four parts of 16: kRunRecs records per run, the run's first
     RunRec *runs;
     // faces with two or more eclipse ranges (opaque discs) sit last, in
@@ -148,7 +149,7 @@ struct PhaseDev {
     float4 *ef;     // (ex, ey, ez, unused) for the mixed sweeps
     uint8_t *type;  // Ginterp::type
     int64_t nent;
-    unsigned long long *pfx;  // phin as a 64-bit fixed-point fraction (mixed)
+    unsigned long long *pfx;  // phin as a 64-bit fixed-point fraction
 };
 
 struct PhaseParams {
