@@ -410,7 +410,7 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
             const EdgeBound B = edge_bound(S, v, lam);
             const double r = sqrt(v.r2);
             double rad = B.rad, K = B.K, fl = fp, extra = 4. * v.tol;
-            double gp = 0., move = 0., t3 = 0.;
+            double gp = 0., move = 0., t3 = 0., cap = 0.;
             bool ok = true;
             if (stage) {
                 // curvature along the line keeps 0.6 h while the point moves by
@@ -434,6 +434,13 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
                 const double db2 = -2. * v.x * v.xp * dir;
                 const double rb = 0.5 * db2 / (kTwoPi * kTwoPi * (1.3 * v.b2 + u2));
                 if (rb < rad) rad = rb;
+                // outwards it shrinks, and one of length acc or less is not searched:
+                // d(b^2)/dw w + 2 (2 pi)^2 |u0|^2 w^2 must leave that much
+                const double two2u = kTwoPi * kTwoPi * u2;
+                const double room =
+                    S.rref2 - v.b2 - 0.25 * acc * acc * (1. + 1e-5) - 1e-12 * (1. + u2);
+                cap = room / (1.1 * db2);
+                if (cap > 0.05 * db2 / two2u) cap = 0.05 * db2 / two2u;
             }
             if (rad * K > 0.8 * fl) rad = 0.8 * fl / K;
             // f (or the minimum) within the zone is f0 + fl w up to K w^2 / 2 and
@@ -455,6 +462,7 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
                 z.hc = pout + dir * w;
                 z.hrad = rad;
                 z.hid = -s0 - off - 4e-15;
+                if (z.hid > 0. && z.hid > cap) z.hid = cap > 0. ? cap : 0.;
                 vis0 = -s0 + off + 4e-15;
                 stage = 1;
                 w -= s0;

@@ -66,6 +66,21 @@ def test_roots_keep_every_decision(root_check, oracle, most, over):
     assert zone >= most * tests, (zone, tests)
 
 
+# small eclipsers and coarse bisections, where the chord through the reference sphere
+# falls to the search's accuracy before the potential reaches its root
+@pytest.mark.parametrize("star,over", [
+    (0, dict(q=0.0428, iangle=83.0, r1=0.17, r2=0.0634, spin1=7.12, delta_phase="7.5e-5")),
+    (1, dict(q=0.794, iangle=83.02, r1=0.087, r2=-1.0, delta_phase="4.64e-5")),
+    (1, dict(q=0.313, iangle=89.4, r1=0.00694, r2=-1.0, spin2=0.484, delta_phase="2.49e-6")),
+    (1, dict(q=2.76, iangle=79.39, r1=0.01026, r2=0.2134, spin1=14.8, delta_phase="1.12e-6")),
+    (1, dict(q=0.705, iangle=83.46, r1=0.0983, r2=0.1346, delta_phase="2.58e-5"))])
+def test_short_chords_keep_every_decision(root_check, oracle, star, over):
+    m = W.model(nlat1f=20, nlat2f=34, **over)
+    rc, r = _run(root_check, m, star, oracle.star_grid(m, star)["posn"])
+    assert rc == 0 and r["wrong"] == 0, r
+    assert r["tests"] > 100
+
+
 # the search's second step from less than half of its accuracy to several times it:
 # smaller and larger eclipsers, finer and coarser bisections
 @pytest.mark.parametrize("r2", [0.08, 0.13, 0.17, 0.19, 0.205, 0.22, 0.235])
