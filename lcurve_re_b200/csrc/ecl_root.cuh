@@ -11,7 +11,8 @@
 //     the closest approach to the eclipser's centre; f <= pref answers "hidden"
 //     at once;
 //   * when the lowest potential on the chord exceeds pref, nothing that the
-//     search evaluates can reach it: "not hidden";
+//     search evaluates can reach it: "not hidden" (the lowest on the whole chord,
+//     which its minimum near the midpoint need not be, see EdgeEval);
 //   * in between, the search's second step answers nearly always (narrow_zone).
 //
 // edge_zone finds the root of f(phase) - pref by Newton's method and, with a
@@ -38,8 +39,11 @@ enum { kEdgeFalse = 0, kEdgeTrue = 1, kEdgeUnsure = 2 };
 
 // Potential about the eclipser's centre (the shift moved into pref):
 //   f(u) = -me/|u| - mo/|u - (dx,0,0)| - ss/2 (ux^2 + uy^2) + k ux - pref
+// gap = 1 - rref (no point of the reference sphere is nearer to the other star), er = me / rref,
+// er3 = me / rref^3, bend = 2 mo / gap^3 + ss (the other terms curve down by no more there)
+// and, where er3 exceeds it clearly, ik = 2 / (er3 - bend), else 0.
 struct EdgeStar {
-    double me, mo, dx, ss, k, pref, rref2, cosi, sini;
+    double me, mo, dx, ss, k, pref, rref2, cosi, sini, gap, er, er3, bend, ik;
 };
 
 LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, double sini,
@@ -56,19 +60,38 @@ LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, dou
         s.pref = pref + comp;
     }
     s.rref2 = rref * rref;
+    s.gap = 1. - rref;
+    s.er = s.me / rref;
+    s.er3 = s.er / s.rref2;
+    s.bend = 2. * s.mo / (s.gap * s.gap * s.gap) + s.ss;
+    s.ik = s.er3 - s.bend > 0.04 * s.er3 ? 2. / (s.er3 - s.bend) : 0.;
     s.cosi = cosi;
     s.sini = sini;
     return s;
 }
 
+// Whether the chord has no second well. "Not hidden" follows from the potential's minimum
+// near the midpoint only where no other lies lower: a contact binary's other star, with
+// an extreme mass ratio and the eclipser a slow rotator, digs one at the near end, and
+// Roche::fblink finds it. From a point at a distance t1 from the midpoint where f is at least
+// f0 and its slope outwards at least s0, the eclipser's term E(t) = -me / sqrt(b^2 + t^2) is
+// known exactly and the rest, the other star's and the rotation's, curves down by t2 at most:
+//   f(t) >= M(t) = f0 + E(t) - E(t1) + (s0 - E'(t1)) (t - t1) - t2 (t - t1)^2 / 2.
+// M bends down once at most on the way out, so with s0 >= 0 it is lowest at t1 or at the
+// chord's end, where E is -me / rref. t2 = bend (EdgeStar) serves most eclipsers and both
+// ends. Where the chord lies beyond the other star, which the line passes at a distance p,
+// and its near end w beyond that, 2 w^2 >= 3 p^2, that star's curvature grows all the
+// way to the near end: f itself bends down once at most, so its value there decides, and
+// towards the far end t2 is what it is at t1.
+
 // One evaluation on the line of sight at a phase, a distance t beyond the
 // chord's midpoint: f, df/dphase (t held), slope g and curvature h along the
 // line; squared distances b2 (closest approach), r2 (of the point) from the
-// eclipser's centre and inverse distance io from the other star's; x, the way
-// to the midpoint, and its rate xp; main term ae = m_e / r^3; a bound tol on
-// the rounding of f.
+// eclipser's centre, distance d from the other star's and its inverse io; x, the
+// way to the midpoint, and its rate xp; main term ae = m_e / r^3; a bound tol on
+// the rounding of f; the line's direction (ex, ey, cos i).
 struct EdgeEval {
-    double f, fp, g, h, b2, r2, io, x, xp, ae, tol;
+    double f, fp, g, h, b2, r2, d, io, x, xp, ae, tol, ex, ey;
     int ans;  // kEdge*: what fblink answers at this phase (t = 0)
     bool on;  // the chord exists and f and the rest are set
 };
@@ -121,7 +144,8 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
     const double ux = fma(lam, ex, u0.x), uy = fma(lam, ey, u0.y), uz = fma(lam, ez, u0.z);
     const double vx = ux - S.dx;
     const double rxy = fma(ux, ux, uy * uy), r2 = fma(uz, uz, rxy);
-    const double ie = edge_rsqrt(r2), io = edge_rsqrt(fma(vx, vx, fma(uy, uy, uz * uz)));
+    const double d2 = fma(vx, vx, fma(uy, uy, uz * uz));
+    const double ie = edge_rsqrt(r2), io = edge_rsqrt(d2);
     const double ie2 = ie * ie, io2 = io * io, pe = S.me * ie, po = S.mo * io;
     const double ae = pe * ie2, ao = po * io2;
     r.f = fma(S.k, ux, fma(-0.5 * S.ss, rxy, -(pe + po))) - S.pref;
@@ -136,8 +160,11 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
     r.fp = fma(r.xp, r.g, lam * fma(gx, px, gy * py));
     r.b2 = b2;
     r.r2 = r2;
+    r.d = d2 * io;
     r.io = io;
     r.x = x;
+    r.ex = ex;
+    r.ey = ey;
     r.ae = ae;
     r.tol = 1e-14 * (pe * ie + po * io + pe + po + 1.);
     r.on = true;
@@ -149,11 +176,30 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
     // eclipser's curvature falls by at most 5 (tau / b)^2 of itself (tau <= b / 10)
     // and the other star's changes by at most 6 mo / r^4 per length
     if (r.f > r.tol && r.h > 0.) {
-        const double tau = 2. * fabs(r.g) / r.h, near = 1. / io - tau;
+        const double ag = fabs(r.g), tau = 2. * ag / r.h, near = r.d - tau;
         if (100. * tau * tau <= b2 && tau * tau <= hc2 && near > 0.1) {
             const double c3 = 6. * S.mo / (near * near * near * near);
             const double hmin = r.h - 5. * ae * tau * tau * ie2 - c3 * tau;
-            if (hmin > 0. && r.f - r.g * r.g / (2. * hmin) > r.tol) r.ans = kEdgeFalse;
+            const double low = r.f - ag * ag / (2. * hmin);
+            if (hmin >= 0.5 * r.h && low > r.tol) {
+                // and the rest of the chord, from tau on with f >= low and the slope at
+                // least hmin tau - |g| >= 0 there; hc <= rref spares most their square root
+                const double c = (hmin - ae) * tau - ag, c0 = c < 0. ? c : 0.;
+                const double top = low + pe - 0.5 * ae * tau * tau - S.er - r.tol;
+                if (top + c0 * (1. - S.gap) > 0.5 * S.bend * hc2) {
+                    r.ans = kEdgeFalse;
+                } else {
+                    const double hc = hc2 * edge_rsqrt(hc2), wn = ev - hc, p2 = d2 - ev * ev;
+                    const double curl = r.h < ae ? ae - r.h : 0.;
+                    const double nx = fma(-hc, ex, ux), ny = fma(-hc, ey, uy);
+                    const double fn = fma(S.k, nx, fma(-0.5 * S.ss, fma(nx, nx, ny * ny),
+                                                       -S.mo * edge_rsqrt(fma(wn, wn, p2)))) -
+                                      S.er - S.pref;
+                    if (wn > 0. && 2. * wn * wn >= 3. * p2 && fn > r.tol &&
+                        top + c0 * hc > 0.5 * curl * hc2)
+                        r.ans = kEdgeFalse;
+                }
+            }
         }
     }
     return r;
@@ -276,13 +322,88 @@ LCG_HD EdgeBound edge_bound(const EdgeStar &S, const EdgeEval &v, double lam) {
     return B;
 }
 
+// The part of a phase radius rad around v (edge_zone's stage 1) over which the chord has
+// no second well, 0 for none: M above from the minimum outwards (f >= 0 there from vis on,
+// its slope 0). The minimum lies within a of the midpoint, and f has no other within move of
+// v's point, less that point's own motion. vis < 0 reaches inwards of v. With y half the
+// chord and ae = me / r^3 at the minimum, M is above zero at an end of the chord where
+//   E(y) - E(a) > ae a y + t2 (y + a)^2 / 2.
+// First for both ends with t2 = bend: E(y) - E(a) >= er3 (y^2 - a^2) / 2 makes that so for
+// every y >= need, and a shorter chord is clear while it lies within move, or gone. Where
+// the eclipser's pull at its reference sphere is too weak for that (it fills its lobe), the
+// ends one by one while the chord keeps most of its length: the far one with t2 as it is at
+// the minimum, the near one by f itself, less what it can lose on its way. Of detached
+// binaries' boundaries all but 0.1% are certified, of lobe-filling donors' 5% are not.
+LCG_HD double clear_radius(const EdgeStar &S, V3 u0, const EdgeEval &v, double dir, double t,
+                           double lam, double dt, double drift, double move, double vis,
+                           double rad) {
+    // b^2 grows outwards by 0.8 to 1.2 db2 per phase
+    const double db2 = -2. * v.x * v.xp * dir, bend = kTwoPi * kTwoPi / 1.1 * lam * lam;
+    if (!(db2 > 0.)) return 0.;
+    if (rad * bend > 0.1 * db2) rad = 0.1 * db2 / bend;
+    const double in = vis < 0. ? -2.1 * kTwoPi * lam * lam * vis : 0.;
+    const double hc2 = S.rref2 - v.b2, y2 = hc2 + in, at = fabs(t), ae = 1.1 * v.ae;
+    double a = at + fabs(dt) + drift * rad;
+    if (!(y2 > 0.)) return rad;
+    if (!(in < 0.05 * v.b2 && 110. * a * a < v.b2)) return 0.;
+    if (S.ik > 0.) {
+        const double need = a * (ae + 0.5 * (S.er3 + S.bend)) * S.ik;
+        const double speed = 1.2 * kTwoPi * lam, left = move - at - need;
+        const double room = hc2 - need * need;
+        // gone at y2 / (0.8 db2) at the latest
+        if (left * 0.8 * db2 >= y2 * speed) return rad;
+        if (room > 0.5 * hc2) {
+            const double r0 = room / (1.2 * db2);
+            return rad < r0 ? rad : r0;
+        }
+    }
+    if (!(hc2 > 0.)) return 0.;
+    // the far end: t2 is the other terms' curvature at v, with what it changes by
+    const double ih = edge_rsqrt(hc2), hc = hc2 * ih, io2 = v.io * v.io, ib2 = 1. / db2;
+    const double t0 = v.ae * (1. - 3. * t * t / v.r2) - v.h;
+    const double tv = (t0 > 0. ? t0 : 0.) + 9. * S.mo * io2 * io2 * move;
+    double r1 = 0.;
+#pragma unroll 1
+    for (int i = 0; i < 2; i++) {
+        const double keep = i ? 0.92 : 0.75;
+        r1 = (1. - keep) / 1.2 * hc2 * ib2;
+        if (r1 > rad) r1 = rad;
+        a = at + fabs(dt) + drift * r1;
+        const double tf = tv + 9. * S.mo * io2 * io2 * a +
+                          2. * kTwoPi * r1 * (2.7 * S.mo * io2 * v.io + S.ss);
+        const double yl = (i ? 0.9591 : 0.8660) * hc;
+        const double ib = edge_rsqrt(S.rref2 - yl * yl + a * a);
+        const double ey = S.me * ib - S.er, ey2 = 0.97 * S.me * ib * ib * ib;
+        // and from there on, E growing by at least ey2 / 2 per y^2
+        if (ey > ae * a * yl + 0.5 * tf * (yl + a) * (yl + a) && ey2 * yl > ae * a + tf * (yl + a))
+            break;
+        if (i) return 0.;
+    }
+    const double ex = v.ex, ey = v.ey, ez = S.cosi, l = v.x - hc;
+    const double nx = fma(l, ex, u0.x), ny = fma(l, ey, u0.y), nz = fma(l, ez, u0.z);
+    const double vx = nx - S.dx, dn2 = fma(vx, vx, fma(ny, ny, nz * nz)), ni = edge_rsqrt(dn2);
+    const double wn = fma(ex, vx, fma(ey, ny, ez * nz));
+    const double fn = fma(S.k, nx, fma(-0.5 * S.ss, fma(nx, nx, ny * ny), -S.mo * ni)) - S.er - S.pref;
+    if (!(wn > 0. && dn2 - wn * wn < 0.22 * dn2 && fn > 0.)) return 0.;
+    // the near end's speed along the sphere, and that of the other star's distance; x > hc,
+    // the element being outside the sphere
+    const double vel = kTwoPi * (lam + 1.) + 1.4 * db2 * ih;
+    const double grad = 1.25 * S.mo * ni * ni + fabs(S.k) + 1.1 * S.ss * (1. - S.gap);
+    const double most = 0.1 * dn2 * ni;
+    double r2 = 0.9 * fn;
+    if (r2 > most * grad) r2 = most * grad;
+    if (r1 * vel * grad > r2) r1 = r2 / (vel * grad);
+    if (r1 * (kTwoPi * lam) > 0.1 * v.x) r1 = 0.1 * v.x / (kTwoPi * lam);
+    return r1 < -vis ? 0. : r1;
+}
+
 // What is known at the visible end of a boundary (edge_zone's stage 1), for
 // narrow_zone.
 struct EdgeEnd {
     double t, dt, tol;           // offset of the minimum, its last step; rounding of f
     double s0, off, fp, fl, K, rad;  // the Newton root of the minimum, its error, bounds
     double gp, move, t3, vis0;   // bounds; where f(midpoint) > 0 from on, from hc
-    double r, h, ae, io, b2;     // EdgeEval's
+    double r, h, ae, io, b2, x, ex, ey;  // EdgeEval's
 };
 
 // Between hid and vis fblink searches: f > pref at the midpoint x, the minimum
@@ -316,10 +437,7 @@ LCG_HD void narrow_zone(const EdgeStar &S, V3 u0, double acc, double dir, double
     const double ni = E.io / (1. - 1.1 * hc * E.io), ir = edge_rsqrt(S.rref2);
     const double t2 = 2. * S.mo * ni * ni * ni + S.ss, rise = S.me * ir * ir * ir - t2;
     if (!(rise > 0.3 * t2)) return;
-    double sn, cs;
-    edge_sincos(z.vc, sn, cs);
-    const double ex = S.sini * cs, ey = -S.sini * sn, ez = S.cosi;
-    const double x = -fma(ex, u0.x, fma(ey, u0.y, ez * u0.z));
+    const double ex = E.ex, ey = E.ey, ez = S.cosi, x = E.x;
     const double tm = fabs(E.t + E.dt), sg = E.t + E.dt > 0. ? 1. : -1.;
     // slopes towards the minimum at x (g), u1 (g1) and u2; the value at u2 (f2)
     double g = 0., g1 = 0., d1 = 0., den = 1., step = 0., f2 = 0.;
@@ -451,11 +569,14 @@ LCG_HD EdgeZone edge_zone(const EdgeStar &S, V3 u0, double acc, double delta, do
                 fabs(s0) + off < rad && off <= fine * delta) {
                 // 4e-15: the rounding of phases near 1
                 if (stage) {
+                    const double clear = clear_radius(S, u0, v, dir, t, lam, dt, gp / (0.6 * v.h),
+                                                      move, off - s0, rad);
+                    if (!(fabs(s0) + off < clear)) return z;
                     z.vc = pout + dir * w;
-                    z.vrad = rad;
+                    z.vrad = clear;
                     z.vis = -s0 + off + 4e-15;
                     const EdgeEnd E{t, dt, v.tol, s0, off, fp, fl, K, rad, gp, move, t3, vis0,
-                                    r, v.h, v.ae, v.io, v.b2};
+                                    r, v.h, v.ae, v.io, v.b2, v.x, v.ex, v.ey};
                     narrow_zone(S, u0, acc, dir, lam, E, B, z);
                     return z;
                 }

@@ -113,3 +113,18 @@ def test_radii_are_the_plain_walks(q, spin, radius, acc):
                              capture_output=True, timeout=300)
         n, bad = (int(v) for v in out.stdout.split())
         assert n > 30000 and bad == 0 and out.returncode == 0, (star, bad)
+
+
+# both lobes filled, the mass ratio extreme, the eclipser (large) a slow rotator: the eclipsed
+# star digs a well of its own at the near end of the chord, below the lobe's potential
+@pytest.mark.parametrize("q", [0.003, 0.02, 0.05, 20.0, 47.0, 300.0])
+@pytest.mark.parametrize("spin,iangle,delta", [
+    (0.0, 70.0, "1e-8"), (0.0, 90.0, "1e-7"), (0.2, 84.0, "1e-7"), (0.4, 70.0, "1e-7"),
+    (0.4, 90.0, "1e-8")])
+def test_second_wells_keep_every_decision(root_check, oracle, q, spin, iangle, delta):
+    star = 1 if q < 1.0 else 0
+    over = dict(nlat1f=16, nlat2f=60, spin1=spin) if star else dict(nlat1f=60, nlat2f=16, spin2=spin)
+    m = W.model(q=q, r1=-1.0, r2=-1.0, iangle=iangle, delta_phase=delta, **over)
+    rc, r = _run(root_check, m, star, oracle.star_grid(m, star)["posn"])
+    assert rc == 0 and r["wrong"] == 0, r
+    assert r["tests"] > 10000
