@@ -166,7 +166,9 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
     r.ex = ex;
     r.ey = ey;
     r.ae = ae;
-    r.tol = 1e-14 * (pe * ie + po * io + pe + po + 1.);
+    // the positions' rounding times the gradients, and that of star 2's squared distance,
+    // which Roche::rpot forms as x^2 + y^2 + z^2 + 1 - 2 x (rpot.cpp:37-86)
+    r.tol = 1e-14 * (pe * ie + po * io + pe + po + 1.) + 2e-15 * (S.dx < 0. ? ae : ao);
     r.on = true;
     if (r.f <= -r.tol) {
         r.ans = kEdgeTrue;

@@ -128,3 +128,16 @@ def test_second_wells_keep_every_decision(root_check, oracle, q, spin, iangle, d
     rc, r = _run(root_check, m, star, oracle.star_grid(m, star)["posn"])
     assert rc == 0 and r["wrong"] == 0, r
     assert r["tests"] > 10000
+
+
+# a tiny star 2 as the eclipser: the potential about it carries the rounding of a squared
+# distance of order one, 1e-16 over the star's radius cubed
+@pytest.mark.parametrize("q", [0.02, 0.3])
+@pytest.mark.parametrize("r2", [0.0003, 0.0005, 0.0008, 0.0015])
+@pytest.mark.parametrize("r1,iangle,delta", [(0.01, 90.0, "1e-9"), (0.01, 90.0, "1e-7"),
+                                             (0.1, 87.4, "1e-9"), (0.1, 87.4, "5e-9")])
+def test_tiny_second_stars_keep_every_decision(root_check, oracle, q, r2, r1, iangle, delta):
+    m = W.model(q=q, r1=r1, r2=r2, iangle=iangle, delta_phase=delta, nlat1f=120, nlat2f=12)
+    rc, r = _run(root_check, m, 0, oracle.star_grid(m, 0)["posn"])
+    assert rc == 0 and r["wrong"] == 0, r
+    assert r["tests"] > 100
