@@ -63,7 +63,7 @@ LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, dou
     s.gap = 1. - rref;
     s.er = s.me / rref;
     s.er3 = s.er / s.rref2;
-    s.bend = 2. * s.mo / (s.gap * s.gap * s.gap) + s.ss;
+    s.bend = s.gap > 0. ? 2. * s.mo / (s.gap * s.gap * s.gap) + s.ss : 1e30;
     s.ik = s.er3 - s.bend > 0.04 * s.er3 ? 2. / (s.er3 - s.bend) : 0.;
     s.cosi = cosi;
     s.sini = sini;
@@ -211,9 +211,12 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
 // (both square roots as reciprocals, shared), for the phases between the
 // certified intervals: the same chord, bracket check and dbrent
 // (dbrent.cpp:21-126) steps, so the same answer except where rounding could
-// decide it; there (a value within rounding of pref, a bracket that fails)
-// kEdgeUnsure hands the phase to fblink itself. Of the about 720 FP64
-// instructions of an fblink that searches, some 250 remain.
+// decide it; there kEdgeUnsure hands the phase to fblink itself: a value within rounding of
+// pref or of the one it is compared with, a bracket that fails, and points within mx of
+// where dbrent would choose otherwise (far more than a secant step makes of the slopes'
+// rounding). That is not rare: after a halved step the best point is the bracket's
+// middle, and which way dbrent then moves by acc is the sign of an exact zero. Of the about
+// 720 FP64 instructions of an fblink that searches, some 270 remain.
 LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double phase) {
     double sn, cs;
     edge_sincos(phase, sn, cs);
@@ -221,14 +224,15 @@ LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double p
     const double B = fma(ex, u0.x, fma(ey, u0.y, ez * u0.z)), C = u2 - S.rref2;
     const double fac = B * B - C, tiny = 1e-12 * (1. + u2);
     if (!(B < -tiny && fac > tiny && C > tiny)) return kEdgeUnsure;
-    const double lam2 = sqrt(fac) - B, lam1 = C / lam2;
+    const double lam2 = sqrt(fac) - B, lam1 = C / lam2, mx = 1e-9 * (lam2 - lam1);
     if (!(lam2 - lam1 > acc * (1. + 1e-9))) return kEdgeUnsure;
-    const double tol = 1e-14 * (S.me / S.rref2 * 4. + fabs(S.pref) + S.mo + 10.);
     const double exy2 = fma(ex, ex, ey * ey), uxy = fma(ex, u0.x, ey * u0.y);
+    double ie = 0., io = 0.;
     auto eval = [&](double l, double &f, double &d) {
         const double ux = fma(l, ex, u0.x), uy = fma(l, ey, u0.y), uz = fma(l, ez, u0.z);
         const double vx = ux - S.dx, yz = fma(uy, uy, uz * uz), eu = l + B;
-        const double ie = edge_rsqrt(fma(ux, ux, yz)), io = edge_rsqrt(fma(vx, vx, yz));
+        ie = edge_rsqrt(fma(ux, ux, yz));
+        io = edge_rsqrt(fma(vx, vx, yz));
         const double pe = S.me * ie, po = S.mo * io;
         f = fma(S.k, ux, fma(-0.5 * S.ss, fma(ux, ux, uy * uy), -(pe + po))) - S.pref;
         d = fma(pe * ie * ie, eu,
@@ -236,10 +240,17 @@ LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double p
     };
     double x = lam1 + (lam2 - lam1) / 2., fx, dx, f1, f2, t;
     eval(x, fx, dx);
+    const double ib = ie;  // the midpoint is the point nearest to the eclipser
+    eval(lam2, f2, t);
+    const double i2 = io;
+    eval(lam1, f1, t);
+    // the other star is nearest at an end, unless the line passes it within the chord
+    const double in = io > i2 ? io : i2, is = S.dx < 0. ? ib : in;
+    if (!(fma(-S.dx, ex, lam1 + B) * fma(-S.dx, ex, lam2 + B) > 0.)) return kEdgeUnsure;
+    const double tol = 1e-14 * (S.me * ib * ib + S.mo * in * in + fabs(S.pref) + 10.) +
+                       2e-15 * (S.dx < 0. ? S.me : S.mo) * is * is * is;
     if (fabs(fx) <= tol) return kEdgeUnsure;
     if (fx < 0.) return kEdgeTrue;
-    eval(lam1, f1, t);
-    eval(lam2, f2, t);
     // the first level of fblink's subdivision brackets the minimum
     if (!(fx < f1 - tol && fx < f2 - tol)) return kEdgeUnsure;
     double a = lam1, b = lam2, w = x, v = x, fw = fx, fv = fx, dw = dx, dv = dx;
@@ -247,8 +258,9 @@ LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double p
     const double tol1 = acc, tol2 = 2. * acc;
 #pragma unroll 1
     for (int iter = 0; iter < 100; iter++) {
-        const double xm = 0.5 * (a + b);
-        if (fabs(x - xm) <= tol2 - 0.5 * (b - a)) return kEdgeFalse;
+        const double xm = 0.5 * (a + b), gap = fabs(x - xm) - (tol2 - 0.5 * (b - a));
+        if (fabs(gap) <= mx) return kEdgeUnsure;
+        if (gap < 0.) return kEdgeFalse;
         bool half = true;
         if (fabs(e) > tol1) {
             double d1 = 2. * (b - a), d2 = d1;
@@ -261,9 +273,13 @@ LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double p
             e = d;
             if (ok1 || ok2) {
                 const double dn = ok1 && ok2 ? (fabs(d1) < fabs(d2) ? d1 : d2) : ok1 ? d1 : d2;
-                if (fabs(dn) <= fabs(0.5 * olde)) {
-                    const double u = x + dn;
-                    d = (u - a < tol2 || b - u < tol2) ? dsign(tol1, xm - x) : dn;
+                const double much = fabs(dn) - fabs(0.5 * olde);
+                if (fabs(much) <= mx) return kEdgeUnsure;
+                if (much < 0.) {
+                    const double u = x + dn, la = u - a, lb = b - u;
+                    const double end = (la < lb ? la : lb) - tol2;
+                    d = end < 0. ? dsign(tol1, xm - x) : dn;
+                    if (fabs(end) <= mx || (end < 0. && fabs(xm - x) <= mx)) return kEdgeUnsure;
                     half = false;
                 }
             }
@@ -273,7 +289,7 @@ LCG_HD int fblink_edge(const EdgeStar &S, V3 u0, double u2, double acc, double p
         const double u = far ? x + d : x + dsign(tol1, d);
         double fu, du;
         eval(u, fu, du);
-        if (fabs(fu) <= tol) return kEdgeUnsure;
+        if (fabs(fu) <= tol || fabs(fu - fx) <= tol) return kEdgeUnsure;
         if (fu < 0.) return kEdgeTrue;
         if (!far && fu > fx) return kEdgeFalse;
         if (fu <= fx) {

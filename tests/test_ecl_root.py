@@ -141,3 +141,19 @@ def test_tiny_second_stars_keep_every_decision(root_check, oracle, q, r2, r1, ia
     rc, r = _run(root_check, m, 0, oracle.star_grid(m, 0)["posn"])
     assert rc == 0 and r["wrong"] == 0, r
     assert r["tests"] > 100
+
+
+# coarse bisections of contact binaries: the search's accuracy is a good part of the chord, and
+# dbrent's way after a halved step hangs on the sign of an exact zero
+@pytest.mark.parametrize("q,spin", [(16.9, 1.0), (20.0, 1.0), (47.0, 0.75), (0.0084, 0.9),
+                                    (0.0027, 0.75)])
+@pytest.mark.parametrize("iangle,delta", [(57.0, "6e-5"), (61.0, "5.3e-5"), (66.0, "4.4e-5"),
+                                          (70.0, "6e-5")])
+def test_coarse_searches_keep_every_decision(root_check, oracle, q, spin, iangle, delta):
+    star = 1 if q < 1.0 else 0
+    over = dict(nlat1f=16, nlat2f=90) if star else dict(nlat1f=90, nlat2f=16)
+    m = W.model(q=q, r1=-1.0, r2=-1.0, spin1=spin, spin2=spin, iangle=iangle, delta_phase=delta,
+                **over)
+    rc, r = _run(root_check, m, star, oracle.star_grid(m, star)["posn"])
+    assert rc == 0 and r["wrong"] == 0, r
+    assert r["tests"] > 10000
