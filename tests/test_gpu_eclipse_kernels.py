@@ -27,3 +27,18 @@ def test_eclipse_kernels_agree(over):
             a, b = plain.star_grid(m, star), e.star_grid(m, star)
             for k in ("posn", "neclipse", "ecl_in", "ecl_out"):
                 np.testing.assert_array_equal(a[k], b[k], err_msg="%s of star %d" % (k, star))
+
+
+# both lobes filled: second wells on the chords, searches that rounding decides
+@pytest.mark.parametrize("star,over", [
+    (1, dict(q=0.003, spin1=0.0, iangle=70.0, delta_phase="1e-8")),
+    (1, dict(q=0.05, spin1=0.2, iangle=84.0)), (0, dict(q=300.0, spin2=0.0, iangle=90.0)),
+    (0, dict(q=20.0, iangle=57.0, delta_phase="6e-5")),
+    (1, dict(q=0.0084, spin1=0.9, spin2=0.9, iangle=61.0, delta_phase="5.3e-5"))])
+@pytest.mark.parametrize("nlat", [120, 200])
+def test_contact_eclipses_agree(star, over, nlat):
+    m = W.model(r1=-1.0, r2=-1.0, nlat1f=16 if star else nlat, nlat2f=nlat if star else 16, **over)
+    with Engine(precision="fp64", eclipse_warp=1 << 30) as plain, Engine(precision="mixed") as e:
+        a, b = plain.star_grid(m, star), e.star_grid(m, star)
+        for k in ("neclipse", "ecl_in", "ecl_out"):
+            np.testing.assert_array_equal(a[k], b[k], err_msg=k)
