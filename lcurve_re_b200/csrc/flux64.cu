@@ -322,9 +322,12 @@ __global__ void __launch_bounds__(kThreadsRag)
     unsigned long long A, La;
     warp_arc<1>(&pf, A, La);
     const int lane = threadIdx.x & 31;
-    // every entry of the warp lies within wide of the middle lane's
-    const double cx = __shfl_sync(0xffffffffu, ex, 16), cy = __shfl_sync(0xffffffffu, ey, 16),
-                 cz = __shfl_sync(0xffffffffu, ez, 16);
+    // every entry of the warp lies within wide of the middle lane's, or of the first one's
+    // that is a number: a point whose time is not spoils no other
+    const unsigned real = __ballot_sync(0xffffffffu, ex == ex && ey == ey && ez == ez);
+    const int mid = ((real >> 16) & 1u) || !real ? 16 : __ffs(real) - 1;
+    const double cx = __shfl_sync(0xffffffffu, ex, mid), cy = __shfl_sync(0xffffffffu, ey, mid),
+                 cz = __shfl_sync(0xffffffffu, ez, mid);
     double wide = sqrt((ex - cx) * (ex - cx) + (ey - cy) * (ey - cy) + (ez - cz) * (ez - cz));
     for (int o = 16; o > 0; o >>= 1) wide = fmax(wide, __shfl_xor_sync(0xffffffffu, wide, o));
     wide = 1.0001 * wide + 1e-9;

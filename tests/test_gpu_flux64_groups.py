@@ -72,3 +72,20 @@ def test_disc_sums_do_not_depend_on_the_warp(npts, precision, over):
         a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
         b = e.light_curve_comp(m, d[perm], scale=False, rdata=False, diagnostics=False)[0]
     np.testing.assert_array_equal(a[perm], b)
+
+
+# a point whose time is not a number spoils no other, whichever lane of a warp it is
+@pytest.mark.parametrize("bad", [[16], [1, 16, 33, 48]])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_point_without_a_time_spoils_no_other(bad, precision):
+    from lcurve_re_b200 import workloads as W
+    from lcurve_re_b200.engine import Engine
+    m = W.cv_disc(nlat1f=30, nlat2f=35, nrad=12, nspot=9)
+    d = W.data(64)
+    with Engine(precision=precision) as e:
+        a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0].copy()
+        d["time"][bad] = np.nan
+        b = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
+    rest = np.setdiff1d(np.arange(64), bad)
+    np.testing.assert_array_equal(a[rest], b[rest])
+    assert np.isnan(b[bad]).all()
