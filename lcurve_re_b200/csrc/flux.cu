@@ -81,8 +81,9 @@ __device__ __forceinline__ int run_class(const RunRec &R, float cut, const float
     for (int j = 0; j < PPT; j++) {
         const float e = sqrtf(fmaf(ex[j], ex[j], ey[j] * ey[j]));
         const float z = fmaxf(ez[j] * B.w, ez[j] * zmin);
+        // a bound that is no number (one of its faces is none) does not make a group dark
         some = some ||
-               fmaf(ex[j], B.x, fmaf(ey[j], B.y, fmaf(e, B.z, z))) + 2e-6f >= cut;
+               !(fmaf(ex[j], B.x, fmaf(ey[j], B.y, fmaf(e, B.z, z))) + 2e-6f < cut);
     }
     if (!__any_sync(0xffffffffu, some)) return kGroupDark;
     if constexpr (ECL) return arc_class(R, A, L);
@@ -374,7 +375,7 @@ __device__ __forceinline__ int group_class(const RunRec &R, const float2 *ex, co
 #pragma unroll
     for (int j = 0; j < PPT; j++) {
         const float d = fmaf(ex[j].x, B.x, ey[j].x * B.y);
-        some = some || fmaf(exy[j], B.z, d + B.w) >= 0.f;
+        some = some || !(fmaf(exy[j], B.z, d + B.w) < 0.f);
         every = every && fmaf(-exy[j], B.z, d + cmin) > 0.f;
     }
     if (!__any_sync(0xffffffffu, some)) return kGroupDark;

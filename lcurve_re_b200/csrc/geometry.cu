@@ -1029,14 +1029,19 @@ __global__ void __launch_bounds__(1024) k_interp(const DatumRec *__restrict__ da
 // group: the mean of (nx, ny), the largest distance r from it and the extremes
 // of cz. r and the extremes are widened well past FP32 rounding (1e-6, 1e-5).
 // All-zero records (padding, faces with several ranges) add zeros whatever is
-// concluded and are left out; a group of them alone gets cmax = -1.
+// concluded and are left out; a group of them alone gets cmax = -1. One with a face
+// that is no finite number gets NaN: neither dark nor bright, its faces are tested singly.
 template <int W>
 __device__ __forceinline__ void group_mu(const float *nx, const float *ny, const float *cz,
                                          const bool *use, RunRec &R) {
     const unsigned full = 0xffffffffu;
     float sx = 0.f, sy = 0.f, cnt = 0.f;
     for (int k = 0; k < 2; k++)
-        if (use[k]) { sx += nx[k]; sy += ny[k]; cnt += 1.f; }
+        if (use[k]) {
+            sx += nx[k] + 0.f * (nx[k] + ny[k] + cz[k]);
+            sy += ny[k];
+            cnt += 1.f;
+        }
     for (int o = W / 2; o > 0; o >>= 1) {
         sx += __shfl_xor_sync(full, sx, o);
         sy += __shfl_xor_sync(full, sy, o);
