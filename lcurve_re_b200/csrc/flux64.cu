@@ -258,6 +258,11 @@ __global__ void __launch_bounds__(kThreads64, 4)
     W.exy = sqrtf(W.ex * W.ex + W.ey * W.ey);
     const unsigned long long pf = ph.pfx[e];
     warp_arc<1>(&pf, W.A, W.L);
+    // the arc holds phases of one turn; with others among them ranges are tested singly
+    if (!__all_sync(0xffffffffu, E.pn >= 0. && E.pn <= 1.)) {
+        W.A = 0ull;
+        W.L = ~0ull;
+    }
     const Consts64 L{k.c[0], k.c[1], k.c[2], k.c[3], k.base, k.mucrit,
                      k.beam, k.spin, k.vfac, k.xcofm, k.rlens1};
     // a warp leaves together whether its copies arrived or the wait gave up,

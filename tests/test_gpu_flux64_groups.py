@@ -89,3 +89,19 @@ def test_a_point_without_a_time_spoils_no_other(bad, precision):
     rest = np.setdiff1d(np.arange(64), bad)
     np.testing.assert_array_equal(a[rest], b[rest])
     assert np.isnan(b[bad]).all()
+
+
+# phases outside one turn, as a caller of the face-list sweep may hand them in: the ranges are
+# compared with them as they are
+@pytest.mark.parametrize("scale,shift", [(1.0, 1.0), (1.0, -1.0), (1.0, 0.5), (3.0, -1.0)])
+@pytest.mark.parametrize("n,n0,nent", [(65, 0, 33), (1025, 17, 1300)])
+def test_phases_outside_one_turn(engine_fp64, oracle, n, n0, nent, scale, shift):
+    flat = flat_grid(n, n0, False)
+    ph = scale * np.linspace(0, 1, nent, endpoint=False) + shift
+    si, ci = np.sin(np.radians(85.0)), np.cos(np.radians(85.0))
+    phases = dict(ex=si * np.cos(2 * np.pi * ph), ey=-si * np.sin(2 * np.pi * ph),
+                  ez=np.full(nent, ci), phin=ph)
+    kw = dict(ldc=[0.4, 0.1, 0.05, 0.02], ltype=1, spin=1.1, vfac=1e-3, xcofm=0.2)
+    for star in (0, 1):
+        np.testing.assert_array_equal(oracle.sum_star_multi(star, flat, phases, **kw),
+                                      engine_fp64.sum_star_multi(star, flat, phases, **kw))

@@ -1,7 +1,7 @@
 """The mixed general sweep over face lists with entries that a caller may hand in.
 
 Groups of faces are left out by bounds over their normals; a face that is no
-number, or a normal longer than one, must not take its neighbours along.
+number must not take its neighbours along.
 """
 import numpy as np
 import pytest
