@@ -963,7 +963,8 @@ lcg_status lcg_mlp_pca_chisq(void *stream, const float *coef, int32_t m, int32_t
     const size_t smem = (size_t)kPcaRows * keep * sizeof(double) +
                         (size_t)ncoef * kPcaRows * (anchor ? 2 : 1) * sizeof(float);
     auto kern = anchor ? k_pca_chisq<true> : k_pca_chisq<false>;
-    if (smem > 48 * 1024 &&
+    // 48 KB are a CTA's without asking, the kernel's static arrays among them
+    if (smem > 47 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))
         return LCG_E_CUDA;
     kern<<<(unsigned)((m + kPcaRows - 1) / kPcaRows), kPcaThreads, smem, (cudaStream_t)stream>>>(

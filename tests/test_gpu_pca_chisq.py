@@ -6,6 +6,9 @@ remains are double sums of npts terms: npts 2^-53 of the summed magnitudes, and
 the scale's error enters chi**2 once more, twice: 4 npts 2^-53 bounds both.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -55,3 +58,17 @@ def test_chi2_of_exact_curves(rows, npts, nc, anchored):
     want = (w * ((y - s[:, None] * f) / e) ** 2).sum(1)
     mag = (w * ((y.abs() + (s[:, None] * f).abs()) / e) ** 2).sum(1)
     assert ((chi - want).abs() <= tol * mag).all()
+
+
+# curves and coefficients that fill the 48 KB a CTA has without asking, or all but the
+# kernel's own static arrays; in a process of its own, since a kernel that was given
+# more once keeps it
+def test_chi2_at_the_default_shared_memory():
+    sizes = [(2944, True), (3000, True), (3007, True), (3008, True), (3032, False), (3040, False)]
+    code = "import test_gpu_pca_chisq as t\n" + "".join(
+        "t.test_chi2_of_exact_curves(3, %d, 64, %s)\n" % s for s in sizes)
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                         env=env)
+    assert out.returncode == 0, out.stderr[-2000:]
