@@ -66,3 +66,14 @@ def test_general_sums_do_not_depend_on_the_warp(over, npts, span):
         a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
         b = e.light_curve_comp(m, d[perm], scale=False, rdata=False, diagnostics=False)[0]
     np.testing.assert_array_equal(a[perm], b)
+
+
+# a beamed curve whose chunk of 1024 faces takes 48 KB of shared memory, what a CTA has
+# without asking, its barrier aside
+def test_general_sweep_at_the_default_shared_memory():
+    m = W.model(nlat1f=20, nlat2f=220, beam_factor1=1.3, beam_factor2=1.6)
+    d = W.data(12500)
+    with Engine(precision="mixed") as e, Engine(precision="fp64") as e64:
+        a = e.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
+        b = e64.light_curve_comp(m, d, scale=False, rdata=False, diagnostics=False)[0]
+    np.testing.assert_allclose(a, b, rtol=1e-5)
