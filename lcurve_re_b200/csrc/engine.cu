@@ -416,28 +416,26 @@ lcg_status build_geometry(lcg_ctx *c, const lcg_model &m, int star, int fine, Gr
                           cudaStream_t st) {
     Fail f{0, ""};
     // A grid without infill has the ring table of its strip count, the one on the
-    // device if it had as many strips before.
+    // device if it had as many strips before. ring_nlat names that table only while it
+    // is whole: what a failed call leaves belongs to no strip count.
     StarSetup &s = g.setup;
     const int32_t nlat = star == kStar1 ? (fine ? m.nlat1f : m.nlat1c) : (fine ? m.nlat2f : m.nlat2c);
     const bool plain = star == kStar1 || !fine || !m.npole ||
                        (m.nlatfill <= 0 && m.nlngfill <= 0);
     const bool rings_on = plain && g.ring_nlat == nlat && nlat > 0;
     const int nface = s.nface;
-    if (!prepare_star(m, star, fine, s, f, !rings_on)) {
-        g.ring_nlat = 0;
-        return c->fail(f.code, "%s", f.msg.c_str());
-    }
+    g.ring_nlat = 0;
+    if (!prepare_star(m, star, fine, s, f, !rings_on)) return c->fail(f.code, "%s", f.msg.c_str());
     if (rings_on) s.nface = nface;
     cudaError_t e;
     if ((e = g.alloc_points(s.nface)) != cudaSuccess) return c->cuda_fail(e, "grid allocation");
     g.ntiled = s.ntiled;
-    if (!rings_on) {
-        g.ring_nlat = 0;
-        if ((e = g.rings.ensure(s.rings.size())) != cudaSuccess) return c->cuda_fail(e, "rings");
-        cudaMemcpyAsync(g.rings.p, s.rings.data(), s.rings.size() * sizeof(RingRec),
-                        cudaMemcpyHostToDevice, st);
-        if (plain) g.ring_nlat = nlat;
-    }
+    if (!rings_on && ((e = g.rings.ensure(s.rings.size())) ||
+                      (e = cudaMemcpyAsync(g.rings.p, s.rings.data(),
+                                           s.rings.size() * sizeof(RingRec),
+                                           cudaMemcpyHostToDevice, st))))
+        return c->cuda_fail(e, "rings");
+    if (plain) g.ring_nlat = nlat;
     GridParams gp{};
     gp.star = star;
     gp.roche = star == kStar1 ? m.roche1 : m.roche2;

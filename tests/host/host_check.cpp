@@ -1,0 +1,247 @@
+// The engine's host side (engine.cu) on the CPU, with allocations that fail.
+//
+// engine.cu holds no device code: it is compiled here with the host compiler against a
+// runtime in which device memory is host memory and the n-th allocation of a call returns
+// cudaErrorMemoryAllocation. The kernels' launchers are replaced by checks of what they are
+// given: that every array lives and is large enough, that the ring table belongs to
+// the grid, and that a sweep reads the fluxes of the model it is launched for.
+//
+//   host_check rings|cache|data   (stdin: lcg_model A, lcg_model B)
+//
+// A call with A, one with B whose k-th allocation fails, then A again (mode data: points for
+// the first call, more of them for the second), in a new context for every k until the second
+// call has none left to fail. Prints the number of failures tried and of what was wrong;
+// exits 1 if anything was.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+
+#include "../../lcurve_re_b200/csrc/engine.cu"
+
+static std::map<char *, size_t> g_mem;
+static long g_countdown = -1;  // allocations until one fails
+static int g_wrong = 0;
+static const lcg_model *g_model = nullptr;
+static std::map<const void *, double> g_flux_t, g_flat_t;  // by array: the model's temperature
+
+static void wrong(const char *what) {
+    g_wrong++;
+    fprintf(stderr, "wrong: %s\n", what);
+}
+static size_t room(const void *p) {  // bytes left in the allocation that p points into
+    auto it = g_mem.upper_bound((char *)p);
+    if (!p || it == g_mem.begin()) return 0;
+    --it;
+    const size_t at = (size_t)((char *)p - it->first);
+    return at < it->second ? it->second - at : 0;
+}
+template <class T>
+static void need(const T *p, int64_t n, const char *what) {
+    if (room(p) < (size_t)n * sizeof(T)) wrong(what);
+}
+static cudaError_t get(void **p, size_t n) {
+    if (g_countdown > 0 && --g_countdown == 0) {
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
+    *p = calloc(1, n);
+    g_mem[(char *)*p] = n;
+    return cudaSuccess;
+}
+static cudaError_t drop(void *p) {
+    g_mem.erase((char *)p);
+    free(p);
+    return cudaSuccess;
+}
+
+extern "C" {
+cudaError_t cudaMalloc(void **p, size_t n) { return get(p, n); }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return get(p, n); }
+cudaError_t cudaFree(void *p) { return drop(p); }
+cudaError_t cudaFreeHost(void *p) { return drop(p); }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+    if (k == cudaMemcpyHostToDevice && room(d) < n) {
+        wrong("a copy past its destination");
+        return cudaErrorInvalidValue;
+    }
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy2DAsync(void *, size_t, const void *, size_t, size_t, size_t, cudaMemcpyKind,
+                              cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) {
+    if (room(p) < n) wrong("a clear past its array");
+    else memset(p, v, n);
+    return cudaSuccess;
+}
+cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp *p, int) {
+    memset(p, 0, sizeof *p);
+    p->major = 10;
+    p->multiProcessorCount = 148;
+    return cudaSuccess;
+}
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = nullptr; return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = nullptr; return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = nullptr; return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *t, cudaEvent_t, cudaEvent_t) { *t = 0.f; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t) { return "allocation failed by the test"; }
+lcg_status lcg_light_curve_batch_resident(lcg_ctx *, const lcg_model *, int32_t, int32_t, double *,
+                                          double *, double *, double *, int32_t *) {
+    return LCG_E_INVALID;
+}
+}
+
+namespace lcg {
+
+static void need_grid(const GridDev &g) {
+    for (const double *p : {g.px, g.py, g.pz, g.nx, g.ny, g.nz, g.ein, g.eout}) need(p, g.n, "grid");
+    for (const float *p : {g.area, g.grav, g.flux}) need(p, g.n, "grid");
+    need(g.necl, g.n, "grid");
+}
+void launch_grid(const GridParams &p, const RingRec *r, GridDev g, int32_t *cnt, DevStatus *,
+                 cudaStream_t) {
+    need_grid(g);
+    need(cnt, 8, "counters");
+    if (room(r) < (size_t)p.nrings * sizeof(RingRec) || p.nrings < 1) {
+        wrong("a ring table shorter than its grid's rings");
+        return;
+    }
+    const RingRec &last = r[p.nrings - 1];
+    if (last.off + last.nphi != g.ntiled || last.hoff + (last.nphi + 1) / 2 != p.nhalf)
+        wrong("a ring table of another grid");
+    if (llabs(g.n - g.ntiled) > 4) wrong("a face count of another grid");
+}
+void launch_eclipse(const EclParams &, int32_t, GridDev g, int32_t *q, int32_t *c, double4 *es,
+                    int32_t *h, DevStatus *, int, int32_t, cudaStream_t) {
+    need_grid(g);
+    need(q, g.n, "queue"); need(c, 8, "counters"); need(es, g.n, "states"); need(h, g.n, "hits");
+}
+int64_t cont_blocks(int64_t n) { return (n + 255) / 256; }
+void launch_continuum(const ContParams &p, GridDev g, int32_t *cnt, double *dsum, cudaStream_t) {
+    need_grid(g);
+    if (cnt) need(cnt, 2 * cont_blocks(g.n), "counts");
+    if (dsum) need(dsum, 4 * cont_blocks(g.n), "sums");
+    g_flux_t[g.flux] = p.t_own;
+}
+void launch_flatten(GridDev g, FlatDev f, const int32_t *cnt, int mixed, int need_pos,
+                    const FastCoef &fc, cudaStream_t) {
+    need_grid(g);
+    need(cnt, 2 * cont_blocks(g.n), "counts");
+    if (need_pos && mixed) need(f.pos, f.npad, "positions");
+    if (mixed && fc.on) need(f.fp, 8 * f.npad, "records");
+    g_flat_t[f.n0] = g_flux_t[g.flux];
+}
+void launch_phases(const PhaseParams &, const DatumRec *d, const int64_t *off, int32_t n, PhaseDev ph,
+                   bool, V3, double, cudaStream_t) {
+    need(d, n, "points");
+    need(off, n + 1, "offsets");
+    if (room(off) >= (size_t)(n + 1) * 8 && off[n] > ph.nent) wrong("entries of other points");
+    for (const double *p : {ph.ex, ph.ey, ph.ez, ph.phin, ph.w1, ph.w2}) need(p, ph.nent, "entries");
+}
+void launch_scatter(const ScatterParams &, const ReduceParams &, const PhaseDev &, const DatumRec *d,
+                    const int64_t *, int32_t n, double *calc, cudaStream_t) {
+    need(d, n, "points");
+    need(calc, n, "curve");
+}
+void launch_finalize(int32_t, const DatumRec *, int32_t, double *, double, const TailIn &, TailOut *,
+                     cudaStream_t) {}
+void launch_tail(const TailIn &, TailOut *, cudaStream_t) {}
+void launch_interp(const DatumRec *, int32_t, const int64_t *, int32_t, const double *, double *,
+                   int32_t, double *, cudaStream_t) {}
+void launch_iscale(int32_t, int32_t, const DatumRec *, int32_t, const double *, double *, double *,
+                   double *, double *, cudaStream_t) {}
+void launch_pack_flat(FlatDev, int64_t, int, cudaStream_t) {}
+void launch_pack_phases(PhaseDev, cudaStream_t) {}
+void launch_run_bounds64(const FlatDev &, cudaStream_t) {}
+void launch_run_bounds_geo(const FlatDev &, cudaStream_t) {}
+FluxPlan plan_flux(int mixed, int fast, int64_t nface, int64_t nent, int) {
+    FluxPlan p{};
+    p.fast = mixed && fast;
+    p.ppt = 1;
+    p.threads = 256;
+    p.chunk = p.group = 1024;
+    p.nchunk = (nface + 1023) / 1024;
+    p.ntile = (nent + 255) / 256;
+    return p;
+}
+void launch_flux(int mixed, int star, const FluxConsts &, const FlatDev &f, const PhaseDev &,
+                 const FluxPlan &, double *part, int64_t ldp, DevStatus *, cudaStream_t) {
+    if (mixed) need(f.ecl, f.npad, "ranges");
+    need(part, ldp, "partial sums");
+    if (g_flat_t[f.n0] != (star == 0 ? g_model->t1 : g_model->t2))
+        wrong("a sweep over another model's fluxes");
+}
+void launch_flux_ragged(int, const FluxConsts &, const FlatDev &, const GridDev &, const PhaseDev &,
+                        int64_t, int64_t, double *, int64_t, cudaStream_t) {}
+void launch_components(const CompParams &, ElemRec *, double4 *, DevStatus *, cudaStream_t) {}
+void launch_disc_faces(const DiscGeom &, const GridDev &, uint8_t *, double2 *, int32_t *, DevStatus *,
+                       cudaStream_t) {}
+void launch_comp_sums(const ElemRec *, int32_t, int32_t, int32_t, double, double, PhaseDev const &,
+                      double *, double *, int64_t, cudaStream_t) {}
+int64_t comp_sums_scratch(int32_t, int64_t) { return 1; }
+void launch_fma_probe(float *, int, int, double *, cudaStream_t) {}
+void launch_dfma_probe(double *, int, int, double *, cudaStream_t) {}
+namespace eng {
+void batch_release(BatchState *) {}
+bool comp_setup(const lcg_model &, CompParams &, std::vector<DiscRing> &, Fail &) { return false; }
+}  // namespace eng
+}  // namespace lcg
+
+static lcg_status points(lcg_ctx *c, int n) {
+    std::vector<lcg_datum> d((size_t)n);
+    memset(d.data(), 0, d.size() * sizeof(lcg_datum));
+    for (int i = 0; i < n; i++) {
+        d[i].time = 1e-3 * i;
+        d[i].ferr = d[i].weight = 1.;
+        d[i].ndiv = 1;
+    }
+    return lcg_set_data(c, d.data(), n);
+}
+static lcg_status curve(lcg_ctx *c, const lcg_model &m, int n) {
+    std::vector<double> calc((size_t)n);
+    double sfac[5] = {1., 1., 1., 1., 1.}, out[LCG_NOUT];
+    g_model = &m;
+    return lcg_light_curve_resident(c, &m, 0, sfac, calc.data(), out);
+}
+
+int main(int argc, char **argv) {
+    lcg_model a, b;
+    if (argc < 2 || fread(&a, sizeof a, 1, stdin) != 1 || fread(&b, sizeof b, 1, stdin) != 1) return 2;
+    const bool data = !strcmp(argv[1], "data");
+    int k = 1;
+    for (;; k++) {
+        lcg_ctx *c = nullptr;
+        if (lcg_create(&c, nullptr) || points(c, 100) || curve(c, a, 100)) return 3;
+        g_countdown = k;
+        const lcg_status st = data ? points(c, 5000) : curve(c, b, 100);
+        const bool failed = g_countdown == 0;
+        g_countdown = -1;
+        if (failed != (st != LCG_OK)) wrong("a failed allocation without a status");
+        const lcg_status again = curve(c, a, 5000);
+        // after points that were not taken there are none
+        if (data ? (again == LCG_OK) == failed : again != LCG_OK) {
+            wrong("the call after it");
+            fprintf(stderr, "  %s\n", lcg_last_error(c));
+        }
+        lcg_destroy(c);
+        if (!failed) break;
+    }
+    printf("%d %d\n", k - 1, g_wrong);
+    return g_wrong ? 1 : 0;
+}

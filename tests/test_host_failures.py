@@ -1,0 +1,42 @@
+"""The engine's host side when an allocation fails, on the CPU.
+
+host_check.cpp compiles engine.cu against a fake CUDA runtime in which the k-th
+allocation of a call fails. Whatever k is, that call returns an error and the
+next one runs on arrays, tables and fluxes of its own.
+"""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from lcurve_re_b200 import workloads as W
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+SRC = os.path.join(HERE, "host", "host_check.cpp")
+EXE = os.path.join(HERE, "host", "_build", "host_check")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def host_check():
+    if shutil.which("g++") is None or not os.path.isdir(os.path.join(CUDA, "include")):
+        pytest.skip("g++ or the CUDA headers are not available")
+    os.makedirs(os.path.dirname(EXE), exist_ok=True)
+    subprocess.check_call(["g++", "-x", "c++", "-std=c++17", "-O1", "-I" + os.path.join(CUDA, "include"),
+                           "-I" + os.path.join(ROOT, "include"), "-o", EXE, SRC])
+    return EXE
+
+
+def _run(exe, mode, a, b):
+    blob = bytes(W.model(nlat1f=20, nlat2f=24, **a).to_c()) + bytes(W.model(**b).to_c())
+    out = subprocess.run([exe, mode], input=blob, capture_output=True, timeout=300)
+    assert out.returncode == 0, out.stderr.decode()[-2000:]
+    return int(out.stdout.split()[0])
+
+
+@pytest.mark.parametrize("nlat1,nlat2", [(60, 70), (20, 70), (90, 24)])
+def test_ring_tables_after_a_failed_allocation(host_check, nlat1, nlat2):
+    """A grid's ring table is kept for its strip count: not past another one's failure."""
+    assert _run(host_check, "rings", {}, dict(nlat1f=nlat1, nlat2f=nlat2)) > 15
