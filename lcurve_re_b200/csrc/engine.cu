@@ -1049,6 +1049,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
                           c->cached_mixed_pos == (int)need_pos && !opaque && !c->g1f.disc &&
                           !c->g2f.disc && !c->g1c.disc && !c->g2c.disc;
     if (!cont_hit) {
+        c->has_cont = false;  // until this call has its fluxes
         Grid *gl[] = {&c->g1f, &c->g2f, &c->g1c, &c->g2c};
         const int stars[] = {kStar1, kStar2, kStar1, kStar2};
         const bool use[] = {true, true, !c->copy1, !c->copy2};

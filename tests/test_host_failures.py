@@ -40,3 +40,10 @@ def _run(exe, mode, a, b):
 def test_ring_tables_after_a_failed_allocation(host_check, nlat1, nlat2):
     """A grid's ring table is kept for its strip count: not past another one's failure."""
     assert _run(host_check, "rings", {}, dict(nlat1f=nlat1, nlat2f=nlat2)) > 15
+
+
+@pytest.mark.parametrize("over", [dict(t1=15000.0, t2=3000.0, beam_factor1=1.3),
+                                  dict(t1=15000.0, mucrit1=0.2), dict(t2=3500.0, limb2="Poly")])
+def test_fluxes_after_a_failed_allocation(host_check, over):
+    """The reuse of a model's fluxes ends when another model's call has overwritten them."""
+    _run(host_check, "cache", {}, dict(nlat1f=20, nlat2f=24, **over))
