@@ -821,7 +821,7 @@ lcg_status lcg_set_data(lcg_ctx *c, const lcg_datum *data, int32_t n) {
     // the last ones out of it are done once the stream is.
     cudaError_t e;
     if (c->h_data_n && (e = cudaStreamSynchronize(c->stream))) return c->cuda_fail(e, "stream");
-    c->h_data_n = 0;
+    c->h_data_n = c->data_n = 0;  // none while the buffers grow
     const size_t dbytes = (size_t)n * sizeof(DatumRec), obytes = ((size_t)n + 1) * sizeof(int64_t);
     if ((e = c->h_in.ensure(dbytes + obytes)) || (e = c->data.ensure(n)) ||
         (e = c->off.ensure(n + 1)))

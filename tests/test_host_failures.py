@@ -47,3 +47,8 @@ def test_ring_tables_after_a_failed_allocation(host_check, nlat1, nlat2):
 def test_fluxes_after_a_failed_allocation(host_check, over):
     """The reuse of a model's fluxes ends when another model's call has overwritten them."""
     _run(host_check, "cache", {}, dict(nlat1f=20, nlat2f=24, **over))
+
+
+def test_points_after_a_failed_allocation(host_check):
+    """Points that did not fit are refused, and no call takes the freed ones for them."""
+    assert _run(host_check, "data", {}, dict(nlat1f=20, nlat2f=24)) >= 2
