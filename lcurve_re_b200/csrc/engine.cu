@@ -817,8 +817,8 @@ lcg_status lcg_set_data(lcg_ctx *c, const lcg_datum *data, int32_t n) {
     cudaSetDevice(c->device);
     // per-point offsets of the sub-exposure entries and the time range used
     // by the polynomial factor (light_curve_comp.cpp:351-356). Points and offsets go
-    // to pinned memory first, so that the copies run on while the host goes on;
-    // the last ones out of it are done once the stream is.
+    // to a block of the context's own first, so that the copies may run on while the host
+    // goes on; the last ones out of it are done once the stream is.
     cudaError_t e;
     if (c->h_data_n && (e = cudaStreamSynchronize(c->stream))) return c->cuda_fail(e, "stream");
     c->h_data_n = c->data_n = 0;  // none while the buffers grow
@@ -1220,7 +1220,7 @@ lcg_status lcg_light_curve_resident(lcg_ctx *c, const lcg_model *mp, int32_t fla
             launch_finalize(flags & 3, c->data.p, n, c->calc(), sfac[0], ti, tail, c->stream);
         }
     }
-    // one copy for everything the call returns, through pinned memory
+    // one copy for everything the call returns
     cudaMemcpyAsync(c->h_res.p, c->res.p,
                     sizeof(TailOut) + (calc ? (size_t)n * sizeof(double) : 0),
                     cudaMemcpyDeviceToHost, c->stream);

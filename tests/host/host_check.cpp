@@ -6,8 +6,9 @@
 // given: that every array lives and is large enough, that the ring table belongs to
 // the grid, and that a sweep reads the fluxes of the model it is launched for.
 //
-//   host_check rings|cache|data   (stdin: lcg_model A, lcg_model B)
+//   host_check rings|cache|data|pin   (stdin: lcg_model A, lcg_model B)
 //
+// pin: many calls with A, counting pinned blocks. The others:
 // A call with A, one with B whose k-th allocation fails, then A again (mode data: points for
 // the first call, more of them for the second), in a new context for every k until the second
 // call has none left to fail. Prints the number of failures tried and of what was wrong;
@@ -21,7 +22,7 @@
 
 static std::map<char *, size_t> g_mem;
 static long g_countdown = -1;  // allocations until one fails
-static int g_wrong = 0;
+static int g_wrong = 0, g_pinned = 0, g_pins = 0;
 static const lcg_model *g_model = nullptr;
 static std::map<const void *, double> g_flux_t, g_flat_t;  // by array: the model's temperature
 
@@ -57,9 +58,25 @@ static cudaError_t drop(void *p) {
 
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t n) { return get(p, n); }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return get(p, n); }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+    g_pinned++;
+    g_pins++;
+    return get(p, n);
+}
+cudaError_t cudaHostRegister(void *, size_t, unsigned) {
+    g_pinned++;
+    g_pins++;
+    return cudaSuccess;
+}
+cudaError_t cudaHostUnregister(void *) {
+    g_pinned--;
+    return cudaSuccess;
+}
 cudaError_t cudaFree(void *p) { return drop(p); }
-cudaError_t cudaFreeHost(void *p) { return drop(p); }
+cudaError_t cudaFreeHost(void *p) {
+    g_pinned--;
+    return drop(p);
+}
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t) {
     if (k == cudaMemcpyHostToDevice && room(d) < n) {
         wrong("a copy past its destination");
@@ -223,6 +240,20 @@ static lcg_status curve(lcg_ctx *c, const lcg_model &m, int n) {
 int main(int argc, char **argv) {
     lcg_model a, b;
     if (argc < 2 || fread(&a, sizeof a, 1, stdin) != 1 || fread(&b, sizeof b, 1, stdin) != 1) return 2;
+    if (!strcmp(argv[1], "pin")) {
+        lcg_ctx *c = nullptr;
+        if (lcg_create(&c, nullptr)) return 3;
+        for (int i = 0; i < 200; i++) {
+            if (points(c, 100) || curve(c, a, 100)) return 3;
+            if (i < 20 && g_pins) wrong("pinned memory before it can pay");
+        }
+        if (g_pins != 2) wrong("the points and the results pinned once each");
+        if (points(c, 5000) || curve(c, a, 5000) || g_pinned) wrong("blocks grown, not unpinned");
+        lcg_destroy(c);
+        if (g_pinned) wrong("pinned memory left behind");
+        printf("%d %d\n", g_pins, g_wrong);
+        return g_wrong ? 1 : 0;
+    }
     const bool data = !strcmp(argv[1], "data");
     int k = 1;
     for (;; k++) {

@@ -2,7 +2,8 @@
 
 host_check.cpp compiles engine.cu against a fake CUDA runtime in which the k-th
 allocation of a call fails. Whatever k is, that call returns an error and the
-next one runs on arrays, tables and fluxes of its own.
+next one runs on arrays, tables and fluxes of its own. And what a context costs
+before it has done much.
 """
 import os
 import shutil
@@ -52,3 +53,8 @@ def test_fluxes_after_a_failed_allocation(host_check, over):
 def test_points_after_a_failed_allocation(host_check):
     """Points that did not fit are refused, and no call takes the freed ones for them."""
     assert _run(host_check, "data", {}, dict(nlat1f=20, nlat2f=24)) >= 2
+
+
+def test_pinned_memory_waits_until_it_pays(host_check):
+    """A context of few calls pins nothing; one of many does so once, and undoes it."""
+    _run(host_check, "pin", {}, {})
