@@ -91,7 +91,10 @@ struct Fail {
 };
 
 struct Grid {
-    DBuf<double> px, py, pz, nx, ny, nz, ein, eout;
+    // positions, normals, eclipse phases: eight columns of one allocation (a cudaMalloc of
+    // 2 MB or more takes 0.33 ms, eight of them half of a context's first call)
+    DBuf<double> pts;
+    int64_t stride = 0;
     DBuf<float> area, grav, flux;
     DBuf<uint8_t> necl;
     DBuf<RingRec> rings;
@@ -121,12 +124,10 @@ struct Grid {
         n = nf;
         ntiled = nf;
         cudaError_t e = cudaSuccess;
-        DBuf<double> *d[] = {&px, &py, &pz, &nx, &ny, &nz, &ein, &eout};
-        for (auto *b : d)
-            if ((e = b->ensure(nf)) != cudaSuccess) return e;
-        if ((e = area.ensure(nf)) || (e = grav.ensure(nf)) || (e = flux.ensure(nf)) ||
-            (e = necl.ensure(nf)) || (e = cnt.ensure(2 * cont_blocks(nf))) ||
-            (e = dsum.ensure(4 * cont_blocks(nf))))
+        stride = (nf + 15) / 16 * 16;
+        if ((e = pts.ensure(8 * stride)) || (e = area.ensure(nf)) || (e = grav.ensure(nf)) ||
+            (e = flux.ensure(nf)) || (e = necl.ensure(nf)) ||
+            (e = cnt.ensure(2 * cont_blocks(nf))) || (e = dsum.ensure(4 * cont_blocks(nf))))
             return e;
         return cudaSuccess;
     }
@@ -154,8 +155,10 @@ struct Grid {
         return cudaSuccess;
     }
     GridDev dev() const {
-        return GridDev{px.p, py.p, pz.p, nx.p, ny.p, nz.p, area.p, grav.p, flux.p,
-                       necl.p, ein.p, eout.p, n, ntiled, disc ? ndx.p : nullptr,
+        double *c = pts.p;
+        const int64_t s = stride;
+        return GridDev{c, c + s, c + 2 * s, c + 3 * s, c + 4 * s, c + 5 * s, area.p, grav.p, flux.p,
+                       necl.p, c + 6 * s, c + 7 * s, n, ntiled, disc ? ndx.p : nullptr,
                        disc ? xr.p : nullptr};
     }
     FlatDev flat() const {
@@ -164,8 +167,7 @@ struct Grid {
                        n0.p ? n0.p + 1 : nullptr, ridx.p, rr.p, rn.p};
     }
     void release() {
-        DBuf<double> *d[] = {&px, &py, &pz, &nx, &ny, &nz, &ein, &eout, &fdx, &fdy,
-                             &fdz, &fpx, &fpy, &fpz, &fflux, &fin, &fout};
+        DBuf<double> *d[] = {&pts, &fdx, &fdy, &fdz, &fpx, &fpy, &fpz, &fflux, &fin, &fout};
         for (auto *b : d) b->release();
         area.release(); grav.release(); flux.release(); necl.release(); rings.release();
         queue.release(); counters.release(); es.release(); hits.release();

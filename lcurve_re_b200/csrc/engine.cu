@@ -1383,18 +1383,19 @@ lcg_status lcg_star_grid(lcg_ctx *c, const lcg_model *m, int32_t star, int32_t f
     std::vector<double> px(nface), py(nface), pz(nface), nx(nface), ny(nface), nz(nface);
     std::vector<uint8_t> ne(nface);
     const size_t d8 = (size_t)nface * sizeof(double), f4 = (size_t)nface * sizeof(float);
-    cudaMemcpyAsync(px.data(), g.px.p, d8, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(py.data(), g.py.p, d8, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(pz.data(), g.pz.p, d8, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(nx.data(), g.nx.p, d8, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(ny.data(), g.ny.p, d8, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(nz.data(), g.nz.p, d8, cudaMemcpyDeviceToHost, c->stream);
+    const GridDev gd = g.dev();
+    cudaMemcpyAsync(px.data(), gd.px, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(py.data(), gd.py, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(pz.data(), gd.pz, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(nx.data(), gd.nx, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(ny.data(), gd.ny, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(nz.data(), gd.nz, d8, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(area, g.area.p, f4, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(gravity, g.grav.p, f4, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(flux, g.flux.p, f4, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(ne.data(), g.necl.p, (size_t)nface, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(ecl_in, g.ein.p, d8, cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(ecl_out, g.eout.p, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(ecl_in, gd.ein, d8, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(ecl_out, gd.eout, d8, cudaMemcpyDeviceToHost, c->stream);
     if ((rc = finish_status(c))) return rc;
     for (int i = 0; i < nface; i++) {
         posn[3 * i] = px[i]; posn[3 * i + 1] = py[i]; posn[3 * i + 2] = pz[i];

@@ -6,9 +6,10 @@
 // given: that every array lives and is large enough, that the ring table belongs to
 // the grid, and that a sweep reads the fluxes of the model it is launched for.
 //
-//   host_check rings|cache|data|pin   (stdin: lcg_model A, lcg_model B)
+//   host_check rings|cache|data|pin|first   (stdin: lcg_model A, lcg_model B)
 //
-// pin: many calls with A, counting pinned blocks. The others:
+// pin: many calls with A, counting pinned blocks. first: prints the device allocations of 2 MB
+// or more of a context's first call, with A. The others:
 // A call with A, one with B whose k-th allocation fails, then A again (mode data: points for
 // the first call, more of them for the second), in a new context for every k until the second
 // call has none left to fail. Prints the number of failures tried and of what was wrong;
@@ -22,7 +23,7 @@
 
 static std::map<char *, size_t> g_mem;
 static long g_countdown = -1;  // allocations until one fails
-static int g_wrong = 0, g_pinned = 0, g_pins = 0;
+static int g_wrong = 0, g_pinned = 0, g_pins = 0, g_large = 0;
 static const lcg_model *g_model = nullptr;
 static std::map<const void *, double> g_flux_t, g_flat_t;  // by array: the model's temperature
 
@@ -57,7 +58,10 @@ static cudaError_t drop(void *p) {
 }
 
 extern "C" {
-cudaError_t cudaMalloc(void **p, size_t n) { return get(p, n); }
+cudaError_t cudaMalloc(void **p, size_t n) {
+    g_large += n >= (size_t)2 << 20;
+    return get(p, n);
+}
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
     g_pinned++;
     g_pins++;
@@ -240,6 +244,13 @@ static lcg_status curve(lcg_ctx *c, const lcg_model &m, int n) {
 int main(int argc, char **argv) {
     lcg_model a, b;
     if (argc < 2 || fread(&a, sizeof a, 1, stdin) != 1 || fread(&b, sizeof b, 1, stdin) != 1) return 2;
+    if (!strcmp(argv[1], "first")) {
+        lcg_ctx *c = nullptr;
+        if (lcg_create(&c, nullptr) || points(c, 100) || curve(c, a, 100)) return 3;
+        printf("%d %d\n", g_large, g_wrong);
+        lcg_destroy(c);
+        return g_wrong ? 1 : 0;
+    }
     if (!strcmp(argv[1], "pin")) {
         lcg_ctx *c = nullptr;
         if (lcg_create(&c, nullptr)) return 3;
