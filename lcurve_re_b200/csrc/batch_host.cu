@@ -150,6 +150,7 @@ struct BatchState {
     std::map<int32_t, RingSet> ringsets;
     std::vector<RingRec> h_rings;
     DBuf<RingRec> rings;
+    size_t rings_up = 0;  // how many of h_rings are on the device
     // per-model exact-reuse keys: the last model evaluated in each position,
     // its input scale and the data version its results belong to
     std::vector<lcg_model> key;
@@ -294,7 +295,6 @@ lcg_status relayout(lcg_ctx *c, BatchState &B, const lcg_model *models, int32_t 
     B.flat0.assign(B.nslots + 1, 0);
     B.blk0.assign(B.nslots + 1, 0);
     B.chunk_pre.assign(B.nslots + 1, 0);
-    const size_t nring_before = B.h_rings.size();
     for (int32_t m = 0; m < nmodels; m++) {
         B.nlat[2 * m] = models[m].nlat1f;
         B.nlat[2 * m + 1] = models[m].nlat2f;
@@ -395,10 +395,13 @@ lcg_status relayout(lcg_ctx *c, BatchState &B, const lcg_model *models, int32_t 
         (e = B.sfac.ensure(nm * 5)) || (e = B.out.ensure(nm * 3)) ||
         (e = B.d_tab.ensure(B.tab_bytes)))
         return c->cuda_fail(e, "batch buffers");
-    if (B.h_rings.size() != nring_before || !B.rings.p) {
-        if ((e = B.rings.ensure(B.h_rings.size()))) return c->cuda_fail(e, "ring pool");
-        cudaMemcpyAsync(B.rings.p, B.h_rings.data(), B.h_rings.size() * sizeof(RingRec),
-                        cudaMemcpyHostToDevice, c->stream);
+    if (B.h_rings.size() != B.rings_up) {
+        B.rings_up = 0;
+        if ((e = B.rings.ensure(B.h_rings.size())) ||
+            (e = cudaMemcpyAsync(B.rings.p, B.h_rings.data(), B.h_rings.size() * sizeof(RingRec),
+                                 cudaMemcpyHostToDevice, c->stream)))
+            return c->cuda_fail(e, "ring pool");
+        B.rings_up = B.h_rings.size();
     }
     // an odd pad record or a never-built slot must read as zeros
     cudaMemsetAsync(B.fp.p, 0, 8 * (size_t)B.nflat * sizeof(float), c->stream);

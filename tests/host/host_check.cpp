@@ -1,15 +1,16 @@
-// The engine's host side (engine.cu) on the CPU, with allocations that fail.
+// The engine's host side (engine.cu, batch_host.cu) on the CPU, with allocations that fail.
 //
-// engine.cu holds no device code: it is compiled here with the host compiler against a
+// Neither holds device code: they are compiled here with the host compiler against a
 // runtime in which device memory is host memory and the n-th allocation of a call returns
 // cudaErrorMemoryAllocation. The kernels' launchers are replaced by checks of what they are
 // given: that every array lives and is large enough, that the ring table belongs to
 // the grid, and that a sweep reads the fluxes of the model it is launched for.
 //
-//   host_check rings|cache|data|pin|first   (stdin: lcg_model A, lcg_model B)
+//   host_check rings|cache|data|pin|first|batch|moved   (stdin: lcg_model A, lcg_model B)
 //
 // pin: many calls with A, counting pinned blocks. first: prints the device allocations of 2 MB
-// or more of a context's first call, with A. The others:
+// or more of a context's first call, with A. batch: batched calls in place of single ones.
+// moved: a batch's captured graph after its points moved. The others:
 // A call with A, one with B whose k-th allocation fails, then A again (mode data: points for
 // the first call, more of them for the second), in a new context for every k until the second
 // call has none left to fail. Prints the number of failures tried and of what was wrong;
@@ -17,9 +18,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
+#include <set>
 
 #include "../../lcurve_re_b200/csrc/engine.cu"
+#include "../../lcurve_re_b200/csrc/batch_host.cu"
 
 static std::map<char *, size_t> g_mem;
 static long g_countdown = -1;  // allocations until one fails
@@ -42,18 +46,36 @@ template <class T>
 static void need(const T *p, int64_t n, const char *what) {
     if (room(p) < (size_t)n * sizeof(T)) wrong(what);
 }
+// what a captured stream would run when its graph is launched
+static std::vector<std::function<void()>> g_graph;
+static bool g_capturing = false;
+template <class F>
+static void stream(F f) {
+    if (g_capturing) g_graph.push_back(f);
+    else f();
+}
+static const size_t kKeep = 1 << 20;
+static char *g_arena = nullptr;      // blocks of kKeep bytes, given out lowest address first
+static std::set<char *> g_free;
 static cudaError_t get(void **p, size_t n) {
     if (g_countdown > 0 && --g_countdown == 0) {
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
-    *p = calloc(1, n);
+    if (g_arena && n <= kKeep && !g_free.empty()) {
+        *p = *g_free.begin();
+        g_free.erase(g_free.begin());
+    } else {
+        *p = calloc(1, n);
+    }
     g_mem[(char *)*p] = n;
     return cudaSuccess;
 }
-static cudaError_t drop(void *p) {
-    g_mem.erase((char *)p);
-    free(p);
+static cudaError_t drop(void *v) {
+    char *p = (char *)v;
+    g_mem.erase(p);
+    if (g_arena && p >= g_arena && p < g_arena + 64 * kKeep) g_free.insert(p);
+    else free(p);
     return cudaSuccess;
 }
 
@@ -82,11 +104,10 @@ cudaError_t cudaFreeHost(void *p) {
     return drop(p);
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t) {
-    if (k == cudaMemcpyHostToDevice && room(d) < n) {
-        wrong("a copy past its destination");
-        return cudaErrorInvalidValue;
-    }
-    memcpy(d, s, n);
+    stream([=] {
+        if (room(k == cudaMemcpyHostToDevice ? d : s) < n) wrong("a copy past its array");
+        else memcpy(d, s, n);
+    });
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
@@ -98,10 +119,32 @@ cudaError_t cudaMemcpy2DAsync(void *, size_t, const void *, size_t, size_t, size
     return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) {
-    if (room(p) < n) wrong("a clear past its array");
-    else memset(p, v, n);
+    stream([=] {
+        if (room(p) < n) wrong("a clear past its array");
+        else memset(p, v, n);
+    });
     return cudaSuccess;
 }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    g_capturing = true;
+    g_graph.clear();
+    return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) {
+    g_capturing = false;
+    *g = (cudaGraph_t)&g_graph;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t g, unsigned long long) {
+    *e = (cudaGraphExec_t)g;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
+    for (auto &f : g_graph) f();
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp *p, int) {
     memset(p, 0, sizeof *p);
@@ -122,17 +165,14 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *t, cudaEvent_t, cudaEvent_t) { *t = 0.f; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "allocation failed by the test"; }
-lcg_status lcg_light_curve_batch_resident(lcg_ctx *, const lcg_model *, int32_t, int32_t, double *,
-                                          double *, double *, double *, int32_t *) {
-    return LCG_E_INVALID;
-}
 }
 
 namespace lcg {
 
 static void need_grid(const GridDev &g) {
     for (const double *p : {g.px, g.py, g.pz, g.nx, g.ny, g.nz, g.ein, g.eout}) need(p, g.n, "grid");
-    for (const float *p : {g.area, g.grav, g.flux}) need(p, g.n, "grid");
+    for (const float *p : {g.area, g.grav}) need(p, g.n, "grid");
+    if (g.flux) need(g.flux, g.n, "grid");  // batches keep none
     need(g.necl, g.n, "grid");
 }
 void launch_grid(const GridParams &p, const RingRec *r, GridDev g, int32_t *cnt, DevStatus *,
@@ -218,8 +258,51 @@ void launch_comp_sums(const ElemRec *, int32_t, int32_t, int32_t, double, double
 int64_t comp_sums_scratch(int32_t, int64_t) { return 1; }
 void launch_fma_probe(float *, int, int, double *, cudaStream_t) {}
 void launch_dfma_probe(double *, int, int, double *, cudaStream_t) {}
+void launch_batch_grid(const BatchDev &b, int, cudaStream_t) {
+    stream([=] {
+        for (int k = 0; k < b.counts[0]; k++) {
+            const SlotDev &S = b.slots[b.geo_slot[k]];
+            const RingRec *r = b.rings + S.ring0;
+            if (room(r) < (size_t)S.gp.nrings * sizeof(RingRec)) {
+                wrong("a ring pool shorter than a slot's rings");
+                continue;
+            }
+            const RingRec &last = r[S.gp.nrings - 1];
+            if (last.off + last.nphi != S.ntiled) wrong("a ring table of another slot");
+        }
+    });
+}
+void launch_batch_eclipse(const BatchDev &b, int, int32_t, cudaStream_t) {
+    stream([=] {
+        need_grid(b.g);
+        need(b.queue, b.qcap, "queue");
+        need(b.es, b.qcap, "states");
+    });
+}
+void launch_batch_partition(const BatchDev &, int, cudaStream_t) {}
+void launch_batch_continuum(const BatchDev &b, int, cudaStream_t) {
+    stream([=] { need(b.fp, 8 * b.g.n, "records"); });
+}
+void launch_batch_phases(const BatchDev &, const DatumRec *d, const int64_t *off, int32_t n,
+                         const BatchPhases &, cudaStream_t) {
+    stream([=] {
+        need(d, n, "points");
+        need(off, n + 1, "offsets");
+        if (room(off) >= (size_t)(n + 1) * 8 && (off[0] != 0 || off[n] != n)) wrong("other offsets");
+    });
+}
+void launch_batch_flux(const BatchDev &, const BatchPhases &, const FluxPlan &, double *, int64_t,
+                       cudaStream_t) {}
+void launch_batch_reduce(const BatchDev &, const BatchPhases &, const double *, int64_t, double *,
+                         const DatumRec *d, const int64_t *off, int32_t n, int32_t, double *, double *,
+                         double *, cudaStream_t) {
+    stream([=] {
+        need(d, n, "points");
+        need(off, n + 1, "offsets");
+    });
+}
+void launch_gather_rows(const double *, int32_t, const int32_t *, int32_t, double *, cudaStream_t) {}
 namespace eng {
-void batch_release(BatchState *) {}
 bool comp_setup(const lcg_model &, CompParams &, std::vector<DiscRing> &, Fail &) { return false; }
 }  // namespace eng
 }  // namespace lcg
@@ -239,6 +322,19 @@ static lcg_status curve(lcg_ctx *c, const lcg_model &m, int n) {
     double sfac[5] = {1., 1., 1., 1., 1.}, out[LCG_NOUT];
     g_model = &m;
     return lcg_light_curve_resident(c, &m, 0, sfac, calc.data(), out);
+}
+
+static lcg_status batch(lcg_ctx *c, const lcg_model &a, const lcg_model &b, int n) {
+    lcg_model m[2] = {a, b};
+    std::vector<double> calc(2 * (size_t)n);
+    double sfac[10], chisq[2], wnok[2];
+    int32_t st[2];
+    for (double &s : sfac) s = 1.;
+    // new temperatures: nothing is reused
+    static double step = 0.;
+    m[0].t1 += (step += 1.);
+    m[1].t1 += step;
+    return lcg_light_curve_batch_resident(c, m, 2, 0, sfac, calc.data(), chisq, wnok, st);
 }
 
 int main(int argc, char **argv) {
@@ -265,17 +361,41 @@ int main(int argc, char **argv) {
         printf("%d %d\n", g_pins, g_wrong);
         return g_wrong ? 1 : 0;
     }
-    const bool data = !strcmp(argv[1], "data");
+    if (!strcmp(argv[1], "moved")) {
+        // three blocks in a row, the points in the first and the offsets in the third; then the
+        // second becomes free, and larger points get the first and the second
+        lcg_ctx *c = nullptr;
+        if (lcg_create(&c, nullptr)) return 3;
+        g_arena = (char *)calloc(64, kKeep);
+        for (int i = 0; i < 64; i++) g_free.insert(g_arena + i * kKeep);
+        void *blk[3];
+        for (void *&p : blk) cudaMalloc(&p, 64);
+        cudaFree(blk[0]);
+        cudaFree(blk[2]);
+        if (points(c, 100) || c->data.p != blk[0] || (void *)c->off.p != blk[2]) return 4;
+        for (int i = 0; i < 3; i++)
+            if (batch(c, a, a, 100)) return 3;
+        cudaFree(blk[1]);
+        if (points(c, 5000) || c->data.p != blk[0] || (void *)c->off.p != blk[1]) return 4;
+        if (points(c, 100) || batch(c, a, a, 100)) return 3;
+        lcg_destroy(c);
+        printf("1 %d\n", g_wrong);
+        return g_wrong ? 1 : 0;
+    }
+    const bool data = !strcmp(argv[1], "data"), many = !strcmp(argv[1], "batch");
     int k = 1;
     for (;; k++) {
         lcg_ctx *c = nullptr;
-        if (lcg_create(&c, nullptr) || points(c, 100) || curve(c, a, 100)) return 3;
+        if (lcg_create(&c, nullptr) || points(c, 100)) return 3;
+        for (int i = 0; i < (many ? 3 : 1); i++)
+            if (many ? batch(c, a, a, 100) : curve(c, a, 100)) return 3;
         g_countdown = k;
-        const lcg_status st = data ? points(c, 5000) : curve(c, b, 100);
+        const lcg_status st = data ? points(c, 5000) : many ? batch(c, a, b, 100) : curve(c, b, 100);
         const bool failed = g_countdown == 0;
         g_countdown = -1;
         if (failed != (st != LCG_OK)) wrong("a failed allocation without a status");
-        const lcg_status again = curve(c, a, 5000);
+        lcg_status again = many ? batch(c, a, b, 100) : curve(c, a, 5000);
+        for (int i = 0; i < 3 && many && !again; i++) again = batch(c, i ? b : a, a, 100);
         // after points that were not taken there are none
         if (data ? (again == LCG_OK) == failed : again != LCG_OK) {
             wrong("the call after it");

@@ -1,6 +1,6 @@
 """The engine's host side when an allocation fails, on the CPU.
 
-host_check.cpp compiles engine.cu against a fake CUDA runtime in which the k-th
+host_check.cpp compiles engine.cu and batch_host.cu against a fake CUDA runtime in which the k-th
 allocation of a call fails. Whatever k is, that call returns an error and the
 next one runs on arrays, tables and fluxes of its own. And what a context costs
 before it has done much.
@@ -25,7 +25,8 @@ def host_check():
     if shutil.which("g++") is None or not os.path.isdir(os.path.join(CUDA, "include")):
         pytest.skip("g++ or the CUDA headers are not available")
     os.makedirs(os.path.dirname(EXE), exist_ok=True)
-    subprocess.check_call(["g++", "-x", "c++", "-std=c++17", "-O1", "-I" + os.path.join(CUDA, "include"),
+    subprocess.check_call(["g++", "-x", "c++", "-std=c++17", "-O1", "-pthread",
+                           "-I" + os.path.join(CUDA, "include"),
                            "-I" + os.path.join(ROOT, "include"), "-o", EXE, SRC])
     return EXE
 
@@ -64,3 +65,9 @@ def test_first_calls_make_few_large_allocations(host_check):
     """Each takes a third of a millisecond: per grid of 326,000 faces its points, the state of
     its eclipse candidates, its records and their ranges."""
     assert _run(host_check, "first", dict(nlat1f=506, nlat2f=506), {}) <= 8
+
+
+@pytest.mark.parametrize("nlat1,nlat2", [(60, 70), (20, 70), (90, 24)])
+def test_batches_after_a_failed_allocation(host_check, nlat1, nlat2):
+    """Ring tables that a failed layout added to the pool reach the device with the next one."""
+    assert _run(host_check, "batch", {}, dict(nlat1f=nlat1, nlat2f=nlat2)) >= 8
