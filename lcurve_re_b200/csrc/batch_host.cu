@@ -136,7 +136,7 @@ struct BatchState {
     // layout key
     int32_t nmodels = -1, n = 0, flags = 0, want_calc = 0;
     int64_t nent = 0;
-    const void *data_p = nullptr;
+    const void *data_p = nullptr, *off_p = nullptr;  // what the captured graph reads
     std::vector<int32_t> nlat;  // nlat1f, nlat2f per model
     // layout
     int32_t nslots = 0;
@@ -286,6 +286,7 @@ lcg_status relayout(lcg_ctx *c, BatchState &B, const lcg_model *models, int32_t 
     B.n = c->data_n;
     B.nent = c->data_nent;
     B.data_p = c->data.p;
+    B.off_p = c->off.p;
     B.flags = flags;
     B.want_calc = want_calc;
     B.nslots = 2 * nmodels;
@@ -428,7 +429,8 @@ lcg_status relayout(lcg_ctx *c, BatchState &B, const lcg_model *models, int32_t 
 bool same_layout(const BatchState &B, const lcg_ctx *c, const lcg_model *models,
                  int32_t nmodels, int32_t flags, int want_calc) {
     if (B.nmodels != nmodels || B.n != c->data_n || B.nent != c->data_nent ||
-        B.data_p != (const void *)c->data.p || B.flags != flags || B.want_calc != want_calc)
+        B.data_p != (const void *)c->data.p || B.off_p != (const void *)c->off.p ||
+        B.flags != flags || B.want_calc != want_calc)
         return false;
     for (int32_t m = 0; m < nmodels; m++)
         if (B.nlat[2 * m] != models[m].nlat1f || B.nlat[2 * m + 1] != models[m].nlat2f)

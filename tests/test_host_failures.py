@@ -71,3 +71,9 @@ def test_first_calls_make_few_large_allocations(host_check):
 def test_batches_after_a_failed_allocation(host_check, nlat1, nlat2):
     """Ring tables that a failed layout added to the pool reach the device with the next one."""
     assert _run(host_check, "batch", {}, dict(nlat1f=nlat1, nlat2f=nlat2)) >= 8
+
+
+def test_batches_after_their_points_moved(host_check):
+    """Points that grew and shrank back lie in the same block, their offsets in another: the
+    captured graph goes with both."""
+    _run(host_check, "moved", {}, {})
