@@ -39,25 +39,28 @@ struct DBuf {
 };
 
 // Host memory that grows, for the copies of a call; its contents do not survive growth. It
-// is pinned where it lies once kPinAfter calls found it large enough: pinning takes 0.4 ms
-// and undoing it 0.2, while a call gains 2 us (500 points) to 10 us (10,000), so a context
-// of few calls should not pay for it (blocks of cudaHostAlloc, 1 to 3 ms each, made the first
-// call of a context on 81/163 strips and 2,411 points 3.3 to 4.8 ms instead of 2.2).
+// is pinned where it lies once kPinAfter bytes went through it, a call counting as kPerCall
+// more: pinning takes 0.4 ms and undoing it 0.2, and saves 2-5 us a call and 0.04-0.05 us per
+// KB (30,000 points 100 us), so that is when it has paid for itself. A context of few calls
+// does not pay (blocks of cudaHostAlloc, 1 to 3 ms each, made the first call of a context on 81/163
+// strips and 2,411 points 3.3 to 4.8 ms instead of 2.2).
 struct HBuf {
-    static constexpr int kPinAfter = 64;
+    static constexpr size_t kPinAfter = 12u << 20, kPerCall = 64u << 10;
     unsigned char *p = nullptr;
-    size_t cap = 0;
-    int calls = 0;
-    bool pinned = false;
+    size_t cap = 0, used = 0;
+    bool tried = false, pinned = false;
     cudaError_t ensure(size_t bytes) {
         if (bytes <= cap) {
-            if (++calls == kPinAfter) {
+            used += bytes + kPerCall;
+            if (used >= kPinAfter && !tried) {
+                tried = true;
                 pinned = cudaHostRegister(p, cap, cudaHostRegisterDefault) == cudaSuccess;
                 if (!pinned) cudaGetLastError();  // the copies work without, only slower
             }
             return cudaSuccess;
         }
         release();
+        used = bytes;
         bytes += bytes / 2;  // a fit's light curves come in a few sizes
         bytes = (bytes + 4095) / 4096 * 4096;
         p = (unsigned char *)aligned_alloc(4096, bytes);
@@ -69,9 +72,8 @@ struct HBuf {
         if (pinned) cudaHostUnregister(p);
         free(p);
         p = nullptr;
-        cap = 0;
-        calls = 0;
-        pinned = false;
+        cap = used = 0;
+        tried = pinned = false;
     }
 };
 

@@ -350,12 +350,12 @@ int main(int argc, char **argv) {
     if (!strcmp(argv[1], "pin")) {
         lcg_ctx *c = nullptr;
         if (lcg_create(&c, nullptr)) return 3;
-        for (int i = 0; i < 200; i++) {
-            if (points(c, 100) || curve(c, a, 100)) return 3;
+        for (int i = 0; i < 400; i++) {  // 320 KB of points a call, 40 KB of results
+            if (points(c, 5000) || curve(c, a, 5000)) return 3;
             if (i < 20 && g_pins) wrong("pinned memory before it can pay");
         }
         if (g_pins != 2) wrong("the points and the results pinned once each");
-        if (points(c, 5000) || curve(c, a, 5000) || g_pinned) wrong("blocks grown, not unpinned");
+        if (points(c, 20000) || curve(c, a, 20000) || g_pinned) wrong("blocks grown, not unpinned");
         lcg_destroy(c);
         if (g_pinned) wrong("pinned memory left behind");
         printf("%d %d\n", g_pins, g_wrong);
