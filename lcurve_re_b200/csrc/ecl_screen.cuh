@@ -1,4 +1,5 @@
-// ecl_screen.cuh — an FP32 screen of the eclipse line-of-sight test.
+// ecl_screen.cuh — an FP32 screen of the eclipse line-of-sight test. No kernel uses it since
+// the boundaries come from their roots (ecl_root.cuh); its test on the CPU does.
 //
 // Roche::fblink (fblink.cpp:34-104) decides whether the line of sight from a
 // point towards the earth passes inside the companion's Roche lobe: it cuts

@@ -369,7 +369,8 @@ __device__ __noinline__ bool fblink(int star, double q, double spin, double acc,
 // of 60-400 strips: 13.8 ms; with the intervals of edge_zone alone, and 3.3 searches
 // per M-dwarf boundary for what they leave, 5.4; with narrow_zone 3.8. One curve on
 // 400/200 strips: 103 -> 60 us a star by narrow_zone. With the FP32 screen kept for
-// the tests outside the intervals the batch took 0.4 ms more. (Times before the cap on short chords, 3%.)
+// the tests outside the intervals the batch took 0.4 ms more. (Times before the cap on
+// short chords, 3%, and the certificate of the whole chord, 11%.)
 template <class Ecl>
 __device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pin, double pout,
                                               double acc, V3 pos, int &s) {
@@ -425,8 +426,9 @@ __device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pi
 namespace lcg {
 namespace {
 
-// Warp-cooperative Roche::ingress_egress, for grids with few eclipse
-// candidates, where one thread per face leaves the GPU idle. Lane 0 runs the
+// Warp-cooperative Roche::ingress_egress by the plain bisection, on request only (a lane
+// per boundary, from its root, is faster at any number of candidates): what the other
+// kernels are tested against. Lane 0 runs the
 // sphere test and pot_min; then lanes 0-15 bisect the ingress and lanes 16-31
 // the egress. Each half evaluates at once the 15 midpoints of the next four
 // bisection steps (a complete binary tree of brackets in heap order: child 2n

@@ -14,7 +14,8 @@
 //    faces; all lanes read the same face record (shared-memory broadcast).
 //  * element math in FP32; sums over at most 64 faces in FP32, folded into
 //    FP64 accumulators; one FP64 partial per (chunk, entry) is written and
-//    merged in chunk order by k_scatter (deterministic, no atomics).
+//    added by k_reduce_chunks, eighths of the chunks in order (deterministic, no
+//    atomics).
 //  * eclipse test in 64-bit fixed-point phase: visible iff (phase - ingress)
 //    mod 2^64 >= width + 1 (ecl_fx64, geometry.cu), the reference's double
 //    comparisons decision for decision.
@@ -773,7 +774,8 @@ FluxPlan plan_flux(int mixed, int fast, int64_t nface, int64_t nent, int nsm) {
         while (p.group > 64 && (nface + p.group - 1) / p.group < want) p.group >>= 1;
         // The chunk only regroups FP64 sums: the one whose whole waves, three CTAs an SM
         // (80 registers), cost least, a CTA's faces plus some 32 faces' worth of loading
-        // and ending. 9,003 entries and 18,600 faces: 256 faces fill 1.5 waves, 136 us;
+        // and ending. (At eight entries a thread, 162 to 232 registers, one CTA fits; waves
+        // counted so were within 2% of these at 16,384 to 60,000 entries.) 9,003 entries and 18,600 faces: 256 faces fill 1.5 waves, 136 us;
         // 128 three, 111. Above 1024 the shared memory would turn CTAs away.
         const int64_t slots = 3 * (int64_t)nsm;
         int64_t best = INT64_MAX;

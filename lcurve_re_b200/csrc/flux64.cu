@@ -3,7 +3,7 @@
 // Same sums as sum_star{1,2}_multi_t (comp_light_flat.cpp:241-372): faces in
 // blocks of 1024 (FACE_BLOCK, :239) in FlatGrid order; per block and phase
 // entry, element values of s1_elem / s2_elem (:109-168) are added in
-// ascending face order; k_scatter then adds the block partials in block
+// ascending face order; k_reduce_chunks then adds the block partials in block
 // order. Compiled with --fmad=false, every operation rounds as in the
 // reference, so given the same FlatGrid and phases the result is
 // bit-identical (sqrt and division are IEEE on both sides).

@@ -1463,8 +1463,8 @@ __global__ void __launch_bounds__(128, 4) k_ecl_potmin_b(BatchDev b, int32_t war
     }
 }
 
-// 6 blocks of 4 warps per SM (a sweep of 4, 5, 6 and 8 on B200 chose 6: more
-// warps hide the FP64 latency, fewer registers spill more)
+// 4 blocks of 4 warps per SM (bisect_blocks_per_sm; the registers of 6 spill, 8.41 ms at 4
+// and 8.36 at 6 for two batches of 256 models, 4 faster on small ones)
 template <int NB>
 __global__ void __launch_bounds__(128, NB)
     k_ecl_bisect_b(__grid_constant__ const BatchDev b, int32_t warp_max) {
