@@ -39,11 +39,11 @@ enum { kEdgeFalse = 0, kEdgeTrue = 1, kEdgeUnsure = 2 };
 
 // Potential about the eclipser's centre (the shift moved into pref):
 //   f(u) = -me/|u| - mo/|u - (dx,0,0)| - ss/2 (ux^2 + uy^2) + k ux - pref
-// gap = 1 - rref (no point of the reference sphere is nearer to the other star), er = me / rref,
-// er3 = me / rref^3, bend = 2 mo / gap^3 + ss (the other terms curve down by no more there)
-// and, where er3 exceeds it clearly, ik = 2 / (er3 - bend), else 0.
+// er = me / rref. round: the eclipser's pull exceeds three times what the other terms can
+// bend f down by anywhere in the reference sphere (see EdgeEval).
 struct EdgeStar {
-    double me, mo, dx, ss, k, pref, rref2, cosi, sini, gap, er, er3, bend, ik;
+    double me, mo, dx, ss, k, pref, rref2, cosi, sini, rref, er;
+    int32_t round;
 };
 
 LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, double sini,
@@ -60,11 +60,10 @@ LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, dou
         s.pref = pref + comp;
     }
     s.rref2 = rref * rref;
-    s.gap = 1. - rref;
+    s.rref = rref;
     s.er = s.me / rref;
-    s.er3 = s.er / s.rref2;
-    s.bend = s.gap > 0. ? 2. * s.mo / (s.gap * s.gap * s.gap) + s.ss : 1e30;
-    s.ik = s.er3 - s.bend > 0.04 * s.er3 ? 2. / (s.er3 - s.bend) : 0.;
+    const double gap = 1. - rref;  // no point of the sphere is nearer to the other star
+    s.round = gap > 0. && s.er / s.rref2 > 3. * (2. * s.mo / (gap * gap * gap) + s.ss);
     s.cosi = cosi;
     s.sini = sini;
     return s;
@@ -73,16 +72,20 @@ LCG_HD EdgeStar make_edge_star(int star, double q, double spin, double cosi, dou
 // Whether the chord has no second well. "Not hidden" follows from the potential's minimum
 // near the midpoint only where no other lies lower: a contact binary's other star, with
 // an extreme mass ratio and the eclipser a slow rotator, digs one at the near end, and
-// Roche::fblink finds it. From a point at a distance t1 from the midpoint where f is at least
-// f0 and its slope outwards at least s0, the eclipser's term E(t) = -me / sqrt(b^2 + t^2) is
-// known exactly and the rest, the other star's and the rotation's, curves down by t2 at most:
-//   f(t) >= M(t) = f0 + E(t) - E(t1) + (s0 - E'(t1)) (t - t1) - t2 (t - t1)^2 / 2.
-// M bends down once at most on the way out, so with s0 >= 0 it is lowest at t1 or at the
-// chord's end, where E is -me / rref. t2 = bend (EdgeStar) serves most eclipsers and both
-// ends. Where the chord lies beyond the other star, which the line passes at a distance p,
-// and its near end w beyond that, 2 w^2 >= 3 p^2, that star's curvature grows all the
-// way to the near end: f itself bends down once at most, so its value there decides, and
-// towards the far end t2 is what it is at t1.
+// Roche::fblink finds it. Along the chord f = E + T, the eclipser's term E(t) = -me /
+// sqrt(b^2 + t^2), whose slope P(t) = me t / r^3 is at least er3 t, er3 = me / rref^3, and the
+// other star's and the rotation's, which bend down by T'' >= -c, c = 2 mo / (1 - rref)^3 + ss.
+//   * Round eclipsers, er3 > 3 c, where rref^2 < 1.6 b^2 and the minimum tm lies within b / 9 of
+//     the midpoint: past k tm, k = (me / b^3 - c) / (er3 - c) < 2.6, the slope is at least
+//     (er3 - c) t - (me / b^3 - c) tm > 0; up to there P' > er3 / 2 > c; on the other side of
+//     the midpoint P alone outweighs c. f falls to tm and rises after it: nothing else to see.
+//   * Otherwise from a point t1 with f >= f0 and a slope outwards of at least s0 >= 0,
+//       f(t) >= M(t) = f0 + E(t) - E(t1) + (s0 - P(t1)) (t - t1) - t2 (t - t1)^2 / 2
+//     while T'' >= -t2. M bends down once at most on the way out, so it is lowest at t1 or at
+//     the chord's end, where E = -me / rref. Where the chord lies beyond the other star,
+//     which the line passes at a distance p, and its near end w beyond that, 2 w^2 >= 3 p^2,
+//     T'' falls all the way to the near end: f itself bends down once at most, so its value
+//     there decides, and towards the far end t2 is what it is at t1.
 
 // One evaluation on the line of sight at a phase, a distance t beyond the
 // chord's midpoint: f, df/dphase (t held), slope g and curvature h along the
@@ -184,21 +187,19 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
             const double hmin = r.h - 5. * ae * tau * tau * ie2 - c3 * tau;
             const double low = r.f - ag * ag / (2. * hmin);
             if (hmin >= 0.5 * r.h && low > r.tol) {
-                // and the rest of the chord, from tau on with f >= low and the slope at
-                // least hmin tau - |g| >= 0 there; hc <= rref spares most their square root
-                const double c = (hmin - ae) * tau - ag, c0 = c < 0. ? c : 0.;
-                const double top = low + pe - 0.5 * ae * tau * tau - S.er - r.tol;
-                if (top + c0 * (1. - S.gap) > 0.5 * S.bend * hc2) {
+                if (S.round && S.rref2 < 1.6 * b2) {
                     r.ans = kEdgeFalse;
                 } else {
+                    // the chord's ends, from tau on, where the slope is at least hmin tau - |g|
                     const double hc = hc2 * edge_rsqrt(hc2), wn = ev - hc, p2 = d2 - ev * ev;
-                    const double curl = r.h < ae ? ae - r.h : 0.;
+                    const double c = (hmin - ae) * tau - ag, curl = r.h < ae ? ae - r.h : 0.;
                     const double nx = fma(-hc, ex, ux), ny = fma(-hc, ey, uy);
                     const double fn = fma(S.k, nx, fma(-0.5 * S.ss, fma(nx, nx, ny * ny),
                                                        -S.mo * edge_rsqrt(fma(wn, wn, p2)))) -
                                       S.er - S.pref;
-                    if (wn > 0. && 2. * wn * wn >= 3. * p2 && fn > r.tol &&
-                        top + c0 * hc > 0.5 * curl * hc2)
+                    const double far = low + pe - 0.5 * ae * tau * tau - S.er +
+                                       (c < 0. ? c : 0.) * hc - 0.5 * curl * hc2;
+                    if (wn > 0. && 2. * wn * wn >= 3. * p2 && fn > r.tol && far > r.tol)
                         r.ans = kEdgeFalse;
                 }
             }
@@ -341,40 +342,27 @@ LCG_HD EdgeBound edge_bound(const EdgeStar &S, const EdgeEval &v, double lam) {
 }
 
 // The part of a phase radius rad around v (edge_zone's stage 1) over which the chord has
-// no second well, 0 for none: M above from the minimum outwards (f >= 0 there from vis on,
-// its slope 0). The minimum lies within a of the midpoint, and f has no other within move of
-// v's point, less that point's own motion. vis < 0 reaches inwards of v. With y half the
-// chord and ae = me / r^3 at the minimum, M is above zero at an end of the chord where
-//   E(y) - E(a) > ae a y + t2 (y + a)^2 / 2.
-// First for both ends with t2 = bend: E(y) - E(a) >= er3 (y^2 - a^2) / 2 makes that so for
-// every y >= need, and a shorter chord is clear while it lies within move, or gone. Where
-// the eclipser's pull at its reference sphere is too weak for that (it fills its lobe), the
-// ends one by one while the chord keeps most of its length: the far one with t2 as it is at
-// the minimum, the near one by f itself, less what it can lose on its way. Of detached
-// binaries' boundaries all but 0.1% are certified, of lobe-filling donors' 5% are not.
+// no second well, 0 for none: above, from the minimum, which lies within a of the midpoint
+// and is above zero from vis on (vis < 0 reaches inwards of v). For a round eclipser that is
+// all of rad, over which b keeps 0.9 of itself. Else, while the chord keeps most of its
+// length y, by its far end, where M is above zero if
+//   E(y) - E(a) > (me / r^3) a y + t2 (y + a)^2 / 2
+// with t2 as it is at the minimum, and by f at the near end, less what it can lose on its
+// way. Of detached binaries' boundaries all but 0.1% are certified, of lobe-filling donors' 5%
+// are not.
 LCG_HD double clear_radius(const EdgeStar &S, V3 u0, const EdgeEval &v, double dir, double t,
                            double lam, double dt, double drift, double move, double vis,
                            double rad) {
+    const double at = fabs(t), hc2 = S.rref2 - v.b2;
+    double a = at + fabs(dt) + drift * rad;
+    if (S.round && S.rref2 < 1.3 * v.b2 && 100. * a * a < v.b2) return rad;
     // b^2 grows outwards by 0.8 to 1.2 db2 per phase
     const double db2 = -2. * v.x * v.xp * dir, bend = kTwoPi * kTwoPi / 1.1 * lam * lam;
     if (!(db2 > 0.)) return 0.;
     if (rad * bend > 0.1 * db2) rad = 0.1 * db2 / bend;
-    const double in = vis < 0. ? -2.1 * kTwoPi * lam * lam * vis : 0.;
-    const double hc2 = S.rref2 - v.b2, y2 = hc2 + in, at = fabs(t), ae = 1.1 * v.ae;
-    double a = at + fabs(dt) + drift * rad;
-    if (!(y2 > 0.)) return rad;
+    const double in = vis < 0. ? -2.1 * kTwoPi * lam * lam * vis : 0., ae = 1.1 * v.ae;
+    a = at + fabs(dt) + drift * rad;
     if (!(in < 0.05 * v.b2 && 110. * a * a < v.b2)) return 0.;
-    if (S.ik > 0.) {
-        const double need = a * (ae + 0.5 * (S.er3 + S.bend)) * S.ik;
-        const double speed = 1.2 * kTwoPi * lam, left = move - at - need;
-        const double room = hc2 - need * need;
-        // gone at y2 / (0.8 db2) at the latest
-        if (left * 0.8 * db2 >= y2 * speed) return rad;
-        if (room > 0.5 * hc2) {
-            const double r0 = room / (1.2 * db2);
-            return rad < r0 ? rad : r0;
-        }
-    }
     if (!(hc2 > 0.)) return 0.;
     // the far end: t2 is the other terms' curvature at v, with what it changes by
     const double ih = edge_rsqrt(hc2), hc = hc2 * ih, io2 = v.io * v.io, ib2 = 1. / db2;
@@ -406,7 +394,7 @@ LCG_HD double clear_radius(const EdgeStar &S, V3 u0, const EdgeEval &v, double d
     // the near end's speed along the sphere, and that of the other star's distance; x > hc,
     // the element being outside the sphere
     const double vel = kTwoPi * (lam + 1.) + 1.4 * db2 * ih;
-    const double grad = 1.25 * S.mo * ni * ni + fabs(S.k) + 1.1 * S.ss * (1. - S.gap);
+    const double grad = 1.25 * S.mo * ni * ni + fabs(S.k) + 1.1 * S.ss * S.rref;
     const double most = 0.1 * dn2 * ni;
     double r2 = 0.9 * fn;
     if (r2 > most * grad) r2 = most * grad;
