@@ -197,8 +197,10 @@ LCG_HD EdgeEval eval_edge(const EdgeStar &S, V3 u0, double u2, double acc, doubl
                     const double fn = fma(S.k, nx, fma(-0.5 * S.ss, fma(nx, nx, ny * ny),
                                                        -S.mo * edge_rsqrt(fma(wn, wn, p2)))) -
                                       S.er - S.pref;
-                    const double far = low + pe - 0.5 * ae * tau * tau - S.er +
-                                       (c < 0. ? c : 0.) * hc - 0.5 * curl * hc2;
+                    // (towards the far end it rises from the midpoint on where g > 0)
+                    const double up = r.g > 0. ? r.f + ag * hc
+                                               : low - 0.5 * ae * tau * tau + (c < 0. ? c : 0.) * hc;
+                    const double far = up + pe - S.er - 0.5 * curl * hc2;
                     if (wn > 0. && 2. * wn * wn >= 3. * p2 && fn > r.tol && far > r.tol)
                         r.ans = kEdgeFalse;
                 }
@@ -348,8 +350,7 @@ LCG_HD EdgeBound edge_bound(const EdgeStar &S, const EdgeEval &v, double lam) {
 // length y, by its far end, where M is above zero if
 //   E(y) - E(a) > (me / r^3) a y + t2 (y + a)^2 / 2
 // with t2 as it is at the minimum, and by f at the near end, less what it can lose on its
-// way. Of detached binaries' boundaries all but 0.1% are certified, of lobe-filling donors' 5%
-// are not.
+// way. Of lobe-filling donors' boundaries 99.9% are certified so.
 LCG_HD double clear_radius(const EdgeStar &S, V3 u0, const EdgeEval &v, double dir, double t,
                            double lam, double dt, double drift, double move, double vis,
                            double rad) {
@@ -360,10 +361,9 @@ LCG_HD double clear_radius(const EdgeStar &S, V3 u0, const EdgeEval &v, double d
     const double db2 = -2. * v.x * v.xp * dir, bend = kTwoPi * kTwoPi / 1.1 * lam * lam;
     if (!(db2 > 0.)) return 0.;
     if (rad * bend > 0.1 * db2) rad = 0.1 * db2 / bend;
-    const double in = vis < 0. ? -2.1 * kTwoPi * lam * lam * vis : 0., ae = 1.1 * v.ae;
-    a = at + fabs(dt) + drift * rad;
-    if (!(in < 0.05 * v.b2 && 110. * a * a < v.b2)) return 0.;
-    if (!(hc2 > 0.)) return 0.;
+    const double in = vis < 0. ? -2.1 * kTwoPi * lam * lam * vis : 0.;
+    if (!(in < 0.05 * v.b2 && hc2 > 0.)) return 0.;
+    const double ae = 1.15 * v.ae;  // of the minimum, anywhere in the zone
     // the far end: t2 is the other terms' curvature at v, with what it changes by
     const double ih = edge_rsqrt(hc2), hc = hc2 * ih, io2 = v.io * v.io, ib2 = 1. / db2;
     const double t0 = v.ae * (1. - 3. * t * t / v.r2) - v.h;
@@ -379,9 +379,12 @@ LCG_HD double clear_radius(const EdgeStar &S, V3 u0, const EdgeEval &v, double d
                           2. * kTwoPi * r1 * (2.7 * S.mo * io2 * v.io + S.ss);
         const double yl = (i ? 0.9591 : 0.8660) * hc;
         const double ib = edge_rsqrt(S.rref2 - yl * yl + a * a);
-        const double ey = S.me * ib - S.er, ey2 = 0.97 * S.me * ib * ib * ib;
+        const double ey = S.me * ib - S.er, ey2 = (1. - 3.2 * a * a / v.b2) * S.me * ib * ib * ib;
+        // the eclipser's pull at the minimum counts against the end on its own side only
+        const double pull = t + (a - at) < 0. ? 0. : ae * a;
         // and from there on, E growing by at least ey2 / 2 per y^2
-        if (ey > ae * a * yl + 0.5 * tf * (yl + a) * (yl + a) && ey2 * yl > ae * a + tf * (yl + a))
+        if (25. * a * a < v.b2 && ey > pull * yl + 0.5 * tf * (yl + a) * (yl + a) &&
+            ey2 * yl > pull + tf * (yl + a))
             break;
         if (i) return 0.;
     }
