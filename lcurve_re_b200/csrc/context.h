@@ -40,12 +40,12 @@ struct DBuf {
 
 // Host memory that grows, for the copies of a call; its contents do not survive growth. It
 // is pinned where it lies once kPinAfter bytes went through it, a call counting as kPerCall
-// more: pinning takes 0.4 ms and undoing it 0.2, and saves 2-5 us a call and 0.04-0.05 us per
+// more: pinning takes 0.4 ms and undoing it 0.2, and saves 2-6 us a call and 0.04-0.05 us per
 // KB (30,000 points 100 us), so that is when it has paid for itself. A context of few calls
 // does not pay (blocks of cudaHostAlloc, 1 to 3 ms each, made the first call of a context on 81/163
 // strips and 2,411 points 3.3 to 4.8 ms instead of 2.2).
 struct HBuf {
-    static constexpr size_t kPinAfter = 12u << 20, kPerCall = 64u << 10;
+    static constexpr size_t kPinAfter = 12u << 20, kPerCall = 128u << 10;
     unsigned char *p = nullptr;
     size_t cap = 0, used = 0;
     bool tried = false, pinned = false;
