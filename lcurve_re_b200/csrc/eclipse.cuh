@@ -370,7 +370,7 @@ __device__ __noinline__ bool fblink(int star, double q, double spin, double acc,
 // per M-dwarf boundary for what they leave, 5.4; with narrow_zone 3.8. One curve on
 // 400/200 strips: 103 -> 60 us a star by narrow_zone. With the FP32 screen kept for
 // the tests outside the intervals the batch took 0.4 ms more. (Times before the cap on
-// short chords, 3%, and the certificate of the whole chord, 11%.)
+// short chords, 3%, and the certificate of the whole chord, 9%.)
 template <class Ecl>
 __device__ __forceinline__ double bisect_warp(const Ecl &p, bool live, double pin, double pout,
                                               double acc, V3 pos, int &s) {
