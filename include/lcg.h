@@ -191,8 +191,8 @@ lcg_status lcg_light_curve(lcg_ctx *ctx, const lcg_model *model,
 
 /* Resident-data form of lcg_light_curve for callers that evaluate many
  * models over the same points (samplers, Jacobians): lcg_set_data copies the
- * points to the device once; lcg_light_curve_resident then evaluates a model
- * over them. calc may be NULL, leaving the curve on the device only
+ * points to the device once (after a failure none are resident);
+ * lcg_light_curve_resident then evaluates a model over them. calc may be NULL, leaving the curve on the device only
  * (lcg_device_calc). lcg_light_curve is lcg_set_data followed by
  * lcg_light_curve_resident. The reference passes the Data on every call
  * (light_curve_comp.cpp:119); these two split that call. */
