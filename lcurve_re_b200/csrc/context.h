@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -38,21 +39,66 @@ struct DBuf {
     }
 };
 
-// Host memory that grows, for the copies of a call; its contents do not survive growth. It
-// is pinned where it lies once kPinAfter bytes went through it, a call counting as kPerCall
-// more: pinning takes 0.4 ms and undoing it 0.2, and saves 2-6 us a call and 0.04-0.05 us per
-// KB (30,000 points 100 us), so that is when it has paid for itself. A context of few calls
-// does not pay (blocks of cudaHostAlloc, 1 to 3 ms each, made the first call of a context on 81/163
-// strips and 2,411 points 3.3 to 4.8 ms instead of 2.2).
+// Pinned memory for the copies of calls, shared by the contexts of the process: pinning takes
+// 1 to 3 ms, and a call gains 2 us (500 points) to 10 us (10,000) by it, so a block of its own
+// would make each context's first call pay for hundreds of later ones (81/163 strips and
+// 2,411 points: 3.3 to 4.8 ms instead of 2.1). One block of kBytes is made with the first
+// context and kept; contexts take runs of its pages and give them back. Any thread, any
+// device (portable); without it, or when it is full, blocks are pageable at first.
+struct PinnedPool {
+    static constexpr size_t kBytes = 8u << 20, kPage = 32u << 10;
+    static constexpr int kPages = (int)(kBytes / kPage);
+    static PinnedPool &get() {
+        static PinnedPool pool;
+        return pool;
+    }
+    void open() {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (tried_) return;
+        tried_ = true;
+        if (cudaHostAlloc((void **)&base_, kBytes, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            base_ = nullptr;
+        }
+    }
+    // the first run of pages that holds bytes; NULL if there is none
+    unsigned char *take(size_t bytes) {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (!base_ || bytes > kBytes) return nullptr;
+        const int want = (int)((bytes + kPage - 1) / kPage);
+        for (int i = 0, run = 0; i < kPages; i++) {
+            run = used_[i] ? 0 : run + 1;
+            if (run < want) continue;
+            for (int k = i - want + 1; k <= i; k++) used_[k] = true;
+            return base_ + (size_t)(i - want + 1) * kPage;
+        }
+        return nullptr;
+    }
+    void give(unsigned char *p, size_t bytes) {
+        std::lock_guard<std::mutex> lk(mu_);
+        const int first = (int)((size_t)(p - base_) / kPage);
+        for (int k = 0; k < (int)((bytes + kPage - 1) / kPage); k++) used_[first + k] = false;
+    }
+
+  private:
+    std::mutex mu_;
+    unsigned char *base_ = nullptr;
+    bool tried_ = false, used_[kPages] = {};
+};
+
+// Host memory that grows, for the copies of a call; its contents do not survive growth.
+// From the pool while that has room. Else it is pinned where it lies once kPinAfter bytes
+// went through it, a call counting as kPerCall more, which is when the 0.4 ms of pinning and
+// 0.2 of undoing it have been earned back, at 2-6 us a call and 0.04-0.05 us per KB.
 struct HBuf {
     static constexpr size_t kPinAfter = 12u << 20, kPerCall = 128u << 10;
     unsigned char *p = nullptr;
     size_t cap = 0, used = 0;
-    bool tried = false, pinned = false;
+    bool pooled = false, tried = false, pinned = false;
     cudaError_t ensure(size_t bytes) {
         if (bytes <= cap) {
             used += bytes + kPerCall;
-            if (used >= kPinAfter && !tried) {
+            if (used >= kPinAfter && !pooled && !tried) {
                 tried = true;
                 pinned = cudaHostRegister(p, cap, cudaHostRegisterDefault) == cudaSuccess;
                 if (!pinned) cudaGetLastError();  // the copies work without, only slower
@@ -63,17 +109,20 @@ struct HBuf {
         used = bytes;
         bytes += bytes / 2;  // a fit's light curves come in a few sizes
         bytes = (bytes + 4095) / 4096 * 4096;
-        p = (unsigned char *)aligned_alloc(4096, bytes);
+        p = PinnedPool::get().take(bytes);
+        pooled = p != nullptr;
+        if (!p) p = (unsigned char *)aligned_alloc(4096, bytes);
         if (!p) return cudaErrorMemoryAllocation;
         cap = bytes;
         return cudaSuccess;
     }
     void release() {
         if (pinned) cudaHostUnregister(p);
-        free(p);
+        if (pooled) PinnedPool::get().give(p, cap);
+        else free(p);
         p = nullptr;
         cap = used = 0;
-        tried = pinned = false;
+        pooled = tried = pinned = false;
     }
 };
 

@@ -735,6 +735,7 @@ lcg_status lcg_create(lcg_ctx **out, const lcg_options *opt) {
         delete c;
         return LCG_E_CUDA;
     }
+    PinnedPool::get().open();
     *out = c;
     return LCG_OK;
 }

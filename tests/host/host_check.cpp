@@ -8,7 +8,7 @@
 //
 //   host_check rings|cache|data|pin|first|batch|moved   (stdin: lcg_model A, lcg_model B)
 //
-// pin: many calls with A, counting pinned blocks. first: prints the device allocations of 2 MB
+// pin: many contexts and calls with A, counting pinned blocks. first: prints the device allocations of 2 MB
 // or more of a context's first call, with A. batch: batched calls in place of single ones.
 // moved: a batch's captured graph after its points moved. The others:
 // A call with A, one with B whose k-th allocation fails, then A again (mode data: points for
@@ -348,16 +348,30 @@ int main(int argc, char **argv) {
         return g_wrong ? 1 : 0;
     }
     if (!strcmp(argv[1], "pin")) {
-        lcg_ctx *c = nullptr;
-        if (lcg_create(&c, nullptr)) return 3;
-        for (int i = 0; i < 400; i++) {  // 320 KB of points a call, 40 KB of results
-            if (points(c, 5000) || curve(c, a, 5000)) return 3;
-            if (i < 20 && g_pins) wrong("pinned memory before it can pay");
+        // contexts one after another and side by side share one block
+        lcg_ctx *c[20];
+        for (int i = 0; i < 50; i++) {
+            if (lcg_create(&c[0], nullptr) || points(c[0], 5000) || curve(c[0], a, 5000)) return 3;
+            lcg_destroy(c[0]);
         }
-        if (g_pins != 2) wrong("the points and the results pinned once each");
-        if (points(c, 20000) || curve(c, a, 20000) || g_pinned) wrong("blocks grown, not unpinned");
-        lcg_destroy(c);
-        if (g_pinned) wrong("pinned memory left behind");
+        if (g_pins != 1) wrong("more than one block pinned, or none");
+        // 15 pages each of 256: the block is full with the 17th
+        for (lcg_ctx *&x : c)
+            if (lcg_create(&x, nullptr) || points(x, 5000) || curve(x, a, 5000)) return 3;
+        std::set<const void *> at;
+        for (lcg_ctx *x : c) at.insert(x->h_in.p), at.insert(x->h_res.p);
+        if (at.size() != 40) wrong("two contexts in the same pages");
+        if (!c[0]->h_in.pooled || c[19]->h_in.pooled) wrong("the block's size");
+        if (g_pins != 1) wrong("pinned memory before it can pay");
+        for (int i = 0; i < 400; i++)
+            if (points(c[19], 5000) || curve(c[19], a, 5000)) return 3;
+        if (!c[19]->h_in.pinned) wrong("a block that has paid for it, not pinned");
+        for (lcg_ctx *x : c) lcg_destroy(x);
+        if (g_pinned != 1) wrong("pinned memory left behind");
+        if (lcg_create(&c[0], nullptr) || points(c[0], 80000) || !c[0]->h_in.pooled)
+            wrong("pages not given back");
+        if (points(c[0], 200000) || c[0]->h_in.pooled) wrong("more than the block holds");
+        lcg_destroy(c[0]);
         printf("%d %d\n", g_pins, g_wrong);
         return g_wrong ? 1 : 0;
     }

@@ -57,7 +57,8 @@ def test_points_after_a_failed_allocation(host_check):
 
 
 def test_pinned_memory_waits_until_it_pays(host_check):
-    """A context of few calls pins nothing; one of many does so once, and undoes it."""
+    """Contexts share one pinned block; past it a context of few calls pins nothing, and one of
+    many does so once, and undoes it."""
     _run(host_check, "pin", {}, {})
 
 
